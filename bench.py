@@ -543,11 +543,11 @@ def run_ours(args):
     n_ms, l_ms = per
     form = FORM_NAMES[net.step_form]  # the form the timed steps ran in (auto: the one it chose)
     if form == "dense":
-        # the synapse pass moves the 14 bytes per synaptic event (index 4, delay 2,
-        # weight read + write 8), the neuron pass the 16 per neuron
-        kernels = {"k_dense_synapses": n_ms, "k_dense_neurons": l_ms}
-        dominant = "k_dense_synapses" if n_ms >= l_ms else "k_dense_neurons"
-        alg = 14.0 * ev_per_step_k if dominant == "k_dense_synapses" else 16.0 * N_NEURONS
+        # one kernel per step: 14 bytes per synaptic event (index 4, delay 2, weight read +
+        # write 8) and 16 per neuron
+        kernels = {"k_dense_step": n_ms}
+        dominant = "k_dense_step"
+        alg = 14.0 * ev_per_step_k + 16.0 * N_NEURONS
     else:
         kernels = {"k_neuron_step": n_ms, "k_spike_launch": l_ms}
         dominant = "k_neuron_step" if n_ms >= l_ms else "k_spike_launch"
@@ -575,7 +575,8 @@ def run_ours(args):
                   "mean_rate_hz": fires / (N_NEURONS * args.steps * S / 1000.0),
                   "timed_steps": f"{args.warmup * S + 1}-{(args.warmup + args.steps) * S}",
                   "step_alg_gbs": step_alg},
-        "gpu_launches": 2 * args.steps * S,  # two kernels per simulation step in either form
+        # kernels per simulation step: one in the dense form, two in the event form
+        "gpu_launches": (1 if form == "dense" else 2) * args.steps * S,
         "clocks": clk.summary(),
         "roofline": {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,

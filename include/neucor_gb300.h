@@ -78,11 +78,11 @@ typedef struct {
 #define NC_ORDER_ID 1
 
 /* Form of the step kernels.  Results never depend on it.
- *   NC_STEP_DENSE  (default) two launches per step: a synapse pass that streams every
- *                  in-synapse row in order, making the launch decisions, the plasticity
- *                  and the arrival window there, and a neuron pass.  Its cost grows with
- *                  the synapse count: the faster form when a large share of neurons fires
- *                  every step.
+ *   NC_STEP_DENSE  (default) one launch per step that streams every target's in-row in
+ *                  order, deciding launches, plasticity and the arrival window there, and
+ *                  sums and updates the neurons beside it.  Its cost grows with the
+ *                  synapse count, not with activity: the fast form when a large share
+ *                  of neurons fires every step.
  *   NC_STEP_EVENT  two launches per step; fired neurons are compacted into a list and
  *                  only their out-synapses and the arrived spikes are touched.  Its cost
  *                  grows with the synaptic events: the faster form for sparse activity.
@@ -329,16 +329,16 @@ typedef struct {
 /* Launch configuration of an engine (the autotuner's search space). */
 typedef struct {
     int32_t neuron_block;        /* threads per block of the neuron update, or of the dense step
-                                    (32..256, multiple of 32) */
+                                    (32..256, multiple of 32; the dense step takes 64 at least) */
     int32_t launch_blocks;       /* event form: blocks of the spike launch */
     int32_t launch_block;        /* event form: threads per block of the spike launch (32..256) */
     int32_t graph_steps;         /* steps per captured CUDA graph */
-    int32_t dense_blocks;        /* dense form: blocks of the synapse pass (a grid-stride loop over
-                                    256-synapse spans); 0 = one wave of resident blocks */
-    int32_t steps_per_launch;    /* dense form: 0 = each step is two launches (replayed through CUDA
+    int32_t dense_blocks;        /* dense form: blocks of the step (each takes every dense_blocks-th
+                                    share of the rows); 0 = one per share, a wave of resident blocks */
+    int32_t steps_per_launch;    /* dense form: 0 = each step is one launch (replayed through CUDA
                                     graphs of graph_steps steps); k > 0 = k whole steps per
-                                    persistent cooperative launch (grid barriers between the
-                                    passes; networks with periodic input firers use graphs) */
+                                    persistent cooperative launch (a grid barrier after each;
+                                    networks with periodic input firers use graphs) */
 } nc_launch_config;
 
 int nc_batch_create(int32_t n_nets, const nc_net_spec* specs, nc_batch** out);
@@ -353,7 +353,7 @@ int nc_batch_get_launch(nc_batch* batch, nc_launch_config* out);
 int nc_batch_set_launch(nc_batch* batch, const nc_launch_config* cfg);
 /* Times `steps_per_trial` steps under each candidate configuration, three times each
  * after a warm-up trial, and keeps the one with the lowest median; *best receives it.
- * The candidates cover block sizes, the synapse pass's grid, graph length and (dense
+ * The candidates cover block sizes, graph length and (dense
  * form) steps per persistent launch.  The simulation advances during the trials; the
  * results do not depend on the configuration. */
 int nc_batch_autotune(nc_batch* batch, int32_t steps_per_trial, nc_launch_config* best);
@@ -458,8 +458,8 @@ int nc_run_noalloc(nc_net* net, int32_t n_steps, void* stream);
 /* Times n_steps of the handle's step kernels with CUDA events on its stream;
  * *ms receives the elapsed device time, *kernel_ms (may be NULL) two entries:
  * the mean time of one neuron-update and one spike-launch launch over a separate
- * instrumented pass of min(n_steps, 200) steps (dense form: the synapse pass and the
- * neuron pass). */
+ * instrumented pass of min(n_steps, 200) steps (dense form: the step is one kernel: its
+ * time, and 0). */
 int nc_time_steps(nc_net* net, int32_t n_steps, float* ms, float* kernel_ms);
 
 #ifdef __cplusplus

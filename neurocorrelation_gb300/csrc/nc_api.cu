@@ -150,8 +150,8 @@ int nc_create(int32_t n_neurons, const float* xyz, int64_t n_synapses, const int
     nc::NetHost& h = net->host;
     std::vector<uint32_t>().swap(h.out_ringpos);
     std::vector<int32_t>().swap(h.csc_pre);
-    std::vector<int32_t>().swap(h.csc_post);
-    std::vector<uint16_t>().swap(h.csc_dl);
+    std::vector<uint32_t>().swap(h.key);
+    std::vector<uint8_t>().swap(h.qrow);
     std::vector<float>().swap(h.w);
     std::vector<int64_t>().swap(h.in_ptr);
     std::vector<int32_t>().swap(h.ring_off);
@@ -206,13 +206,17 @@ static int ensure_host_tables(nc_net* net)
     const auto& P = net->eng.P;
     std::vector<int64_t> i2c((size_t)S);
     std::vector<int32_t> to((size_t)S);
-    std::vector<uint16_t> dl((size_t)S);
+    std::vector<uint32_t> key((size_t)h.sp);
     NC_CALL(net->eng, download, i2c.data(), (const int64_t*)net->dev_i2c, (size_t)S);
     NC_CALL(net->eng, download, to.data(), (const int32_t*)net->dev_to, (size_t)S);
-    NC_CALL(net->eng, download, (int16_t*)dl.data(), (const int16_t*)P.csc_dl, (size_t)S);
-    h.csc_delay.resize((size_t)S);
-    for (int64_t c = 0; c < S; ++c) h.csc_delay[(size_t)c] = dl[(size_t)c] & 0x3fff;
-    h.inh_bits.assign((size_t)((S + 31) / 32), 0u);  // U[0,1) weights: none inhibitory
+    // the words with the delays: the second range of a wide net
+    const int64_t wide = h.wide ? (h.sp + 31) / 32 * 32 : 0;
+    const uint32_t low = h.wide ? ~0u : (1u << h.key_shift) - 1u;
+    NC_CALL(net->eng, download, key.data(), (const uint32_t*)P.key + wide, (size_t)h.sp);
+    h.csc_delay.resize((size_t)h.sp);
+    for (int64_t c = 0; c < h.sp; ++c) 
+        h.csc_delay[(size_t)c] = (int32_t)((key[(size_t)c] & low) >> NC_KEY_DELAY_SHIFT);
+    h.inh_bits.assign((size_t)((h.sp + 31) / 32), 0u);  // U[0,1) weights: none inhibitory
     // out-synapses of the source in slot s: its k in creation order
     h.out_ptr.resize((size_t)h.n + 1);
     for (int32_t s = 0; s <= h.n; ++s) h.out_ptr[(size_t)s] = (int64_t)s * k;
@@ -224,9 +228,9 @@ static int ensure_host_tables(nc_net* net)
         for (int32_t m = 0; m < k; ++m) {
             const int64_t e = (int64_t)i * k + m, q = (int64_t)s * k + m;
             const int64_t c = i2c[(size_t)e];
-            h.out_csc[(size_t)q] = (int32_t)c;
+            h.out_csc[(size_t)q] = (int32_t)(uint32_t)c;
             h.out_post[(size_t)q] = h.slot_of[(size_t)to[(size_t)e]];
-            h.out_delay[(size_t)q] = (int16_t)dl[(size_t)c];
+            h.out_delay[(size_t)q] = (int16_t)h.csc_delay[(size_t)c];
         }
     }
     h.input_to_csc = std::move(i2c);
@@ -664,8 +668,8 @@ int nc_read_weights(nc_net* net, float* out_s)
     const nc::NetHost& h = net->host;
     if (!out_s && h.n_input) return fail(NC_ERR_INVALID, "null output");
     NC_CALL0(net->eng, flush_plasticity);
-    std::vector<float> w((size_t)h.s);
-    NC_CALL(net->eng, download, w.data(), (const float*)net->eng.P.w + net->eng.slots[0].syn_base, (size_t)h.s);
+    std::vector<float> w((size_t)h.sp);
+    NC_CALL(net->eng, download, w.data(), (const float*)net->eng.P.w + net->eng.slots[0].syn_base, (size_t)h.sp);
     for (int64_t k = 0; k < h.n_input; ++k) {
         const int64_t c = h.input_to_csc[(size_t)k];
         out_s[k] = c < 0 ? NAN : w[(size_t)c];
@@ -711,11 +715,14 @@ int nc_read_synapse_snapshots(nc_net* net, nc_synapse_snapshot* out, int64_t cap
     NC_CALL0(net->eng, flush_plasticity);
     const auto& sl = net->eng.slots[0];
     const auto& P = net->eng.P;
-    std::vector<float> w((size_t)h.s);
-    std::vector<int32_t> la((size_t)h.s);  // CSC order (dense form) or out-synapse order (event form)
-    NC_CALL(net->eng, download, w.data(), (const float*)P.w + sl.syn_base, (size_t)h.s);
+    std::vector<float> w((size_t)h.sp);
+    NC_CALL(net->eng, download, w.data(), (const float*)P.w + sl.syn_base, (size_t)h.sp);
+    // last accepted arrivals: states in CSC order (dense form), steps in out-synapse order
+    // (event form)
     const bool dense = net->eng.dense;
-    NC_CALL(net->eng, download, la.data(), (const int32_t*)(dense ? P.la_c : P.last_arr) + sl.syn_base, (size_t)h.s);
+    std::vector<int32_t> la((size_t)(dense ? h.sp : h.s));
+    NC_CALL(net->eng, download, la.data(), (dense ? (const int32_t*)P.state : (const int32_t*)P.last_arr) + sl.syn_base,
+            la.size());
     const float T = net->time;
     const int64_t t = net->step;
     int64_t q = 0;
@@ -723,7 +730,7 @@ int nc_read_synapse_snapshots(nc_net* net, nc_synapse_snapshot* out, int64_t cap
         const int32_t si = h.slot_of[(size_t)i];
         for (int64_t k = h.out_ptr[(size_t)si]; k < h.out_ptr[(size_t)si + 1]; ++k) {
             nc_synapse_snapshot& o = out[q++];
-            const int32_t c = h.out_csc[(size_t)k];
+            const int64_t c = (uint32_t)h.out_csc[(size_t)k];
             const float weight = w[(size_t)c];
             o.from_id = i;
             o.to_id = h.orig_id[(size_t)h.out_post[(size_t)k]];
@@ -731,7 +738,8 @@ int nc_read_synapse_snapshots(nc_net* net, nc_synapse_snapshot* out, int64_t cap
             o.inhibitory = weight < 0.0f;
             o.pre_potential = 0.0f;
             o.post_potential = 0.0f;
-            const int32_t a = la[(size_t)(dense ? c : k)];
+            int32_t a = la[(size_t)(dense ? c : k)];
+            if (dense && !h.wide) a = (int32_t)t - nc_state_age((uint32_t)a, (int32_t)t);
             // in flight (AP_fireTime != 0) until its target's update KC steps after arrival
             if (a == NC_NEVER || t - a >= h.kc) continue;
             const int32_t d = (int32_t)((uint16_t)h.out_delay[(size_t)k] & 0x3fffu);

@@ -67,7 +67,10 @@ int nc_batch_create(int32_t n_nets, const nc_net_spec* specs, nc_batch** out)
     std::atomic<int32_t> next{0};
     auto worker = [&]() {
         for (int32_t q = next++; q < n_nets; q = next++) {
-            const nc_net_spec& sp = specs[q];
+            nc_net_spec sp = specs[q];
+            // an engine runs one form, its first network's: every network is laid out for it
+            if (sp.params.step_mode == NC_STEP_DENSE || sp.params.step_mode == NC_STEP_EVENT)
+                sp.params.step_mode = specs[0].params.step_mode;
             int rc = nc::build_net(sp.n_neurons, sp.xyz, sp.n_synapses, sp.syn_from, sp.syn_to, sp.syn_weight,
                                    sp.syn_length, sp.syn_inhibitory, sp.params, b->hosts[(size_t)q], errs[(size_t)q]);
             if (rc == NC_OK) rc = nc::set_groups(b->hosts[(size_t)q], sp.n_groups, sp.groups, errs[(size_t)q]);
@@ -109,7 +112,8 @@ int nc_batch_create(int32_t n_nets, const nc_net_spec* specs, nc_batch** out)
         std::vector<int64_t>().swap(h.in_ptr);
         std::vector<int32_t>().swap(h.ring_off);
         std::vector<int32_t>().swap(h.csc_pre);
-        std::vector<uint16_t>().swap(h.csc_dl);
+        std::vector<uint32_t>().swap(h.key);
+        std::vector<uint8_t>().swap(h.qrow);
     }
     *out = b;
     return NC_OK;
@@ -191,9 +195,7 @@ int nc_batch_autotune(nc_batch* b, int32_t steps_per_trial, nc_launch_config* be
                                   b->eng.graph_ticks, b->eng.L.dense_blocks, b->eng.L.fused_ticks};
     if (b->eng.dense) {
         for (int nb : {64, 128, 256})
-            for (int dbm : {0, 2})
-                for (int g : {16, 64})
-                    cands.push_back(nc_launch_config{nb, cur.launch_blocks, cur.launch_block, g, sms * dbm, 0});
+            for (int g : {16, 64}) cands.push_back(nc_launch_config{nb, cur.launch_blocks, cur.launch_block, g, 0, 0});
         if (b->eng.P.n_firers == 0)
             for (int k : {4, 16, 64})
                 cands.push_back(nc_launch_config{128, cur.launch_blocks, cur.launch_block, 16, 0, k});
@@ -268,8 +270,8 @@ int nc_batch_read_weights(nc_batch* b, int32_t net, float* out)
     if (!out && h.n_input) return bfail(NC_ERR_INVALID, "null output");
     B_CALL0(b->eng, flush_plasticity);
     const auto& sl = b->eng.slots[(size_t)net];
-    std::vector<float> w((size_t)h.s);
-    B_CALL(b->eng, download, w.data(), (const float*)b->eng.P.w + sl.syn_base, (size_t)h.s);
+    std::vector<float> w((size_t)h.sp);
+    B_CALL(b->eng, download, w.data(), (const float*)b->eng.P.w + sl.syn_base, (size_t)h.sp);
     for (int64_t k = 0; k < h.n_input; ++k) {
         const int64_t c = h.input_to_csc[(size_t)k];
         out[k] = c < 0 ? NAN : w[(size_t)c];

@@ -12,13 +12,15 @@
 //      an atomic scatter of the edges into their target's row and a per-row bitonic
 //      sort by source id (warp per row), then the dense form's streams: source and target
 //      slots, weight, delay (coord3::getDist, rounded to whole steps) and the same-step
-//      order flags.
+//      order flags.  The longest distance is known from the search, so the form of the
+//      keys is chosen before the pools are allocated.
 // Storage order (Morton codes, an O(n log n) sort of the positions) and the constant
 // tables stay on the host.  Capacities are bounded (candidates per point, ties, row
 // length); past them the build reports it and the host builder takes over.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -35,7 +37,7 @@ constexpr int kRowCap = 2048;         // in-synapses per row sorted in shared me
 constexpr int kRowWarps = 4;
 
 // build failure flags
-constexpr uint32_t kFlagCandidates = 1u, kFlagTies = 2u, kFlagRow = 4u, kFlagDelay = 8u;
+constexpr uint32_t kFlagCandidates = 1u, kFlagTies = 2u, kFlagRow = 4u;
 
 __device__ __forceinline__ float dist3(const float* a, const float* b)
 {
@@ -161,7 +163,8 @@ struct KnnShared {
 __global__ void __launch_bounds__(32 * kKnnWarps) k_knn(int32_t n, int32_t k, float h, int32_t g, uint32_t k0,
                                                         uint32_t k1, const float* xyz, const int32_t* cstart,
                                                         const int32_t* members, unsigned long long* scratch,
-                                                        int32_t* to, float* weight, uint32_t* flags)
+                                                        int32_t* to, float* weight, uint32_t* flags,
+                                                        uint32_t* far)
 {
     __shared__ KnnShared sh;
     const int lane = threadIdx.x & 31;
@@ -222,6 +225,8 @@ __global__ void __launch_bounds__(32 * kKnnWarps) k_knn(int32_t n, int32_t k, fl
             if (lane == 0) atomicOr(flags, kFlagCandidates);
             continue;
         }
+        // distances are >= 0: their bits are ordered as they are
+        if (lane == 0) atomicMax(far, kth);
         // the k smallest (distance, id): every candidate below the k-th distance, then the
         // smallest ids at exactly that distance
         if (lane == 0) {
@@ -287,10 +292,18 @@ __global__ void k_scatter_rows(int64_t edges, int32_t k, const int32_t* to, cons
     rows[pos] = ((unsigned long long)(uint32_t)from << 32) | (uint32_t)e;
 }
 
-// Warp per target row: sort by source id, then the dense form's in-synapse streams.
-__global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t n, int32_t k, float dt,
-                                                              const float* xyz, const int32_t* to,
-                                                              const float* weight, const int32_t* slot_of,
+// AP_fireTime = length * AP_speed in whole steps (nc::delay_steps).
+__device__ __forceinline__ float delay_of(float length, float dt)
+{
+    return floorf(__fadd_rn(__fdiv_rn(__fmul_rn(length, 2.0f), dt), 0.5f));
+}
+
+// Warp per target row: sort by source id, then the dense form's in-synapses (the engine has
+// set the state words).  cursor: the end of each row's edges.
+__global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t n, int32_t pad, int32_t key_shift,
+                                                              int64_t wide, float dt, const float* xyz,
+                                                              const int32_t* to, const float* weight,
+                                                              const int32_t* slot_of, const unsigned long long* cursor,
                                                               const unsigned long long* rows, int64_t* input_to_csc,
                                                               uint32_t* flags)
 {
@@ -301,7 +314,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t
     const int nw = gridDim.x * kRowWarps;
     for (int32_t tj = gw; tj < n; tj += nw) {
         const int64_t s0 = P.in_ptr[tj], s1 = P.in_ptr[tj + 1];
-        const int len = (int)(s1 - s0);
+        const int len = (int)((int64_t)cursor[tj] - s0);
         if (len > kRowCap) {
             if (lane == 0) atomicOr(flags, kFlagRow);
             continue;
@@ -311,28 +324,27 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t
         for (int q = lane; q < p; q += 32) sh[wib][q] = q < len ? rows[s0 + q] : ~0ull;
         __syncwarp();
         warp_bitonic(sh[wib], p, lane);
-        for (int q = lane; q < len; q += 32) {
+        for (int q = lane; q < (int)(s1 - s0); q += 32) {
+            const int64_t c = s0 + q;
+            if ((q & 3) == 0) P.qrow[c >> 2] = (uint8_t)(tj & 31);
+            if (q >= len) {  // the row's padding
+                P.key[c] = (uint32_t)pad << key_shift;
+                if (wide) P.key[wide + c] = 0u;
+                P.w[c] = 0.0f;
+                continue;
+            }
             const unsigned long long key = sh[wib][q];
             const int32_t from = (int32_t)(key >> 32);
             const int64_t e = (int64_t)(uint32_t)key;
             const int32_t target = to[e];
-            const int64_t c = s0 + q;
-            // AP_fireTime = length * AP_speed in whole steps (nc::delay_steps)
-            const float len_ = dist3(xyz + 3 * (int64_t)from, xyz + 3 * (int64_t)target);
-            const float qd = floorf(__fadd_rn(__fdiv_rn(__fmul_rn(len_, 2.0f), dt), 0.5f));
-            int32_t d = 1;
-            if (qd >= 1.0f) d = (int32_t)qd;
-            if (qd > 16383.0f) {
-                atomicOr(flags, kFlagDelay);
-                d = 1;
-            }
-            const uint32_t fl = (target > from ? 1u << 14 : 0u) | (target < from ? 1u << 15 : 0u);
-            P.csc_pre[c] = slot_of[from];
-            P.csc_post[c] = tj;
-            P.csc_dl[c] = (uint16_t)((uint32_t)d | fl);
+            const float qd = delay_of(dist3(xyz + 3 * (int64_t)from, xyz + 3 * (int64_t)target), dt);
+            uint32_t d = 1u;
+            if (qd >= 1.0f) d = (uint32_t)qd;
+            const uint32_t hi = d << NC_KEY_DELAY_SHIFT | (target > from ? NC_KEY_AFTER : 0u) |
+                                (target < from ? NC_KEY_BEFORE : 0u);
+            P.key[c] = (uint32_t)slot_of[from] << key_shift | (wide ? 0u : hi);
+            if (wide) P.key[wide + c] = hi;
             P.w[c] = weight[e];
-            P.t_arr[c] = NC_NEVER;
-            P.la_c[c] = NC_NEVER;
             input_to_csc[e] = c;
         }
         __syncwarp();
@@ -393,7 +405,7 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     int32_t* d_members = dalloc<int32_t>((size_t)n, own.v, e);
     int32_t* d_to = dalloc<int32_t>((size_t)edges, own.v, e);
     float* d_w = dalloc<float>((size_t)edges, own.v, e);
-    uint32_t* d_flags = dalloc<uint32_t>(1, own.v, e);
+    uint32_t* d_flags = dalloc<uint32_t>(2, own.v, e);  // failure flags, the longest distance's bits
     const int knn_blocks = std::max(1, sms * 8);
     unsigned long long* d_scratch = dalloc<unsigned long long>((size_t)knn_blocks * kKnnWarps * kCandCap, own.v, e);
     if (e != cudaSuccess) {
@@ -401,7 +413,7 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
         return e == cudaErrorMemoryAllocation ? NC_ERR_NOMEM : NC_ERR_CUDA;
     }
     cudaMemset(d_count, 0, sizeof(int32_t) * ((size_t)cells + 1));
-    cudaMemset(d_flags, 0, sizeof(uint32_t));
+    cudaMemset(d_flags, 0, 2 * sizeof(uint32_t));
     k_positions<<<(n + 255) / 256, 256>>>(n, k0, k1, G.side, G.h, G.g, d_xyz, d_cell, d_count);
     // cell starts (host scan of the counts)
     std::vector<int32_t> cstart((size_t)cells + 1, 0);
@@ -416,14 +428,14 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     }
     k_fill_cells<<<(n + 255) / 256, 256>>>(n, d_cell, d_cursor, d_members);
     k_knn<<<knn_blocks, 32 * kKnnWarps>>>(n, k, G.h, G.g, k0, k1, d_xyz, d_count, d_members, d_scratch, d_to, d_w,
-                                          d_flags);
-    uint32_t flags = 0;
-    e = cudaMemcpy(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost);
+                                          d_flags, d_flags + 1);
+    uint32_t found[2] = {0, 0};
+    e = cudaMemcpy(found, d_flags, sizeof(found), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         err = cuda_msg("device kNN build (search)", e);
         return NC_ERR_CUDA;
     }
-    if (flags) {
+    if (found[0]) {
         err = "device kNN build: candidate capacity exceeded";
         return NC_ERR_UNSUPPORTED;
     }
@@ -458,16 +470,27 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
         return NC_ERR_CUDA;
     }
     h.in_ptr.assign((size_t)n + 1, 0);
-    for (int32_t j = 0; j < n; ++j) h.in_ptr[(size_t)j + 1] = h.in_ptr[(size_t)j] + deg[(size_t)j];
+    for (int32_t j = 0; j < n; ++j) {
+        const int64_t end = h.in_ptr[(size_t)j] + deg[(size_t)j], align = row_align(j);
+        h.in_ptr[(size_t)j + 1] = (end + align - 1) / align * align;
+    }
     h.s = edges;
+    h.sp = h.in_ptr[(size_t)n];
     h.n_input = edges;
-    h.max_delay = 1;
+    float far = 0.0f;
+    std::memcpy(&far, &found[1], sizeof(far));
+    h.max_delay = delay_steps(far, h.dt);
+    if (h.max_delay < 0 || h.max_delay > kMaxDelay) {
+        err = "synapse delay exceeds 16383 steps";
+        return NC_ERR_INVALID;
+    }
+    choose_key(h);
     // device pools; the synapse streams are written below
     std::vector<const NetHost*> nets{&h};
     rc = net->eng.build(nets, 64, err, nullptr, true);
     if (rc != NC_OK) return rc;
     unsigned long long* d_cur = dalloc<unsigned long long>((size_t)n, own.v, e);
-    unsigned long long* d_rows = dalloc<unsigned long long>((size_t)edges, own.v, e);
+    unsigned long long* d_rows = dalloc<unsigned long long>((size_t)h.sp, own.v, e);
     int64_t* d_i2c = dalloc<int64_t>((size_t)edges, own.v, e);
     if (e == cudaSuccess)
         e = cudaMemcpy(d_cur, h.in_ptr.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice);
@@ -476,16 +499,14 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
         return e == cudaErrorMemoryAllocation ? NC_ERR_NOMEM : NC_ERR_CUDA;
     }
     k_scatter_rows<<<eb, 256>>>(edges, k, d_to, d_slot, d_cur, d_rows);
-    k_fill_rows<<<std::max(1, sms * 8), 32 * kRowWarps>>>(net->eng.P, n, k, h.dt, d_xyz, d_to, d_w, d_slot, d_rows,
-                                                          d_i2c, d_flags);
+    const int64_t wide = h.wide ? (h.sp + 31) / 32 * 32 : 0;  // the net's second range (Engine::build)
+    k_fill_rows<<<std::max(1, sms * 8), 32 * kRowWarps>>>(net->eng.P, n, pad_slot(n), h.key_shift, wide, h.dt, d_xyz,
+                                                          d_to, d_w, d_slot, d_cur, d_rows, d_i2c, d_flags);
+    uint32_t flags = 0;
     e = cudaMemcpy(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         err = cuda_msg("device kNN build (rows)", e);
         return NC_ERR_CUDA;
-    }
-    if (flags & kFlagDelay) {
-        err = "synapse delay exceeds 16383 steps";
-        return NC_ERR_INVALID;
     }
     if (flags) {
         err = "device kNN build: row capacity exceeded";

@@ -1,37 +1,55 @@
-// nc_dense.cu — the dense form of the NeuCor step: a synapse pass and a neuron pass.
+// nc_dense.cu — the dense form of the NeuCor step: one kernel per step.
 //
 // The event form (nc_kernels.cu) pushes every launched spike from its source into the
-// target's CSC row: scattered term writes and ring atomics per synaptic event.  When a
-// large share of neurons fires every step (the kNN / U[0,1]-weight networks saturate
-// near one fire per refractory period), nearly every in-row is touched every step
-// anyway, and streaming the rows in order is cheaper than scattering into them.
+// target's CSC row: scattered writes and ring atomics per synaptic event.  When a large
+// share of neurons fires every step (the kNN / U[0,1]-weight networks saturate near one
+// fire per refractory period), nearly every in-row is touched every step anyway, and
+// streaming the rows in order is cheaper than scattering into them.
 //
-//   k_dense_synapses (warp per span of 8 x 32 in-synapses, CSC order; the span's
-//   streams arrive by bulk copies into shared memory, the next ones in flight while a
-//   warp works), for the step prev = t-1 of the span's net:
-//     Synapse::fire of every in-synapse whose source fired at prev (src/NeuCor.cpp:
-//     727-738): dropped while busy, otherwise it captures fl(fl(0.2f*52)*w) and its
-//     arrival step; then the plasticity of prev (src/NeuCor.cpp:740-761): post-spike
-//     branch on the rows of targets that fired at prev, arrival branch on synapses
-//     whose spike arrived at prev.  Launched terms are computed 32 at a time from a
-//     per-warp queue so the two FP64 multiplies run on full warps.  Each chunk's
-//     ballot of "arrived in t-KC .. t-1" is one word of the window bitmap.
-//   k_dense_neurons (lane per neuron): charge_insynapses in ascending source order
-//     from the window bitmap, charge_passive, threshold, AP, background draws (as the
-//     event form's k_neuron_step); a neuron inside its AP skips its fold.  It also
-//     writes each neuron's post state for the next synapse pass.
-//   k_dense_fused: both passes of several steps in one cooperative launch, with grid
-//     barriers between them (batched engines).
+//   k_dense_step, step t, prev = t-1: a block works through the tiles (up to 32
+//   consecutive neurons and their in-rows) of its even share of the quads; its last warp
+//   is the neuron warp, the others stream.
+//     rows (neuron warp): whether each neuron fired at prev, and the weight change an
+//       arrival at prev makes (its trace at prev), into shared memory;
+//     synapses (stream warps), a quad (four positions of one row) per thread: Synapse::fire
+//       of those whose source fired at prev (src/NeuCor.cpp:727-738): dropped while busy,
+//       otherwise it captures deltaT * fl(fl(0.2f*52)*w) and its arrival; the plasticity of
+//       prev (src/NeuCor.cpp:740-761): post-spike branch on the rows of neurons that fired
+//       at prev, arrival branch on synapses whose spike arrived at prev; and four window
+//       bits, "arrived in t-KC .. t-1", into a byte of shared memory;
+//     neurons (neuron warp, while the others stream the next tile): charge_insynapses in
+//       ascending source order from the window bits, charge_passive, threshold, AP, input
+//       requests and background draws, fired bits.
+//   The kernel boundary between two steps is the only point where neurons meet: the
+//   fired bits of t are read by the tiles of t+1.
+//   k_dense_fused: several steps in one cooperative launch, a grid barrier after each
+//   (batched engines).
 //
 // Launches of the fires of prev happen at the start of step t instead of the end of
 // step prev; nothing between those points reads what they write (a spike launched at
-// prev arrives at prev+1 at the earliest and joins the fold from prev+2), so the
-// results are the event form's bit for bit.  The launch decision reads the same rule:
-// accepted iff prev - last_arrival >= KC + [target caller id > source caller id], and
-// the captured weight includes the target's post-spike plasticity of prev when the
-// target fired at prev and its caller id is below the source's.  A flush (before
-// read-back) runs the synapse pass early; the step then finds it done (stdp_done) and
-// its window bitmap already written.
+// prev arrives at t at the earliest and joins the fold from t+1), so the results are the
+// event form's bit for bit.  The launch decision reads the same rule: accepted iff
+// prev - last_arrival >= KC + [target caller id > source caller id], and the captured
+// weight includes the target's post-spike plasticity of prev when the target fired at
+// prev and its caller id is below the source's.  A flush (before read-back) streams
+// early; the step then finds it done (stdp_done) and only gathers the window bits.
+//
+// What bounds it, and why this shape.  The step streams 12.25 bytes a synapse (key, state,
+// weight; a row byte per quad) and writes what changed; on networks past the L2 cache that
+// is 23 bytes a synapse of DRAM traffic at 5.2 TB/s (2M x 200: 2,815 -> 1,640 us a step),
+// on smaller ones instruction issue and, below some 10k neurons, the chain of dependent
+// loads.  The two passes before it (synapses, then neurons) read 22 bytes a synapse, took
+// 184 warp instructions per 32 synapses against 75, and exchanged window bits, captured
+// terms and traces through memory.  100k x 100: 92 -> 48 us; 1k x 50: 18.0 -> 7.4;
+// 20k x 100 with inhibitory synapses: 45.8 -> 26; 30k x 73 at dt 0.5: 33 -> 16.5.
+//   - Rows padded to quads: a thread's four synapses share their target's values, and move
+//     with one 16-byte access per array; every eighth row ends on a 128-byte line.
+//   - A warp of its own sums, so the others never wait for a sum: with block barriers
+//     between the two halves the 100k x 100 step took 78 us.
+//   - 96 threads (two stream warps to a neuron warp), 80 registers, 8 blocks an SM, the
+//     rest of shared memory left to the L1 (all of it for shared memory: 57 -> 66 us).
+//     128 threads: 49 us, and 19.6 us against 16.5 on 30k x 73, whose shares get uneven;
+//     64 registers spill (60 us).
 #include "nc_device.cuh"
 #include "nc_engine.cuh"
 
@@ -44,497 +62,82 @@ namespace {
 
 using namespace nc_dev;
 
-constexpr int kMaxWarps = 8;  // 256 threads per block at most
-constexpr int kQueue = 64;    // launched-term queue per warp
+constexpr int kMaxThreads = 256;
+// Quads whose window bits fit in the block's shared memory (a tile of 32 rows of 256
+// synapses); a tile with more keeps them in its slice of NcPools::nib.
+constexpr int kNibCap = 2048;
+// Quads under way per thread, the current one included (cp.async into the thread's own
+// slots of shared memory).  Two leave the memory idle (400k x 100: 215 us a step against
+// 180), four take L1 from the gathers of fired bits (188).
+constexpr int kRing = 3;
 
-// Programmatic dependent launch: each pass of the dense step is launched so that its
-// blocks may be scheduled while the previous pass drains, and waits here, before it
-// reads anything, until that pass has completed and its writes are visible.  (A kernel
-// launched without the attribute passes the wait at once.)
-#ifndef NC_PDL
-#define NC_PDL 1
-#endif
-__device__ __forceinline__ void wait_previous_pass()
-{
-    if (NC_PDL) asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-// The synapse pass lets the neuron pass's blocks be scheduled once its own wait has
-// passed (so the neuron pass that follows cannot start before the one that preceded has
-// completed); the neuron pass then reads what no synapse pass writes (step counters, last
-// fires, potentials, row bounds, input draws) before its own wait.
-#ifndef NC_NEURON_EARLY_START
-#define NC_NEURON_EARLY_START 1
-#endif
-__device__ __forceinline__ void release_next_pass()
-{
-    if (NC_PDL && NC_NEURON_EARLY_START) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-__device__ __forceinline__ int warp_sum(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
-}
-
-// Adds each warp's per-net counters (K of them, into stats[first ..]) to the nets'
-// stats, summed per net over the block first.
-template <int K>
-__device__ void block_counters(const NcPools& P, int* s_net, unsigned long long (*s_acc)[2], int wib, int lane,
-                               int acc_net, const unsigned long long* acc, int first)
-{
-    if (lane == 0) {
-        s_net[wib] = acc_net;
-#pragma unroll
-        for (int k = 0; k < K; ++k) s_acc[wib][k] = acc[k];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int wpb = blockDim.x >> 5;
-        for (int w = 0; w < wpb; ++w) {
-            const int n = s_net[w];
-            if (n < 0) continue;
-            unsigned long long tot[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) tot[k] = s_acc[w][k];
-            for (int v = w + 1; v < wpb; ++v) {
-                if (s_net[v] != n) continue;
-#pragma unroll
-                for (int k = 0; k < K; ++k) tot[k] += s_acc[v][k];
-                s_net[v] = -1;
-            }
-            unsigned long long* st = P.nets[n].stats;
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                if (tot[k]) atomicAdd(st + first + k, tot[k]);
-        }
-    }
-}
-
-// ---------------------------------------------------------------- staged synapse pass
-// The same pass with the six in-synapse streams staged into shared memory by the
-// bulk-copy (TMA) engine.  A warp works through its spans in units of half a span
-// (4 chunks, 128 synapses) and keeps the next unit's copies in flight while it works
-// on the current one (a ring of stage buffers, one mbarrier each): the memory system
-// sees the copies in flight whatever the warp's registers hold, and 24 warps per SM
-// (8 per block, 3 blocks) cover the compute's own latencies.  Shapes measured on the
-// 100k x 100 network (us per pass, before the span-level values were shared by a
-// span's units): 8 warps / half-span units / 2 stages 103, 6 / whole spans / 2 stages
-// 104, 4 / whole / 2 105, 6 / half / 3 110, 4 / half / 4 119, 4 / whole / 3 136; after:
-// a unit's four chunks gathered together 95.5 against two at a time 99.3, and 3 stages
-// 104.8.
-
-#ifndef NC_STAGE_WARPS
-#define NC_STAGE_WARPS 8
-#endif
-#ifndef NC_STAGE_UNIT
-#define NC_STAGE_UNIT 4
-#endif
-#ifndef NC_STAGE_DEPTH
-#define NC_STAGE_DEPTH 2
-#endif
-constexpr int kStageWarps = NC_STAGE_WARPS;  // warps per block
-constexpr int kUnitChunks = NC_STAGE_UNIT;   // chunks per staged unit
-constexpr int kUnitSyn = kUnitChunks * 32;
-constexpr int kUnitsPerSpan = NC_SPAN_CHUNKS / kUnitChunks;
-constexpr int kStages = NC_STAGE_DEPTH;      // units in flight per warp, the current one included
-#ifndef NC_STAGE_UNROLL
-#define NC_STAGE_UNROLL 4
-#endif
-constexpr int kStageUnroll = NC_STAGE_UNROLL;  // chunks whose gathers are in flight together
-static_assert(NC_SPAN_CHUNKS % kUnitChunks == 0 && kUnitChunks % kStageUnroll == 0, "unit shape");
-
-struct StageBuf {                 // one unit, as laid out in the pools (16-byte multiples)
-    int32_t pre[kUnitSyn];
-    int32_t post[kUnitSyn];
-    int32_t la[kUnitSyn];
-    float w[kUnitSyn];
-    int32_t ta[kUnitSyn];
-    uint16_t dl[kUnitSyn];
+struct RowState {
+    float chg;      // weight change of an arrival at prev, before the clamp
+    uint32_t tf;    // the neuron fired at prev
 };
 
-struct NetConst {                 // a span's net constants (see the staged pass)
-    const uint32_t* fprev;        // fired bits of prev
-    const float* pst;             // per neuron: post trace at prev, -0.0 when it fired at prev
-    const float* tab_pre;         // presynaptic trace table
-    double e_term;
-    int32_t t, kc, tab_pre_len;
-    float dt, c52;
-    Rates R;
+struct BlockShared {
+    RowState row[2][NC_TILE_ROWS];               // of two tiles: one streamed, one summed
+    __align__(16) uint8_t nib[2][kNibCap];       // window bits of their quads
+    int ok;
 };
 
-// Lane 0's memo of the last span and net it staged: the second half of a span, and
-// every span of a net after its first, are issued without reloading the span table
-// and the net's descriptor (two dependent loads ahead of the copies).
-// (Kept in the warp's shared memory: only lane 0 uses it.)
-struct StageMemo {
-    int64_t base;    // syn_base
-    int64_t chunks;  // 32-synapse chunks of the net
-    NcTile span;
-    int sp;
-    int net;
-    int ok;          // the net runs its synapse pass in this launch
-    int pad;
-};
+constexpr int kRingBytes = kRing * (3 * 16 + 4);  // dynamic shared memory per stream thread
+size_t ring_bytes(int threads) { return (size_t)threads * kRingBytes; }
 
-struct __align__(16) WarpStage {
-    StageBuf buf[kStages];
-    StageMemo memo;
-    NetConst nc;
-    unsigned long long bar[kStages];  // mbarriers: the copies of buf[k] have landed
-    int32_t qs[kQueue];               // launched synapse, relative to its span's first
-    float qx[kQueue];
-};
-
-constexpr size_t kStageSmem = sizeof(WarpStage) * kStageWarps;
-constexpr uint32_t kWaitLimit = 1u << 22;  // try_wait polls before a stage gives up
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p)
+// Named barriers between the neuron warp and the stream warps, two of each: `ready` once a
+// tile's rows are in shared memory and its window bits may be written, `full` once they are.
+// (Constant ids: with an id in a register a block reserves all 16 barriers, and an SM then
+// holds 4 blocks.)
+template <int kId>
+__device__ __forceinline__ void bar_sync_id()
 {
-    return (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("bar.sync %0, %1;" ::"n"(kId), "r"(blockDim.x) : "memory");
 }
-
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, unsigned long long* bar)
+template <int kId>
+__device__ __forceinline__ void bar_arrive_id()
 {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
+    asm volatile("bar.arrive %0, %1;" ::"n"(kId), "r"(blockDim.x) : "memory");
 }
-
-#ifndef NC_STAGE_MEMO
-#define NC_STAGE_MEMO 1
-#endif
-
-// Lane 0: copies unit `half` of span `sp` into b (all six streams), completing on *bar.
-// Returns 0 when nothing is copied: the span's net is skipped this launch, or the unit
-// lies past the net's last synapse.
-__device__ int stage_unit(const NcPools& P, int sp, int half, bool flush, StageBuf* b, unsigned long long* bar,
-                          StageMemo& m)
+template <int kId>
+__device__ __forceinline__ void bar_sync(int b)  // barrier kId + b, b = 0 or 1
 {
-    if (!NC_STAGE_MEMO || sp != m.sp) {
-        m.span = P.spans[sp];
-        m.sp = sp;
-    }
-    if (!NC_STAGE_MEMO || m.span.net != m.net) {
-        const NcNetDesc& D = P.nets[m.span.net];
-        const int32_t t = D.t, prev = t - 1;
-        m.ok = D.active && prev >= 1 && D.stdp_done < prev && (flush || t <= D.t_end);
-        m.base = D.syn_base;
-        m.chunks = (D.n_syn + 31) / 32;
-        m.net = m.span.net;
-    }
-    if (!m.ok) return 0;
-    const int64_t c0 = m.span.first + (int64_t)half * kUnitChunks;
-    const int64_t nch = min((int64_t)kUnitChunks, m.chunks - c0);
-    if (nch <= 0) return 0;
-    const int64_t s = m.base + c0 * 32;
-    const uint32_t b4 = (uint32_t)(nch * 128), b2 = (uint32_t)(nch * 64);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_addr(bar)), "r"(5 * b4 + b2)
-                 : "memory");
-    bulk_copy(b->pre, P.csc_pre + s, b4, bar);
-    bulk_copy(b->post, P.csc_post + s, b4, bar);
-    bulk_copy(b->la, P.la_c + s, b4, bar);
-    bulk_copy(b->w, P.w + s, b4, bar);
-    bulk_copy(b->ta, P.t_arr + s, b4, bar);
-    bulk_copy(b->dl, P.csc_dl + s, b2, bar);
-    return 1;
+    if (b) bar_sync_id<kId + 1>();
+    else bar_sync_id<kId>();
 }
-
-#ifndef NC_FULL_UNIT
-#define NC_FULL_UNIT 1
-#endif
-template <bool B>
-struct BoolTag {
-    static constexpr bool value = B;
-};
-
-// All lanes: bounded wait for the phase of *bar.
-__device__ __forceinline__ bool stage_wait(unsigned long long* bar, uint32_t phase)
+template <int kId>
+__device__ __forceinline__ void bar_arrive(int b)
 {
-    const uint32_t a = smem_addr(bar);
-    for (uint32_t it = 0; it < kWaitLimit; ++it) {
-        uint32_t done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(done) : "r"(a), "r"(phase) : "memory");
-        if (done) return true;
-    }
-    return false;
+    if (b) bar_arrive_id<kId + 1>();
+    else bar_arrive_id<kId>();
 }
+constexpr int kBarReady = 1, kBarFull = 3;
 
-// The block's shared memory besides the stage buffers, used by both passes.
-struct PassShared {
-    int s_net[kMaxWarps];
-    unsigned long long s_acc[kMaxWarps][2];
-    int s_last;
-    int s_ok;
-    int s_cnt[kMaxWarps];
-    uint16_t s_list[kMaxWarps * 32];
-    float s_pot[kMaxWarps * 32];
-};
+// Programmatic dependent launch: a step's blocks may be scheduled while the previous step
+// drains, and wait here, before they read anything that a step writes, until it has
+// completed and its writes are visible.  (A kernel launched without the attribute passes
+// the wait at once.)
+__device__ __forceinline__ void wait_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next step's blocks be scheduled as this one's leave (it waits in turn).
+__device__ __forceinline__ void release_next_step() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Lane 0 initialises the warp's stage barriers (once per launch).
-__device__ __forceinline__ void init_stages(WarpStage& ws, int lane)
+__device__ __forceinline__ void async16(uint32_t dst, const void* src)
 {
-    if (lane == 0) {
-        for (int k = 0; k < kStages; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_addr(&ws.bar[k])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncwarp();
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-
-// The synapse pass of every span (see k_dense_synapses), each warp striding over the
-// grid's spans.  phases: the parity of each stage slot's next completion, carried from
-// one pass to the next within a launch.  All threads of the block call it.
-template <bool kFlush>
-__device__ __forceinline__ void synapse_pass(const NcPools& P, WarpStage& ws, PassShared& sh, uint32_t& phases)
+__device__ __forceinline__ void async4(uint32_t dst, const void* src)
 {
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * kStageWarps + wib;
-    const int nw = gridDim.x * kStageWarps;
-    const int n_spans = P.n_spans_dev ? *P.n_spans_dev : P.n_spans;
-
-    // unit k of this warp: half k % kUnitsPerSpan of span gw + (k / kUnitsPerSpan) * nw,
-    // staged in slot k % kStages
-    int iss = 0;  // lane 0: bit j set = slot j holds an issued unit not yet consumed
-    StageMemo& memo = ws.memo;
-    if (lane == 0) {
-        memo.sp = -1;
-        memo.net = -1;
-    }
-    if (lane == 0)
-        for (int k = 0; k < kStages - 1; ++k) {
-            const int sp = gw + (k / kUnitsPerSpan) * nw;
-            if (sp < n_spans && stage_unit(P, sp, k % kUnitsPerSpan, kFlush, &ws.buf[k], &ws.bar[k], memo))
-                iss |= 1 << k;
-        }
-
-    int acc_net = -1, cur_net = -1;
-    unsigned long long acc[2] = {0, 0};  // launched, dropped
-    bool ok = true;
-    int qn = 0, nl = 0, nd = 0;
-    for (int i = 0;; ++i) {
-        const int sp = gw + i * nw;
-        if (sp >= n_spans) break;
-        // the span's values, once for its units
-        const NcTile span = P.spans[sp];
-        const NcNetDesc& D = P.nets[span.net];
-        const int32_t t = D.t;
-        const int32_t prev = t - 1;
-        if (span.net != acc_net) {
-            if (acc_net >= 0 && lane == 0) {
-                unsigned long long* st = P.nets[acc_net].stats;
-                atomicAdd(st + 1, acc[0]);
-                atomicAdd(st + 2, acc[1]);
-            }
-            acc_net = span.net;
-            acc[0] = acc[1] = 0;
-        }
-        const int64_t sb = D.syn_base;
-        const int64_t nsyn = D.n_syn;
-        const int64_t s_span = sb + (int64_t)span.first * 32;
-        if (span.net != cur_net) {
-            // the net's constants, once per warp in shared memory: reading them there needs
-            // no reload after each global store (which could alias the descriptor) and no
-            // registers across the chunk loop
-            if (lane == 0) {
-                NetConst& c = ws.nc;
-                c.fprev = P.fired + (int64_t)(prev & 1) * P.total_words + D.word_base;
-                c.pst = P.pst + D.neuron_base;
-                c.tab_pre = P.tables + D.table_base;
-                c.e_term = D.e_term;
-                c.t = t;
-                c.kc = D.kc;
-                c.tab_pre_len = D.tab_pre_len;
-                c.dt = D.dt;
-                c.c52 = D.c52;
-                c.R = rates_of(D);
-            }
-            __syncwarp();
-            cur_net = span.net;
-        }
-        const NetConst& C = ws.nc;
-#pragma unroll 1
-        for (int half = 0; half < kUnitsPerSpan; ++half) {
-            const int k = i * kUnitsPerSpan + half;
-            const int slot = k % kStages;
-            {
-                // the slot consumed last iteration takes unit k + kStages - 1
-                const int kn = k + kStages - 1, sn = kn % kStages;
-                const int spn = gw + (kn / kUnitsPerSpan) * nw;
-                if (lane == 0) {
-                    iss &= ~(1 << sn);
-                    if (spn < n_spans &&
-                        stage_unit(P, spn, kn % kUnitsPerSpan, kFlush, &ws.buf[sn], &ws.bar[sn], memo))
-                        iss |= 1 << sn;
-                }
-            }
-            const int bits = __shfl_sync(kFull, iss, 0);
-            if ((bits >> slot) & 1) {
-                if (!stage_wait(&ws.bar[slot], (phases >> slot) & 1u)) {
-                    if (lane == 0) atomicOr(P.dev_err, NC_DEV_ERR_STAGE_TIMEOUT);
-                    ok = false;
-                    break;
-                }
-                phases ^= 1u << slot;
-                const StageBuf& B = ws.buf[slot];
-                // this unit's synapses start at ubase; offsets within it are 32-bit
-                const int64_t c0 = span.first + (int64_t)half * kUnitChunks;
-                const int64_t ubase = sb + c0 * 32;
-                const int32_t u_rem = (int32_t)min((int64_t)kUnitSyn, nsyn - c0 * 32);  // synapses in the unit
-                int32_t* la_u = P.la_c + ubase;
-                float* w_u = P.w + ubase;
-                int32_t* ta_u = P.t_arr + ubase;
-                uint32_t* win_u = P.win + (ubase >> 5);
-                const uint32_t* inh_u = P.inh + (ubase >> 5);
-                const int32_t qoff = half * kUnitSyn;  // the unit's first synapse, relative to the span
-                const int32_t prev_c = C.t - 1;
-                // the chunks of the unit; a full unit (all but a net's last) is compiled
-                // without the per-lane bounds tests
-                auto chunks = [&](auto all_tag) {
-                constexpr bool kAll = decltype(all_tag)::value;
-                for (int h = 0; h < kUnitChunks; h += kStageUnroll) {
-                    uint32_t fword[kStageUnroll], ihw[kStageUnroll];
-                    float pstv[kStageUnroll];
-    #pragma unroll
-                    for (int u = 0; u < kStageUnroll; ++u) {
-                        const int q = (h + u) * 32 + lane;
-                        fword[u] = 0u;
-                        pstv[u] = 0.0f;
-                        ihw[u] = 0u;
-                        if (kAll || q < u_rem) {
-                            fword[u] = C.fprev[B.pre[q] >> 5];
-                            pstv[u] = C.pst[B.post[q]];
-                            ihw[u] = __ldg(inh_u + h + u);
-                        }
-                    }
-    #pragma unroll
-                    for (int u = 0; u < kStageUnroll; ++u) {
-                        const int q = (h + u) * 32 + lane;
-                        const bool in = kAll || q < u_rem;
-                        const int32_t la = B.la[q];
-                        int32_t lac = in ? la : NC_NEVER;
-                        bool launch = false, srcf = false;
-                        float x = 0.0f;
-                        if (in) {
-                            const uint32_t dl = B.dl[q];
-                            // target fired at prev: the sign of its post state
-                            const bool tf = __float_as_uint(pstv[u]) == 0x80000000u;
-                            srcf = (fword[u] >> (B.pre[q] & 31)) & 1u;
-                            const bool arrived = la == prev_c;
-                            const int32_t after = (int32_t)((dl >> 14) & 1u);
-                            // free: never launched (NC_NEVER is INT32_MIN, far below) or
-                            // prev - la >= KC + after
-                            launch = srcf && la + C.kc + after <= prev_c;
-                            const bool ih = (ihw[u] >> lane) & 1u;
-                            const float lo = ih ? -1.0f : 0.0f, hi = ih ? 0.0f : 1.0f;
-                            const float w0 = B.w[q];
-                            float w1 = w0;
-                            if (tf) w1 = plasticity_b(w0, lo, hi, trace_at_u(C.tab_pre, C.tab_pre_len, prev_c, B.ta[q]),
-                                                      0.0f, C.R);
-                            if (launch) {
-                                // target below the source in caller order and fired at prev:
-                                // its update ran first, post-spike plasticity included
-                                const float cap = (((dl >> 15) & 1u) && tf) ? w1 : w0;
-                                // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
-                                x = C.dt * (C.c52 * cap);
-                                lac = prev_c + (int32_t)(dl & 0x3fffu);
-                                la_u[q] = lac;
-                            }
-                            float w2 = w1;
-                            if (arrived) {
-                                // the target's post trace at prev (0 when it fired at prev)
-                                w2 = plasticity_b(w1, lo, hi, 0.0f, fabsf(pstv[u]), C.R);
-                                ta_u[q] = prev_c;
-                            }
-                            if (tf || arrived) w_u[q] = w2;
-                        }
-                        // arrived t-KC .. t-1: in the fold of step t (NC_NEVER and later
-                        // arrivals wrap past KC)
-                        const bool win = (uint32_t)prev_c - (uint32_t)lac < (uint32_t)C.kc;
-                        const uint32_t wm = __ballot_sync(kFull, win);
-                        if (lane == 0 && (kAll || (h + u) * 32 < u_rem)) win_u[h + u] = wm;
-                        const uint32_t lm = __ballot_sync(kFull, launch);
-                        // launched and dropped, counted once per warp
-                        const int nlm = __popc(lm);
-                        nl += nlm;
-                        nd += __popc(__ballot_sync(kFull, srcf)) - nlm;
-                        if (lm) {
-                            if (launch) {
-                                const int pos = qn + __popc(lm & ((1u << lane) - 1u));
-                                ws.qs[pos] = qoff + q;
-                                ws.qx[pos] = x;
-                            }
-                            qn += __popc(lm);
-                            if (qn >= 32) {
-                                __syncwarp();
-                                P.term[s_span + ws.qs[lane]] = make_term(ws.qx[lane], C.e_term);
-                                __syncwarp();
-                                if (lane < qn - 32) {
-                                    ws.qs[lane] = ws.qs[32 + lane];
-                                    ws.qx[lane] = ws.qx[32 + lane];
-                                }
-                                __syncwarp();
-                                qn -= 32;
-                            }
-                        }
-                    }
-                }
-                };
-                if (NC_FULL_UNIT && u_rem == kUnitSyn) chunks(BoolTag<true>{});
-                else chunks(BoolTag<false>{});
-                // the queue holds offsets into this span: drain it before the warp moves on
-                // to another span (the span's next unit follows when it was issued)
-                const bool more = half + 1 < kUnitsPerSpan && ((bits >> ((k + 1) % kStages)) & 1);
-                if (!more) {
-                    __syncwarp();
-                    if (lane < qn) P.term[s_span + ws.qs[lane]] = make_term(ws.qx[lane], C.e_term);
-                    qn = 0;
-                    acc[0] += (unsigned long long)nl;
-                    acc[1] += (unsigned long long)nd;
-                    nl = nd = 0;
-                }
-            }
-            // the slot is refilled next iteration: finish reading it first, and order those
-            // reads before the copy engine's writes
-            __syncwarp();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-        if (!ok) break;
-    }
-    if (!ok) {
-        // let this warp's copies in flight land (bounded) before the block's shared
-        // memory goes away: the one that timed out and the ones issued behind it
-        const int bits = __shfl_sync(kFull, iss, 0);
-        for (int j = 0; j < kStages; ++j)
-            if ((bits >> j) & 1) stage_wait(&ws.bar[j], (phases >> j) & 1u);
-    }
-    block_counters<2>(P, sh.s_net, sh.s_acc, wib, lane, acc_net, acc, 1);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory"); }
 
-#ifndef NC_STAGE_MIN_BLOCKS
-#define NC_STAGE_MIN_BLOCKS 4
-#endif
-
-template <bool kFlush>
-__global__ void __launch_bounds__(32 * kStageWarps, NC_STAGE_MIN_BLOCKS) k_dense_synapses(NcPools P)
-{
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
-    __shared__ PassShared sh;
-    WarpStage& ws = reinterpret_cast<WarpStage*>(dyn_smem)[threadIdx.x >> 5];
-    init_stages(ws, threadIdx.x & 31);
-    wait_previous_pass();
-    release_next_pass();
-    uint32_t phases = 0u;  // bit j: parity of slot j's next completion
-    synapse_pass<kFlush>(P, ws, sh, phases);
-}
-
-// charge_insynapses (src/NeuCor.cpp:688-700) of neuron j of net D: the terms of the
-// spikes that arrived t-1 .. t-KC, in ascending source id, folded into pot.  The row's
-// window bits are read 256 synapses (8 words) at a time and streamed in batches of 8
-// across word boundaries, so that a warp's batch count is its busiest lane's, not a sum
-// of per-word maxima.
+// charge_insynapses (src/NeuCor.cpp:688-700) of one row: the terms of the spikes that
+// arrived t-1 .. t-KC, in ascending source id, folded into pot.  nib: the tile's window
+// bits, four to a byte; q0, nq: the row's quads; x0: the tile's captured charges.  The bits
+// are read eight quads at a time and streamed in batches of 8 terms across word
+// boundaries, so that a warp's batch count is its busiest lane's, not a sum of per-word
+// maxima.
 //
 // When no term of the net can be negative (nonneg_terms), the running sum only grows
 // (each `float += double` rounds a larger value, and rounding keeps the order), and so
@@ -542,269 +145,588 @@ __global__ void __launch_bounds__(32 * kStageWarps, NC_STAGE_MIN_BLOCKS) k_dense
 // whatever the remaining terms are, and its potential is then replaced by the AP table
 // (src/NeuCor.cpp:682-686, 706-714): the fold stops there and returns the partial sum,
 // which leads the update to the same decision.
-__device__ __forceinline__ float fold_row(const NcPools& P, const NcNetDesc& D, int32_t j, float pot)
+__device__ __forceinline__ float fold_row(const uint8_t* nib, int q0, int nq, const float* x0, float pot, float leak,
+                                          const TermFactor& F, bool stop)
 {
-    const int64_t s0 = P.in_ptr[D.ptr_base + j];
-    const int64_t s1 = P.in_ptr[D.ptr_base + j + 1];
-    if (s1 <= s0) return pot;
-    const bool stop = NC_FOLD_EARLY_EXIT && D.nonneg_terms;
-    const float leak = D.leak;
-    double pd = (double)pot;
-    const int64_t wa0 = s0 >> 5, wa1 = (s1 - 1) >> 5;
-    for (int64_t wb = wa0; wb <= wa1; wb += 8) {
-        unsigned long long m[4];
+    if (nq <= 0) return pot;
+    const int skip = (int)((uintptr_t)(nib + q0) & 7);  // quads of the first word before the row
+    const unsigned long long* words = (const unsigned long long*)(nib + q0 - skip);
+    const int nw = (skip + nq + 7) >> 3;
+    const unsigned long long last = ((skip + nq) & 7) ? (1ull << (8 * ((skip + nq) & 7))) - 1ull : ~0ull;
+    const float* x = x0 + 4 * (int64_t)(q0 - skip);
+    unsigned long long m = words[0] & (~0ull << (8 * skip));
+    if (nw == 1) m &= last;
+    int w = 0;
+    while (true) {
+        float xv[8];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int64_t wq = wb + 2 * q;
-            uint32_t x = wq <= wa1 ? P.win[wq] : 0u;
-            uint32_t y = wq + 1 <= wa1 ? P.win[wq + 1] : 0u;
-            if (wq == wa0) x &= ~0u << (s0 & 31);
-            if (wq == wa1 && (s1 & 31)) x &= (1u << (s1 & 31)) - 1u;
-            if (wq + 1 == wa1 && (s1 & 31)) y &= (1u << (s1 & 31)) - 1u;
-            m[q] = x | ((unsigned long long)y << 32);
-        }
-        const double* tp = P.term + wb * 32;
-        unsigned long long m0 = m[0], m1 = m[1], m2 = m[2], m3 = m[3];
-        int base = 0;
-        while (m0 | m1 | m2 | m3) {
-            int b[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                // on to the next pair when this one is spent (an empty pair costs a slot)
-                if (m0 == 0ull) {
-                    m0 = m1;
-                    m1 = m2;
-                    m2 = m3;
-                    m3 = 0ull;
-                    base += 64;
-                }
-                b[k] = m0 ? base + __ffsll((long long)m0) - 1 : -1;
-                m0 &= m0 - 1ull;
+        for (int k = 0; k < 8; ++k) {
+            // on to the next word when this one is spent (an empty word costs a slot)
+            if (m == 0ull && w + 1 < nw) {
+                ++w;
+                m = words[w];
+                if (w + 1 == nw) m &= last;
             }
-            double v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (b[k] >= 0) v[k] = tp[b[k]];
-            pd = fold8(pd, v, b, tp);
-            // pd holds a float value exactly
-            if (stop && fires_at((float)pd, leak)) return (float)pd;
+            const int p = __ffsll((long long)m) - 1;
+            xv[k] = -0.0f;
+            if (m) xv[k] = x[w * 32 + ((p >> 1) & ~3) + (p & 3)];
+            m &= m - 1ull;
         }
+        pot = fold8(pot, xv, F);
+        if (m == 0ull && w + 1 >= nw) return pot;
+        if (stop && fires_at(pot, leak)) return pot;
     }
-    return __double2float_rn(pd);
 }
 
-// Lane per neuron (warp per tile of 32, a block per group of tiles).  Inside its AP
-// (t - lastFire < KC) a neuron's potential comes from the AP table whatever its sum is,
-// and it cannot cross the threshold, so its fold is skipped.  The block's remaining
-// folds are packed onto its first threads before they run: a warp's FP64 add costs the
-// same however few lanes are active, and at saturation two neurons in three are in
-// their AP.
-#ifndef NC_DNEURON_MAXT
-#define NC_DNEURON_MAXT 256
-#endif
-#ifndef NC_DNEURON_MINB
-#define NC_DNEURON_MINB NC_NEURON_MIN_BLOCKS
-#endif
-// The neuron pass of every tile (see k_dense_neurons), each block striding over groups
-// of tiles; the last block to finish advances the nets' step counters.  All threads of
-// the block call it.
-#ifndef NC_NEURON_EARLY
-#define NC_NEURON_EARLY 1
-#endif
+// What a net's quads share.
+struct TileConst {
+    const uint32_t* fprev;   // fired bits of prev
+    const float* tab_pre;    // presynaptic trace table
+    int32_t tab_pre_len;
+    int32_t prev, kc;
+    int32_t key_shift;
+    float dt, c52;
+    float post0;             // postsynaptic factor * 0: the absent trace of a post-spike update
+    float pre, lr;
+    bool refresh;            // set old ages back in this step (NC_AGE_PERIOD)
+    int64_t wide;
+};
 
-#ifndef NC_FOLD_PACK
-#define NC_FOLD_PACK 1
-#endif
-
-__device__ __forceinline__ void neuron_pass(const NcPools& P, PassShared& sh)
+// The clamp of synapticPlasticity (src/NeuCor.cpp:757-761): hi = 1, lo = 0 for an excitatory
+// synapse, hi = 0, lo = -1 for an inhibitory one.  fminf is the compare and select of the
+// upper bound (a NaN becomes hi); the lower one keeps a negative zero, as the reference's.
+__device__ __forceinline__ float clamp_weight(float v, float lo, float hi)
 {
-    int* s_net = sh.s_net;
-    int* s_cnt = sh.s_cnt;
-    uint16_t* s_list = sh.s_list;
-    float* s_pot = sh.s_pot;
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int wpb = blockDim.x >> 5;
-    const int n_tiles = P.n_tiles_dev ? *P.n_tiles_dev : P.n_tiles;
+    const float m = fminf(v, hi);
+    return (m >= lo) ? m : lo;
+}
 
-    int acc_net = -1;
-    unsigned long long acc[1] = {0};  // fires
-    for (int tb = blockIdx.x; tb * wpb < n_tiles; tb += gridDim.x) {
-        // which of the block's neurons fold, packed in tile order
-        const int tix = tb * wpb + wib;
-        bool need = false;
-        // NC_NEURON_EARLY: the input requests and the background draw of each lane, which
-        // do not depend on its potential, are made before the block's folds, so the warps
-        // that do not fold make them while the others fold
-        bool early_req = false;
-        uint32_t early_bg = ~0u;  // slot of the background target for t+1, or ~0u
-        if (tix < n_tiles) {
-            const NcTile tile = P.tiles[tix];
-            const NcNetDesc& D = P.nets[tile.net];
-            const int32_t t = D.t;
-            const int32_t j = tile.first + lane;
-            if (D.active && t <= D.t_end && j < D.n) {
-                const int32_t lf = P.lf[D.neuron_base + j];
-                need = !(lf != NC_NEVER && t - lf < D.kc) &&
-                       P.in_ptr[D.ptr_base + j + 1] > P.in_ptr[D.ptr_base + j];
-                // with no negative term, a neuron already over the threshold fires whatever
-                // its sum (see fold_row)
-                if (NC_FOLD_EARLY_EXIT && need && D.nonneg_terms && fires_at(P.pot[D.neuron_base + j], D.leak))
-                    need = false;
-                if (NC_NEURON_EARLY) {
-                    const int32_t pj = D.neuron_base + j;
-                    const int32_t cid = D.permuted ? P.orig_id[pj] : j;
-                    if (D.n_groups) early_req = input_request(P, D, cid, t);
-                    if (D.bg_period > 0) {
-                        uint32_t o[4];
-                        philox((uint32_t)cid, (uint32_t)t, NC_STREAM_BACKGROUND, 0u, D, o);
-                        if (o[0] % (uint32_t)D.bg_period == 0u) {
-                            uint32_t tgt = o[1] % (uint32_t)D.n;
-                            if (D.permuted) tgt = (uint32_t)P.slot_of[D.neuron_base + tgt];
-                            early_bg = tgt;
-                        }
-                    }
+// Quad Q (pool index) of a row: launches and plasticity of prev.  Returns the
+// quad's window bits.  Branches are per quad (the row fired; something to store); the four
+// synapses run side by side on selects, so that their gathers are under way together.
+// f: bit 0 of each, its source fired at prev.  kInh: the net has inhibitory synapses.
+template <bool kWide, bool kInh>
+__device__ __forceinline__ uint32_t quad_update(const NcPools& P, const TileConst& C, uint32_t Q, const RowState row,
+                                                const uint4 key, const uint4 st, const uint4 w, const uint32_t (&f)[4],
+                                                unsigned& nl, unsigned& nf)
+{
+    uint32_t h[4], s[4] = {st.x, st.y, st.z, st.w}, bf[4];
+    const uint32_t k[4] = {key.x, key.y, key.z, key.w};
+    const float w0[4] = {__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)};
+    if (kWide) {
+        const uint4 hi4 = __ldg((const uint4*)(P.key + C.wide) + Q);
+        const uint4 before4 = *((const uint4*)(P.state + C.wide) + Q);
+        h[0] = hi4.x, h[1] = hi4.y, h[2] = hi4.z, h[3] = hi4.w;
+        bf[0] = before4.x, bf[1] = before4.y, bf[2] = before4.z, bf[3] = before4.w;
+    }
+    const uint32_t dmask = kWide ? ~0u : (1u << C.key_shift) - 1u;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (!kWide) h[u] = k[u];
+    // steps since the accepted arrival, negative while the spike travels
+    int32_t age[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) age[u] = kWide ? C.prev - (int32_t)s[u] : nc_state_age(s[u], C.prev);
+    float lo[4], hi[4], w1[4], w2[4], cap[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const bool inh = kInh && (h[u] & NC_KEY_INH) != 0u;
+        lo[u] = inh ? -1.0f : 0.0f;
+        hi[u] = inh ? 0.0f : 1.0f;
+        w1[u] = cap[u] = w0[u];
+    }
+    if (row.tf) {
+        // post-spike branch: the trace since the last arrival before prev
+        float tr[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int32_t since =
+                age[u] > 0 ? age[u] : (kWide ? C.prev - (int32_t)bf[u] : age[u] + (int32_t)(s[u] & 0xffffu));
+            tr[u] = since < C.tab_pre_len ? __ldg(C.tab_pre + since) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            w1[u] = clamp_weight(w0[u] + (C.pre * tr[u] - C.post0) * C.lr, lo[u], hi[u]);
+            // target below the source in caller order: its update of prev ran before the launch
+            if (h[u] & NC_KEY_BEFORE) cap[u] = w1[u];
+        }
+    }
+    uint32_t win = 0u;
+    bool arrived = false;
+    const unsigned nl0 = nl;
+    float* xq = P.x + 4 * (int64_t)Q;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const bool fs = f[u] & 1u;
+        // free: prev - arrival >= KC + [target above source]
+        const bool launch = fs && age[u] >= C.kc + (int32_t)(h[u] & NC_KEY_AFTER);
+        const bool now = age[u] == 0;
+        win |= (uint32_t)age[u] < (uint32_t)C.kc ? 1u << u : 0u;
+        // arrival branch
+        const float v = clamp_weight(w1[u] + row.chg, lo[u], hi[u]);
+        w2[u] = now ? v : w1[u];
+        // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
+        if (launch) xq[u] = C.dt * (C.c52 * cap[u]);
+        const int32_t d = (int32_t)((h[u] & dmask) >> NC_KEY_DELAY_SHIFT);
+        if (kWide) {
+            bf[u] = launch ? s[u] : bf[u];
+            s[u] = launch ? (uint32_t)(C.prev + d) : s[u];
+        } else {
+            // nc_state_word(prev, -d, d + age)
+            const uint32_t ns = (uint32_t)d * 65537u + (((uint32_t)C.prev << 16) + (uint32_t)age[u]);
+            s[u] = launch ? ns : s[u];
+        }
+        arrived |= now;
+        nl += launch ? 1u : 0u;
+        nf += fs ? 1u : 0u;
+    }
+    if (!kWide && C.refresh) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (nc_state_age(s[u], C.prev) >= NC_AGE_LIMIT) s[u] = nc_state_word(C.prev, NC_AGE_OLD, 0);
+    }
+    if (row.tf || arrived) *((float4*)P.w + Q) = make_float4(w2[0], w2[1], w2[2], w2[3]);
+    if (nl != nl0 || (!kWide && C.refresh)) {
+        *((uint4*)P.state + Q) = make_uint4(s[0], s[1], s[2], s[3]);
+        if (kWide) *((uint4*)(P.state + C.wide) + Q) = make_uint4(bf[0], bf[1], bf[2], bf[3]);
+    }
+    return win;
+}
+
+// This stream thread's slots of the ring: components apart, so that a warp's 16-byte
+// accesses are contiguous; then the word that holds the quad's row byte.  (.ca copies: a
+// .cg copy of 16 bytes per lane fetched every 32-byte sector twice.)
+struct Ring {
+    uint32_t quad;     // shared address of slot 0's key
+    uint32_t part;     // bytes between components
+    uint32_t row;      // shared address of slot 0's row word
+    __device__ __forceinline__ Ring(unsigned char* dyn, uint32_t threads)
+    {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(dyn);
+        part = 16u * threads;
+        quad = base + 16u * threadIdx.x;
+        row = base + kRing * 3u * part + 4u * threadIdx.x;
+    }
+    __device__ __forceinline__ uint4 load(int slot, int c) const
+    {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(quad + (slot * 3 + c) * part));
+        return v;
+    }
+    __device__ __forceinline__ uint32_t load_row(int slot) const
+    {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(row + slot * (part >> 2)));
+        return v;
+    }
+    __device__ __forceinline__ void fetch(const NcPools& P, int slot, uint32_t Q) const
+    {
+        const uint32_t to = quad + slot * 3 * part;
+        async16(to, (const uint4*)P.key + Q);
+        async16(to + part, (const uint4*)P.state + Q);
+        async16(to + 2 * part, (const uint4*)P.w + Q);
+        async4(row + slot * (part >> 2), (const uint32_t*)P.qrow + (Q >> 2));
+    }
+};
+
+// The tiles of a block that are due in a launch, in order: blocks take the plan's shares
+// blockIdx.x, blockIdx.x + gridDim.x, ...  Every other step goes through a share backwards:
+// what a step touched last is what the L2 cache still holds when the next one begins
+// (100k x 100, 160 MB of arrays against 129 MB of L2: 53.4 -> 48.5 us a step).
+template <bool kFlush>
+struct Tiles {
+    const NcPools& P;
+    int share, ti, begin, end;  // begin <= ti < end
+    bool back;
+    int single;  // one net: 1 when it is due, 0 when not; -1: several nets
+    __device__ __forceinline__ static bool due_net(const NcNetDesc& D)
+    {
+        const int32_t t = D.t;
+        return D.active && (kFlush ? t >= 2 && D.stdp_done < t - 1 : t <= D.t_end);
+    }
+    __device__ __forceinline__ explicit Tiles(const NcPools& p) : P(p), share(blockIdx.x)
+    {
+        single = P.n_nets == 1 ? (due_net(P.nets[0]) ? 1 : 0) : -1;
+        back = P.nets[0].t & 1;
+        enter();
+        settle();
+    }
+    __device__ __forceinline__ void enter()
+    {
+        begin = end = ti = 0;
+        if (share >= P.row_blocks) return;
+        begin = P.rstart[share];
+        end = P.rstart[share + 1];
+        ti = back ? end - 1 : begin;
+    }
+    // to the first due tile from ti on; ti = -1 past the last
+    __device__ __forceinline__ void settle()
+    {
+        while (true) {
+            if (share >= P.row_blocks || single == 0) {
+                ti = -1;
+                return;
+            }
+            if (ti >= begin && ti < end) {
+                if (single > 0 || due_net(P.nets[P.rtiles[ti].net])) return;
+                ti += back ? -1 : 1;
+                continue;
+            }
+            share += gridDim.x;
+            enter();
+        }
+    }
+    __device__ __forceinline__ void next()
+    {
+        ti += back ? -1 : 1;
+        settle();
+    }
+};
+
+// Adds a stream warp's counts to its net's.
+__device__ __forceinline__ void count_events(const NcNetDesc& D, unsigned nl, unsigned nf, int lane)
+{
+    nl = __reduce_add_sync(kFull, nl);
+    nf = __reduce_add_sync(kFull, nf);
+    if (lane == 0 && nl) atomicAdd(D.stats + 1, (unsigned long long)nl);
+    if (lane == 0 && nf != nl) atomicAdd(D.stats + 2, (unsigned long long)(nf - nl));
+}
+
+// Fired words of prev of a quad's four sources, and their bits.
+template <bool kWide>
+__device__ __forceinline__ void fired_words(const TileConst& C, const uint4& key, uint32_t (&f)[4])
+{
+    const uint32_t k[4] = {key.x, key.y, key.z, key.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) f[u] = C.fprev[kWide ? k[u] >> 5 : k[u] >> (C.key_shift + 5)];
+}
+template <bool kWide>
+__device__ __forceinline__ void fired_bits(const TileConst& C, const uint4& key, uint32_t (&f)[4])
+{
+    const uint32_t k[4] = {key.x, key.y, key.z, key.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) f[u] = __funnelshift_r(f[u], 0u, kWide ? k[u] : k[u] >> C.key_shift);  // (slot mod 32)
+}
+
+// The quads of one tile.  The block's quads of one net are consecutive, [run0, run0 + run):
+// this thread takes every threads-th of them, from Q on in steps of `step`, whichever tiles
+// they fall into (Q is left at its first past the tile), and keeps its next ones under way.
+template <bool kFlush, bool kWide, bool kInh>
+__device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst& C, uint32_t q0, uint32_t nq,
+                                              uint32_t run0, uint32_t run, bool due, const RowState* row,
+                                              uint32_t row0, uint8_t* nib, const Ring& ring, uint32_t step,
+                                              uint32_t& Q, int& slot, uint32_t (&f)[4], unsigned& nl, unsigned& nf)
+{
+    for (; Q - q0 < nq; Q += step) {
+        async_wait();
+        const int ahead = slot + 1 == kRing ? 0 : slot + 1;
+        const uint4 st = ring.load(slot, 1);
+        uint32_t win = 0u;
+        if (due) {
+            const uint4 key = ring.load(slot, 0);
+            uint32_t fired[4] = {f[0], f[1], f[2], f[3]};
+            fired_bits<kWide>(C, key, fired);
+            // the next quad's fired words while this one is worked on
+            if (Q + step - run0 < run) fired_words<kWide>(C, ring.load(ahead, 0), f);
+            const uint4 w = ring.load(slot, 2);
+            const uint32_t rb = ring.load_row(slot) >> (8 * (Q & 3u));
+            win = quad_update<kWide, kInh>(P, C, Q, row[(rb - row0) & 31u], key, st, w, fired, nl, nf);
+        } else {
+            const uint32_t s[4] = {st.x, st.y, st.z, st.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int32_t age = kWide ? C.prev - (int32_t)s[u] : nc_state_age(s[u], C.prev);
+                win |= (uint32_t)age < (uint32_t)C.kc ? 1u << u : 0u;
+            }
+        }
+        if (!kFlush) nib[Q] = (uint8_t)win;
+        // the slot has been read: refill it
+        const uint32_t next = Q + kRing * step;
+        if (next - run0 < run) ring.fetch(P, slot, next);
+        async_commit();
+        slot = ahead;
+    }
+}
+
+// The stream warps' part of a step (or of the flush of the last one).
+template <bool kFlush>
+__device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, unsigned char* dyn)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t threads = blockDim.x - 32;
+    const Ring ring(dyn, threads);
+    Tiles<kFlush> at(P);
+    TileConst C;
+    int net = -1, share = -1, slot = 0;
+    const uint32_t step = at.back ? 0u - threads : threads;
+    uint32_t Q = 0u, run0 = 0u, run = 0u;
+    uint32_t f[4] = {0u, 0u, 0u, 0u};  // fired words of this thread's next quad
+    bool due = false, inh = false;
+    unsigned nl = 0u, nf = 0u;  // launches, and synapses whose source fired
+    for (int n = 0; at.ti >= 0; at.next(), ++n) {
+        const NcRowTile tile = P.rtiles[at.ti];
+        const bool new_run = tile.net != net || at.share != share;
+        if (new_run) {
+            // the next run of consecutive quads: fetch this thread's first ones
+            share = at.share;
+            int other = at.back ? at.begin : at.end - 1;  // the run's last tile in this order
+            while (P.rtiles[other].net != tile.net) other += at.back ? 1 : -1;
+            const NcRowTile& last = P.rtiles[other];
+            run0 = at.back ? last.q0 : tile.q0;
+            run = (at.back ? tile.q0 + (uint32_t)tile.nq : last.q0 + (uint32_t)last.nq) - run0;
+            // chunks of `threads` quads from run0 on, the last one short
+            Q = run0 + threadIdx.x + (at.back && run ? (run - 1u) / threads * threads : 0u);
+            if (at.back && Q - run0 >= run) Q -= threads;
+#pragma unroll 1
+            for (int k = 0; k < kRing; ++k) {
+                const uint32_t q = Q + k * step;
+                if (q - run0 < run) ring.fetch(P, slot + k < kRing ? slot + k : slot + k - kRing, q);
+                async_commit();
+            }
+        }
+        if (tile.net != net) {
+            if (net >= 0) count_events(P.nets[net], nl, nf, lane);
+            nl = nf = 0u;
+            net = tile.net;
+            const NcNetDesc& D = P.nets[net];
+            const int32_t prev = D.t - 1;
+            due = prev >= 1 && D.stdp_done < prev;  // launches and plasticity of prev
+            inh = !D.nonneg_terms;
+            C.fprev = P.fired + (int64_t)(prev & 1) * P.total_words + D.word_base;
+            C.tab_pre = P.tables + D.table_base;
+            C.tab_pre_len = D.tab_pre_len;
+            C.prev = prev;
+            C.kc = D.kc;
+            C.key_shift = D.key_shift;
+            C.dt = D.dt;
+            C.c52 = D.c52;
+            C.pre = D.pre_factor;
+            C.lr = D.lr;
+            C.post0 = D.post_factor * 0.0f;
+            C.refresh = prev % NC_AGE_PERIOD == 0;
+            C.wide = D.wide;
+        }
+        if (new_run && due) {  // the first quad's fired words
+            async_wait();
+            if (Q - run0 < run) {
+                if (C.wide) fired_words<true>(C, ring.load(slot, 0), f);
+                else fired_words<false>(C, ring.load(slot, 0), f);
+            }
+        }
+        const int b = n & 1;
+        uint8_t* nib = (tile.nq <= kNibCap ? sh.nib[b] - tile.q0 : P.nib);  // by pool index of the quad
+        bar_sync<kBarReady>(b);
+        const uint32_t row0 = (uint32_t)tile.first, nq = (uint32_t)tile.nq;
+        if (C.wide)
+            tile_synapses<kFlush, true, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
+                                              slot, f, nl, nf);
+        else if (inh)
+            tile_synapses<kFlush, false, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
+                                              slot, f, nl, nf);
+        else
+            tile_synapses<kFlush, false, false>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
+                                              slot, f, nl, nf);
+        bar_arrive<kBarFull>(b);
+    }
+    if (net >= 0) count_events(P.nets[net], nl, nf, lane);
+    else if (!kFlush) bar_arrive<kBarFull>(0);  // nothing to do: the step counters have been read
+}
+
+// Every block has read the step counters: one warp moves them on.
+__device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
+{
+    for (int n = lane; n < P.n_nets; n += 32) {
+        NcNetDesc* D = P.nets + n;
+        if (D->active && D->t <= D->t_end) {
+            if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
+            D->stats[3] += 1ull;
+            D->t += 1;
+            D->tsum = __fadd_rn(D->tsum, D->dt);  // currentTime = targetTime (src/NeuCor.cpp:616)
+        }
+    }
+    if (lane == 0) *P.done_ctr = 0u;
+}
+
+// Rows of tile `ti` into sh.row[b], and the buffer handed to the stream warps.
+__device__ __forceinline__ void give_rows(const NcPools& P, BlockShared& sh, int ti, int b, int lane)
+{
+    if (lane < P.rtiles[ti].count) {
+        const NcNetDesc& D = P.nets[P.rtiles[ti].net];
+        const int32_t i = P.rtiles[ti].neuron + lane;
+        // the target's trace at prev; the arriving synapse's own is 0
+        const int32_t lf = P.lf[i];
+        const float trT = P.pst[i];
+        sh.row[b][lane] = RowState{(D.pre_factor * 0.0f - D.post_factor * trT) * D.lr, lf == D.t - 1 ? 1u : 0u};
+    }
+    bar_arrive<kBarReady>(b);
+}
+
+// The neuron warp's part of a step.
+template <bool kFlush>
+__device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh)
+{
+    const int lane = threadIdx.x & 31;
+    Tiles<kFlush> at(P);
+    // the tile whose rows are given next: up to two ahead of the one being summed
+    Tiles<kFlush> ahead = at;
+    int given = 0;
+    for (; given < 2 && ahead.ti >= 0; ++given, ahead.next()) give_rows(P, sh, ahead.ti, given & 1, lane);
+    unsigned arrived = 0u;
+    unsigned fires = 0u;
+    int net = -1;
+    bool counted = false;
+    for (int n = 0; at.ti >= 0; ++n) {
+        const int b = n & 1;
+        const NcRowTile tile = P.rtiles[at.ti];
+        at.next();
+        if (kFlush) {
+            bar_sync<kBarFull>(b);
+            if (ahead.ti >= 0) {
+                give_rows(P, sh, ahead.ti, b, lane);
+                ahead.next();
+            }
+            continue;
+        }
+        const NcNetDesc& D = P.nets[tile.net];
+        if (tile.net != net) {
+            if (net >= 0 && lane == 0 && fires) atomicAdd(P.nets[net].stats + 0, (unsigned long long)fires);
+            net = tile.net;
+            fires = 0u;
+        }
+        const int32_t t = D.t;
+        const int32_t kc = D.kc;
+        const int32_t i = tile.first + lane, pj = tile.neuron + lane;
+        const bool live = lane < tile.count;
+        const bool stop = D.nonneg_terms != 0;
+        const float leak = D.leak;
+        const float* tables = P.tables + D.table_base;
+        uint8_t* fired_t = (uint8_t*)(P.fired + (int64_t)(t & 1) * P.total_words + D.word_base);
+        uint8_t* forced_t = (uint8_t*)(P.forced + (int64_t)(t & 1) * P.total_words + D.word_base);
+        uint8_t* ufire_t = (uint8_t*)(P.ufire + (int64_t)(t & 1) * P.total_words + D.word_base);
+        uint32_t* forced_n = P.forced + (int64_t)((t + 1) & 1) * P.total_words + D.word_base;
+        int32_t lf = NC_NEVER;
+        float pot = 0.0f, ap = 0.0f, ap0 = 0.0f, trace = 0.0f;
+        bool forced = false, input = false;
+        int q0 = 0, nq = 0;
+        if (live) {
+            lf = P.lf[pj];
+            pot = P.pot[pj];
+            q0 = (int)((__ldg(P.in_ptr + tile.ptr + lane) >> 2) - (int64_t)tile.q0);
+            nq = (int)((__ldg(P.in_ptr + tile.ptr + lane + 1) >> 2) - (int64_t)tile.q0) - q0;
+            forced = (forced_t[i >> 3] >> (i & 7)) & 1u;
+            input = (ufire_t[i >> 3] >> (i & 7)) & 1u;
+            // the AP table's entries now and after a fire, the trace without one
+            if (lf != NC_NEVER && t - lf < kc) ap = __ldg(P.tables + D.ap_base + (t - lf));
+            ap0 = __ldg(P.tables + D.ap_base);
+            trace = trace_at_u(tables + D.tab_pre_len, D.tab_post_len, t, lf);
+            // input requests; background fires for step t+1 (src/NeuCor.cpp:604-607), drawn per
+            // caller id
+            const int32_t cid = D.permuted ? __ldg(P.orig_id + pj) : i;
+            if (D.n_groups && input_request(P, D, cid, t)) forced = true;
+            if (D.bg_period > 0) {
+                uint32_t o[4];
+                philox((uint32_t)cid, (uint32_t)t, NC_STREAM_BACKGROUND, 0u, D, o);
+                if (o[0] % (uint32_t)D.bg_period == 0u) {
+                    uint32_t bg = o[1] % (uint32_t)D.n;
+                    if (D.permuted) bg = (uint32_t)P.slot_of[D.neuron_base + bg];
+                    atomicOr(forced_n + (bg >> 5), 1u << (bg & 31));
                 }
             }
         }
-        // everything above reads state no synapse pass writes; the folds and the update
-        // below need the synapse pass of this step
-        if (NC_NEURON_EARLY_START) wait_previous_pass();
-        if (NC_FOLD_PACK) {
-            const uint32_t need_m = __ballot_sync(kFull, need);
-            if (lane == 0) s_cnt[wib] = __popc(need_m);
-            __syncthreads();
-            int base = 0, total = 0;
-            for (int w = 0; w < wpb; ++w) {
-                base += w < wib ? s_cnt[w] : 0;
-                total += s_cnt[w];
-            }
-            if (need) s_list[base + __popc(need_m & ((1u << lane) - 1u))] = (uint16_t)(wib * 32 + lane);
-            __syncthreads();
-            for (int r = threadIdx.x; r < total; r += blockDim.x) {
-                const int ent = s_list[r];
-                const NcTile tile = P.tiles[tb * wpb + (ent >> 5)];
-                const NcNetDesc& D = P.nets[tile.net];
-                const int32_t j = tile.first + (ent & 31);
-                s_pot[ent] = fold_row(P, D, j, P.pot[D.neuron_base + j]);
-            }
-            __syncthreads();
-        } else if (need) {
-            // each lane folds its own neuron (no packing, no block barrier)
-            const NcTile tile = P.tiles[tix];
-            const NcNetDesc& D = P.nets[tile.net];
-            const int32_t j = tile.first + lane;
-            s_pot[wib * 32 + lane] = fold_row(P, D, j, P.pot[D.neuron_base + j]);
+        // inside its AP (t - lastFire < KC) a neuron's potential comes from the AP table
+        // whatever its sum is, and it cannot cross the threshold; with no negative term a
+        // neuron already over the threshold fires whatever its sum
+        const bool can = lf == NC_NEVER || t - lf >= kc;
+        const bool need = live && can && !(stop && fires_at(pot, leak));
+        bar_sync<kBarFull>(b);
+        if (at.ti < 0) {  // the block's last tile: all its warps have read the step counters
+            counted = true;
+            if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
         }
-        if (tix >= n_tiles) continue;
-        const NcTile tile = P.tiles[tix];
-        const NcNetDesc& D = P.nets[tile.net];
-        const int32_t t = D.t;
-        if (!(D.active && t <= D.t_end)) continue;
-        if (tile.net != acc_net) {
-            if (acc_net >= 0 && lane == 0) atomicAdd(P.nets[acc_net].stats + 0, acc[0]);
-            acc_net = tile.net;
-            acc[0] = 0;
+        const uint8_t* nib = tile.nq <= kNibCap ? sh.nib[b] : P.nib + tile.q0;
+        if (need) pot = fold_row(nib, q0, nq, P.x + 4 * (int64_t)tile.q0, pot, leak, term_factor(D), stop);
+        __syncwarp();
+        if (ahead.ti >= 0) {
+            give_rows(P, sh, ahead.ti, b, lane);
+            ahead.next();
         }
-        const int32_t first = tile.first;
-        const int32_t j = first + lane;
-        const bool live = j < D.n;
-        const int32_t pj = D.neuron_base + j;
-        const int64_t word = D.word_base + (first >> 5);
-        const int32_t kc = D.kc;
         bool fired = false;
         if (live) {
-            int32_t lf = P.lf[pj];
-            float pot = need ? s_pot[wib * 32 + lane] : P.pot[pj];
-            const uint32_t fw = P.forced[(int64_t)(t & 1) * P.total_words + word];
-            const uint32_t uw = P.ufire[(int64_t)(t & 1) * P.total_words + word];
-            bool forced = (fw >> lane) & 1u;
-            if (NC_NEURON_EARLY) forced = forced || early_req;
-            else if (!forced && D.n_groups) forced = input_request(P, D, D.permuted ? P.orig_id[pj] : j, t);
             // charge_passive (src/NeuCor.cpp:677-680)
-            pot = (pot - -70.0f) * D.leak + -70.0f;
-            // charge_thresholdCheck (src/NeuCor.cpp:682-686); vesicles stay positive
-            const bool can = (lf == NC_NEVER) || (t - lf >= kc);
-            // an input firer's Neuron::fire has no threshold or refractory test
-            fired = ((uw >> lane) & 1u) || ((-55.0f < pot || forced) && can);
-            if (fired) {
-                lf = t;
-                P.lf[pj] = t;
-                P.firings[pj] += 1u;
-            }
+            pot = (pot - -70.0f) * leak + -70.0f;
+            // charge_thresholdCheck (src/NeuCor.cpp:682-686); vesicles stay positive.  An input
+            // firer's Neuron::fire has no threshold or refractory test
+            fired = input || ((-55.0f < pot || forced) && can);
             // AP (src/NeuCor.cpp:706-714)
-            if (lf != NC_NEVER && t - lf < kc) pot = __ldg(P.tables + D.ap_base + (t - lf));
+            if (fired) {
+                P.lf[pj] = t;
+                atomicAdd(P.firings + pj, 1u);  // (nothing waits for a value)
+                pot = ap0;
+            } else if (!can) {
+                pot = ap;
+            }
             P.pot[pj] = pot;
-            // the post state the next synapse pass reads: getTrace at t (src/NeuCor.cpp:671-675,
-            // 0 when it fired at t), its sign set when it fired at t
-            P.pst[pj] = fired ? -0.0f : trace_at(P.tables + D.table_base + D.tab_pre_len, D.tab_post_len, t, lf);
+            // getTrace at t (src/NeuCor.cpp:671-675; 0 when it fired at t) for the next step
+            P.pst[pj] = fired ? 0.0f : trace;
         }
         const uint32_t fmask = __ballot_sync(kFull, fired);
-        if (lane == 0) {
-            P.fired[(int64_t)(t & 1) * P.total_words + word] = fmask;
-            P.forced[(int64_t)(t & 1) * P.total_words + word] = 0u;
-            P.ufire[(int64_t)(t & 1) * P.total_words + word] = 0u;
+        // a tile may hold part of a word: bytes (8 neurons) are written on their own
+        if (lane < 4 && 8 * lane < tile.count) {
+            const int32_t at_byte = tile.first / 8 + lane;
+            const uint8_t v = (uint8_t)(fmask >> (8 * lane));
+            fired_t[at_byte] = v;
+            forced_t[at_byte] = 0;
+            ufire_t[at_byte] = 0;
             if (D.raster_len > 0 && t >= D.raster_t0 && t - D.raster_t0 < D.raster_len)
-                D.raster[(int64_t)(t - D.raster_t0) * D.n_words + (first >> 5)] = fmask;
+                ((uint8_t*)(D.raster + (int64_t)(t - D.raster_t0) * D.n_words))[at_byte] = v;
         }
-        acc[0] += (unsigned long long)__popc(fmask);
-        // background fires for step t+1 (src/NeuCor.cpp:604-607), drawn per caller id
-        if (NC_NEURON_EARLY && early_bg != ~0u)
-            atomicOr(P.forced + (int64_t)((t + 1) & 1) * P.total_words + D.word_base + (early_bg >> 5),
-                     1u << (early_bg & 31));
-        if (!NC_NEURON_EARLY && live && D.bg_period > 0) {
-            uint32_t o[4];
-            philox((uint32_t)(D.permuted ? P.orig_id[pj] : j), (uint32_t)t, NC_STREAM_BACKGROUND, 0u, D, o);
-            if (o[0] % (uint32_t)D.bg_period == 0u) {
-                uint32_t tgt = o[1] % (uint32_t)D.n;
-                if (D.permuted) tgt = (uint32_t)P.slot_of[D.neuron_base + tgt];
-                atomicOr(P.forced + (int64_t)((t + 1) & 1) * P.total_words + D.word_base + (tgt >> 5),
-                         1u << (tgt & 31));
-            }
-        }
+        fires += __popc(fmask);
     }
-    // (a block with no tile of its own still waits before the step counters can move)
-    if (NC_NEURON_EARLY_START) wait_previous_pass();
-    block_counters<1>(P, s_net, sh.s_acc, wib, lane, acc_net, acc, 0);
-    // the last block to finish advances the step counters
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) sh.s_last = (atomicAdd(P.done_ctr, 1u) == gridDim.x - 1u);
-    __syncthreads();
-    if (sh.s_last) {
-        __threadfence();
-        for (int n = threadIdx.x; n < P.n_nets; n += blockDim.x) {
-            NcNetDesc* D = P.nets + n;
-            if (D->active && D->t <= D->t_end) {
-                if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
-                D->stats[3] += 1ull;
-                D->t += 1;
-                D->tsum = __fadd_rn(D->tsum, D->dt);  // currentTime = targetTime (src/NeuCor.cpp:616)
-            }
-        }
-        if (threadIdx.x == 0) *P.done_ctr = 0u;
+    if (kFlush) return;
+    if (net >= 0 && lane == 0 && fires) atomicAdd(P.nets[net].stats + 0, (unsigned long long)fires);
+    if (!counted) {  // a block with nothing to do (its other warps have read the counters)
+        bar_sync<kBarFull>(0);
+        if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
+    }
+    if (__shfl_sync(kFull, arrived, 0) == gridDim.x - 1u) advance_steps(P, lane);
+}
+
+// One step (or the flush of the last one) of every tile of this block.
+template <bool kFlush>
+__device__ __forceinline__ void dense_pass(const NcPools& P, BlockShared& sh, unsigned char* dyn)
+{
+    if (threadIdx.x >= blockDim.x - 32) {
+        neuron_role<kFlush>(P, sh);
+    } else {
+        stream_role<kFlush>(P, sh, dyn);
     }
 }
 
-__global__ void __launch_bounds__(NC_DNEURON_MAXT, NC_DNEURON_MINB) k_dense_neurons(NcPools P)
+#ifndef NC_DENSE_MIN_BLOCKS
+#define NC_DENSE_MIN_BLOCKS 3
+#endif
+template <bool kFlush>
+__global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_step(NcPools P)
 {
-    __shared__ PassShared sh;
-    if (!NC_NEURON_EARLY_START) wait_previous_pass();
-    neuron_pass(P, sh);
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ BlockShared sh;
+    wait_previous_step();
+    release_next_step();
+    dense_pass<kFlush>(P, sh, dyn);
 }
 
 // ---------------------------------------------------------------- fused multi-step launch
-// `ticks` whole steps of every net in one cooperative launch: synapse pass, grid
-// barrier, neuron pass (whose last block advances the step counters), grid barrier.
+// `ticks` whole steps of every net in one cooperative launch, a grid barrier after each.
 // The grid is at most one wave (cudaLaunchCooperativeKernel refuses more), so every
 // block reaches every barrier; each barrier wait is still bounded, and one that gives
-// up sets NC_DEV_ERR_BARRIER and ends its block.  It saves the per-step launches and
-// their drain and fill for batches of small networks.  (No periodic input firers: they
-// run as their own kernel before a step.)
+// up sets NC_DEV_ERR_BARRIER and ends its block.  (No periodic input firers: they run as
+// their own kernel before a step.)
 constexpr uint32_t kBarrierPolls = 1u << 24;  // polls (64 ns sleeps) before a barrier gives up
 
 // bar[0]: arrivals, bar[1]: generation.  gen: this block's view of the generation.
-__device__ bool grid_barrier(unsigned* bar, unsigned& gen, uint32_t* dev_err, PassShared& sh)
+__device__ bool grid_barrier(unsigned* bar, unsigned& gen, uint32_t* dev_err, BlockShared& sh)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -828,36 +750,26 @@ __device__ bool grid_barrier(unsigned* bar, unsigned& gen, uint32_t* dev_err, Pa
         }
         __threadfence();
         gen = g + 1u;
-        sh.s_ok = ok;
+        sh.ok = ok;
     }
     __syncthreads();
-    return sh.s_ok != 0;
+    return sh.ok != 0;
 }
 
-#ifndef NC_FUSED_MIN_BLOCKS
-#define NC_FUSED_MIN_BLOCKS 3  // the neuron pass needs ~80 registers
-#endif
-__global__ void __launch_bounds__(32 * kStageWarps, NC_FUSED_MIN_BLOCKS) k_dense_fused(NcPools P, int32_t ticks,
-                                                                                     unsigned* bar)
+__global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_fused(NcPools P, int32_t ticks,
+                                                                                unsigned* bar)
 {
-    extern __shared__ __align__(128) unsigned char dyn_smem[];
-    __shared__ PassShared sh;
-    WarpStage& ws = reinterpret_cast<WarpStage*>(dyn_smem)[threadIdx.x >> 5];
-    init_stages(ws, threadIdx.x & 31);
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ BlockShared sh;
     unsigned gen = 0u;
     if (threadIdx.x == 0) gen = atomicAdd(&bar[1], 0u);
-    uint32_t phases = 0u;
     for (int32_t k = 0; k < ticks; ++k) {
-        synapse_pass<false>(P, ws, sh, phases);
+        dense_pass<false>(P, sh, dyn);
         if (!grid_barrier(bar, gen, P.dev_err, sh)) return;
-        neuron_pass(P, sh);
-        if (!grid_barrier(bar, gen, P.dev_err, sh)) return;
-        // the next pass's bulk copies read what other blocks stored in this launch
-        asm volatile("fence.proxy.async.global;" ::: "memory");
     }
 }
 
-// After a flush: the synapse pass of every active net's last step is done.
+// After a flush: the launches and plasticity of every active net's last step are done.
 __global__ void k_dense_mark_flushed(NcPools P)
 {
     for (int n = threadIdx.x; n < P.n_nets; n += blockDim.x) {
@@ -866,140 +778,87 @@ __global__ void k_dense_mark_flushed(NcPools P)
     }
 }
 
-// The synapse pass's grid: the launch configuration's, else a persistent grid of as
-// many blocks as fit on the GPU at once (one wave; each warp strides over many spans,
-// and keeps its next units' copies in flight meanwhile).  A grid of one span per warp
-// measured 25% slower.  (A form of the pass on register loads instead of bulk copies
-// measured 5% slower and was dropped.)
-struct SynKernel {
-    const void* fn;
-    int threads;
-    size_t smem;
-};
-
-template <bool kFlush>
-SynKernel syn_kernel()
+// Blocks of one wave of kernel `which` (0: a step, 1: several) with `threads` threads on the
+// current device (cached per device and block size).  Returns 0 when the device cannot run
+// it (the launch then reports an error).
+int resident_blocks(int which, int threads)
 {
-    return {(const void*)k_dense_synapses<kFlush>, 32 * kStageWarps, kStageSmem};
-}
-
-SynKernel fused_kernel() { return {(const void*)k_dense_fused, 32 * kStageWarps, kStageSmem}; }
-
-// Blocks of one wave of kernel k on the current device (cached per device and kernel;
-// the shared-memory opt-in is set here, before the first launch).  Returns 0 when the
-// device cannot run it (the launch then reports an error).
-int resident_blocks(const SynKernel& k, int which)
-{
-    static std::atomic<int> cache[3][64];
+    static std::atomic<int> cache[2][64][kMaxThreads / 32 + 1];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    int n = cache[which][dev].load(std::memory_order_relaxed);
+    std::atomic<int>& c = cache[which][dev][threads / 32];
+    int n = c.load(std::memory_order_relaxed);
     if (n == 0) {
-        if (k.smem > 48 * 1024 &&
-            cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem) != cudaSuccess)
-            return 0;
         int sms = 0, per_sm = 0;
+        const void* fn = which ? (const void*)k_dense_fused : (const void*)k_dense_step<false>;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.threads, k.smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, ring_bytes(threads - 32)) !=
+                cudaSuccess ||
             sms * per_sm <= 0)
             return 0;
+        // no more shared memory than the blocks need: the rest is L1 for the gathers
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
+        const size_t need = (size_t)per_sm * (fa.sharedSizeBytes + ring_bytes(threads - 32) + 1024);
+        cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             (int)std::min<size_t>(100, (need * 100 + 233471) / 233472));
         n = sms * per_sm;
-        cache[which][dev].store(n, std::memory_order_relaxed);
+        c.store(n, std::memory_order_relaxed);
     }
     return n;
 }
 
-template <bool kFlush>
-int resident_syn_blocks()
-{
-    return resident_blocks(syn_kernel<kFlush>(), kFlush ? 1 : 0);
-}
-
-// Launches fn<<<grid, block, smem, s>>>(P) as a programmatic dependent launch.
-cudaError_t launch_pdl(const void* fn, int grid, int block, size_t smem, cudaStream_t s, const NcPools& P)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = NC_PDL ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, (void (*)(NcPools))fn, P);
-}
-
-template <bool kFlush>
-int launch_syn(const NcPools& P, const nc::LaunchShape& L, cudaStream_t s)
-{
-    const SynKernel k = syn_kernel<kFlush>();
-    const int wpb = k.threads / 32;
-    const int full = (P.n_spans + wpb - 1) / wpb;
-    if (full <= 0) return 0;
-    const int resident = resident_syn_blocks<kFlush>();
-    if (resident <= 0) return -1;
-    const int blocks = L.dense_blocks > 0 ? L.dense_blocks : (full < resident ? full : resident);
-    return launch_pdl(k.fn, blocks, k.threads, k.smem, s, P) == cudaSuccess ? 0 : -1;
-}
+// Threads per block: a neuron warp and at least one stream warp.
+int block_threads(const nc::LaunchShape& L) { return std::max(L.neuron_block, 64); }
 
 }  // namespace
 
 namespace nc {
 
-int launch_dense_synapses(const NcPools& P, const LaunchShape& L, void* stream)
+int dense_resident_blocks(int threads) { return resident_blocks(0, std::max(threads, 64)); }
+
+int launch_step_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
-    if (launch_syn<false>(P, L, (cudaStream_t)stream)) return -1;
+    // a net with no neuron has no tile, but its step counter still advances
+    const int threads = block_threads(L);
+    const int blocks = L.dense_blocks > 0 ? std::min(L.dense_blocks, P.row_blocks) : P.row_blocks;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = ring_bytes(threads - 32);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_dense_step<false>, P) != cudaSuccess) return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_dense_neurons(const NcPools& P, const LaunchShape& L, void* stream)
-{
-    const int wpb = L.neuron_block / 32;
-    const int blocks = (P.n_tiles + wpb - 1) / wpb;
-    if (blocks > 0 &&
-        launch_pdl((const void*)k_dense_neurons, blocks, L.neuron_block, 0, (cudaStream_t)stream, P) != cudaSuccess)
-        return -1;
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-int prepare_dense_launch()
-{
-    return resident_syn_blocks<false>() > 0 && resident_syn_blocks<true>() > 0 &&
-                   resident_blocks(fused_kernel(), 2) > 0
-               ? 0
-               : -1;
-}
-
-int launch_fused_dense(const NcPools& P, int32_t ticks, unsigned* bar, void* stream)
+int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, unsigned* bar, void* stream)
 {
     if (ticks <= 0) return 0;
-    const int resident = resident_blocks(fused_kernel(), 2);
+    const int threads = block_threads(L);
+    const int resident = resident_blocks(1, threads);
     if (resident <= 0) return -1;
-    // as many blocks as the larger pass has work for, at most one wave: a barrier over
-    // fewer blocks is quicker
-    const int need = std::max((P.n_spans + kStageWarps - 1) / kStageWarps, (P.n_tiles + kStageWarps - 1) / kStageWarps);
-    const int blocks = std::max(1, std::min(resident, need));
+    // at most one wave
+    const int blocks = std::min(resident, P.row_blocks);
     const cudaStream_t s = (cudaStream_t)stream;
     // the arrival count starts at zero (a barrier that gave up may have left it set)
     if (cudaMemsetAsync(bar, 0, sizeof(unsigned), s) != cudaSuccess) return -1;
     NcPools p = P;
     void* args[] = {(void*)&p, (void*)&ticks, (void*)&bar};
-    if (cudaLaunchCooperativeKernel((const void*)k_dense_fused, dim3((unsigned)blocks), dim3(32 * kStageWarps),
-                                    args, kStageSmem, s) != cudaSuccess)
+    if (cudaLaunchCooperativeKernel((const void*)k_dense_fused, dim3((unsigned)blocks), dim3((unsigned)threads), args,
+                                    ring_bytes(threads - 32), s) != cudaSuccess)
         return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_step_dense(const NcPools& P, const LaunchShape& L, void* stream)
-{
-    return launch_dense_synapses(P, L, stream) | launch_dense_neurons(P, L, stream);
-}
-
 int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
-    if (launch_syn<true>(P, L, (cudaStream_t)stream)) return -1;
+    const int threads = block_threads(L);
+    k_dense_step<true><<<P.row_blocks, threads, ring_bytes(threads - 32), (cudaStream_t)stream>>>(P);
     k_dense_mark_flushed<<<1, 256, 0, (cudaStream_t)stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -76,40 +76,70 @@ static __device__ __forceinline__ float plasticity(float w, bool inh, float trac
     return plasticity(w, inh, traceS, traceT, rates_of(D));
 }
 
-// The charge_insynapses term of a launch, deltaT*AP_depolFac*0.9943*exp(0.3702*deltaT)
-// (src/NeuCor.cpp:695) for x = deltaT*AP_depolFac.
+// The charge_insynapses term of a captured charge x = deltaT*AP_depolFac,
+// x*0.9943*exp(0.3702*deltaT) (src/NeuCor.cpp:695).
 static __device__ __forceinline__ double make_term(float x, double e_term)
 {
     return __dmul_rn(__dmul_rn((double)x, 0.9943), e_term);
 }
 
-// RN32 of a double, returned as the (exactly representable) double: the 52-bit
-// fraction is rounded to 23 bits, half to even, with integer operations, so the one
-// double add of `float += double` (src/NeuCor.cpp:695) stays the only FP64 instruction
-// of a fold.  `rare` is set for the magnitudes the integer path does not cover —
-// nonzero values below the float normal range, values from 2^127 up, infinities and
-// NaN — and the caller then redoes its batch with the hardware conversion.
-static __device__ __forceinline__ double rn32_int(double d, bool& rare)
+// The factor of every term of a net, 0.9943*exp(0.3702*deltaT), as a float and the float
+// of what it leaves (within 2^-49 of it together), and the binary64 factor of the exact form.
+struct TermFactor {
+    float hi, lo;
+    double e_term;
+};
+static __device__ __forceinline__ TermFactor term_factor(const NcNetDesc& D)
 {
-    unsigned long long u = (unsigned long long)__double_as_longlong(d);
-    const unsigned e = (unsigned)(u >> 52) & 0x7ffu;
-    rare |= (e - 897u > 1149u - 897u) && (u << 1) != 0ull;
-    u += 0x0FFFFFFFull + ((u >> 29) & 1ull);
-    u &= ~0x1FFFFFFFull;
-    return __longlong_as_double((long long)u);
+    return TermFactor{D.term_hi, D.term_lo, D.e_term};
 }
 
-// Exact `float += double` of the terms tp[b_k] (b_k >= 0, in k order) with the
-// hardware conversion.  Kept out of line so that the rare redo below is a branch and
-// its conversions are not issued with every batch.
-static __device__ __noinline__ double fold_exact8(double pd, const double* tp, int b0, int b1, int b2, int b3, int b4,
-                                                  int b5, int b6, int b7)
+// `p += term` of the charge x (src/NeuCor.cpp:695: a binary64 sum rounded to float) on float
+// arithmetic alone, by Ziv's rounding test: the term as a float pair th + tl within 2^-46 of
+// itself, p + th exactly as s + e (Knuth's TwoSum), and s + (e + tl) rounded from either end
+// of an interval that holds the exact sum, the binary64 rounding included.  Where both ends
+// round to the same float that float is the result; otherwise `ok` is cleared and the
+// caller redoes its batch exactly (6 in a million terms of ordinary networks; sums near
+// zero, infinities and NaN always).  An FP64 instruction takes a scheduler 64 cycles here
+// and a dependent add about 300: a batch of 8 took 2,400 cycles in a chain of binary64 adds
+// and takes 400 so.  (tests/test_fold_add.py compares the same arithmetic on the CPU.)
+static __device__ __forceinline__ float add_term(float p, float x, const TermFactor& F, bool& ok)
 {
-    const int b[8] = {b0, b1, b2, b3, b4, b5, b6, b7};
+    const float th = x * F.hi;
+    const float tl = __fmaf_rn(x, F.hi, -th) + x * F.lo;
+    const float s = p + th;
+    const float bb = s - p;
+    const float e = (p - (s - bb)) + (th - bb);
+    const float r = e + tl;
+    // half the interval: eight times the errors of r, tl and the binary64 rounding of the sum
+    const float base = __fmaf_rn(fabsf(s), 0x1p-50f, __fmaf_rn(fabsf(th), 0x1p-43f, 0x1p-120f));
+    const float d = __fmaf_rn(fabsf(r), 0x1p-21f, base);
+    const float a = s + (r + d);
+    ok = ok && a == s + (r - d);
+    return a;
+}
+
+// The exact form of fold8, on binary64.  Kept out of line: a rare redo.
+static __device__ __noinline__ float fold_exact8(float p, float x0, float x1, float x2, float x3, float x4, float x5,
+                                                 float x6, float x7, double e_term)
+{
+    const float x[8] = {x0, x1, x2, x3, x4, x5, x6, x7};
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        if (b[k] >= 0) pd = (double)__double2float_rn(__dadd_rn(pd, tp[b[k]]));
-    return pd;
+        p = __double2float_rn(__dadd_rn((double)p, make_term(x[k], e_term)));
+    return p;
+}
+
+// Folds the terms of the charges x[0..8) into p, in order.  An absent term is the charge
+// -0.0, which adds the term -0.0 and changes no p.
+static __device__ __forceinline__ float fold8(float p, const float x[8], const TermFactor& F)
+{
+    const float p0 = p;
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p = add_term(p, x[k], F, ok);
+    if (__builtin_expect(!ok, 0)) p = fold_exact8(p0, x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7], F.e_term);
+    return p;
 }
 
 // Whether a neuron out of its AP with potential `pot` (its sum so far) fires:
@@ -124,24 +154,6 @@ static __device__ __noinline__ double fold_exact8(double pd, const double* tp, i
 static __device__ __forceinline__ bool fires_at(float pot, float leak)
 {
     return -55.0f < (pot - -70.0f) * leak + -70.0f;
-}
-
-// Folds v[k] = tp[b[k]] for every k with b[k] >= 0 (ascending) into pd, the float
-// accumulator held as a double: `potential += term`, one double add and an integer
-// rounding to float per term.  (A fold on float arithmetic alone — the term split into
-// its float rounding and an integer tail, Fast2Sum and a tie test — is exact too, but
-// measured slower on this GPU: a warp's double add costs the issue of about 55 integer
-// instructions here, and the float path's fallback near a potential's zero crossing
-// costs more.)
-static __device__ __forceinline__ double fold8(double pd, const double v[8], const int b[8], const double* tp)
-{
-    const double pd0 = pd;
-    bool rare = false;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-        if (b[k] >= 0) pd = rn32_int(__dadd_rn(pd, v[k]), rare);
-    if (__builtin_expect(rare, 0)) pd = fold_exact8(pd0, tp, b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7]);
-    return pd;
 }
 
 static __device__ __forceinline__ void philox(uint32_t a, uint32_t b, uint32_t stream, uint32_t c, const NcNetDesc& D,

@@ -9,15 +9,20 @@
 // Per net, in HBM:
 //   neurons   pot, lf (last fire step), firings, act_start     SoA, pool-indexed
 //   in_ptr    CSC row starts (n+1): in-synapses of target j, ascending source id
-//             — the order of the reference's std::map inSynapses (src/NeuCor.h:212)
-//   w, t_arr, term          per in-synapse (CSC order): weight, last arrival step,
-//                           contribution term captured at launch (double)
-//   inh                     one bit per in-synapse: Synapse::inhibitory
-//   out_ptr   CSR row starts (n+1) and per out-synapse (CSR order): target,
-//             CSC index, delay (bits 0-13; bit 14/15: the target's caller id is
-//             above/below the source's), ring bit position, last accepted arrival step
+//             — the order of the reference's std::map inSynapses (src/NeuCor.h:212).
+//             Every row is padded to a multiple of 4 positions (a quad) with synapses
+//             that no source drives, so a quad belongs to one target and one thread
+//             moves it with 16-byte accesses.
+//   w, x      per in-synapse (CSC order): weight, and deltaT*AP_depolFac of the last
+//             accepted launch (the contribution term is formed from it when summed)
+//   dense form   key, state per in-synapse, qrow per quad (see NcPools)
+//   event form   t_arr (last arrival step) and inh (one bit: Synapse::inhibitory) per
+//                in-synapse; out_ptr CSR row starts (n+1) and per out-synapse (CSR
+//                order): target, CSC index, delay (bits 0-13; bit 14/15: the target's
+//                caller id is above/below the source's), ring bit position, last
+//                accepted arrival step
 //   Neurons sit in device slots (Morton order of positions by default); every rule
-//   that depends on ids uses the caller's ids (orig_id, the out_delay flags, the
+//   that depends on ids uses the caller's ids (orig_id, the order flags, the
 //   in-synapse order).
 //   ring      R slots x W words: bit b of target j's words in slot a mod R set when
 //             the spike on j's b-th in-synapse arrives at step a
@@ -35,7 +40,6 @@
 #define NC_NEVER INT32_MIN
 
 // Device error codes (NcPools::dev_err).
-#define NC_DEV_ERR_STAGE_TIMEOUT 1u  // a bulk copy into shared memory did not complete in time
 #define NC_DEV_ERR_FIRER_LOOP 2u     // an input firer's schedule did not advance (capped)
 #define NC_DEV_ERR_BARRIER 4u        // a grid barrier of the fused multi-step launch gave up
 
@@ -63,7 +67,7 @@ struct NcNetDesc {
     int32_t ptr_base;     // pool index of in_ptr/out_ptr/ring_off entry 0 (n+1 entries)
     int32_t word_base;    // pool index of this net's first bitset word
     int32_t n_words;      // ceil(n/32)
-    int64_t syn_base;     // pool index of synapse 0 (CSC and CSR arrays)
+    int64_t syn_base;     // pool index of synapse 0 (CSC and CSR arrays; a multiple of 32)
     int64_t ring_base;    // pool word index of ring slot 0
     int32_t ring_words;   // words per slot
     int32_t ring_mask;    // slots - 1
@@ -85,15 +89,47 @@ struct NcNetDesc {
     float c52;            // float(0.2f * 52.0) (src/NeuCor.cpp:729-730)
     float lr, pre_factor, post_factor;
     double e_term;        // 0.9943 is applied separately; this is exp(0.3702*dt) (src/NeuCor.cpp:695)
+    float term_hi, term_lo; // both factors as one: a float and the float of what it leaves
     uint32_t* raster;     // device raster rows of n_words words
     unsigned long long* stats; // 4 counters: fires, launched, dropped, steps
-    int64_t n_syn;        // synapses (the pool range is padded to a multiple of 32)
+    int64_t n_syn;        // synapses (out-synapse entries)
+    int64_t wide;         // dense form: 0, or the offset of the second range (NcPools::key)
     float tsum;           // NeuCor::currentTime after t-1 steps: the float sum of t-1 runSpeeds
     int32_t nonneg_terms; // 1: no launch can add a negative term (no inhibitory synapse, no
                           // negative weight), so a neuron's sum only grows within a step
     int32_t group_lo;     // caller ids [group_lo, group_hi) hold every input group's members
     int32_t group_hi;
+    int32_t key_shift;    // dense form: first bit of the source's slot in a key
 };
+
+// Dense form: how a synapse's last two arrivals are kept.  A launch is accepted only after
+// the previous spike has arrived (src/NeuCor.cpp:697, 728), so the last arrival of a
+// synapse is its last accepted one once that has arrived and the one before it until
+// then.  One 32-bit word holds both: bits 16-31 the accepted arrival step modulo 2^16,
+// bits 0-15 its distance from the arrival before.  With prev the step whose spikes are
+// being delivered, age = prev - arrival is negative while the spike travels (delays are
+// below 2^14).  Ages grow by one a step and every step visits every synapse: every
+// NC_AGE_PERIOD steps those past NC_AGE_LIMIT are set back to NC_AGE_OLD, an age at which
+// they already count as never launched (free, outside the fold window, trace underflowed
+// to zero), so that 16 bits never wrap.
+#define NC_AGE_PERIOD 1024
+#define NC_AGE_LIMIT 30000
+#define NC_AGE_OLD 21808
+// The age of a synapse whose state word is s.
+NC_HD inline int32_t nc_state_age(uint32_t s, int32_t prev)
+{
+    return (int32_t)((((uint32_t)prev << 16) | 0xffffu) - s) >> 16;
+}
+// The state of a synapse whose accepted spike arrives at prev - age, gap steps after the
+// arrival before it.
+NC_HD inline uint32_t nc_state_word(int32_t prev, int32_t age, int32_t gap)
+{
+    return ((uint32_t)(prev - age) << 16) | (uint32_t)gap;
+}
+// Never launched, for a network whose next step is 1.
+NC_HD inline uint32_t nc_state_never() { return nc_state_word(0, NC_AGE_OLD, 0); }
+// The same for a network that keeps whole step counters (NcNetDesc::wide).
+#define NC_WIDE_NEVER (-(1 << 30))
 
 // The smallest id range holding the members of groups g[0..n) (empty when n is 0).
 inline void nc_group_range(const NcGroupDev* g, int n, int32_t& lo, int32_t& hi)
@@ -113,12 +149,23 @@ inline void nc_group_range(const NcGroupDev* g, int n, int32_t& lo, int32_t& hi)
     }
 }
 
-struct NcTile {          // 32 consecutive neurons of one net, or (span table) 8 chunks of
-    int32_t net;         // 32 in-synapses
-    int32_t first;       // local id of the first neuron (multiple of 32), or first chunk
+struct NcTile {          // event form: 32 consecutive neurons of one net
+    int32_t net;
+    int32_t first;       // local id of the first neuron (multiple of 32)
 };
 
-constexpr int NC_SPAN_CHUNKS = 8;  // 32-synapse chunks per span of the dense synapse pass
+struct alignas(16) NcRowTile {  // dense form: up to NC_TILE_ROWS consecutive neurons and their rows
+    uint32_t q0;         // pool index of the first quad of its rows
+    int32_t nq;          // quads
+    int32_t net;
+    int32_t first;       // local id of the first neuron (a multiple of 8)
+    int32_t neuron;      // pool index of the first neuron
+    int32_t ptr;         // pool index of its row start
+    int32_t count;       // neurons
+    int32_t pad;
+};
+
+constexpr int NC_TILE_ROWS = 32;  // neurons of a dense tile at most: one per lane
 
 struct NcFirer {         // periodic input firer (InputFirer, src/NeuCor.cpp:305-345)
     int32_t net;
@@ -128,6 +175,12 @@ struct NcFirer {         // periodic input firer (InputFirer, src/NeuCor.cpp:305
     int32_t near_end;
     int32_t first;       // set before the net's first step: the run call at time 0 evaluates it too
 };
+
+// Low bits of a key.
+#define NC_KEY_AFTER 1u    // the target's caller id is above the source's
+#define NC_KEY_BEFORE 2u   // it is below
+#define NC_KEY_INH 4u      // Synapse::inhibitory
+#define NC_KEY_DELAY_SHIFT 3
 
 struct NcPools {
     // neurons
@@ -143,27 +196,32 @@ struct NcPools {
     int32_t* ring_off;   // word offset within a slot
     // in-synapses (CSC); every net's synapse base is a multiple of 32
     float* w;
-    uint32_t* inh;       // Synapse::inhibitory, one bit per synapse
-    int32_t* t_arr;
-    double* term;        // last launch's charge_insynapses term (src/NeuCor.cpp:695)
+    float* x;            // deltaT*AP_depolFac of the last accepted launch (src/NeuCor.cpp:695, 729-731)
     // out-synapses (CSR)
     int32_t* out_post;   // local target id
     int32_t* out_csc;    // CSC index relative to syn_base
     int16_t* out_delay;
     uint32_t* out_ringpos; // (word within slot) << 5 | bit
     int32_t* last_arr;
-    // dense form: in-synapse (CSC) order
-    int32_t* csc_pre;    // source's device slot (local to the net)
-    int32_t* csc_post;   // target's device slot (local to the net)
-    uint16_t* csc_dl;    // delay | target-above-source << 14 | target-below-source << 15
-    int32_t* la_c;       // arrival step of the last accepted launch
-    float* pst;          // per neuron, written by the neuron pass of step t for the synapse
-                         // pass of t+1: the postsynaptic trace at t (getTrace), or -0.0
-                         // when the neuron fired at t
-    uint32_t* win;       // bit per synapse: arrived within the fold window of the net's step
-    NcTile* spans;       // work items of the synapse pass
-    int32_t n_spans;
-    int32_t* n_spans_dev; // when set, the span count is read from device memory (served engine)
+    uint32_t* inh;       // event form, CSC: Synapse::inhibitory, one bit per synapse
+    int32_t* t_arr;      // event form, CSC: last arrival step
+    // dense form: in-synapse (CSC) order, one quad of four per thread.
+    //   key    NC_KEY_* flags, the delay in steps and, from bit key_shift up, the source's
+    //          device slot (a padding position: a slot past the last, whose fired bit is
+    //          never set)
+    //   state  last accepted arrival and its distance from the one before (nc_state_age)
+    // A net whose slots and delays do not fit one word, or whose trace outlasts
+    // NC_AGE_OLD steps, takes a second range of both (wide = its offset): key holds the
+    // slot alone and key[wide + s] the flags and delay; state the whole arrival step and
+    // state[wide + s] the one before it.
+    uint32_t* key;
+    uint32_t* state;
+    float* pst;          // per neuron: its trace at its last step (src/NeuCor.cpp:671-675)
+    uint8_t* qrow;       // per quad: low 5 bits of its target's slot
+    uint8_t* nib;        // per quad: window bits of tiles too large for shared memory
+    NcRowTile* rtiles;   // in the order of the blocks that run them
+    int32_t* rstart;     // first tile of each of row_blocks blocks (row_blocks + 1 entries)
+    int32_t row_blocks;
     // ring and bitsets
     uint32_t* ring;
     uint32_t* fired;     // 2 parities x total_words
@@ -232,44 +290,41 @@ namespace nc {
 #ifndef NC_NEURON_MIN_BLOCKS
 #define NC_NEURON_MIN_BLOCKS 3
 #endif
-#ifndef NC_DENSE_MIN_BLOCKS
-#define NC_DENSE_MIN_BLOCKS 4
-#endif
-#ifndef NC_DNEURON_BLOCK
-#define NC_DNEURON_BLOCK 128  // threads per block of the dense neuron pass
+#ifndef NC_DENSE_BLOCK
+#define NC_DENSE_BLOCK 96  // threads per block of the dense step: one warp sums, the others stream
 #endif
 #ifndef NC_LAUNCH_MIN_BLOCKS
 #define NC_LAUNCH_MIN_BLOCKS 4
 #endif
 
 struct LaunchShape {
-    int neuron_block;    // threads per block of the neuron-update kernel (multiple of 32)
+    int neuron_block;    // threads per block of the neuron update or of the dense step (multiple of 32)
     int launch_blocks;   // blocks of the spike-launch kernel
     int launch_block;    // threads per block of the spike-launch kernel
-    int dense_blocks = 0; // blocks of the dense synapse pass (0: one warp per span)
-    int fused_ticks = 0;  // dense form: steps per fused cooperative launch (0: two launches
+    int dense_blocks = 0; // dense form: blocks of the step (0: one wave, or one per tile)
+    int fused_ticks = 0;  // dense form: steps per fused cooperative launch (0: one launch
                           // per step, replayed through CUDA graphs)
 };
 int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream);
 int launch_spike_launch(const NcPools& P, const LaunchShape& L, void* stream);
 int launch_stdp_flush(const NcPools& P, const LaunchShape& L, void* stream);
-// Dense form (nc_dense.cu): the synapse pass and the neuron pass of one step, and the
-// plasticity flush (the synapse pass of the last step's fires) before read-back.
-int launch_dense_synapses(const NcPools& P, const LaunchShape& L, void* stream);
-int launch_dense_neurons(const NcPools& P, const LaunchShape& L, void* stream);
-// Sizes the dense synapse pass's persistent grid (and sets its shared-memory opt-in) on
-// the current device; called before a stream capture, where neither may happen.
-int prepare_dense_launch();
+// Dense form (nc_dense.cu): one step in one launch, and the plasticity flush (the launches
+// and plasticity of the last step's fires) before read-back.
 int launch_step_dense(const NcPools& P, const LaunchShape& L, void* stream);
+// Blocks of `threads` threads of the dense step that fit on the current device at once (0:
+// the device cannot run it); called before a stream capture, where it may not be asked.
+int dense_resident_blocks(int threads);
 // `ticks` whole dense steps of every net in one cooperative launch (no periodic input
 // firers); bar: two zero-initialised words of device memory for its grid barrier.
-int launch_fused_dense(const NcPools& P, int32_t ticks, unsigned* bar, void* stream);
+int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, unsigned* bar, void* stream);
 // Conversion of net `net`'s per-synapse arrival state between the forms (nc_form.cu),
 // after the current form's plasticity flush.  ring_words: the words of the whole ring
 // pool (cleared first).
 int launch_form_to_event(const NcPools& P, int net, int64_t n_syn, int64_t ring_words, void* stream);
 int launch_form_to_dense(const NcPools& P, int net, int64_t n_syn, void* stream);
 int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream);
+// count words of a set to v.
+int launch_fill_words(uint32_t* a, int64_t count, uint32_t v, void* stream);
 int launch_background_prologue(const NcPools& P, int net, int n_neurons, void* stream);
 int launch_force_bits(const NcPools& P, int net, const int32_t* d_ids, int count, void* stream);
 // Input firers (nc_inputs.cu), launched before a step's kernels: each firer's schedule

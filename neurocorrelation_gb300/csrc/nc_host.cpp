@@ -110,11 +110,12 @@ int64_t NetHost::device_bytes() const
 {
     const int64_t per_neuron = 4 + 4 + 4 + 4 + 8 + 8 + 4;             // pot lf firings act_start in_ptr out_ptr ring_off
     const bool dense = p.step_mode != NC_STEP_EVENT, event = p.step_mode != NC_STEP_DENSE;
-    // w t_arr term | csc_pre csc_post csc_dl la_c (dense) and/or out_post out_csc delay ringpos last_arr (event)
-    const int64_t per_syn = 4 + 4 + 8 + (dense ? 4 + 4 + 2 + 4 : 0) + (event ? 4 + 4 + 2 + 4 + 4 : 0);
+    // w x | key state (dense) and/or t_arr out_post out_csc delay ringpos last_arr (event); rows are
+    // padded to quads, and a quad has a row byte and a window byte
+    const int64_t per_syn = 4 + 4 + (dense ? 8 * key_words(*this) + 1 : 0) + (event ? 4 + 4 + 4 + 2 + 4 + 4 : 0);
     const int64_t words = ((int64_t)n + 31) / 32;
     const int64_t ring_bytes = event ? 4 * (int64_t)ring_slots * ring_words : 0;
-    return per_neuron * (n + 1) + per_syn * s + ring_bytes + 4 * 4 * words +
+    return per_neuron * (n + 1) + per_syn * sp + ring_bytes + 4 * 4 * words +
            8 * 2 * (int64_t)n + 4 * (int64_t)tables.size() + (int64_t)sizeof(NcGroupDev) * (int64_t)groups.size();
 }
 
@@ -224,8 +225,7 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
     h.csc_pre.reserve((size_t)n_syn);
     h.csc_delay.reserve((size_t)n_syn);
     h.w.reserve((size_t)n_syn);
-    std::vector<int64_t> csc_input;
-    csc_input.reserve((size_t)n_syn);
+    std::vector<int64_t> row_end((size_t)n, 0);
     for (int32_t j = 0; j < n; ++j) {
         auto b = order.begin() + bstart[j], e = order.begin() + bstart[j + 1];
         std::stable_sort(b, e, [&](int64_t x, int64_t y) { return from[x] < from[y]; });
@@ -236,7 +236,6 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
             last_pre = from[k];
             const int64_t c = (int64_t)h.csc_pre.size();
             h.input_to_csc[(size_t)k] = c;
-            csc_input.push_back(k);
             h.csc_pre.push_back(h.slot_of[(size_t)from[k]]);
             const float len = length ? length[k] : get_dist(&h.xyz[3 * (size_t)from[k]], &h.xyz[3 * (size_t)to[k]]);
             const int32_t d = delay_steps(len, h.dt);
@@ -245,14 +244,22 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
             h.max_delay = std::max(h.max_delay, d);
             h.w.push_back(weight[k]);
         }
+        h.s += (int64_t)h.csc_pre.size() - h.in_ptr[j];
+        row_end[(size_t)j] = (int64_t)h.csc_pre.size();
+        while (h.csc_pre.size() & (size_t)(row_align(j) - 1)) {
+            h.csc_pre.push_back(pad_slot(n));
+            h.csc_delay.push_back(0);
+            h.w.push_back(0.0f);
+        }
         h.in_ptr[j + 1] = (int64_t)h.csc_pre.size();
     }
-    h.s = (int64_t)h.csc_pre.size();
+    h.sp = (int64_t)h.csc_pre.size();
+    if (h.s >= (1ll << 31) || h.sp >= (1ll << 32)) { err = "too many synapses in one network"; return NC_ERR_INVALID; }
 
     // ring words per target: one bit per in-synapse
     h.ring_off.assign((size_t)n + 1, 0);
     for (int32_t j = 0; j < n; ++j) {
-        const int64_t fan = h.in_ptr[j + 1] - h.in_ptr[j];
+        const int64_t fan = row_end[(size_t)j] - h.in_ptr[j];
         const int64_t words = (fan + 31) / 32;
         if ((int64_t)h.ring_off[j] + words >= (1ll << 27)) { err = "network too large for one ring slot"; return NC_ERR_INVALID; }
         h.ring_off[j + 1] = h.ring_off[j] + (int32_t)words;
@@ -261,45 +268,67 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
     h.ring_slots = 1;
     while (h.ring_slots < h.max_delay + h.kc + 1) h.ring_slots <<= 1;
 
+    // tables: presynaptic trace, postsynaptic trace, AP shape
+    h.tables.clear();
+    if (!trace_table(p.presynaptic_trace_decay, h.dt, h.tables, h.tab_pre_len) ||
+        !trace_table(p.postsynaptic_trace_decay, h.dt, h.tables, h.tab_post_len)) {
+        err = "trace table does not underflow";
+        return NC_ERR_INVALID;
+    }
+    h.ap_len = h.kc;
+    for (int32_t k = 0; k < h.kc; ++k) h.tables.push_back(ap_value(step_ms(k, h.dt)));
+
+    choose_key(h);
+    const bool dense = p.step_mode != NC_STEP_EVENT;
+    if (dense) {
+        h.key.resize((size_t)(h.sp * key_words(h)));
+        h.qrow.resize((size_t)(h.sp / 4));
+        for (int64_t c = 0; c < h.sp; ++c) h.key[(size_t)c] = (uint32_t)h.csc_pre[(size_t)c] << h.key_shift;
+        for (int32_t j = 0; j < n; ++j)
+            for (int64_t q = h.in_ptr[j] / 4; q < h.in_ptr[j + 1] / 4; ++q) h.qrow[(size_t)q] = (uint8_t)(j & 31);
+    }
+
     // CSR: each source's out-synapses in creation order (Neuron::outSynapses)
     h.out_ptr.assign((size_t)n + 1, 0);
-    for (int64_t c = 0; c < h.s; ++c) h.out_ptr[(size_t)h.csc_pre[c] + 1]++;
+    for (int32_t j = 0; j < n; ++j)
+        for (int64_t c = h.in_ptr[j]; c < row_end[(size_t)j]; ++c) h.out_ptr[(size_t)h.csc_pre[c] + 1]++;
     for (int32_t i = 0; i < n; ++i) h.out_ptr[i + 1] += h.out_ptr[i];
     h.out_post.assign((size_t)h.s, 0);
     h.out_csc.assign((size_t)h.s, 0);
     h.out_delay.assign((size_t)h.s, 0);
-    h.out_ringpos.assign((size_t)h.s, 0);
-    h.csc_dl.assign((size_t)h.s, 0);
+    const bool event = p.step_mode != NC_STEP_DENSE;
+    if (event) h.out_ringpos.assign((size_t)h.s, 0);
     {
         std::vector<int64_t> fill(h.out_ptr.begin(), h.out_ptr.end() - 1);
-        std::vector<int32_t>& csc_post = h.csc_post;
-        csc_post.assign((size_t)h.s, 0);
-        for (int32_t j = 0; j < n; ++j)
-            for (int64_t c = h.in_ptr[j]; c < h.in_ptr[j + 1]; ++c) csc_post[(size_t)c] = j;
         for (int64_t k = 0; k < n_syn; ++k) {
             const int64_t c = h.input_to_csc[(size_t)k];
             if (c < 0) continue;
-            const int32_t i = h.csc_pre[(size_t)c], j = csc_post[(size_t)c];
+            const int32_t i = h.csc_pre[(size_t)c], j = h.slot_of[(size_t)to[k]];
             const int64_t q = fill[i]++;
             const int64_t b = c - h.in_ptr[j];
             h.out_post[(size_t)q] = j;
-            h.out_csc[(size_t)q] = (int32_t)c;
+            h.out_csc[(size_t)q] = (int32_t)(uint32_t)c;
             // the same-step order rules compare the caller's ids of target and source
             const uint32_t flags = (to[k] > from[k] ? 1u << kAfterBit : 0u) | (to[k] < from[k] ? 1u << kBeforeBit : 0u);
             h.out_delay[(size_t)q] = (int16_t)(uint16_t)((uint32_t)h.csc_delay[(size_t)c] | flags);
-            h.csc_dl[(size_t)c] = (uint16_t)((uint32_t)h.csc_delay[(size_t)c] | flags);
+            if (dense) {
+                const uint32_t hi = (uint32_t)h.csc_delay[(size_t)c] << NC_KEY_DELAY_SHIFT |
+                                    (to[k] > from[k] ? NC_KEY_AFTER : 0u) | (to[k] < from[k] ? NC_KEY_BEFORE : 0u);
+                if (h.wide) h.key[(size_t)(h.sp + c)] = hi;
+                else h.key[(size_t)c] |= hi;
+            }
+            if (!event) continue;
             h.out_ringpos[(size_t)q] = ((uint32_t)(h.ring_off[j] + (int32_t)(b >> 5)) << 5) | (uint32_t)(b & 31);
         }
     }
-    if (h.s >= (1ll << 31)) { err = "too many synapses in one network"; return NC_ERR_INVALID; }
 
     // Synapse::inhibitory: setWeight's sign (src/NeuCor.cpp:576-579), lost by synapses
     // the vector growth copied (rule COPY_LOSS), or the caller's own flags
-    h.inh_bits.assign((size_t)((h.s + 31) / 32), 0u);
+    h.inh_bits.assign((size_t)((h.sp + 31) / 32), 0u);
     for (int32_t i = 0; i < n; ++i) {
         const int64_t size = h.out_ptr[i + 1] - h.out_ptr[i];
         for (int64_t m = 0; m < size; ++m) {
-            const int64_t c = h.out_csc[(size_t)(h.out_ptr[i] + m)];
+            const int64_t c = (uint32_t)h.out_csc[(size_t)(h.out_ptr[i] + m)];
             bool inh = h.w[(size_t)c] < 0.0f;
             if (p.inhibitory_rule == NC_INHIBITORY_COPY_LOSS && grown_copy(m, size)) inh = false;
             if (inh) h.inh_bits[(size_t)(c >> 5)] |= 1u << (c & 31);
@@ -321,16 +350,66 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
     for (uint32_t b : h.inh_bits) h.nonneg_terms = h.nonneg_terms && b == 0u;
     for (float x : h.w) h.nonneg_terms = h.nonneg_terms && x >= 0.0f;
 
-    // tables: presynaptic trace, postsynaptic trace, AP shape
-    h.tables.clear();
-    if (!trace_table(p.presynaptic_trace_decay, h.dt, h.tables, h.tab_pre_len) ||
-        !trace_table(p.postsynaptic_trace_decay, h.dt, h.tables, h.tab_post_len)) {
-        err = "trace table does not underflow";
-        return NC_ERR_INVALID;
+    if (dense) {
+        for (size_t w = 0; w < h.inh_bits.size(); ++w)
+            for (uint32_t m = h.inh_bits[w]; m; m &= m - 1u) {
+                int b = 0;
+                while (!((m >> b) & 1u)) ++b;
+                h.key[(h.wide ? (size_t)h.sp : 0) + 32 * w + (size_t)b] |= NC_KEY_INH;
+            }
     }
-    h.ap_len = h.kc;
-    for (int32_t k = 0; k < h.kc; ++k) h.tables.push_back(ap_value(step_ms(k, h.dt)));
     return NC_OK;
+}
+
+void choose_key(NetHost& h)
+{
+    auto bits = [](uint32_t v) {
+        int32_t b = 0;
+        while (b < 32 && v >> b) ++b;
+        return b;
+    };
+    // one word per synapse holds slot, flags and delay, and one the last two arrivals, unless
+    // the delay needs more bits than the slot leaves or an age that still matters (a trace
+    // not yet underflowed, the fold window) could pass NC_AGE_OLD
+    const int32_t slot_bits = std::max(1, bits((uint32_t)pad_slot(h.n)));
+    h.wide = slot_bits + NC_KEY_DELAY_SHIFT + bits((uint32_t)h.max_delay) > 32 || h.tab_pre_len > NC_AGE_OLD ||
+             h.kc + 1 > NC_AGE_OLD;
+    h.key_shift = h.wide ? 0 : 32 - slot_bits;
+}
+
+void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTile>& tiles,
+               std::vector<int32_t>& start)
+{
+    // a run of 8 neurons weighs its quads and a little for the neurons themselves
+    constexpr int64_t kNeuronWeight = 2;
+    int64_t total = 0, done = 0;
+    for (const RowNet& r : nets) total += r.h->sp / 4 + kNeuronWeight * r.h->n;
+    tiles.clear();
+    start.assign(1, 0);
+    for (const RowNet& r : nets) {
+        const NetHost& h = *r.h;
+        bool open = false;  // the last tile may grow
+        for (int32_t f = 0; f < h.n; f += 8) {
+            const int32_t count = std::min(h.n - f, 8);
+            const int64_t a = h.in_ptr[(size_t)f], b = h.in_ptr[(size_t)(f + count)];
+            const int64_t weight = (b - a) / 4 + kNeuronWeight * count;
+            // the block its middle falls to
+            const int64_t block = std::min<int64_t>(blocks - 1, (int64_t)((done + 0.5 * weight) * blocks / total));
+            done += weight;
+            while ((int64_t)start.size() <= block) {
+                start.push_back((int32_t)tiles.size());
+                open = false;
+            }
+            if (!open || tiles.back().count + count > NC_TILE_ROWS) {
+                tiles.push_back(NcRowTile{(uint32_t)((r.syn_base + a) / 4), 0, r.net, f, r.neuron_base + f,
+                                          r.ptr_base + f, 0, 0});
+                open = true;
+            }
+            tiles.back().nq += (int32_t)((b - a) / 4);
+            tiles.back().count += count;
+        }
+    }
+    while ((int)start.size() <= blocks) start.push_back((int32_t)tiles.size());
 }
 
 int set_groups(NetHost& h, int32_t n_groups, const nc_group* groups, std::string& err)

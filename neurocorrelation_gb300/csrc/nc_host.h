@@ -14,6 +14,7 @@ namespace nc {
 struct NetHost {
     int32_t n = 0;
     int64_t s = 0;        // synapses kept
+    int64_t sp = 0;       // in-synapse (CSC) positions: s and the padding of the rows to quads
     int64_t n_input = 0;  // synapses given
     nc_params p{};
     float dt = 1.0f;
@@ -29,16 +30,20 @@ struct NetHost {
     std::vector<int32_t> slot_of;           // caller's id -> device slot
     bool permuted = false;
     // Below, neurons are device slots.  The in-synapses of a target are sorted by the
-    // caller's source id; out_delay packs the delay (bits 0-13) and whether the target's
+    // caller's source id, each row padded to a multiple of 4 positions; out_delay packs the delay (bits 0-13) and whether the target's
     // caller id is above (bit 14) or below (bit 15) the source's.
     std::vector<int64_t> in_ptr, out_ptr;   // n+1
     std::vector<int32_t> ring_off;          // n+1
     std::vector<float> w;                   // CSC
     std::vector<uint32_t> inh_bits;         // CSC, bit per synapse: Synapse::inhibitory
     std::vector<int32_t> csc_pre, csc_delay;
-    std::vector<uint16_t> csc_dl;           // CSC: delay | flags, as out_delay (dense form)
-    std::vector<int32_t> csc_post;          // CSC: target slot (dense form)
-    std::vector<int32_t> out_post, out_csc;
+    // dense form: key of every in-synapse (NcPools::key; when wide, of sp slots and then
+    // of sp flags and delays), row of every quad
+    std::vector<uint32_t> key;
+    std::vector<uint8_t> qrow;
+    int32_t key_shift = 0;
+    bool wide = false;
+    std::vector<int32_t> out_post, out_csc; // out_csc: below 2^32, read as unsigned
     std::vector<int16_t> out_delay;
     std::vector<uint32_t> out_ringpos;
     std::vector<int64_t> input_to_csc;      // -1 for ignored duplicates
@@ -50,6 +55,37 @@ struct NetHost {
     int64_t device_bytes() const;
 };
 
+// Source slot of a padding position: past the net's last slot, in the spare word of its
+// fired bits (nothing ever sets it).
+inline int32_t pad_slot(int32_t n) { return (n + 31) / 32 * 32; }
+// Rows end at a multiple of 4 positions, and every eighth at one of 32: tiles start at
+// multiples of 8 neurons, so a warp's 16-byte accesses start on a 128-byte line.
+inline int64_t row_align(int32_t j) { return (j & 7) == 7 ? 32 : 4; }
+// Chooses key_shift and wide from the net's size, longest delay and tables.
+void choose_key(NetHost& h);
+// Whether the dense form's arrays hold whole step counters and a second range of keys
+// (NcPools::key); the words they take per position.
+inline int64_t key_words(const NetHost& h) { return h.wide ? 2 : 1; }
+// 0.9943*exp(0.3702*dt) as a float and the float of what it leaves.
+inline void term_pair(const NetHost& h, float& hi, float& lo)
+{
+    const double k = 0.9943 * h.e_term;
+    hi = (float)k;
+    lo = (float)(k - (double)hi);
+}
+// Initial state word (never launched) of the net's positions.
+inline uint32_t initial_state(const NetHost& h) { return h.wide ? (uint32_t)NC_WIDE_NEVER : nc_state_never(); }
+// The row tiles of an engine's nets, and the first tile of each of `blocks` blocks (blocks
+// + 1 entries): consecutive runs of neurons with an even share of the quads each, cut at
+// multiples of 8 neurons and into tiles of at most NC_TILE_ROWS.
+struct RowNet {              // a net and its pool indexes
+    const NetHost* h;
+    int32_t net;
+    int64_t syn_base;
+    int32_t neuron_base, ptr_base;
+};
+void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTile>& tiles,
+               std::vector<int32_t>& start);
 // Builds the layout; returns NC_OK or an NC_ERR_* code with `err` set.
 int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, const int32_t* to,
               const float* weight, const float* length, const uint8_t* inhibitory, const nc_params& p,

@@ -16,8 +16,8 @@
 //
 //   k_spike_launch (one warp per fired neuron)
 //     Synapse::fire (src/NeuCor.cpp:727-738) on each out-synapse: drop if busy,
-//     capture fl(fl(0.2f*52)*w), compute the contribution term, mark the ring bit of
-//     the arrival step.  The last block advances every net's step counter.
+//     capture fl(fl(0.2f*52)*w) times deltaT (the fold forms the contribution term from
+//     it), mark the ring bit of the arrival step.  The last block advances every net's step counter.
 //
 // The CPU restatement runs neurons in ascending id, each update firing at once.
 // Two rules make the split launches produce the same bits:
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
                 // cross the threshold, so only its sum is skipped.
                 const bool in_ap = lf != NC_NEVER && t - lf < D.kc;
                 if (r1 > r0) {
-                    double pd = (double)pot;
+                    const TermFactor F = term_factor(D);
                     // the sum is not needed inside the AP, nor, when no term can be
                     // negative, once the neuron is certain to fire (fires_at)
                     const bool stop = NC_FOLD_EARLY_EXIT && D.nonneg_terms;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
                         const int64_t sb = s0 + (int64_t)(wi - r0) * 32;
                         unsigned long long ih = 0ull;
                         if (arr) ih = inh_bits32(P, sb) | ((unsigned long long)(two ? inh_bits32(P, sb + 32) : 0u) << 32);
-                        // arrival branch first (it touches w and t_arr only, the fold reads term)
+                        // arrival branch first (it touches w and t_arr only, the fold reads x)
                         unsigned long long am = arr;
                         while (am) {
                             int b[8];
@@ -229,13 +229,11 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
                         while (bits) {
                             int b[8];
                             pop8_64(&bits, b);
-                            double v[8];
-                            const double* tp = P.term + sb;
+                            float xv[8];
 #pragma unroll
-                            for (int k = 0; k < 8; ++k)
-                                if (b[k] >= 0) v[k] = tp[b[k]];
-                            pd = fold8(pd, v, b, tp);
-                            if (stop && fires_at((float)pd, D.leak)) {
+                            for (int k = 0; k < 8; ++k) xv[k] = b[k] >= 0 ? P.x[sb + b[k]] : -0.0f;
+                            pot = fold8(pot, xv, F);
+                            if (stop && fires_at(pot, D.leak)) {
                                 settled = true;
                                 bits = 0ull;
                             }
@@ -247,7 +245,6 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
                             if (two && ohi) orow[1] = 0u;
                         }
                     }
-                    pot = __double2float_rn(pd);
                 }
                 // charge_passive (src/NeuCor.cpp:677-680)
                 pot = (pot - -70.0f) * D.leak + -70.0f;
@@ -356,7 +353,6 @@ __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPo
         const int64_t syn_base = D.syn_base, ring_words = D.ring_words;
         const float dt = D.dt, c52 = D.c52;
         const Rates R = rates_of(D);
-        const double e_term = D.e_term;
         int nl = 0, nd = 0;
         // four out-synapses per lane in flight: table loads, then weight loads, then writes
         for (int64_t kb = k0; kb < k1; kb += 128) {
@@ -379,7 +375,7 @@ __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPo
             for (int u = 0; u < 4; ++u) {
                 // freed by the target's update at t only if the target's id is not above
                 acc[u] = ok[u] && (la[u] == NC_NEVER || t - la[u] >= kc + (int32_t)((dl[u] >> 14) & 1u));
-                if (acc[u]) wv[u] = P.w[syn_base + cs[u]];
+                if (acc[u]) wv[u] = P.w[syn_base + (uint32_t)cs[u]];
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -389,7 +385,7 @@ __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPo
                     continue;
                 }
                 const int64_t k = kb + lane + 32 * u;
-                const int64_t s = syn_base + cs[u];
+                const int64_t s = syn_base + (uint32_t)cs[u];
                 float w = wv[u];
                 if ((dl[u] >> 15) & 1u) {  // target id below the source's: its update ran first
                     const int32_t j = P.out_post[k];
@@ -398,8 +394,7 @@ __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPo
                 }
                 // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
                 const float depol = c52 * w;
-                // deltaT*AP_depolFac*0.9943*exp(0.3702*deltaT)  (src/NeuCor.cpp:695)
-                P.term[s] = make_term(dt * depol, e_term);
+                P.x[s] = dt * depol;
                 const int32_t d = (int32_t)(dl[u] & 0x3fffu);
                 P.last_arr[k] = t + d;
                 const uint32_t pos = P.out_ringpos[k];
@@ -513,6 +508,12 @@ __global__ void k_background_prologue(NcPools P, int net)
     }
 }
 
+__global__ void k_fill_words(uint32_t* a, int64_t count, uint32_t v)
+{
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < count; k += (int64_t)gridDim.x * blockDim.x)
+        a[k] = v;
+}
+
 // Forced fire requests for the net's next step (Neuron::scheduleFire).
 __global__ void k_force_bits(NcPools P, int net, const int32_t* ids, int count)
 {
@@ -582,6 +583,14 @@ int launch_stdp_flush(const NcPools& P, const LaunchShape& L, void* stream)
     const int blocks = (P.n_tiles + warps_per_block - 1) / warps_per_block;
     if (blocks > 0) k_stdp_flush<<<blocks, L.neuron_block, 0, (cudaStream_t)stream>>>(P);
     k_mark_flushed<<<1, 256, 0, (cudaStream_t)stream>>>(P);
+    return check_launch();
+}
+
+int launch_fill_words(uint32_t* a, int64_t count, uint32_t v, void* stream)
+{
+    if (count <= 0) return 0;
+    const int64_t blocks = (count + 1023) / 1024;
+    k_fill_words<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, (cudaStream_t)stream>>>(a, count, v);
     return check_launch();
 }
 

@@ -80,6 +80,19 @@ static cudaError_t upload(T* dev, const std::vector<T>& host, size_t offset, cud
     return cudaMemcpyAsync(dev + offset, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
+template <class T>
+static cudaError_t upload_part(T* dev, const std::vector<T>& host, int64_t at, int64_t from, int64_t count,
+                               cudaStream_t s)
+{
+    if (count <= 0) return cudaSuccess;
+    return cudaMemcpyAsync(dev + at, host.data() + from, (size_t)count * sizeof(T), cudaMemcpyHostToDevice, s);
+}
+
+int dense_blocks(int64_t neurons, int threads)
+{
+    return (int)std::max<int64_t>(1, std::min<int64_t>(dense_resident_blocks(threads), (neurons + 7) / 8));
+}
+
 void Engine::set_launch(const LaunchShape& shape, int ticks_per_graph)
 {
     release_graph();
@@ -97,14 +110,11 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     dense = nets.empty() || nets[0]->p.step_mode != NC_STEP_EVENT;
     both = !nets.empty() && nets[0]->p.step_mode == NC_STEP_AUTO;
     const bool event_tables = !dense || both;
-    // the dense neuron pass is one wave: 128-thread blocks spread it more evenly over the
-    // SMs (measured 2% faster on the 100k x 100 network than 256)
-    L.neuron_block = dense ? NC_DNEURON_BLOCK : 256;
     L.launch_block = 256;
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_MIN_BLOCKS);
 
     // pool sizes
-    int64_t neurons = 0, ptrs = 0, words = 0, syn = 0, ring = 0, tables = 0, tiles = 0, spans = 0;
+    int64_t neurons = 0, ptrs = 0, words = 0, syn = 0, ring = 0, tables = 0, tiles = 0;
     const int ngroups_each = std::max(group_capacity, 1);
     slots.clear();
     std::vector<NcNetDesc> desc;
@@ -157,17 +167,20 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         d.pre_factor = h.p.presynaptic_factor;
         d.post_factor = h.p.postsynaptic_factor;
         d.e_term = h.e_term;
+        term_pair(h, d.term_hi, d.term_lo);
         d.n_syn = h.s;
+        d.key_shift = h.key_shift;
+        const int64_t range = (h.sp + 31) / 32 * 32;  // keeps every net's inhibitory bits word-aligned
+        d.wide = dense && h.wide ? range : 0;
         desc.push_back(d);
         slots.push_back(sl);
         neurons += h.n;
         ptrs += h.n + 1;
-        words += sl.n_words;
-        syn += (h.s + 31) / 32 * 32;  // keeps every net's inhibitory bits word-aligned
+        words += sl.n_words + 1;  // a spare word: the fired bits of the rows' padding
+        syn += d.wide ? 2 * range : range;
         if (event_tables) ring += (int64_t)h.ring_slots * h.ring_words;
         tables += (int64_t)h.tables.size();
         tiles += sl.n_words;
-        spans += ((h.s + 31) / 32 + NC_SPAN_CHUNKS - 1) / NC_SPAN_CHUNKS;
         if (h.groups.size() > (size_t)ngroups_each) {
             err = "more input groups than reserved";
             return NC_ERR_INVALID;
@@ -186,19 +199,18 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     NC_ALLOC(P.slot_of, int32_t, neurons);
     NC_ALLOC(P.in_ptr, int64_t, ptrs);
     NC_ALLOC(P.w, float, syn);
-    NC_ALLOC(P.inh, uint32_t, (syn + 31) / 32 + 1);  // one spare word for 32-bit windows
-    NC_ALLOC(P.t_arr, int32_t, syn);
-    NC_ALLOC(P.term, double, syn);
+    NC_ALLOC(P.x, float, syn);
     if (dense) {
-        NC_ALLOC(P.csc_pre, int32_t, syn);
-        NC_ALLOC(P.csc_post, int32_t, syn);
-        NC_ALLOC(P.csc_dl, uint16_t, syn);
-        NC_ALLOC(P.la_c, int32_t, syn);
+        NC_ALLOC(P.key, uint32_t, syn);
+        NC_ALLOC(P.state, uint32_t, syn);
+        NC_ALLOC(P.qrow, uint8_t, syn / 4);
         NC_ALLOC(P.pst, float, neurons);
-        NC_ALLOC(P.win, uint32_t, syn / 32 + 1);
-        NC_ALLOC(P.spans, NcTile, spans);
+        NC_ALLOC(P.nib, uint8_t, syn / 4 + 8);  // read in 8-byte words
     }
+    L.neuron_block = dense ? NC_DENSE_BLOCK : 256;
     if (event_tables) {
+        NC_ALLOC(P.inh, uint32_t, (syn + 31) / 32 + 1);  // one spare word for 32-bit windows
+        NC_ALLOC(P.t_arr, int32_t, syn);
         NC_ALLOC(P.out_ptr, int64_t, ptrs);
         NC_ALLOC(P.ring_off, int32_t, ptrs);
         NC_ALLOC(P.out_post, int32_t, syn);
@@ -219,7 +231,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     NC_ALLOC(P.tables, float, tables);
     NC_ALLOC(P.groups, NcGroupDev, nets.size() * ngroups_each);
     NC_ALLOC(P.nets, NcNetDesc, nets.size());
-    NC_ALLOC(P.tiles, NcTile, tiles);
+    if (event_tables) NC_ALLOC(P.tiles, NcTile, tiles);
     NC_ALLOC(P.tick, int32_t, 1);
     NC_ALLOC(P.done_ctr, uint32_t, 1);
     NC_ALLOC(P.dev_err, uint32_t, 1);
@@ -227,11 +239,10 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     NC_ALLOC(d_stats_, unsigned long long, 4 * nets.size());
     P.n_nets = (int32_t)nets.size();
     P.n_tiles = (int32_t)tiles;
-    P.n_spans = dense ? (int32_t)spans : 0;
 
     // contents
-    std::vector<NcTile> tile_host, span_host;
-    tile_host.reserve((size_t)tiles);
+    std::vector<NcTile> tile_host;
+    std::vector<RowNet> row_nets;
     for (size_t q = 0; q < nets.size(); ++q) {
         const NetHost& h = *nets[q];
         const NetSlot& sl = slots[q];
@@ -247,41 +258,52 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         for (auto& v : inp) v += sl.syn_base;
         for (auto& v : outp) v += sl.syn_base;
         NC_CK(upload(P.in_ptr, inp, sl.ptr_base, stream));
-        if (dense && device_synapses) {
-            const int32_t chunks = (int32_t)((h.s + 31) / 32);
-            for (int32_t c = 0; c < chunks; c += NC_SPAN_CHUNKS) span_host.push_back(NcTile{(int32_t)q, c});
-        } else {
-        NC_CK(upload(P.w, h.w, sl.syn_base, stream));
-        NC_CK(upload(P.inh, h.inh_bits, sl.syn_base / 32, stream));
-        std::vector<int32_t> never((size_t)h.s, NC_NEVER);
-        NC_CK(upload(P.t_arr, never, sl.syn_base, stream));
-        if (dense) {
-            NC_CK(upload(P.csc_pre, h.csc_pre, sl.syn_base, stream));
-            NC_CK(upload(P.csc_post, h.csc_post, sl.syn_base, stream));
-            NC_CK(upload(P.csc_dl, h.csc_dl, sl.syn_base, stream));
-            NC_CK(upload(P.la_c, never, sl.syn_base, stream));
-            const int32_t chunks = (int32_t)((h.s + 31) / 32);
-            for (int32_t c = 0; c < chunks; c += NC_SPAN_CHUNKS) span_host.push_back(NcTile{(int32_t)q, c});
+        row_nets.push_back(RowNet{&h, (int32_t)q, sl.syn_base, sl.neuron_base, sl.ptr_base});
+        std::vector<int32_t> never;
+        if (dense && launch_fill_words(P.state + sl.syn_base, d.wide + h.sp, initial_state(h), stream)) {
+            err = cuda_msg("initial states", cudaGetLastError());
+            return NC_ERR_CUDA;
         }
-        if (event_tables) {
-            NC_CK(upload(P.out_ptr, outp, sl.ptr_base, stream));
-            NC_CK(upload(P.ring_off, h.ring_off, sl.ptr_base, stream));
-            NC_CK(upload(P.last_arr, never, sl.syn_base, stream));
-            NC_CK(upload(P.out_post, h.out_post, sl.syn_base, stream));
-            NC_CK(upload(P.out_csc, h.out_csc, sl.syn_base, stream));
-            NC_CK(upload(P.out_delay, h.out_delay, sl.syn_base, stream));
-            NC_CK(upload(P.out_ringpos, h.out_ringpos, sl.syn_base, stream));
-        }
+        if (!device_synapses) {
+            NC_CK(upload(P.w, h.w, sl.syn_base, stream));
+            if (dense) {
+                for (int64_t part = 0; part < key_words(h); ++part)
+                    NC_CK(upload_part(P.key, h.key, sl.syn_base + part * d.wide, part * h.sp, h.sp, stream));
+                NC_CK(upload(P.qrow, h.qrow, sl.syn_base / 4, stream));
+            }
+            if (event_tables) {
+                never.assign((size_t)h.sp, NC_NEVER);
+                NC_CK(upload(P.inh, h.inh_bits, sl.syn_base / 32, stream));
+                NC_CK(upload(P.t_arr, never, sl.syn_base, stream));
+                NC_CK(upload(P.out_ptr, outp, sl.ptr_base, stream));
+                NC_CK(upload(P.ring_off, h.ring_off, sl.ptr_base, stream));
+                NC_CK(upload_part(P.last_arr, never, sl.syn_base, 0, h.s, stream));
+                NC_CK(upload(P.out_post, h.out_post, sl.syn_base, stream));
+                NC_CK(upload(P.out_csc, h.out_csc, sl.syn_base, stream));
+                NC_CK(upload(P.out_delay, h.out_delay, sl.syn_base, stream));
+                NC_CK(upload(P.out_ringpos, h.out_ringpos, sl.syn_base, stream));
+            }
         }
         NC_CK(upload(P.tables, h.tables, d.table_base, stream));
         if (!h.groups.empty()) NC_CK(upload(P.groups, h.groups, sl.group_base, stream));
-        for (int32_t f = 0; f < h.n; f += 32) tile_host.push_back(NcTile{(int32_t)q, f});
+        if (event_tables)
+            for (int32_t f = 0; f < h.n; f += 32) tile_host.push_back(NcTile{(int32_t)q, f});
         // the vectors above must stay alive until the copies finish
         NC_CK(cudaStreamSynchronize(stream));
     }
     NC_CK(upload(P.nets, desc, 0, stream));
     NC_CK(upload(P.tiles, tile_host, 0, stream));
-    if (dense) NC_CK(upload(P.spans, span_host, 0, stream));
+    if (dense) {
+        std::vector<NcRowTile> rows;
+        std::vector<int32_t> start;
+        P.row_blocks = dense_blocks(neurons, L.neuron_block);
+        plan_rows(row_nets, P.row_blocks, rows, start);
+        NC_ALLOC(P.rtiles, NcRowTile, rows.size());
+        NC_ALLOC(P.rstart, int32_t, start.size());
+        NC_CK(upload(P.rtiles, rows, 0, stream));
+        NC_CK(upload(P.rstart, start, 0, stream));
+        NC_CK(cudaStreamSynchronize(stream));
+    }
     NC_CK(cudaStreamSynchronize(stream));
     for (size_t q = 0; q < nets.size(); ++q) {
         if (launch_background_prologue(P, (int)q, nets[q]->n, stream) != 0) {
@@ -303,7 +325,6 @@ int Engine::capture_graph(std::string& err)
 {
     release_graph();
     cudaGraph_t g = nullptr;
-    if (dense) prepare_dense_launch();
     NC_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
     for (int k = 0; k < graph_ticks && rc == 0; ++k) rc |= launch_tick(stream);
@@ -330,7 +351,7 @@ int Engine::step(int64_t ticks, std::string& err)
         // several whole steps per cooperative launch
         while (ticks > 0) {
             const int32_t m = (int32_t)std::min<int64_t>(ticks, L.fused_ticks);
-            if (launch_fused_dense(P, m, d_bar_, stream)) {
+            if (launch_fused_dense(P, m, L, d_bar_, stream)) {
                 err = cuda_msg("fused step launch", cudaGetLastError());
                 return NC_ERR_CUDA;
             }
@@ -428,31 +449,36 @@ int Engine::step_timed(int64_t ticks, float* ms, std::string& err)
 
 int Engine::time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::string& err)
 {
-    std::vector<cudaEvent_t> ev(3 * (size_t)std::max(ticks, 0));
+    // the dense form's step is one kernel: its time, and 0
+    const int marks = dense ? 2 : 3;
+    std::vector<cudaEvent_t> ev((size_t)marks * (size_t)std::max(ticks, 0));
     for (auto& e : ev) NC_CK(cudaEventCreate(&e));
     for (int k = 0; k < ticks; ++k) {
+        cudaEvent_t* at = &ev[(size_t)(marks * k)];
         if (P.n_firers > 0 && launch_input_firers(P, stream)) {
             err = "launch";
             return NC_ERR_CUDA;
         }
-        NC_CK(cudaEventRecord(ev[3 * k], stream));
-        if (dense ? launch_dense_synapses(P, L, stream) : launch_neuron_step(P, L, stream)) {
+        NC_CK(cudaEventRecord(at[0], stream));
+        if (dense ? launch_step_dense(P, L, stream) : launch_neuron_step(P, L, stream)) {
             err = "launch";
             return NC_ERR_CUDA;
         }
-        NC_CK(cudaEventRecord(ev[3 * k + 1], stream));
-        if (dense ? launch_dense_neurons(P, L, stream) : launch_spike_launch(P, L, stream)) {
+        NC_CK(cudaEventRecord(at[1], stream));
+        if (dense) continue;
+        if (launch_spike_launch(P, L, stream)) {
             err = "launch";
             return NC_ERR_CUDA;
         }
-        NC_CK(cudaEventRecord(ev[3 * k + 2], stream));
+        NC_CK(cudaEventRecord(at[2], stream));
     }
     NC_CK(cudaStreamSynchronize(stream));
     double sa = 0, sb = 0;
     for (int k = 0; k < ticks; ++k) {
+        const cudaEvent_t* at = &ev[(size_t)(marks * k)];
         float x = 0, y = 0;
-        NC_CK(cudaEventElapsedTime(&x, ev[3 * k], ev[3 * k + 1]));
-        NC_CK(cudaEventElapsedTime(&y, ev[3 * k + 1], ev[3 * k + 2]));
+        NC_CK(cudaEventElapsedTime(&x, at[0], at[1]));
+        if (!dense) NC_CK(cudaEventElapsedTime(&y, at[1], at[2]));
         sa += x;
         sb += y;
     }
@@ -488,7 +514,6 @@ int Engine::set_form(bool to_dense, std::string& err)
     }
     release_graph();
     dense = to_dense;
-    if (dense) prepare_dense_launch();
     return sync(err);
 }
 

@@ -40,7 +40,7 @@ public:
     int step_timed(int64_t ticks, float* ms, std::string& err);
     // Mean device time of one neuron-update and one spike-launch launch over `ticks`
     // individually timed ticks (these ticks also advance the nets).
-    // (dense form: the synapse pass and the neuron pass)
+    // (dense form: the step kernel, and 0)
     int time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::string& err);
     int flush_plasticity(std::string& err);
     int sync(std::string& err);
@@ -92,6 +92,9 @@ private:
     int64_t ring_words_total_ = 0;
 };
 
+// Blocks of `threads` threads that the rows of `neurons` neurons are shared out to: one wave,
+// or a block for each 8 neurons.
+int dense_blocks(int64_t neurons, int threads);
 std::string cuda_msg(const char* what, cudaError_t e);
 // Records the calling thread's last error (nc_last_error) and returns `code`.
 int set_last_error(int code, const std::string& msg);

@@ -119,10 +119,13 @@ constexpr int kGroupsPerNet = 16;
 constexpr int64_t kBuiltHostCap = 8ll << 30;
 // host bytes of a prepared request's tables (CSC, CSR, weights, maps)
 int64_t host_bytes(const nc::NetHost& h) { return h.s * 64 + (int64_t)h.n * 64; }
-// per synapse: w t_arr term inh | out_* last_arr (event form) or csc_pre csc_dl la_c (dense)
-constexpr double kSynBytesEvent = 4 + 4 + 8 + 4 + 4 + 2 + 4 + 4 + 0.125;
-constexpr double kSynBytesDense = 4 + 4 + 8 + 4 + 4 + 2 + 4 + 0.125 + 0.125;  // + csc_post, window bit
-constexpr double kNeuronBytes = 4 * 6 + 16 + 20 + 0.5 + 0.25;         // state, fired list, pointers, bitsets, tiles
+// per in-synapse position: w x | t_arr inh out_* last_arr (event form) or key state and a
+// quad's row and window bytes (dense)
+constexpr double kSynBytesEvent = 4 + 4 + 4 + 0.125 + 4 + 4 + 2 + 4 + 4;
+constexpr double kSynBytesDense = 4 + 4 + 4 + 4 + 0.5;
+// state, row starts, bitsets, tiles | fired list, out-row and ring starts (event form)
+constexpr double kNeuronBytesDense = 4 * 7 + 8 + 0.75 + 1;
+constexpr double kNeuronBytesEvent = 4 * 6 + 8 + 0.75 + 0.25 + 16 + 12;
 
 }  // namespace
 
@@ -133,15 +136,13 @@ struct nc_server {
     NcPools P{};
     nc::LaunchShape L{};
     std::vector<void*> allocs;
-    int64_t syn_cap = 0, neuron_cap = 0, ptr_cap = 0, word_cap = 0, ring_cap = 0, table_cap = 0, tile_cap = 0;
+    int64_t syn_cap = 0, neuron_cap = 0, ptr_cap = 0, word_cap = 0, ring_cap = 0, table_cap = 0, tile_cap = 0, rtile_cap = 0;
     bool dense = true;
-    double syn_bytes = kSynBytesDense;
+    double syn_bytes = kSynBytesDense, neuron_bytes = kNeuronBytesDense;
     RangeAlloc a_neuron, a_ptr, a_word, a_syn, a_ring, a_table;
     std::vector<int32_t> free_slots;
     unsigned long long* d_stats = nullptr;
     int32_t* d_ntiles = nullptr;
-    int32_t* d_nspans = nullptr;
-    int64_t span_cap = 0;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -208,22 +209,24 @@ int nc_server::init(std::string& err)
     int sms = 0;
     S_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     // pool capacities carved from the budget: the trace/AP tables first (~600 floats per
-    // network at dt = 1 ms), then ~80% (event form) or ~87% (dense form, which keeps no
-    // ring buffers) of the rest for synapse arrays, then neurons (fan-out of at least 16
-    // assumed) and the event form's ring buffers
+    // network at dt = 1 ms), then ~80% (event form) or ~94% (dense form, which keeps no
+    // ring buffers) of the rest for synapse arrays, then neurons (an average fan-out of at
+    // least 16, or 32 in the denser arrays of the dense form) and the event form's ring
+    // buffers
     const double budget = (double)cfg.memory_budget_bytes;
     dense = cfg.step_mode == NC_STEP_DENSE;
     syn_bytes = dense ? kSynBytesDense : kSynBytesEvent;
+    neuron_bytes = dense ? kNeuronBytesDense : kNeuronBytesEvent;
     const int32_t nets = cfg.max_networks;
     table_cap = (int64_t)nets * 8192 + 65536;
     const double avail = budget - 4.0 * (double)table_cap;
-    syn_cap = avail > 0 ? (int64_t)((dense ? 0.87 : 0.80) * avail / syn_bytes) / 32 * 32 : 0;
-    neuron_cap = std::max<int64_t>(1024, syn_cap / 16);
+    syn_cap = avail > 0 ? (int64_t)((dense ? 0.94 : 0.80) * avail / syn_bytes) / 32 * 32 : 0;
+    neuron_cap = std::max<int64_t>(1024, syn_cap / (dense ? 32 : 16));
     ptr_cap = neuron_cap + nets;
-    word_cap = neuron_cap / 32 + nets;
-    tile_cap = word_cap;
+    word_cap = neuron_cap / 32 + 2 * nets;  // and a spare word each: the rows' padding
+    tile_cap = neuron_cap / 32 + nets;
     ring_cap = dense ? 0 : (int64_t)(0.07 * budget / 4.0);
-    const double used = syn_cap * syn_bytes + neuron_cap * kNeuronBytes + ring_cap * 4.0 + table_cap * 4.0;
+    const double used = syn_cap * syn_bytes + neuron_cap * neuron_bytes + ring_cap * 4.0 + table_cap * 4.0;
     if (syn_cap < 32 || used > 1.05 * budget) {
         err = "memory budget too small";
         return NC_ERR_BUDGET;
@@ -239,20 +242,22 @@ int nc_server::init(std::string& err)
     S_AL(P.slot_of, int32_t, neuron_cap);
     S_AL(P.in_ptr, int64_t, ptr_cap);
     S_AL(P.w, float, syn_cap);
-    S_AL(P.inh, uint32_t, syn_cap / 32 + 1);
-    S_AL(P.t_arr, int32_t, syn_cap);
-    S_AL(P.term, double, syn_cap);
+    S_AL(P.x, float, syn_cap);
     if (dense) {
-        span_cap = syn_cap / (32 * NC_SPAN_CHUNKS) + nets;
-        S_AL(P.csc_pre, int32_t, syn_cap);
-        S_AL(P.csc_post, int32_t, syn_cap);
-        S_AL(P.csc_dl, uint16_t, syn_cap);
-        S_AL(P.la_c, int32_t, syn_cap);
+        S_AL(P.key, uint32_t, syn_cap);
+        S_AL(P.state, uint32_t, syn_cap);
+        S_AL(P.qrow, uint8_t, syn_cap / 4);
         S_AL(P.pst, float, neuron_cap);
-        S_AL(P.win, uint32_t, syn_cap / 32 + 1);
-        S_AL(P.spans, NcTile, span_cap);
-        S_AL(d_nspans, int32_t, 1);
+        S_AL(P.nib, uint8_t, syn_cap / 4 + 8);
+        // every block may cut a tile short, and every network's last one is
+        L.neuron_block = NC_DENSE_BLOCK;
+        P.row_blocks = nc::dense_blocks(neuron_cap, L.neuron_block);
+        rtile_cap = tile_cap + P.row_blocks;
+        S_AL(P.rtiles, NcRowTile, rtile_cap);
+        S_AL(P.rstart, int32_t, P.row_blocks + 1);
     } else {
+        S_AL(P.inh, uint32_t, syn_cap / 32 + 1);
+        S_AL(P.t_arr, int32_t, syn_cap);
         S_AL(P.out_ptr, int64_t, ptr_cap);
         S_AL(P.ring_off, int32_t, ptr_cap);
         S_AL(P.out_post, int32_t, syn_cap);
@@ -272,7 +277,7 @@ int nc_server::init(std::string& err)
     S_AL(P.tables, float, table_cap);
     S_AL(P.groups, NcGroupDev, (int64_t)nets * kGroupsPerNet);
     S_AL(P.nets, NcNetDesc, nets);
-    S_AL(P.tiles, NcTile, tile_cap);
+    if (!dense) S_AL(P.tiles, NcTile, tile_cap);
     S_AL(P.tick, int32_t, 1);
     S_AL(P.done_ctr, uint32_t, 1);
     S_AL(P.dev_err, uint32_t, 1);
@@ -282,8 +287,6 @@ int nc_server::init(std::string& err)
     P.n_nets = nets;
     P.n_tiles = 0;
     P.n_tiles_dev = d_ntiles;
-    P.n_spans = 0;
-    P.n_spans_dev = d_nspans;
     a_neuron.reset(neuron_cap);
     a_ptr.reset(ptr_cap);
     a_word.reset(word_cap);
@@ -291,38 +294,26 @@ int nc_server::init(std::string& err)
     a_ring.reset(ring_cap);
     a_table.reset(table_cap);
     for (int32_t q = nets - 1; q >= 0; --q) free_slots.push_back(q);
-    L.neuron_block = dense ? NC_DNEURON_BLOCK : 256;
+    if (!dense) L.neuron_block = 256;
     L.launch_block = 256;
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_MIN_BLOCKS);
-    L.dense_blocks = 0;  // the synapse pass's persistent grid (its warps stride the span table)
     S_CK(cudaStreamSynchronize(stream));
     return capture(err);
 }
 
 int nc_server::capture(std::string& err)
 {
-    // the neuron update strides over the tile table, so its grid need not follow it
+    // the event form's kernels stride over the tile table, whose live length they read from
+    // the device, and the dense step's blocks find their tiles there: the grids need not
+    // follow the resident networks
     NcPools G = P;
-    G.n_tiles = (int32_t)std::min<int64_t>(tile_cap, 1 << 30);
-    // likewise the synapse pass strides over the span table (its kernels read the live
-    // counts from the device): grids are sized from the capacities
-    G.n_spans = (int32_t)std::min<int64_t>(span_cap, 1 << 30);
-    nc::LaunchShape shape = L;
+    G.n_tiles = (int32_t)std::min<int64_t>(tile_cap, 152 * 16 * (L.neuron_block / 32));
     cudaGraph_t g = nullptr;
-    if (dense) nc::prepare_dense_launch();
     S_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
-    const int nb_tiles = 152 * 16 * (shape.neuron_block / 32);  // grid of the captured neuron update
-    NcPools Gg = G;
-    Gg.n_tiles = (int32_t)std::min<int64_t>(G.n_tiles, nb_tiles);
     for (int k = 0; k < cfg.steps_per_batch && rc == 0; ++k) {
-        if (dense) {
-            rc |= nc::launch_dense_synapses(G, shape, stream);
-            rc |= nc::launch_dense_neurons(Gg, shape, stream);
-        } else {
-            rc |= nc::launch_neuron_step(Gg, shape, stream);
-            rc |= nc::launch_spike_launch(G, shape, stream);
-        }
+        if (dense) rc |= nc::launch_step_dense(G, L, stream);
+        else rc |= nc::launch_neuron_step(G, L, stream) | nc::launch_spike_launch(G, L, stream);
     }
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     if (rc != 0 || e != cudaSuccess) {
@@ -387,6 +378,10 @@ void nc_server::builder_loop()
             if (rc != NC_OK) err = "bad kNN request";
             sp.n_synapses = (int64_t)m;
         }
+        // laid out for the server's form, whichever the request names
+        if (sp.params.step_mode == NC_STEP_DENSE || sp.params.step_mode == NC_STEP_EVENT ||
+            sp.params.step_mode == NC_STEP_AUTO)
+            sp.params.step_mode = cfg.step_mode;
         if (rc == NC_OK)
             rc = nc::build_net(sp.n_neurons, rq->xyz.empty() ? nullptr : rq->xyz.data(), sp.n_synapses,
                                rq->from.data(), rq->to.data(), rq->weight.data(),
@@ -405,15 +400,15 @@ void nc_server::builder_loop()
         }
         if (rc == NC_OK) {
             const nc::NetHost& h = r->host;
-            r->syn_len = (h.s + 31) / 32 * 32;
+            r->syn_len = (h.sp + 31) / 32 * 32 * (dense ? nc::key_words(h) : 1);
             r->ring_len = dense ? 0 : (int64_t)h.ring_slots * h.ring_words;
             r->table_len = (int64_t)h.tables.size();
-            r->words = (h.n + 31) / 32;
+            r->words = (h.n + 31) / 32 + 1;
             if (h.n > neuron_cap || r->syn_len > syn_cap || r->ring_len > ring_cap || r->table_len > table_cap) {
                 rc = NC_ERR_BUDGET;
                 err = "network larger than the server's memory budget";
             }
-            r->bytes = (int64_t)(r->syn_len * syn_bytes + h.n * kNeuronBytes + r->ring_len * 4.0 + r->table_len * 4.0);
+            r->bytes = (int64_t)(r->syn_len * syn_bytes + h.n * neuron_bytes + r->ring_len * 4.0 + r->table_len * 4.0);
         }
         r->status = rc;
         r->err = err;
@@ -457,7 +452,8 @@ int nc_server::admit(Resident& r, std::string& err)
     r.table0 = tb;
     // upload: the same per-network layout as the static engine, state reset
     std::vector<float> pot((size_t)h.n, -70.0f);
-    std::vector<int32_t> never_n((size_t)h.n, NC_NEVER), never_s((size_t)h.s, NC_NEVER);
+    std::vector<int32_t> never_n((size_t)h.n, NC_NEVER), never_s(dense ? 0 : (size_t)h.sp, NC_NEVER);
+    const int64_t wide = dense && h.wide ? r.syn_len / 2 : 0;
     std::vector<int64_t> inp(h.in_ptr), outp(h.out_ptr);
     for (auto& v : inp) v += sb;
     for (auto& v : outp) v += sb;
@@ -469,15 +465,21 @@ int nc_server::admit(Resident& r, std::string& err)
     S_CK(put(P.slot_of, h.slot_of, nb, stream));
     S_CK(put(P.in_ptr, inp, pb, stream));
     S_CK(put(P.w, h.w, sb, stream));
-    S_CK(put(P.inh, h.inh_bits, sb / 32, stream));
-    S_CK(put(P.t_arr, never_s, sb, stream));
     if (dense) {
-        S_CK(put(P.csc_pre, h.csc_pre, sb, stream));
-        S_CK(put(P.csc_post, h.csc_post, sb, stream));
-        S_CK(put(P.csc_dl, h.csc_dl, sb, stream));
-        S_CK(put(P.la_c, never_s, sb, stream));
-        S_CK(cudaMemsetAsync(P.win + sb / 32, 0, sizeof(uint32_t) * (r.syn_len / 32), stream));
+        for (int64_t part = 0; part < nc::key_words(h); ++part) {
+            const size_t bytes = sizeof(uint32_t) * (size_t)h.sp;
+            const int64_t at = sb + part * wide, from = part * h.sp;
+            if (!bytes) break;
+            S_CK(cudaMemcpyAsync(P.key + at, h.key.data() + from, bytes, cudaMemcpyHostToDevice, stream));
+        }
+        if (nc::launch_fill_words(P.state + sb, wide + h.sp, nc::initial_state(h), stream)) {
+            err = nc::cuda_msg("initial states", cudaGetLastError());
+            return NC_ERR_CUDA;
+        }
+        S_CK(put(P.qrow, h.qrow, sb / 4, stream));
     } else {
+        S_CK(put(P.inh, h.inh_bits, sb / 32, stream));
+        S_CK(put(P.t_arr, never_s, sb, stream));
         S_CK(put(P.out_ptr, outp, pb, stream));
         S_CK(put(P.ring_off, h.ring_off, pb, stream));
         S_CK(put(P.last_arr, never_s, sb, stream));
@@ -504,7 +506,7 @@ int nc_server::admit(Resident& r, std::string& err)
     d.neuron_base = (int32_t)nb;
     d.ptr_base = (int32_t)pb;
     d.word_base = (int32_t)wb;
-    d.n_words = (int32_t)r.words;
+    d.n_words = (h.n + 31) / 32;
     d.syn_base = sb;
     d.ring_base = rb;
     d.ring_words = h.ring_words;
@@ -530,7 +532,10 @@ int nc_server::admit(Resident& r, std::string& err)
     d.pre_factor = h.p.presynaptic_factor;
     d.post_factor = h.p.postsynaptic_factor;
     d.e_term = h.e_term;
+    nc::term_pair(h, d.term_hi, d.term_lo);
     d.n_syn = h.s;
+    d.key_shift = h.key_shift;
+    d.wide = wide;
     d.stats = d_stats + 4 * (int64_t)r.slot;
     S_CK(cudaMemcpyAsync(P.nets + r.slot, &d, sizeof(d), cudaMemcpyHostToDevice, stream));
     if (nc::launch_background_prologue(P, r.slot, h.n, stream)) {
@@ -560,6 +565,22 @@ int nc_server::retire(Resident& r, std::string& err)
 
 int nc_server::upload_tiles(std::string& err)
 {
+    if (dense) {
+        std::vector<nc::RowNet> nets;
+        std::vector<NcRowTile> rows;
+        std::vector<int32_t> start;
+        for (const auto& r : active)
+            nets.push_back(nc::RowNet{&r->host, r->slot, r->syn0, (int32_t)r->neuron0, (int32_t)r->ptr0});
+        nc::plan_rows(nets, P.row_blocks, rows, start);
+        if ((int64_t)rows.size() > rtile_cap) {
+            err = "tile table overflow";
+            return NC_ERR_INVALID;
+        }
+        S_CK(put(P.rtiles, rows, 0, stream));
+        S_CK(put(P.rstart, start, 0, stream));
+        S_CK(cudaStreamSynchronize(stream));
+        return NC_OK;
+    }
     std::vector<NcTile> tiles;
     for (const auto& r : active)
         for (int32_t f = 0; f < r->host.n; f += 32) tiles.push_back(NcTile{r->slot, f});
@@ -568,24 +589,8 @@ int nc_server::upload_tiles(std::string& err)
         return NC_ERR_INVALID;
     }
     const int32_t n = (int32_t)tiles.size();
-    if (n) S_CK(cudaMemcpyAsync(P.tiles, tiles.data(), tiles.size() * sizeof(NcTile), cudaMemcpyHostToDevice, stream));
+    S_CK(put(P.tiles, tiles, 0, stream));
     S_CK(cudaMemcpyAsync(d_ntiles, &n, sizeof(n), cudaMemcpyHostToDevice, stream));
-    std::vector<NcTile> spans;
-    if (dense) {
-        for (const auto& r : active) {
-            const int32_t chunks = (int32_t)((r->host.s + 31) / 32);
-            for (int32_t c = 0; c < chunks; c += NC_SPAN_CHUNKS) spans.push_back(NcTile{r->slot, c});
-        }
-        if ((int64_t)spans.size() > span_cap) {
-            err = "span table overflow";
-            return NC_ERR_INVALID;
-        }
-        const int32_t ns = (int32_t)spans.size();
-        if (ns)
-            S_CK(cudaMemcpyAsync(P.spans, spans.data(), spans.size() * sizeof(NcTile), cudaMemcpyHostToDevice, stream));
-        S_CK(cudaMemcpyAsync(d_nspans, &ns, sizeof(ns), cudaMemcpyHostToDevice, stream));
-        P.n_spans = ns;
-    }
     S_CK(cudaStreamSynchronize(stream));
     P.n_tiles = n;
     return NC_OK;
@@ -674,7 +679,6 @@ void nc_server::scheduler_loop()
         if (!done.empty()) {
             NcPools F = P;  // flush launched directly with the current tile count
             F.n_tiles_dev = nullptr;
-            F.n_spans_dev = nullptr;
             if (dense ? nc::launch_flush_dense(F, L, stream) : nc::launch_stdp_flush(F, L, stream)) return;
             cudaStreamSynchronize(stream);
         }
@@ -693,8 +697,8 @@ void nc_server::scheduler_loop()
             Kept k;
             if (cfg.keep_results) {
                 const nc::NetHost& h = r->host;
-                std::vector<float> w((size_t)h.s), pot((size_t)h.n);
-                cudaMemcpyAsync(w.data(), P.w + r->syn0, sizeof(float) * h.s, cudaMemcpyDeviceToHost, stream);
+                std::vector<float> w((size_t)h.sp), pot((size_t)h.n);
+                cudaMemcpyAsync(w.data(), P.w + r->syn0, sizeof(float) * h.sp, cudaMemcpyDeviceToHost, stream);
                 cudaMemcpyAsync(pot.data(), P.pot + r->neuron0, sizeof(float) * h.n, cudaMemcpyDeviceToHost, stream);
                 cudaStreamSynchronize(stream);
                 k.weights.resize((size_t)h.n_input);
