@@ -199,15 +199,16 @@ int nc_create_knn(int32_t n, int32_t k, float density, uint64_t seed, const nc_p
 // position, delays, inhibitory bits, out-synapse tables), fetched on first use.
 static int ensure_host_tables(nc_net* net)
 {
-    if (!net->dev_i2c) return NC_OK;
+    if (!net->dev_to) return NC_OK;
     nc::NetHost& h = net->host;
     const int64_t S = h.s;
     const int32_t k = net->knn_k;
     const auto& P = net->eng.P;
-    std::vector<int64_t> i2c((size_t)S);
+    std::vector<uint32_t> index((size_t)S);
     std::vector<int32_t> to((size_t)S);
     std::vector<uint32_t> key((size_t)h.sp);
-    NC_CALL(net->eng, download, i2c.data(), (const int64_t*)net->dev_i2c, (size_t)S);
+    NC_CALL(net->eng, download, index.data(), (const uint32_t*)net->dev_i2c, (size_t)S);
+    std::vector<int64_t> i2c(index.begin(), index.end());
     NC_CALL(net->eng, download, to.data(), (const int32_t*)net->dev_to, (size_t)S);
     // the words with the delays: the second range of a wide net
     const int64_t wide = h.wide ? (h.sp + 31) / 32 * 32 : 0;
@@ -234,9 +235,7 @@ static int ensure_host_tables(nc_net* net)
         }
     }
     h.input_to_csc = std::move(i2c);
-    cudaFree(net->dev_i2c);
     cudaFree(net->dev_to);
-    net->dev_i2c = nullptr;
     net->dev_to = nullptr;
     return NC_OK;
 }
@@ -550,18 +549,12 @@ int nc_record_raster(nc_net* net, int32_t max_steps)
     if (net->d_raster && max_steps != net->raster_cap) {
         cudaFree(net->d_raster);
         net->d_raster = nullptr;
-        if (net->d_raster_ids) cudaFree(net->d_raster_ids);
-        net->d_raster_ids = nullptr;
         net->raster_cap = 0;
     }
     if (max_steps > 0 && !net->d_raster) {
         const size_t words = (size_t)max_steps * net->eng.slots[0].n_words;
         cudaError_t e = cudaMalloc(&net->d_raster, std::max<size_t>(words, 1) * sizeof(uint32_t));
         if (e != cudaSuccess) return fail(NC_ERR_NOMEM, nc::cuda_msg("cudaMalloc raster", e));
-        if (net->host.permuted) {
-            e = cudaMalloc(&net->d_raster_ids, std::max<size_t>(words, 1) * sizeof(uint32_t));
-            if (e != cudaSuccess) return fail(NC_ERR_NOMEM, nc::cuda_msg("cudaMalloc raster", e));
-        }
         e = cudaMemset(net->d_raster, 0, std::max<size_t>(words, 1) * sizeof(uint32_t));
         if (e != cudaSuccess) return fail(NC_ERR_CUDA, nc::cuda_msg("cudaMemset raster", e));
         net->raster_cap = max_steps;
@@ -576,24 +569,11 @@ int nc_read_raster(nc_net* net, uint8_t* out, int64_t capacity_bytes, int32_t* s
     if (!steps) return fail(NC_ERR_INVALID, "null steps");
     const int64_t done = net->step - net->raster_t0 + 1;
     const int32_t rows = (int32_t)std::max<int64_t>(0, std::min<int64_t>(done, net->raster_cap));
-    const int32_t nw = net->eng.slots[0].n_words;
     const int64_t row_bytes = ((int64_t)net->host.n + 7) / 8;
     *steps = rows;
     if (!out) return NC_OK;
     if (capacity_bytes < rows * row_bytes) return fail(NC_ERR_INVALID, "raster buffer too small");
-    const nc::NetHost& h = net->host;
-    const uint32_t* src = net->d_raster;
-    if (h.permuted && rows > 0) {
-        const auto& sl = net->eng.slots[0];
-        if (nc::launch_raster_to_ids(net->d_raster, net->d_raster_ids, net->eng.P.slot_of + sl.neuron_base, h.n, nw,
-                                     rows, net->eng.stream))
-            return fail(NC_ERR_CUDA, nc::cuda_msg("raster reorder", cudaGetLastError()));
-        src = net->d_raster_ids;
-    }
-    std::vector<uint32_t> buf((size_t)rows * nw);
-    NC_CALL(net->eng, download, buf.data(), src, buf.size());
-    for (int32_t r = 0; r < rows; ++r)
-        std::memcpy(out + (int64_t)r * row_bytes, buf.data() + (size_t)r * nw, (size_t)row_bytes);
+    NC_CALL(net->eng, read_raster, 0, (const uint32_t*)net->d_raster, rows, out);
     return NC_OK;
 }
 
@@ -601,44 +581,15 @@ int nc_read_potentials(nc_net* net, float* out_n)
 {
     NC_NEED(net);
     if (!out_n && net->host.n) return fail(NC_ERR_INVALID, "null output");
-    const auto& sl = net->eng.slots[0];
-    std::vector<float> pot((size_t)sl.n);
-    NC_CALL(net->eng, download, pot.data(), (const float*)net->eng.P.pot + sl.neuron_base, (size_t)sl.n);
-    nc::to_caller_order(net->host, pot.data(), out_n);
+    NC_CALL(net->eng, read_potentials, 0, out_n);
     return NC_OK;
 }
 
 int nc_read_potact(nc_net* net, float* out_2n)
 {
     NC_NEED_COUNTERS(net);
-    const int32_t n = net->host.n;
-    if (!out_2n && n) return fail(NC_ERR_INVALID, "null output");
-    std::vector<float> pot((size_t)n);
-    std::vector<uint32_t> fir((size_t)n);
-    std::vector<int32_t> start((size_t)n);
-    const auto& sl = net->eng.slots[0];
-    NC_CALL(net->eng, download, pot.data(), (const float*)net->eng.P.pot + sl.neuron_base, (size_t)n);
-    NC_CALL(net->eng, download, fir.data(), (const uint32_t*)net->eng.P.firings + sl.neuron_base, (size_t)n);
-    NC_CALL(net->eng, download, start.data(), (const int32_t*)net->eng.P.act_start + sl.neuron_base, (size_t)n);
-    const float dt = net->host.dt;
-    const int64_t t = net->step;
-    std::vector<float> pot_c((size_t)n);
-    std::vector<uint32_t> fir_c((size_t)n);
-    std::vector<int32_t> start_c((size_t)n);
-    nc::to_caller_order(net->host, pot.data(), pot_c.data());
-    nc::to_caller_order(net->host, fir.data(), fir_c.data());
-    nc::to_caller_order(net->host, start.data(), start_c.data());
-    pot.swap(pot_c);
-    fir.swap(fir_c);
-    start.swap(start_c);
-    for (int32_t j = 0; j < n; ++j) {
-        out_2n[2 * (size_t)j] = pot[j];
-        // setActivity(firings/(((float) currentT-activityStartTime)/10.0)) at the last update
-        float act = 0.0f;
-        if (t >= 1 && t > start[j])
-            act = (float)(fir[j] / (((float)nc::step_ms(t, dt) - nc::step_ms(start[j], dt)) / 10.0));
-        out_2n[2 * (size_t)j + 1] = act;
-    }
+    if (!out_2n && net->host.n) return fail(NC_ERR_INVALID, "null output");
+    NC_CALL(net->eng, read_potact, 0, net->step, out_2n);
     return NC_OK;
 }
 
@@ -654,20 +605,25 @@ int nc_read_last_fire(nc_net* net, float* out_n)
     NC_NEED(net);
     const int32_t n = net->host.n;
     if (!out_n && n) return fail(NC_ERR_INVALID, "null output");
-    std::vector<int32_t> lf_s((size_t)n), lf((size_t)n);
-    NC_CALL(net->eng, download, lf_s.data(), (const int32_t*)net->eng.P.lf + net->eng.slots[0].neuron_base, (size_t)n);
-    nc::to_caller_order(net->host, lf_s.data(), lf.data());
-    for (int32_t j = 0; j < n; ++j) out_n[j] = lf[j] == NC_NEVER ? NAN : nc::step_ms(lf[j], net->host.dt);
+    NC_CALL(net->eng, read_last_fire, 0, out_n);
     return NC_OK;
 }
 
 int nc_read_weights(nc_net* net, float* out_s)
 {
     NC_NEED(net);
-    if (int rc = ensure_host_tables(net)) return rc;
     const nc::NetHost& h = net->host;
     if (!out_s && h.n_input) return fail(NC_ERR_INVALID, "null output");
     NC_CALL0(net->eng, flush_plasticity);
+    if (!net->dev_i2c) net->dev_i2c = nc::upload_index(h.input_to_csc);
+    if (net->dev_i2c) {
+        std::string err;
+        const int rc = net->eng.read_weights(0, net->dev_i2c, h.n_input, out_s, err);
+        if (rc == NC_OK) return NC_OK;
+        if (rc != NC_ERR_NOMEM) return fail(rc, err);
+    }
+    // no device memory for the gather: reorder on the host
+    if (int rc = ensure_host_tables(net)) return rc;
     std::vector<float> w((size_t)h.sp);
     NC_CALL(net->eng, download, w.data(), (const float*)net->eng.P.w + net->eng.slots[0].syn_base, (size_t)h.sp);
     for (int64_t k = 0; k < h.n_input; ++k) {

@@ -18,7 +18,13 @@ struct nc_batch {
     std::vector<nc::NetHost> hosts;
     std::vector<int32_t> horizon;
     nc::Engine eng;
-    int64_t ticks = 0;  // launch pairs issued
+    int64_t ticks = 0;  // steps issued
+    std::vector<uint32_t*> index;  // per net, once its weights have been read (nc::upload_index)
+    ~nc_batch()
+    {
+        for (uint32_t* p : index)
+            if (p) cudaFree(p);
+    }
 };
 
 #define B_NEED(b)                                                    \
@@ -255,10 +261,7 @@ int nc_batch_read_potentials(nc_batch* b, int32_t net, float* out)
 {
     B_NEED(b);
     if (!out || net < 0 || net >= (int32_t)b->hosts.size()) return bfail(NC_ERR_INVALID, "bad net index");
-    const auto& sl = b->eng.slots[(size_t)net];
-    std::vector<float> pot((size_t)sl.n);
-    B_CALL(b->eng, download, pot.data(), (const float*)b->eng.P.pot + sl.neuron_base, (size_t)sl.n);
-    nc::to_caller_order(b->hosts[(size_t)net], pot.data(), out);
+    B_CALL(b->eng, read_potentials, net, out);
     return NC_OK;
 }
 
@@ -269,6 +272,16 @@ int nc_batch_read_weights(nc_batch* b, int32_t net, float* out)
     const nc::NetHost& h = b->hosts[(size_t)net];
     if (!out && h.n_input) return bfail(NC_ERR_INVALID, "null output");
     B_CALL0(b->eng, flush_plasticity);
+    if (b->index.empty()) b->index.resize(b->hosts.size(), nullptr);
+    uint32_t*& index = b->index[(size_t)net];
+    if (!index) index = nc::upload_index(h.input_to_csc);
+    if (index) {
+        std::string err;
+        const int rc = b->eng.read_weights(net, index, h.n_input, out, err);
+        if (rc == NC_OK) return NC_OK;
+        if (rc != NC_ERR_NOMEM) return bfail(rc, err);
+    }
+    // no device memory for the gather: reorder on the host
     const auto& sl = b->eng.slots[(size_t)net];
     std::vector<float> w((size_t)h.sp);
     B_CALL(b->eng, download, w.data(), (const float*)b->eng.P.w + sl.syn_base, (size_t)h.sp);
@@ -283,11 +296,7 @@ int nc_batch_read_last_fire(nc_batch* b, int32_t net, float* out)
 {
     B_NEED(b);
     if (!out || net < 0 || net >= (int32_t)b->hosts.size()) return bfail(NC_ERR_INVALID, "bad net index");
-    const auto& sl = b->eng.slots[(size_t)net];
-    std::vector<int32_t> lf_s((size_t)sl.n), lf((size_t)sl.n);
-    B_CALL(b->eng, download, lf_s.data(), (const int32_t*)b->eng.P.lf + sl.neuron_base, (size_t)sl.n);
-    nc::to_caller_order(b->hosts[(size_t)net], lf_s.data(), lf.data());
-    for (int32_t j = 0; j < sl.n; ++j) out[j] = lf[(size_t)j] == NC_NEVER ? NAN : nc::step_ms(lf[(size_t)j], sl.dt);
+    B_CALL(b->eng, read_last_fire, net, out);
     return NC_OK;
 }
 

@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t
                                                               int64_t wide, float dt, const float* xyz,
                                                               const int32_t* to, const float* weight,
                                                               const int32_t* slot_of, const unsigned long long* cursor,
-                                                              const unsigned long long* rows, int64_t* input_to_csc,
+                                                              const unsigned long long* rows, uint32_t* input_to_csc,
                                                               uint32_t* flags)
 {
     __shared__ unsigned long long sh[kRowWarps][kRowCap];
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t
             P.key[c] = (uint32_t)slot_of[from] << key_shift | (wide ? 0u : hi);
             if (wide) P.key[wide + c] = hi;
             P.w[c] = weight[e];
-            input_to_csc[e] = c;
+            input_to_csc[e] = (uint32_t)c;
         }
         __syncwarp();
     }
@@ -491,7 +491,7 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     if (rc != NC_OK) return rc;
     unsigned long long* d_cur = dalloc<unsigned long long>((size_t)n, own.v, e);
     unsigned long long* d_rows = dalloc<unsigned long long>((size_t)h.sp, own.v, e);
-    int64_t* d_i2c = dalloc<int64_t>((size_t)edges, own.v, e);
+    uint32_t* d_i2c = dalloc<uint32_t>((size_t)edges, own.v, e);
     if (e == cudaSuccess)
         e = cudaMemcpy(d_cur, h.in_ptr.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {

@@ -334,6 +334,11 @@ int launch_input_firers(const NcPools& P, void* stream);
 // Mean potential of each detector's near neurons (caller ids; near_ptr has count+1 entries).
 int launch_detector_voltages(const NcPools& P, int32_t neuron_base, const int32_t* near, const int32_t* near_ptr,
                              int32_t count, float* out, void* stream);
-int launch_raster_to_ids(const uint32_t* in, uint32_t* out, const int32_t* slot_of, int32_t n, int32_t n_words,
-                         int32_t rows, void* stream);
+// Read-backs in the caller's order, into device buffers (nc_read.cu): n neurons from
+// caller's id `first` on, rows of a raster.
+int launch_gather(const float* src, const uint32_t* index, int64_t count, float* out, void* stream);
+int launch_potact(const NcPools& P, int32_t neuron_base, int32_t first, int32_t n, int64_t t, float dt, float* out, void* stream);
+int launch_last_fire(const NcPools& P, int32_t neuron_base, int32_t first, int32_t n, float dt, float* out, void* stream);
+int launch_raster_bytes(const uint32_t* in, uint8_t* out, const int32_t* slot_of, int32_t n, int32_t n_words,
+                        int32_t rows, void* stream);
 }  // namespace nc

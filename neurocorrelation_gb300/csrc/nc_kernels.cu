@@ -524,38 +524,9 @@ __global__ void k_force_bits(NcPools P, int net, const int32_t* ids, int count)
     atomicOr(P.forced + (int64_t)(D.t & 1) * P.total_words + D.word_base + (j >> 5), 1u << (j & 31));
 }
 
-// Raster rows from device-slot order to caller-id order: thread per output word.
-__global__ void k_raster_to_ids(const uint32_t* in, uint32_t* out, const int32_t* slot_of, int32_t n, int32_t n_words,
-                                int32_t rows)
-{
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (int64_t)rows * n_words) return;
-    const int32_t r = (int32_t)(q / n_words), w = (int32_t)(q % n_words);
-    const uint32_t* row = in + (int64_t)r * n_words;
-    uint32_t v = 0;
-    for (int b = 0; b < 32; ++b) {
-        const int32_t i = w * 32 + b;
-        if (i >= n) break;
-        const int32_t s = __ldg(slot_of + i);
-        v |= ((__ldg(row + (s >> 5)) >> (s & 31)) & 1u) << b;
-    }
-    out[q] = v;
-}
-
 }  // namespace
 
 namespace nc {
-
-int launch_raster_to_ids(const uint32_t* in, uint32_t* out, const int32_t* slot_of, int32_t n, int32_t n_words,
-                         int32_t rows, void* stream)
-{
-    const int64_t total = (int64_t)rows * n_words;
-    if (total <= 0) return 0;
-    k_raster_to_ids<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(in, out, slot_of, n, n_words,
-                                                                                       rows);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
 
 static int check_launch()
 {

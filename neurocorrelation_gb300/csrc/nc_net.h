@@ -20,7 +20,6 @@ struct nc_net {
     uint64_t auto_fires = 0;
     int64_t auto_steps = 0;
     uint32_t* d_raster = nullptr;
-    uint32_t* d_raster_ids = nullptr;  // the same rows in caller-id order (read-back staging)
     int32_t raster_cap = 0;
     int32_t raster_t0 = 0;
     // periodic input firers (InputFirer): positions, radii and near lists (device slots)
@@ -30,17 +29,18 @@ struct nc_net {
     std::vector<int32_t> det_near, det_ptr{0};
     int32_t* d_det = nullptr;      // det_near then det_ptr on the device
     float* d_volt = nullptr;
-    // built on the device (nc_create_knn): targets in creation order and the CSC position
-    // of every synapse, kept there until a read-back needs the host tables
+    // CSC position of every input synapse on the device (~0: not kept): from nc_create_knn, or
+    // uploaded by the first weight read-back
+    uint32_t* dev_i2c = nullptr;
+    // built on the device (nc_create_knn): targets in creation order, kept until a read-back
+    // needs the host tables
     int32_t* dev_to = nullptr;
-    int64_t* dev_i2c = nullptr;
     int32_t knn_k = 0;
     ~nc_net()
     {
         if (dev_to) cudaFree(dev_to);
         if (dev_i2c) cudaFree(dev_i2c);
         if (d_raster) cudaFree(d_raster);
-        if (d_raster_ids) cudaFree(d_raster_ids);
         if (d_det) cudaFree(d_det);
         if (d_volt) cudaFree(d_volt);
     }

@@ -104,5 +104,6 @@ extern "C" int nc_run_noalloc(nc_net* net, int32_t n_steps, void* stream)
     // the launches above are not tracked by the handle once issued: later calls on the
     // handle read the step counter and simulated time back from the device
     net->counters_on_device = true;
+    net->eng.steps_unseen();
     return NC_OK;
 }

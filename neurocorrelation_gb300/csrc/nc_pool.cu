@@ -28,6 +28,7 @@ Engine::~Engine()
     if (stream) cudaStreamSynchronize(stream);
     if (firers_buf_) cudaFree(firers_buf_);
     if (near_buf_) cudaFree(near_buf_);
+    if (d_ids_) cudaFree(d_ids_);
     for (void* p : allocs_) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
 }
@@ -237,6 +238,10 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     NC_ALLOC(P.dev_err, uint32_t, 1);
     NC_ALLOC(d_bar_, unsigned, 2);
     NC_ALLOC(d_stats_, unsigned long long, 4 * nets.size());
+    for (const NetHost* h : nets)
+        scratch_bytes_ = std::max(scratch_bytes_, std::max(sizeof(float) * (size_t)h->n_input, 8 * (size_t)h->n));
+    scratch_bytes_ = std::max<size_t>(256, std::min(scratch_bytes_, kScratchMax));
+    NC_ALLOC(scratch_, char, scratch_bytes_);
     P.n_nets = (int32_t)nets.size();
     P.n_tiles = (int32_t)tiles;
 
@@ -347,6 +352,7 @@ int Engine::capture_graph(std::string& err)
 int Engine::step(int64_t ticks, std::string& err)
 {
     if (ticks <= 0) return NC_OK;
+    flushed_ = false;
     if (dense && L.fused_ticks > 0 && P.n_firers == 0) {
         // several whole steps per cooperative launch
         while (ticks > 0) {
@@ -450,6 +456,7 @@ int Engine::step_timed(int64_t ticks, float* ms, std::string& err)
 int Engine::time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::string& err)
 {
     // the dense form's step is one kernel: its time, and 0
+    flushed_ = false;
     const int marks = dense ? 2 : 3;
     std::vector<cudaEvent_t> ev((size_t)marks * (size_t)std::max(ticks, 0));
     for (auto& e : ev) NC_CK(cudaEventCreate(&e));
@@ -490,11 +497,97 @@ int Engine::time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::str
 
 int Engine::flush_plasticity(std::string& err)
 {
+    if (flushed_ && !unseen_) return NC_OK;
     if (dense ? launch_flush_dense(P, L, stream) : launch_stdp_flush(P, L, stream)) {
         err = cuda_msg("plasticity flush", cudaGetLastError());
         return NC_ERR_CUDA;
     }
+    flushed_ = true;
     return NC_OK;
+}
+
+// Runs `launch(first, count, buffer)` for `items` items of per_item bytes, as many at a time
+// as the buffer holds, and copies each part to out.
+template <class F>
+static int read_parts(int64_t items, size_t per_item, void* buf, size_t buf_bytes, void* out, cudaStream_t stream,
+                      F&& launch, std::string& err)
+{
+    const int64_t part = std::max<int64_t>(1, (int64_t)(buf_bytes / std::max<size_t>(per_item, 1)));
+    for (int64_t a = 0; a < items && per_item; a += part) {
+        const int64_t m = std::min(part, items - a);
+        if (launch(a, m, buf)) {
+            err = cuda_msg("read-back", cudaGetLastError());
+            return NC_ERR_CUDA;
+        }
+        NC_CK(cudaMemcpyAsync((char*)out + a * (int64_t)per_item, buf, (size_t)m * per_item, cudaMemcpyDeviceToHost,
+                              stream));
+    }
+    NC_CK(cudaStreamSynchronize(stream));
+    return NC_OK;
+}
+
+int Engine::read_potentials(int net, float* out, std::string& err)
+{
+    const NetSlot& sl = slots[(size_t)net];
+    // slot_of is a permutation of 0 .. n-1: an index of the same bits
+    return read_parts(sl.n, sizeof(float), scratch_, scratch_bytes_, out, stream,
+                      [&](int64_t a, int64_t m, void* buf) {
+                          return launch_gather(P.pot + sl.neuron_base,
+                                               (const uint32_t*)P.slot_of + sl.neuron_base + a, m, (float*)buf, stream);
+                      },
+                      err);
+}
+
+int Engine::read_potact(int net, int64_t t, float* out_2n, std::string& err)
+{
+    const NetSlot& sl = slots[(size_t)net];
+    return read_parts(sl.n, 2 * sizeof(float), scratch_, scratch_bytes_, out_2n, stream,
+                      [&](int64_t a, int64_t m, void* buf) {
+                          return launch_potact(P, sl.neuron_base, (int32_t)a, (int32_t)m, t, sl.dt, (float*)buf, stream);
+                      },
+                      err);
+}
+
+int Engine::read_last_fire(int net, float* out, std::string& err)
+{
+    const NetSlot& sl = slots[(size_t)net];
+    return read_parts(sl.n, sizeof(float), scratch_, scratch_bytes_, out, stream,
+                      [&](int64_t a, int64_t m, void* buf) {
+                          return launch_last_fire(P, sl.neuron_base, (int32_t)a, (int32_t)m, sl.dt, (float*)buf, stream);
+                      },
+                      err);
+}
+
+int Engine::read_weights(int net, const uint32_t* index, int64_t count, float* out, std::string& err)
+{
+    const float* w = P.w + slots[(size_t)net].syn_base;
+    return read_parts(count, sizeof(float), scratch_, scratch_bytes_, out, stream,
+                      [&](int64_t a, int64_t m, void* buf) { return launch_gather(w, index + a, m, (float*)buf, stream); },
+                      err);
+}
+
+int Engine::read_raster(int net, const uint32_t* d_raster, int32_t rows, uint8_t* out, std::string& err)
+{
+    const NetSlot& sl = slots[(size_t)net];
+    return read_parts(rows, ((size_t)sl.n + 7) / 8, scratch_, scratch_bytes_, out, stream,
+                      [&](int64_t a, int64_t m, void* buf) {
+                          return launch_raster_bytes(d_raster + a * sl.n_words, (uint8_t*)buf, P.slot_of + sl.neuron_base,
+                                                     sl.n, sl.n_words, (int32_t)m, stream);
+                      },
+                      err);
+}
+
+uint32_t* upload_index(const std::vector<int64_t>& input_to_csc)
+{
+    std::vector<uint32_t> index(input_to_csc.begin(), input_to_csc.end());  // -1 becomes ~0
+    void* d = nullptr;
+    if (cudaMalloc(&d, sizeof(uint32_t) * std::max<size_t>(index.size(), 1)) != cudaSuccess ||
+        cudaMemcpy(d, index.data(), sizeof(uint32_t) * index.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        if (d) cudaFree(d);
+        return nullptr;
+    }
+    return (uint32_t*)d;
 }
 
 int Engine::set_form(bool to_dense, std::string& err)

@@ -42,7 +42,18 @@ public:
     // individually timed ticks (these ticks also advance the nets).
     // (dense form: the step kernel, and 0)
     int time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::string& err);
+    // (nothing is launched when nothing has been stepped since the last one)
     int flush_plasticity(std::string& err);
+    // Steps are launched that this object does not see (nc_run_noalloc's may be replayed).
+    void steps_unseen() { unseen_ = true; }
+    // Read-backs of a net's neurons and weights in the caller's order (nc_read.cu): gathered
+    // into the engine's scratch a part at a time and copied to the host.
+    int read_potentials(int net, float* out, std::string& err);
+    int read_potact(int net, int64_t t, float* out_2n, std::string& err);
+    int read_last_fire(int net, float* out, std::string& err);
+    // index: device array, the CSC position of each synapse (~0: not kept)
+    int read_weights(int net, const uint32_t* index, int64_t count, float* out, std::string& err);
+    int read_raster(int net, const uint32_t* d_raster, int32_t rows, uint8_t* out, std::string& err);
     int sync(std::string& err);
 
     int set_groups(int net, const std::vector<NcGroupDev>& groups, std::string& err);
@@ -81,6 +92,12 @@ private:
     void release_graph();
     template <class T>
     T* alloc(size_t count, std::string& err);
+    // Read-back scratch on the device, allocated with the pools: a net's largest read-back,
+    // or kScratchMax of it at a time.
+    static constexpr size_t kScratchMax = 64 << 20;
+    void* scratch_ = nullptr;
+    size_t scratch_bytes_ = 0;
+    bool flushed_ = false, unseen_ = false;
     std::vector<void*> allocs_;
     cudaGraphExec_t graph_ = nullptr;
     void* firers_buf_ = nullptr;
@@ -95,6 +112,9 @@ private:
 // Blocks of `threads` threads that the rows of `neurons` neurons are shared out to: one wave,
 // or a block for each 8 neurons.
 int dense_blocks(int64_t neurons, int threads);
+// The CSC positions of a net's input synapses on the device (freed by the caller), or null
+// when there is no memory for them: the read-back then reorders on the host.
+uint32_t* upload_index(const std::vector<int64_t>& input_to_csc);
 std::string cuda_msg(const char* what, cudaError_t e);
 // Records the calling thread's last error (nc_last_error) and returns `code`.
 int set_last_error(int code, const std::string& msg);
