@@ -210,10 +210,11 @@ int nc_schedule_fire(nc_net* net, int32_t count, const int32_t* neuron_ids);
  * the event form when fewer than
  * NC_AUTO_TO_EVENT_PERMILLE per mille of its neurons fired per step in the window, and
  * back to the dense form above NC_AUTO_TO_DENSE_PERMILLE (the measured crossover of the
- * two forms on a 100k-neuron, 100-fan-out network lies between). */
+ * two forms lies between: 100k x 100 at 1.1% of neurons firing per step, 38 us a step in
+ * either form; 50k x 80 at 2.8%, 22.5 us). */
 #define NC_AUTO_WINDOW 256
-#define NC_AUTO_TO_EVENT_PERMILLE 100
-#define NC_AUTO_TO_DENSE_PERMILLE 160
+#define NC_AUTO_TO_EVENT_PERMILLE 10
+#define NC_AUTO_TO_DENSE_PERMILLE 20
 int nc_run(nc_net* net, int32_t n_steps);
 /* The form the network's next steps run in (NC_STEP_DENSE or NC_STEP_EVENT).  A network
  * created with NC_STEP_AUTO may be switched by the caller with nc_set_step_form (form
@@ -433,20 +434,11 @@ int nc_server_destroy(nc_server* server);
  * renderer, a game or robotics engine embedding the simulator) whose own allocator owns
  * the GPU's memory.  For them a cudaMalloc made behind their back can fail when the
  * memory is spoken for, or break their accounting.  nc_run instantiates CUDA graphs on
- * first use and, in the event form (NC_STEP_EVENT), keeps its per-step scratch (the
- * list of neurons that fired, passed from the neuron update to the spike launch) in
- * memory the handle allocated.  This call launches the same kernels directly on
- * `stream` (NULL = the handle's own stream) and calls no cudaMalloc, cudaFree or
- * allocating library routine.  The dense form needs no scratch; the event form uses a
- * fixed scratch array compiled into the library.  That array (4 MiB) is held by every
- * GPU that loads the library until the process exits, and it limits event-form calls
- * to networks of at most NC_NOALLOC_MAX_NEURONS neurons; larger ones are refused with
- * NC_ERR_INVALID.  The first event-form call on a device looks the array's device
- * address up (cudaGetSymbolAddress) and keeps it; make that first call before any
- * stream capture.  Every call clears the array's counters before its kernels run; the
- * array otherwise keeps the last call's contents, and all event-form calls share it,
- * so calls whose kernels overlap on the GPU (other handles, other streams) race: order
- * them.  Order the call after the handle's earlier work, and synchronise `stream`
+ * first use.  This call launches the same kernels directly on `stream` (NULL = the
+ * handle's own stream) and calls no cudaMalloc, cudaFree or allocating library routine;
+ * neither form's kernels need scratch.  In the event form it serves networks of at most
+ * NC_NOALLOC_MAX_NEURONS neurons; larger ones are refused with NC_ERR_INVALID.
+ * Order the call after the handle's earlier work, and synchronise `stream`
  * before any other call on the handle when it is not the handle's stream.  After this
  * call the handle reads its step counter and simulated time back from the device
  * (nc_get_step, nc_get_time and the read-backs wait for the handle's stream to do so).

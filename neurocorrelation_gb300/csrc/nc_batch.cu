@@ -207,7 +207,7 @@ int nc_batch_autotune(nc_batch* b, int32_t steps_per_trial, nc_launch_config* be
                 cands.push_back(nc_launch_config{128, cur.launch_blocks, cur.launch_block, 16, 0, k});
     } else {
         for (int nb : {64, 128, 256})
-            for (int lbm : {2, 4, 8})
+            for (int lbm : {4, 8, 16})
                 for (int lb : {128, 256})
                     for (int g : {16, 64}) cands.push_back(nc_launch_config{nb, sms * lbm, lb, g, 0, 0});
     }

@@ -172,7 +172,7 @@ __device__ __forceinline__ float fold_row(const uint8_t* nib, int q0, int nq, co
             if (m) xv[k] = x[w * 32 + ((p >> 1) & ~3) + (p & 3)];
             m &= m - 1ull;
         }
-        pot = fold8(pot, xv, F);
+        pot = fold_terms(pot, xv, F);
         if (m == 0ull && w + 1 >= nw) return pot;
         if (stop && fires_at(pot, leak)) return pot;
     }
@@ -191,15 +191,6 @@ struct TileConst {
     bool refresh;            // set old ages back in this step (NC_AGE_PERIOD)
     int64_t wide;
 };
-
-// The clamp of synapticPlasticity (src/NeuCor.cpp:757-761): hi = 1, lo = 0 for an excitatory
-// synapse, hi = 0, lo = -1 for an inhibitory one.  fminf is the compare and select of the
-// upper bound (a NaN becomes hi); the lower one keeps a negative zero, as the reference's.
-__device__ __forceinline__ float clamp_weight(float v, float lo, float hi)
-{
-    const float m = fminf(v, hi);
-    return (m >= lo) ? m : lo;
-}
 
 // Quad Q (pool index) of a row: launches and plasticity of prev.  Returns the
 // quad's window bits.  Branches are per quad (the row fired; something to store); the four

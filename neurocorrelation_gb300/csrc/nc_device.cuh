@@ -51,15 +51,12 @@ static __device__ __forceinline__ float plasticity(float w, bool inh, float trac
     return v;
 }
 
-// The same update with the clamp bounds of the synapse's sign given: hi = 1, lo = 0 for an
-// excitatory synapse, hi = 0, lo = -1 for an inhibitory one (the same compares and
-// selects as above, with the bounds chosen once per synapse).
-static __device__ __forceinline__ float plasticity_b(float w, float lo, float hi, float traceS, float traceT,
-                                                     const Rates& R)
+// The clamp of synapticPlasticity (src/NeuCor.cpp:757-761): hi = 1, lo = 0 for an excitatory
+// synapse, hi = 0, lo = -1 for an inhibitory one.  fminf is the compare and select of the
+// upper bound (a NaN becomes hi); the lower one keeps a negative zero, as the reference's.
+static __device__ __forceinline__ float clamp_weight(float v, float lo, float hi)
 {
-    const float weightChange = R.pre * traceS - R.post * traceT;
-    const float v = w + weightChange * R.lr;
-    const float m = (v <= hi) ? v : hi;
+    const float m = fminf(v, hi);
     return (m >= lo) ? m : lo;
 }
 
@@ -119,9 +116,9 @@ static __device__ __forceinline__ float add_term(float p, float x, const TermFac
     return a;
 }
 
-// The exact form of fold8, on binary64.  Kept out of line: a rare redo.
-static __device__ __noinline__ float fold_exact8(float p, float x0, float x1, float x2, float x3, float x4, float x5,
-                                                 float x6, float x7, double e_term)
+// The exact form of fold_terms, on binary64.  Kept out of line: a rare redo.
+static __device__ __noinline__ float fold_exact(float p, float x0, float x1, float x2, float x3, float x4, float x5,
+                                                float x6, float x7, double e_term)
 {
     const float x[8] = {x0, x1, x2, x3, x4, x5, x6, x7};
 #pragma unroll
@@ -132,13 +129,13 @@ static __device__ __noinline__ float fold_exact8(float p, float x0, float x1, fl
 
 // Folds the terms of the charges x[0..8) into p, in order.  An absent term is the charge
 // -0.0, which adds the term -0.0 and changes no p.
-static __device__ __forceinline__ float fold8(float p, const float x[8], const TermFactor& F)
+static __device__ __forceinline__ float fold_terms(float p, const float (&x)[8], const TermFactor& F)
 {
     const float p0 = p;
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 8; ++k) p = add_term(p, x[k], F, ok);
-    if (__builtin_expect(!ok, 0)) p = fold_exact8(p0, x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7], F.e_term);
+    if (__builtin_expect(!ok, 0)) p = fold_exact(p0, x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7], F.e_term);
     return p;
 }
 
@@ -199,15 +196,6 @@ static __device__ __forceinline__ void pop8(uint32_t* m, int b[8])
     for (int k = 0; k < 8; ++k) {
         b[k] = *m ? __ffs(*m) - 1 : -1;
         *m &= *m - 1u;
-    }
-}
-
-static __device__ __forceinline__ void pop8_64(unsigned long long* m, int b[8])
-{
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        b[k] = *m ? __ffsll((long long)*m) - 1 : -1;
-        *m &= *m - 1ull;
     }
 }
 

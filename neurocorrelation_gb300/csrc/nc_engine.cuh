@@ -18,9 +18,7 @@
 //   dense form   key, state per in-synapse, qrow per quad (see NcPools)
 //   event form   t_arr (last arrival step) and inh (one bit: Synapse::inhibitory) per
 //                in-synapse; out_ptr CSR row starts (n+1) and per out-synapse (CSR
-//                order): target, CSC index, delay (bits 0-13; bit 14/15: the target's
-//                caller id is above/below the source's), ring bit position, last
-//                accepted arrival step
+//                order) an NcOut and the last accepted arrival step
 //   Neurons sit in device slots (Morton order of positions by default); every rule
 //   that depends on ids uses the caller's ids (orig_id, the order flags, the
 //   in-synapse order).
@@ -81,6 +79,7 @@ struct NcNetDesc {
     int32_t group_base;
     int32_t n_groups;
     int32_t active;       // 0: skipped by the kernels
+    int32_t live;         // event form: the last neuron step advanced the net (its fires launch)
     int32_t raster_len;   // recorded steps capacity (0 = off)
     int32_t raster_t0;    // first recorded step
     int32_t permuted;     // neurons are stored in a different order than the caller's ids
@@ -167,6 +166,13 @@ struct alignas(16) NcRowTile {  // dense form: up to NC_TILE_ROWS consecutive ne
 
 constexpr int NC_TILE_ROWS = 32;  // neurons of a dense tile at most: one per lane
 
+struct alignas(16) NcOut {  // event form, per out-synapse
+    uint32_t csc;        // its in-synapse position, relative to syn_base
+    int32_t post;        // target's device slot
+    uint32_t ringpos;    // (word within a ring slot) << 5 | bit
+    uint32_t delay;      // bits 0-13; bit 14/15: the target's caller id is above/below the source's
+};
+
 struct NcFirer {         // periodic input firer (InputFirer, src/NeuCor.cpp:305-345)
     int32_t net;
     float last;          // InputFirer::lastFire, ms
@@ -198,10 +204,7 @@ struct NcPools {
     float* w;
     float* x;            // deltaT*AP_depolFac of the last accepted launch (src/NeuCor.cpp:695, 729-731)
     // out-synapses (CSR)
-    int32_t* out_post;   // local target id
-    int32_t* out_csc;    // CSC index relative to syn_base
-    int16_t* out_delay;
-    uint32_t* out_ringpos; // (word within slot) << 5 | bit
+    NcOut* out;
     int32_t* last_arr;
     uint32_t* inh;       // event form, CSC: Synapse::inhibitory, one bit per synapse
     int32_t* t_arr;      // event form, CSC: last arrival step
@@ -231,10 +234,6 @@ struct NcPools {
     int32_t n_firers;
     int32_t* firer_near;
     int64_t total_words;
-    // fired list (global, 2 parities)
-    int2* fired_list;    // (net, local id)
-    int32_t* fired_count;// [2]
-    int64_t fired_cap;
     // constants
     float* tables;
     NcGroupDev* groups;
@@ -243,9 +242,10 @@ struct NcPools {
     NcTile* tiles;
     int32_t n_tiles;
     int32_t* n_tiles_dev; // when set, the tile count is read from device memory (served engine)
+    int32_t warp_rows;   // event form: neurons per warp of the neuron step: 8, 16 or 32
+    int32_t launch_rows; // and of the spike launch: 1, 2, 4 or 8
     // engine
-    int32_t* tick;       // engine tick (parity of the fired list)
-    uint32_t* done_ctr;  // last-block detection
+    uint32_t* done_ctr;  // blocks (event form: warps) that have read the step counters
     uint32_t* dev_err;   // nonzero: a bounded device wait gave up (NC_DEV_ERR_*)
 };
 
@@ -284,17 +284,22 @@ NC_HD inline void nc_philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, 
 
 // Kernel launchers (nc_kernels.cu).
 namespace nc {
-// Resident 256-thread blocks per SM the step kernels' register allocation is held to
-// (3 keep every tile of a 100k-neuron net in one wave for the event form's neuron
-// update); the spike-launch grid defaults to NC_LAUNCH_MIN_BLOCKS blocks per SM.
+// Resident 256-thread blocks per SM the event form's neuron step is held to: 128 registers
+// (at 80 it spills: 100k-neuron step 112 -> 89 us without).
 #ifndef NC_NEURON_MIN_BLOCKS
-#define NC_NEURON_MIN_BLOCKS 3
+#define NC_NEURON_MIN_BLOCKS 2
 #endif
 #ifndef NC_DENSE_BLOCK
 #define NC_DENSE_BLOCK 96  // threads per block of the dense step: one warp sums, the others stream
 #endif
+#ifndef NC_EVENT_BLOCK
+#define NC_EVENT_BLOCK 64  // threads per block of the event form's neuron step
+#endif
 #ifndef NC_LAUNCH_MIN_BLOCKS
 #define NC_LAUNCH_MIN_BLOCKS 4
+#endif
+#ifndef NC_LAUNCH_BLOCKS
+#define NC_LAUNCH_BLOCKS 16  // 128-thread blocks per SM of the spike launch's grid
 #endif
 
 struct LaunchShape {

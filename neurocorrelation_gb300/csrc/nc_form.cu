@@ -25,7 +25,8 @@ __global__ void k_form_to_event(NcPools P, int net)
     const int64_t sb = D.syn_base;
     uint32_t* ring = P.ring + D.ring_base;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < D.n_syn; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = sb + (uint32_t)P.out_csc[sb + k];
+        const NcOut o = P.out[sb + k];
+        const int64_t c = sb + o.csc;
         const uint32_t s = P.state[c];
         const int32_t age = D.wide ? prev - (int32_t)s : nc_state_age(s, prev);
         // steps since the last arrival: the plasticity of prev is done
@@ -34,8 +35,8 @@ __global__ void k_form_to_event(NcPools P, int net)
         P.last_arr[sb + k] = age >= old ? NC_NEVER : prev - age;
         P.t_arr[c] = since >= old ? NC_NEVER : prev - since;
         if (age < kc) {
-            const uint32_t pos = P.out_ringpos[sb + k];
-            atomicOr(ring + (int64_t)((prev - age) & D.ring_mask) * D.ring_words + (pos >> 5), 1u << (pos & 31));
+            atomicOr(ring + (int64_t)((prev - age) & D.ring_mask) * D.ring_words + (o.ringpos >> 5),
+                     1u << (o.ringpos & 31));
         }
     }
 }
@@ -47,7 +48,7 @@ __global__ void k_form_to_dense(NcPools P, int net)
     const int32_t prev = D.t - 1;
     const int64_t sb = D.syn_base;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < D.n_syn; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = sb + (uint32_t)P.out_csc[sb + k];
+        const int64_t c = sb + P.out[sb + k].csc;
         const int32_t la = P.last_arr[sb + k], ta = P.t_arr[c];
         if (D.wide) {
             P.state[c] = (uint32_t)(la == NC_NEVER ? NC_WIDE_NEVER : la);
@@ -76,8 +77,6 @@ int launch_form_to_event(const NcPools& P, int net, int64_t n_syn, int64_t ring_
     const cudaStream_t s = (cudaStream_t)stream;
     if (cudaMemsetAsync(P.ring, 0, sizeof(uint32_t) * (size_t)ring_words, s) != cudaSuccess) return -1;
     k_form_to_event<<<grid_for(n_syn, 256), 256, 0, s>>>(P, net);
-    // the next step's neuron update starts a new fired list
-    if (cudaMemsetAsync(P.fired_count, 0, 2 * sizeof(int32_t), s) != cudaSuccess) return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -110,9 +110,9 @@ int64_t NetHost::device_bytes() const
 {
     const int64_t per_neuron = 4 + 4 + 4 + 4 + 8 + 8 + 4;             // pot lf firings act_start in_ptr out_ptr ring_off
     const bool dense = p.step_mode != NC_STEP_EVENT, event = p.step_mode != NC_STEP_DENSE;
-    // w x | key state (dense) and/or t_arr out_post out_csc delay ringpos last_arr (event); rows are
+    // w x | key state (dense) and/or t_arr out last_arr (event); rows are
     // padded to quads, and a quad has a row byte and a window byte
-    const int64_t per_syn = 4 + 4 + (dense ? 8 * key_words(*this) + 1 : 0) + (event ? 4 + 4 + 4 + 2 + 4 + 4 : 0);
+    const int64_t per_syn = 4 + 4 + (dense ? 8 * key_words(*this) + 1 : 0) + (event ? 4 + 16 + 4 : 0);
     const int64_t words = ((int64_t)n + 31) / 32;
     const int64_t ring_bytes = event ? 4 * (int64_t)ring_slots * ring_words : 0;
     return per_neuron * (n + 1) + per_syn * sp + ring_bytes + 4 * 4 * words +
@@ -375,6 +375,14 @@ void choose_key(NetHost& h)
     h.wide = slot_bits + NC_KEY_DELAY_SHIFT + bits((uint32_t)h.max_delay) > 32 || h.tab_pre_len > NC_AGE_OLD ||
              h.kc + 1 > NC_AGE_OLD;
     h.key_shift = h.wide ? 0 : 32 - slot_bits;
+}
+
+std::vector<NcOut> out_records(const NetHost& h)
+{
+    std::vector<NcOut> out((size_t)h.s);
+    for (size_t q = 0; q < out.size(); ++q)
+        out[q] = NcOut{(uint32_t)h.out_csc[q], h.out_post[q], h.out_ringpos[q], (uint16_t)h.out_delay[q]};
+    return out;
 }
 
 void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTile>& tiles,

@@ -86,6 +86,8 @@ struct RowNet {              // a net and its pool indexes
 };
 void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTile>& tiles,
                std::vector<int32_t>& start);
+// The net's out-synapse records (event form).
+std::vector<NcOut> out_records(const NetHost& h);
 // Builds the layout; returns NC_OK or an NC_ERR_* code with `err` set.
 int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, const int32_t* to,
               const float* weight, const float* length, const uint8_t* inhibitory, const nc_params& p,

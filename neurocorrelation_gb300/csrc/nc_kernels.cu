@@ -2,22 +2,22 @@
 //
 // One simulation step t of every packed net is two launches:
 //
-//   k_neuron_step  (one warp per 32 neurons of one net)
+//   k_neuron_step
 //     a. plasticity deferred from step t-1 (src/NeuCor.cpp:740-761):
 //        post-spike branch for every neuron that fired at t-1 (its whole in-synapse
-//        row, the warp's 32 lanes striding it — coalesced), then the arrival branch
-//        for every spike that arrived at t-1 (Synapse::run, src/NeuCor.cpp:718-726)
+//        row, eight lanes a row), then the arrival branch for every spike that arrived
+//        at t-1 (Synapse::run, src/NeuCor.cpp:718-726)
 //     b. Neuron::run at t (src/NeuCor.cpp:619-641): charge_insynapses folds the
 //        terms of spikes that arrived at t-1..t-KC in ascending source order (the
 //        ring bits are in CSC order, so the fold follows std::map order), charge_passive,
 //        charge_thresholdCheck with the forced-fire requests, AP
 //     c. background fire draws for t+1 (src/NeuCor.cpp:604-607)
-//     d. block-level compaction of the fired neurons into the fired list
+//     d. fired bits; the last warp to have read the step counters advances them
 //
-//   k_spike_launch (one warp per fired neuron)
+//   k_spike_launch (one warp per up to 8 neurons' fired bits)
 //     Synapse::fire (src/NeuCor.cpp:727-738) on each out-synapse: drop if busy,
 //     capture fl(fl(0.2f*52)*w) times deltaT (the fold forms the contribution term from
-//     it), mark the ring bit of the arrival step.  The last block advances every net's step counter.
+//     it), mark the ring bit of the arrival step.
 //
 // The CPU restatement runs neurons in ascending id, each update firing at once.
 // Two rules make the split launches produce the same bits:
@@ -37,50 +37,62 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 namespace {
 
 using namespace nc_dev;
 
+// Programmatic dependent launch: the step's two kernels are scheduled while the one before
+// drains and wait here before they read anything it writes.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Post-spike branch of the plasticity of step `prev` (src/NeuCor.cpp:650-655, 740-761):
-// the whole in-row of every neuron of the tile that fired at prev.  The warp takes the
-// rows two at a time, each lane four synapses of each, so eight loads per lane are in
-// flight per pass (all lanes call).
-__device__ void postfire_rows(const NcPools& P, const NcNetDesc& D, int64_t word, int lane, int64_t s0, int64_t s1,
+// the whole in-row of every neuron of the tile that fired at prev.  Groups of eight lanes
+// take a row each, a quad per lane and up to four quads in flight (all lanes call).
+__device__ void postfire_rows(const NcPools& P, const NcNetDesc& D, uint32_t fired, int lane, int64_t s0, int64_t s1,
                               int32_t prev)
 {
     const float* tab_pre = P.tables + D.table_base;
     const int32_t tpl = D.tab_pre_len;
     const Rates R = rates_of(D);
-    uint32_t m = P.fired[(int64_t)(prev & 1) * P.total_words + word];
-    while (m) {
-        const int ba = __ffs(m) - 1;
-        m &= m - 1;
-        const bool pair = m != 0;
-        const int bb = pair ? __ffs(m) - 1 : ba;
-        if (pair) m &= m - 1;
-        const int64_t a0 = __shfl_sync(kFull, s0, ba), a1 = __shfl_sync(kFull, s1, ba);
-        const int64_t c0 = __shfl_sync(kFull, s0, bb);
-        const int64_t c1 = pair ? __shfl_sync(kFull, s1, bb) : c0;
-        const int64_t len = (a1 - a0) > (c1 - c0) ? (a1 - a0) : (c1 - c0);
-        for (int64_t off = 0; off < len; off += 128) {
-            float wv[8];
-            int32_t ta[8];
-            bool ok[8], ih[8];
+    const bool inh = !D.nonneg_terms;
+    const float post0 = R.post * 0.0f;
+    while (fired) {
+        // the next four rows, one per group
+        int row = -1;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int64_t s = (u < 4 ? a0 : c0) + off + lane + 32 * (u & 3);
-                ok[u] = s < (u < 4 ? a1 : c1);
-                if (ok[u]) {
-                    wv[u] = P.w[s];
-                    ta[u] = P.t_arr[s];
-                    ih[u] = inh_bit(P, s);
-                }
+        for (int g = 0; g < 4; ++g) {
+            const int j = fired ? __ffs(fired) - 1 : -1;
+            fired &= fired - 1u;
+            if (lane >> 3 == g) row = j;
+        }
+        const int64_t a = __shfl_sync(kFull, s0, row < 0 ? 0 : row), e = __shfl_sync(kFull, s1, row < 0 ? 0 : row);
+        const int32_t nq = row < 0 ? 0 : (int32_t)((e - a) >> 2);
+        for (int32_t q0 = lane & 7; q0 < nq; q0 += 32) {
+            float4 w[4];
+            int4 ta[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (q0 + 8 * u >= nq) continue;
+                w[u] = *((const float4*)(P.w + a) + q0 + 8 * u);
+                ta[u] = *((const int4*)(P.t_arr + a) + q0 + 8 * u);
             }
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (!ok[u]) continue;
-                const int64_t s = (u < 4 ? a0 : c0) + off + lane + 32 * (u & 3);
-                P.w[s] = plasticity(wv[u], ih[u], trace_at(tab_pre, tpl, prev, ta[u]), 0.0f, R);
+            for (int u = 0; u < 4; ++u) {
+                if (q0 + 8 * u >= nq) continue;
+                const int64_t s = a + 4 * (int64_t)(q0 + 8 * u);
+                const uint32_t ih = inh ? __ldg(P.inh + (s >> 5)) >> (s & 31) : 0u;
+                float* wv = &w[u].x;
+                const int32_t* tv = &ta[u].x;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const bool neg = (ih >> k) & 1u;
+                    const float tr = trace_at_u(tab_pre, tpl, prev, tv[k]);
+                    wv[k] = clamp_weight(wv[k] + (R.pre * tr - post0) * R.lr, neg ? -1.0f : 0.0f, neg ? 0.0f : 1.0f);
+                }
+                *((float4*)P.w + (s >> 2)) = w[u];
             }
         }
     }
@@ -119,231 +131,336 @@ __device__ void arrival_row(const NcPools& P, const NcNetDesc& D, int64_t s0, in
     }
 }
 
+// Four consecutive ring words of a row, over the steps t-1 .. t-KC.
+struct RowBits {
+    uint32_t win[4];  // arrived t-KC .. t-1: in the fold
+    uint32_t arr[4];  // arrived t-1
+    uint32_t old;     // bit q: word q of slot t-KC, released by this step, is not empty
+};
+
+// Loads the words [wi, min(wi + 4, r1)) of every slot of the window, four slots at a time so
+// that their latencies overlap.
+__device__ __forceinline__ void row_bits(RowBits& B, const uint32_t* ring, int64_t rw, int32_t ring_mask, int32_t wi,
+                                         int32_t r1, int32_t t, int32_t kc)
+{
+    B.old = 0u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) B.win[q] = B.arr[q] = 0u;
+    for (int32_t k0 = 1; k0 <= kc && t - k0 >= 1; k0 += 4) {
+        uint32_t x[4][4];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            const int32_t k = k0 + d;
+            const bool in = k <= kc && t - k >= 1;
+            const uint32_t* row = ring + (int64_t)((t - k) & ring_mask) * rw + wi;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) x[d][q] = in && wi + q < r1 ? row[q] : 0u;
+        }
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                B.win[q] |= x[d][q];
+                if (k0 + d == 1) B.arr[q] = x[d][q];
+                if (k0 + d == kc && x[d][q]) B.old |= 1u << q;
+            }
+    }
+}
+
+// Pops up to kB set bits of the four words m (ascending, -1 when exhausted) into b; base is
+// the bit number of m[0]'s first bit (an empty word costs a slot).
+template <int kB>
+__device__ __forceinline__ void pop_words(uint32_t (&m)[4], int& base, int (&b)[kB])
+{
+#pragma unroll
+    for (int k = 0; k < kB; ++k) {
+        if (m[0] == 0u) {
+            m[0] = m[1];
+            m[1] = m[2];
+            m[2] = m[3];
+            m[3] = 0u;
+            base += 32;
+        }
+        b[k] = m[0] ? base + __ffs((int)m[0]) - 1 : -1;
+        m[0] &= m[0] - 1u;
+    }
+}
+__device__ __forceinline__ bool any_words(const uint32_t (&m)[4]) { return (m[0] | m[1] | m[2] | m[3]) != 0u; }
+
+constexpr int kBatch = 8;  // charges, or weights, of a row gathered together
+
+// Every warp has read the step counters: the last to say so moves them on.  The spike launch
+// that follows works on the step before the counter, for the nets this advanced (live).
+__device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
+{
+    for (int n = lane; n < P.n_nets; n += 32) {
+        NcNetDesc* D = P.nets + n;
+        D->live = D->active && D->t <= D->t_end;
+        if (D->live) {
+            if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
+            D->stats[3] += 1ull;
+            D->t += 1;
+            D->tsum = __fadd_rn(D->tsum, D->dt);  // currentTime = targetTime (src/NeuCor.cpp:616)
+        }
+    }
+    if (lane == 0) *P.done_ctr = 0u;
+}
+
+// One warp per warp_rows (8, 16 or 32) neurons of one net; blocks of any size, no block
+// barrier.  The chain of dependent loads bounds it (about 800 cycles each and more for what
+// is not in L2), so:
+//   - what the spike launch of the step before does not write (everything but charges, ring
+//     bits and arrival steps) is read, and the draws are made, before the wait for it;
+//   - the ring words of the whole window come in one go, then the gathers of the arrivals'
+//     weights and of the sum's charges together;
+//   - a small network gives a warp fewer neurons, so that a warp has fewer fired rows and a
+//     shorter longest sum.
+// Measured with the spike launch, a step (with a list of the fired neurons between the two
+// kernels before): 50k x 80 at 1.7 Hz 26.9 -> 13.6 us, 8k x 50 with inhibitory synapses at
+// 100 Hz 41.7 -> 20.2 us, 60k x 100 at 333 Hz 125 -> 85 us.
 __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPools P)
 {
-    __shared__ int s_cnt[32];
-    __shared__ int s_base;
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
-    const int tick = *P.tick;
-    const int n_tiles = P.n_tiles_dev ? *P.n_tiles_dev : P.n_tiles;
-
-    // blocks stride over the tile table (block-uniform loop: the compaction barriers
-    // below are reached by every thread)
-    for (int base = blockIdx.x * wpb; base < n_tiles; base += gridDim.x * wpb) {
-    const int gw = base + wib;
-    uint32_t fmask = 0;
-    int net = 0, first = 0;
-    if (gw < n_tiles) {
-        const NcTile tile = P.tiles[gw];
+    const int rows = P.warp_rows;
+    const int parts = 32 / rows;  // warps per tile
+    bool waited = false;
+    int n_tiles = P.n_tiles;
+    if (P.n_tiles_dev) {
+        wait_previous();
+        waited = true;
+        n_tiles = *P.n_tiles_dev;
+    }
+    const int units = n_tiles * parts, warps = gridDim.x * wpb;
+    const int me = blockIdx.x * wpb + (threadIdx.x >> 5);
+    for (int u = me; u < units; u += warps) {
+        const NcTile tile = P.tiles[u / parts];
         const NcNetDesc& D = P.nets[tile.net];
-        const int32_t t = D.t;
-        if (D.active && t <= D.t_end) {
-            net = tile.net;
-            first = tile.first;
-            const int32_t j = first + lane;
-            const bool live = j < D.n;
-            const int32_t pj = D.neuron_base + j;
-            const int32_t pb = D.ptr_base + j;
-            const int64_t word = D.word_base + (first >> 5);
-            int32_t lf = NC_NEVER;
-            int64_t s0 = 0, s1 = 0;
-            int32_t r0 = 0, r1 = 0;
-            float pot = 0.0f;
-            uint32_t fw = 0, uw = 0;
-            if (live) {
-                lf = P.lf[pj];
-                s0 = P.in_ptr[pb];
-                s1 = P.in_ptr[pb + 1];
-                r0 = P.ring_off[pb];
-                r1 = P.ring_off[pb + 1];
-                pot = P.pot[pj];
-                fw = P.forced[(int64_t)(t & 1) * P.total_words + word];
-                uw = P.ufire[(int64_t)(t & 1) * P.total_words + word];
+        const int32_t first = tile.first + (u % parts) * rows, j = first + lane;
+        const bool live = lane < rows && j < D.n;
+        const int32_t pj = D.neuron_base + j;
+        const int32_t pb = D.ptr_base + j;
+        const int64_t word = D.word_base + (first >> 5);
+        const int shift = first & 31;
+        const uint32_t mask = (rows == 32 ? ~0u : (1u << rows) - 1u) << shift;
+        uint32_t* ring = P.ring + D.ring_base;
+        const int64_t rw = D.ring_words;
+        const int32_t ring_mask = D.ring_mask, kc = D.kc;
+        // (mutable state past the L1: it may hold what an earlier kernel left)
+        const int32_t t = __ldcg(&D.t), done_to = __ldcg(&D.stdp_done);
+        const bool act = __ldcg(&D.active) && t <= __ldcg(&D.t_end);
+        const int32_t prev = t - 1;
+        int64_t s0 = 0, s1 = 0;
+        int32_t r0 = 0, r1 = 0, cid = j;
+        int32_t lf = NC_NEVER;
+        float pot = 0.0f;
+        if (live) {
+            lf = __ldcg(P.lf + pj);
+            pot = __ldcg(P.pot + pj);
+            s0 = __ldg(P.in_ptr + pb);
+            s1 = __ldg(P.in_ptr + pb + 1);
+            r0 = __ldg(P.ring_off + pb);
+            r1 = __ldg(P.ring_off + pb + 1);
+            if (D.permuted) cid = __ldg(P.orig_id + pj);
+        }
+        const uint32_t was = (__ldcg(P.fired + (int64_t)(prev & 1) * P.total_words + word) & mask) >> shift;
+        const uint32_t fw = (__ldcg(P.forced + (int64_t)(t & 1) * P.total_words + word) & mask) >> shift;
+        const uint32_t uw = (__ldcg(P.ufire + (int64_t)(t & 1) * P.total_words + word) & mask) >> shift;
+        // input requests, and the background target for step t+1 (src/NeuCor.cpp:604-607),
+        // drawn per caller id
+        bool forced = (fw >> lane) & 1u;
+        uint32_t bg = ~0u;
+        if (live && act) {
+            if (!forced && D.n_groups) forced = input_request(P, D, cid, t);
+            if (D.bg_period > 0) {
+                uint32_t o[4];
+                philox((uint32_t)cid, (uint32_t)t, NC_STREAM_BACKGROUND, 0u, D, o);
+                if (o[0] % (uint32_t)D.bg_period == 0u) {
+                    bg = o[1] % (uint32_t)D.n;
+                    if (D.permuted) bg = (uint32_t)__ldg(P.slot_of + D.neuron_base + bg);
+                }
             }
-            const int32_t prev = t - 1;
-            const bool stdp = prev >= 1 && D.stdp_done < prev;
-            if (stdp) postfire_rows(P, D, word, lane, s0, s1, prev);
+        }
+        if (!waited) {
+            wait_previous();
+            release_next();
+            waited = true;
+        }
+        // the last unit's counters are read (the condition needs them): say so
+        unsigned arrived = 0u;
+        const bool last_unit = u + warps >= units;
+        if (!act && !last_unit) continue;
+        if (last_unit && lane == 0) arrived = atomicAdd(P.done_ctr, min(t, done_to) > NC_NEVER ? 1u : 0u);
+        if (act) {
+            const bool stdp = prev >= 1 && done_to < prev;
+            RowBits B;
+            row_bits(B, ring, rw, ring_mask, r0, r1, t, kc);
+            if (bg != ~0u)
+                atomicOr(P.forced + (int64_t)((t + 1) & 1) * P.total_words + D.word_base + (bg >> 5), 1u << (bg & 31));
+            if (stdp && was) postfire_rows(P, D, was, lane, s0, s1, prev);
 
-            bool fired = false;
-            if (live) {
-                bool forced = (fw >> lane) & 1u;
-                if (!forced && D.n_groups) forced = input_request(P, D, D.permuted ? P.orig_id[pj] : j, t);
-                // charge_insynapses (src/NeuCor.cpp:688-700): terms of spikes that arrived
-                // t-1 .. t-KC, ascending source id.  The arrival branch of the deferred
-                // plasticity rides along: the spikes that arrived at prev are the ring
-                // bits of slot prev.  Inside its AP (t - lastFire < KC) a neuron's
-                // potential comes from the AP table whatever the sum is, and it cannot
-                // cross the threshold, so only its sum is skipped.
-                const bool in_ap = lf != NC_NEVER && t - lf < D.kc;
-                if (r1 > r0) {
-                    const TermFactor F = term_factor(D);
-                    // the sum is not needed inside the AP, nor, when no term can be
-                    // negative, once the neuron is certain to fire (fires_at)
-                    const bool stop = NC_FOLD_EARLY_EXIT && D.nonneg_terms;
-                    bool settled = in_ap || (stop && fires_at(pot, D.leak));
-                    uint32_t* ring = P.ring + D.ring_base;
-                    const int64_t rw = D.ring_words;
-                    const int32_t kc = D.kc;
-                    const int32_t oldest = t - kc;
-                    const float trT = trace_at(P.tables + D.table_base + D.tab_pre_len, D.tab_post_len, prev, lf);
-                    const Rates R = rates_of(D);
-                    for (int32_t wi = r0; wi < r1; wi += 2) {
-                        const bool two = wi + 1 < r1;
-                        uint32_t lo = 0, hi = 0, alo = 0, ahi = 0, olo = 0, ohi = 0;
-                        for (int32_t k = 1; k <= kc && t - k >= 1; ++k) {
-                            const uint32_t* row = ring + (int64_t)((t - k) & D.ring_mask) * rw + wi;
-                            const uint32_t x = row[0];
-                            const uint32_t y = two ? row[1] : 0u;
-                            lo |= x;
-                            hi |= y;
-                            if (k == 1) {
-                                alo = x;
-                                ahi = y;
-                            }
-                            olo = x;  // ends as the word of slot t-KC when t-KC >= 1
-                            ohi = y;
-                        }
-                        unsigned long long bits = settled ? 0ull : (lo | ((unsigned long long)hi << 32));
-                        const unsigned long long arr = stdp ? (alo | ((unsigned long long)ahi << 32)) : 0ull;
-                        const int64_t sb = s0 + (int64_t)(wi - r0) * 32;
-                        unsigned long long ih = 0ull;
-                        if (arr) ih = inh_bits32(P, sb) | ((unsigned long long)(two ? inh_bits32(P, sb + 32) : 0u) << 32);
-                        // arrival branch first (it touches w and t_arr only, the fold reads x)
-                        unsigned long long am = arr;
-                        while (am) {
-                            int b[8];
-                            pop8_64(&am, b);
-                            float wv[8];
+            // charge_insynapses (src/NeuCor.cpp:688-700): terms of spikes that arrived
+            // t-1 .. t-KC, ascending source id.  The arrival branch of the deferred
+            // plasticity rides along: the spikes that arrived at prev are the ring bits of
+            // slot prev.  Inside its AP (t - lastFire < KC) a neuron's potential comes from
+            // the AP table whatever the sum is, and it cannot cross the threshold, so only
+            // its sum is skipped; so is the rest of it once a neuron of a net with no
+            // negative term is certain to fire (fires_at).
+            const bool can = lf == NC_NEVER || t - lf >= kc;
+            const bool stop = D.nonneg_terms != 0;
+            const float leak = D.leak;
+            bool settled = !can || (stop && fires_at(pot, leak));
+            const TermFactor F = term_factor(D);
+            const float trT = trace_at_u(P.tables + D.table_base + D.tab_pre_len, D.tab_post_len, prev, lf);
+            const Rates R = rates_of(D);
+            const float chg = (R.pre * 0.0f - R.post * trT) * R.lr;
+            for (int32_t wi = r0; wi < r1;) {
+                const int64_t sb = s0 + (int64_t)(wi - r0) * 32;
+                int ba0 = 0, bw0 = 0;
+                if (!stdp) B.arr[0] = B.arr[1] = B.arr[2] = B.arr[3] = 0u;
+                if (settled) B.win[0] = B.win[1] = B.win[2] = B.win[3] = 0u;
+                int bw[kBatch];
+                float xv[kBatch];
+                pop_words(B.win, bw0, bw);
 #pragma unroll
-                            for (int k = 0; k < 8; ++k)
-                                if (b[k] >= 0) wv[k] = P.w[sb + b[k]];
+                for (int k = 0; k < kBatch; ++k) xv[k] = bw[k] >= 0 ? P.x[sb + bw[k]] : -0.0f;
+                while (any_words(B.arr)) {
+                    int ba[kBatch];
+                    float wv[kBatch];
+                    uint32_t neg = 0u;
+                    pop_words(B.arr, ba0, ba);
 #pragma unroll
-                            for (int k = 0; k < 8; ++k) {
-                                if (b[k] < 0) continue;
-                                P.t_arr[sb + b[k]] = prev;
-                                P.w[sb + b[k]] = plasticity(wv[k], (ih >> b[k]) & 1ull, 0.0f, trT, R);
-                            }
-                        }
-                        while (bits) {
-                            int b[8];
-                            pop8_64(&bits, b);
-                            float xv[8];
+                    for (int k = 0; k < kBatch; ++k) {
+                        if (ba[k] < 0) continue;
+                        wv[k] = P.w[sb + ba[k]];
+                        if (!stop) neg |= inh_bit(P, sb + ba[k]) ? 1u << k : 0u;
+                    }
 #pragma unroll
-                            for (int k = 0; k < 8; ++k) xv[k] = b[k] >= 0 ? P.x[sb + b[k]] : -0.0f;
-                            pot = fold8(pot, xv, F);
-                            if (stop && fires_at(pot, D.leak)) {
-                                settled = true;
-                                bits = 0ull;
-                            }
-                        }
-                        // the spikes that arrived KC steps ago are released (AP_fireTime = 0)
-                        if (oldest >= 1) {
-                            uint32_t* orow = ring + (int64_t)(oldest & D.ring_mask) * rw + wi;
-                            if (olo) orow[0] = 0u;
-                            if (two && ohi) orow[1] = 0u;
-                        }
+                    for (int k = 0; k < kBatch; ++k) {
+                        if (ba[k] < 0) continue;
+                        const bool n = (neg >> k) & 1u;
+                        P.t_arr[sb + ba[k]] = prev;
+                        P.w[sb + ba[k]] = clamp_weight(wv[k] + chg, n ? -1.0f : 0.0f, n ? 0.0f : 1.0f);
                     }
                 }
+                while (true) {
+                    // the next batch's charges are gathered while this one is summed
+                    const bool more = any_words(B.win);
+                    float xn[kBatch];
+                    if (more) {
+                        pop_words(B.win, bw0, bw);
+#pragma unroll
+                        for (int k = 0; k < kBatch; ++k) xn[k] = bw[k] >= 0 ? P.x[sb + bw[k]] : -0.0f;
+                    }
+                    if (!settled) pot = fold_terms(pot, xv, F);
+                    if (stop && !settled) settled = fires_at(pot, leak);
+                    if (!more || settled) break;
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k) xv[k] = xn[k];
+                }
+                // the spikes that arrived KC steps ago are released (AP_fireTime = 0)
+                if (t - kc >= 1) {
+                    uint32_t* orow = ring + (int64_t)((t - kc) & ring_mask) * rw + wi;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if ((B.old >> q) & 1u) orow[q] = 0u;
+                }
+                wi += 4;
+                if (wi < r1) row_bits(B, ring, rw, ring_mask, wi, r1, t, kc);
+            }
+            bool fired = false;
+            if (live) {
                 // charge_passive (src/NeuCor.cpp:677-680)
-                pot = (pot - -70.0f) * D.leak + -70.0f;
-                // charge_thresholdCheck (src/NeuCor.cpp:682-686); vesicles stay positive
-                const bool can = (lf == NC_NEVER) || (t - lf >= D.kc);
-                // an input firer's Neuron::fire has no threshold or refractory test
+                pot = (pot - -70.0f) * leak + -70.0f;
+                // charge_thresholdCheck (src/NeuCor.cpp:682-686); vesicles stay positive.  An
+                // input firer's Neuron::fire has no threshold or refractory test
                 fired = ((uw >> lane) & 1u) || ((-55.0f < pot || forced) && can);
                 if (fired) {
                     lf = t;
                     P.lf[pj] = t;
-                    P.firings[pj] += 1u;
+                    atomicAdd(P.firings + pj, 1u);  // (nothing waits for a value)
                 }
                 // AP (src/NeuCor.cpp:706-714)
-                if (lf != NC_NEVER && t - lf < D.kc) pot = __ldg(P.tables + D.ap_base + (t - lf));
+                if (lf != NC_NEVER && t - lf < kc) pot = __ldg(P.tables + D.ap_base + (t - lf));
                 P.pot[pj] = pot;
             }
-            fmask = __ballot_sync(kFull, fired);
-            if (lane == 0) {
-                P.fired[(int64_t)(t & 1) * P.total_words + word] = fmask;
-                P.forced[(int64_t)(t & 1) * P.total_words + word] = 0u;
-                P.ufire[(int64_t)(t & 1) * P.total_words + word] = 0u;
+            // bytes (8 neurons) of the bitsets: a warp may own part of a word
+            const uint32_t fmask = __ballot_sync(kFull, fired);
+            if (8 * lane < rows && first + 8 * lane < D.n) {
+                const int64_t b = 4 * (D.word_base + (int64_t)(first >> 5)) + (shift >> 3) + lane;
+                const uint8_t v = (uint8_t)(fmask >> (8 * lane));
+                ((uint8_t*)(P.fired + (int64_t)(t & 1) * P.total_words))[b] = v;
+                if ((fw >> (8 * lane)) & 0xffu) ((uint8_t*)(P.forced + (int64_t)(t & 1) * P.total_words))[b] = 0;
+                if ((uw >> (8 * lane)) & 0xffu) ((uint8_t*)(P.ufire + (int64_t)(t & 1) * P.total_words))[b] = 0;
                 if (D.raster_len > 0 && t >= D.raster_t0 && t - D.raster_t0 < D.raster_len)
-                    D.raster[(int64_t)(t - D.raster_t0) * D.n_words + (first >> 5)] = fmask;
-            }
-            // background fires for step t+1 (src/NeuCor.cpp:604-607), drawn per caller id
-            if (live && D.bg_period > 0) {
-                uint32_t o[4];
-                philox((uint32_t)(D.permuted ? P.orig_id[pj] : j), (uint32_t)t, NC_STREAM_BACKGROUND, 0u, D, o);
-                if (o[0] % (uint32_t)D.bg_period == 0u) {
-                    uint32_t tgt = o[1] % (uint32_t)D.n;
-                    if (D.permuted) tgt = (uint32_t)P.slot_of[D.neuron_base + tgt];
-                    atomicOr(P.forced + (int64_t)((t + 1) & 1) * P.total_words + D.word_base + (tgt >> 5),
-                             1u << (tgt & 31));
-                }
+                    ((uint8_t*)(D.raster + (int64_t)(t - D.raster_t0) * D.n_words))[(first >> 3) + lane] = v;
             }
         }
+        if (last_unit && __shfl_sync(kFull, arrived, 0) == (unsigned)min(units, warps) - 1u) advance_steps(P, lane);
     }
-    // block-level compaction of fired neurons
-    const int cnt = __popc(fmask);
-    if (lane == 0) s_cnt[wib] = cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int tot = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            const int c = s_cnt[w];
-            s_cnt[w] = tot;
-            tot += c;
-        }
-        s_base = tot ? atomicAdd(P.fired_count + (tick & 1), tot) : 0;
-    }
-    __syncthreads();
-    if ((fmask >> lane) & 1u) {
-        const int rank = __popc(fmask & ((1u << lane) - 1u));
-        P.fired_list[(int64_t)(tick & 1) * P.fired_cap + s_base + s_cnt[wib] + rank] = make_int2(net, first + lane);
-    }
-    __syncthreads();  // s_cnt and s_base are reused by the next tile group
+    if (units == 0 && blockIdx.x == 0 && threadIdx.x < 32) {  // nets without neurons still step
+        if (!waited) wait_previous();
+        advance_steps(P, lane);
     }
 }
 
-__device__ __forceinline__ int warp_sum(int v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
-}
-
+// Synapse::fire (src/NeuCor.cpp:727-738) on the out-synapses of the neurons that fired at t,
+// a warp per launch_rows (1 to 8) neurons' fired bits, all lanes on a fired neuron's
+// out-synapses, four in flight each.  Its chain of loads bounds it: the fired byte (of both
+// parities, beside the step counter), the 16-byte out-synapse records, the weights and the
+// fired words of targets that came first.
 __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPools P)
 {
-    __shared__ int s_last;
-    __shared__ int s_net[32];
-    __shared__ unsigned long long s_acc[32][3];
+    __shared__ int s_net[8];
+    __shared__ unsigned s_acc[8][3];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const int nwb = blockDim.x >> 5;
-    const int gw = blockIdx.x * nwb + wib;
-    const int nw = gridDim.x * nwb;
-    const int tick = *P.tick;
-    const int par = tick & 1;
-    const int count = P.fired_count[par];
-
+    bool waited = false;
+    int n_tiles = P.n_tiles;
+    if (P.n_tiles_dev) {
+        wait_previous();
+        waited = true;
+        n_tiles = *P.n_tiles_dev;
+    }
+    const int rows = P.launch_rows, parts = 32 / rows;
+    const int units = parts * n_tiles;
     int acc_net = -1;
-    unsigned long long acc_fire = 0, acc_launch = 0, acc_drop = 0;
-    for (int e = gw; e < count; e += nw) {
-        const int2 ent = P.fired_list[(int64_t)par * P.fired_cap + e];
-        const NcNetDesc& D = P.nets[ent.x];
-        const int32_t i = ent.y;
-        const int32_t t = D.t;
-        if (ent.x != acc_net) {
-            if (acc_net >= 0 && lane == 0) {
-                unsigned long long* st = P.nets[acc_net].stats;
-                atomicAdd(st + 0, acc_fire);
-                atomicAdd(st + 1, acc_launch);
-                atomicAdd(st + 2, acc_drop);
-            }
-            acc_net = ent.x;
-            acc_fire = acc_launch = acc_drop = 0;
+    unsigned fires = 0, nl = 0, nd = 0;  // of acc_net; nl, nd per lane
+    for (int u = blockIdx.x * nwb + wib; u < units; u += gridDim.x * nwb) {
+        const NcTile tile = P.tiles[u / parts];
+        const NcNetDesc& D = P.nets[tile.net];
+        const int32_t first = tile.first + (u % parts) * rows;
+        if (first >= D.n) continue;
+        int64_t start = 0;  // row start of neuron first + lane
+        if (lane <= min(rows, D.n - first)) start = __ldg(P.out_ptr + D.ptr_base + first + lane);
+        const int64_t byte = 4 * (D.word_base + (int64_t)(first >> 5)) + ((first & 31) >> 3);
+        if (!waited) {
+            wait_previous();
+            release_next();
+            waited = true;
         }
-        const int64_t k0 = P.out_ptr[D.ptr_base + i];
-        const int64_t k1 = P.out_ptr[D.ptr_base + i + 1];
+        // both parities' bytes beside the counter that picks one
+        const uint32_t f0 = __ldcg((const uint8_t*)P.fired + byte);
+        const uint32_t f1 = __ldcg((const uint8_t*)(P.fired + P.total_words) + byte);
+        const int32_t t = __ldcg(&D.t) - 1;
+        uint32_t fired = ((t & 1 ? f1 : f0) >> (first & 7)) & ((1u << rows) - 1u);
+        if (!fired || !__ldcg(&D.live)) continue;
+        if (tile.net != acc_net) {
+            if (acc_net >= 0) {
+                nl = __reduce_add_sync(kFull, nl);
+                nd = __reduce_add_sync(kFull, nd);
+                if (lane == 0) {
+                    unsigned long long* st = P.nets[acc_net].stats;
+                    atomicAdd(st + 0, (unsigned long long)fires);
+                    atomicAdd(st + 1, (unsigned long long)nl);
+                    atomicAdd(st + 2, (unsigned long long)nd);
+                }
+            }
+            acc_net = tile.net;
+            fires = nl = nd = 0;
+        }
+        fires += __popc(fired);
         const uint32_t* fired_t = P.fired + (int64_t)(t & 1) * P.total_words + D.word_base;
         const float* tab_pre = P.tables + D.table_base;
         uint32_t* ring = P.ring + D.ring_base;
@@ -353,107 +470,81 @@ __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPo
         const int64_t syn_base = D.syn_base, ring_words = D.ring_words;
         const float dt = D.dt, c52 = D.c52;
         const Rates R = rates_of(D);
-        int nl = 0, nd = 0;
-        // four out-synapses per lane in flight: table loads, then weight loads, then writes
-        for (int64_t kb = k0; kb < k1; kb += 128) {
-            int32_t la[4], cs[4];
-            uint32_t dl[4];
-            bool ok[4];
+        for (; fired; fired &= fired - 1u) {
+            const int i = __ffs((int)fired) - 1;
+            const int64_t k0 = __shfl_sync(kFull, start, i), k1 = __shfl_sync(kFull, start, i + 1);
+            for (int64_t kb = k0; kb < k1; kb += 128) {
+                uint4 o[4];
+                int32_t la[4];
+                bool ok[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int64_t k = kb + lane + 32 * u;
-                ok[u] = k < k1;
-                if (ok[u]) {
-                    dl[u] = (uint16_t)P.out_delay[k];
-                    la[u] = P.last_arr[k];
-                    cs[u] = P.out_csc[k];
+                for (int v = 0; v < 4; ++v) {
+                    const int64_t k = kb + lane + 32 * v;
+                    ok[v] = k < k1;
+                    if (ok[v]) {
+                        o[v] = __ldg((const uint4*)P.out + k);
+                        la[v] = P.last_arr[k];
+                    }
                 }
-            }
-            float wv[4];
-            bool acc[4];
+                float wv[4];
+                uint32_t fw[4];
+                bool acc[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                // freed by the target's update at t only if the target's id is not above
-                acc[u] = ok[u] && (la[u] == NC_NEVER || t - la[u] >= kc + (int32_t)((dl[u] >> 14) & 1u));
-                if (acc[u]) wv[u] = P.w[syn_base + (uint32_t)cs[u]];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (!ok[u]) continue;
-                if (!acc[u]) {
-                    ++nd;
-                    continue;
+                for (int v = 0; v < 4; ++v) {
+                    // freed by the target's update at t only if the target's id is not above
+                    acc[v] = ok[v] && (la[v] == NC_NEVER || t - la[v] >= kc + (int32_t)((o[v].w >> 14) & 1u));
+                    fw[v] = 0u;
+                    if (acc[v]) {
+                        wv[v] = P.w[syn_base + o[v].x];
+                        // target id below the source's: its update ran first
+                        if ((o[v].w >> 15) & 1u) fw[v] = fired_t[o[v].y >> 5] >> (o[v].y & 31);
+                    }
+                    nl += acc[v] ? 1u : 0u;
+                    nd += ok[v] && !acc[v] ? 1u : 0u;
                 }
-                const int64_t k = kb + lane + 32 * u;
-                const int64_t s = syn_base + (uint32_t)cs[u];
-                float w = wv[u];
-                if ((dl[u] >> 15) & 1u) {  // target id below the source's: its update ran first
-                    const int32_t j = P.out_post[k];
-                    if ((fired_t[j >> 5] >> (j & 31)) & 1u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    if (!acc[v]) continue;
+                    const int64_t k = kb + lane + 32 * v;
+                    const int64_t s = syn_base + o[v].x;
+                    float w = wv[v];
+                    if (fw[v] & 1u)
                         w = plasticity(w, inh_bit(P, s), trace_at(tab_pre, tpl, t, P.t_arr[s]), 0.0f, R);
+                    // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
+                    P.x[s] = dt * (c52 * w);
+                    const int32_t d = (int32_t)(o[v].w & 0x3fffu);
+                    P.last_arr[k] = t + d;
+                    atomicOr(ring + (int64_t)((t + d) & ring_mask) * ring_words + (o[v].z >> 5), 1u << (o[v].z & 31));
                 }
-                // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
-                const float depol = c52 * w;
-                P.x[s] = dt * depol;
-                const int32_t d = (int32_t)(dl[u] & 0x3fffu);
-                P.last_arr[k] = t + d;
-                const uint32_t pos = P.out_ringpos[k];
-                atomicOr(ring + (int64_t)((t + d) & ring_mask) * ring_words + (pos >> 5), 1u << (pos & 31));
-                ++nl;
             }
         }
-        nl = warp_sum(nl);
-        nd = warp_sum(nd);
-        acc_fire += 1;
-        acc_launch += (unsigned long long)nl;
-        acc_drop += (unsigned long long)nd;
     }
+    if (!waited) wait_previous();
     // per-block reduction of the counters, per net
+    if (!__syncthreads_or(acc_net >= 0)) return;
+    nl = __reduce_add_sync(kFull, nl);
+    nd = __reduce_add_sync(kFull, nd);
     if (lane == 0) {
         s_net[wib] = acc_net;
-        s_acc[wib][0] = acc_fire;
-        s_acc[wib][1] = acc_launch;
-        s_acc[wib][2] = acc_drop;
+        s_acc[wib][0] = fires;
+        s_acc[wib][1] = nl;
+        s_acc[wib][2] = nd;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 0; w < nwb; ++w) {
             const int n = s_net[w];
             if (n < 0) continue;
-            unsigned long long f = s_acc[w][0], l = s_acc[w][1], d = s_acc[w][2];
+            unsigned long long c[3] = {s_acc[w][0], s_acc[w][1], s_acc[w][2]};
             for (int v = w + 1; v < nwb; ++v) {
                 if (s_net[v] != n) continue;
-                f += s_acc[v][0];
-                l += s_acc[v][1];
-                d += s_acc[v][2];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) c[k] += s_acc[v][k];
                 s_net[v] = -1;
             }
-            unsigned long long* st = P.nets[n].stats;
-            atomicAdd(st + 0, f);
-            atomicAdd(st + 1, l);
-            atomicAdd(st + 2, d);
-        }
-    }
-    // the last block to finish advances the step counters
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(P.done_ctr, 1u) == gridDim.x - 1u);
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        for (int n = threadIdx.x; n < P.n_nets; n += blockDim.x) {
-            NcNetDesc* D = P.nets + n;
-            if (D->active && D->t <= D->t_end) {
-                if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
-                D->stats[3] += 1ull;
-                D->t += 1;
-                D->tsum = __fadd_rn(D->tsum, D->dt);  // currentTime = targetTime (src/NeuCor.cpp:616)
-            }
-        }
-        if (threadIdx.x == 0) {
-            P.fired_count[(tick + 1) & 1] = 0;
-            *P.tick = tick + 1;
-            *P.done_ctr = 0u;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (c[k]) atomicAdd(P.nets[n].stats + k, c[k]);
         }
     }
 }
@@ -481,7 +572,8 @@ __global__ void __launch_bounds__(256) k_stdp_flush(NcPools P)
         r0 = P.ring_off[pb];
         r1 = P.ring_off[pb + 1];
     }
-    postfire_rows(P, D, D.word_base + (tile.first >> 5), lane, s0, s1, prev);
+    postfire_rows(P, D, P.fired[(int64_t)(prev & 1) * P.total_words + D.word_base + (tile.first >> 5)], lane, s0, s1,
+                  prev);
     if (live && r1 > r0) arrival_row(P, D, s0, r0, r1, lf, prev);
 }
 
@@ -533,19 +625,32 @@ static int check_launch()
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+// Launches fn<<<grid, block, 0, s>>>(P) as a programmatic dependent launch.
+static int launch_dependent(void (*fn)(NcPools), int grid, int block, void* stream, const NcPools& P)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, fn, P) != cudaSuccess) return -1;
+    return check_launch();
+}
+
 int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream)
 {
-    const int warps_per_block = L.neuron_block / 32;
-    const int blocks = (P.n_tiles + warps_per_block - 1) / warps_per_block;
-    if (blocks == 0) return 0;
-    k_neuron_step<<<blocks, L.neuron_block, 0, (cudaStream_t)stream>>>(P);
-    return check_launch();
+    const int64_t warps = (int64_t)P.n_tiles * (32 / P.warp_rows);
+    const int64_t blocks = (warps + L.neuron_block / 32 - 1) / (L.neuron_block / 32);
+    return launch_dependent(k_neuron_step, (int)std::max<int64_t>(1, blocks), L.neuron_block, stream, P);
 }
 
 int launch_spike_launch(const NcPools& P, const LaunchShape& L, void* stream)
 {
-    k_spike_launch<<<L.launch_blocks, L.launch_block, 0, (cudaStream_t)stream>>>(P);
-    return check_launch();
+    return launch_dependent(k_spike_launch, L.launch_blocks, L.launch_block, stream, P);
 }
 
 int launch_stdp_flush(const NcPools& P, const LaunchShape& L, void* stream)

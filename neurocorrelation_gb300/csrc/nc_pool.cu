@@ -89,6 +89,18 @@ static cudaError_t upload_part(T* dev, const std::vector<T>& host, int64_t at, i
     return cudaMemcpyAsync(dev + at, host.data() + from, (size_t)count * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
+void event_rows(int64_t tiles, int sms, NcPools& P)
+{
+    // 8k neurons: 26.0 us a step with a warp per 32, 23.8 with one per 8; 50k (1,563 tiles):
+    // 15.0 against 27.2
+    P.warp_rows = tiles <= 2 * (int64_t)sms ? 8 : tiles <= 4 * (int64_t)sms ? 16 : 32;
+    // as few neurons per warp of the spike launch as fill its grid once: their fires are
+    // served one after the other
+    P.launch_rows = 8;
+    while (P.launch_rows > 1 && tiles * 32 / (P.launch_rows / 2) <= (int64_t)sms * NC_LAUNCH_BLOCKS * 4)
+        P.launch_rows /= 2;
+}
+
 int dense_blocks(int64_t neurons, int threads)
 {
     return (int)std::max<int64_t>(1, std::min<int64_t>(dense_resident_blocks(threads), (neurons + 7) / 8));
@@ -111,8 +123,8 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     dense = nets.empty() || nets[0]->p.step_mode != NC_STEP_EVENT;
     both = !nets.empty() && nets[0]->p.step_mode == NC_STEP_AUTO;
     const bool event_tables = !dense || both;
-    L.launch_block = 256;
-    L.launch_blocks = std::max(1, sms * NC_LAUNCH_MIN_BLOCKS);
+    L.launch_block = 128;
+    L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
 
     // pool sizes
     int64_t neurons = 0, ptrs = 0, words = 0, syn = 0, ring = 0, tables = 0, tiles = 0;
@@ -208,16 +220,13 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         NC_ALLOC(P.pst, float, neurons);
         NC_ALLOC(P.nib, uint8_t, syn / 4 + 8);  // read in 8-byte words
     }
-    L.neuron_block = dense ? NC_DENSE_BLOCK : 256;
+    L.neuron_block = dense ? NC_DENSE_BLOCK : NC_EVENT_BLOCK;
     if (event_tables) {
         NC_ALLOC(P.inh, uint32_t, (syn + 31) / 32 + 1);  // one spare word for 32-bit windows
         NC_ALLOC(P.t_arr, int32_t, syn);
         NC_ALLOC(P.out_ptr, int64_t, ptrs);
         NC_ALLOC(P.ring_off, int32_t, ptrs);
-        NC_ALLOC(P.out_post, int32_t, syn);
-        NC_ALLOC(P.out_csc, int32_t, syn);
-        NC_ALLOC(P.out_delay, int16_t, syn);
-        NC_ALLOC(P.out_ringpos, uint32_t, syn);
+        NC_ALLOC(P.out, NcOut, syn);
         NC_ALLOC(P.last_arr, int32_t, syn);
         NC_ALLOC(P.ring, uint32_t, ring);
         ring_words_total_ = ring;
@@ -226,14 +235,10 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     NC_ALLOC(P.fired, uint32_t, 2 * P.total_words);
     NC_ALLOC(P.forced, uint32_t, 2 * P.total_words);
     NC_ALLOC(P.ufire, uint32_t, 2 * P.total_words);
-    P.fired_cap = event_tables ? std::max<int64_t>(neurons, 1) : 0;
-    if (event_tables) NC_ALLOC(P.fired_list, int2, 2 * P.fired_cap);
-    NC_ALLOC(P.fired_count, int32_t, 2);
     NC_ALLOC(P.tables, float, tables);
     NC_ALLOC(P.groups, NcGroupDev, nets.size() * ngroups_each);
     NC_ALLOC(P.nets, NcNetDesc, nets.size());
     if (event_tables) NC_ALLOC(P.tiles, NcTile, tiles);
-    NC_ALLOC(P.tick, int32_t, 1);
     NC_ALLOC(P.done_ctr, uint32_t, 1);
     NC_ALLOC(P.dev_err, uint32_t, 1);
     NC_ALLOC(d_bar_, unsigned, 2);
@@ -243,7 +248,8 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     scratch_bytes_ = std::max<size_t>(256, std::min(scratch_bytes_, kScratchMax));
     NC_ALLOC(scratch_, char, scratch_bytes_);
     P.n_nets = (int32_t)nets.size();
-    P.n_tiles = (int32_t)tiles;
+    P.n_tiles = event_tables ? (int32_t)tiles : 0;
+    event_rows(tiles, sms, P);
 
     // contents
     std::vector<NcTile> tile_host;
@@ -265,6 +271,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         NC_CK(upload(P.in_ptr, inp, sl.ptr_base, stream));
         row_nets.push_back(RowNet{&h, (int32_t)q, sl.syn_base, sl.neuron_base, sl.ptr_base});
         std::vector<int32_t> never;
+        std::vector<NcOut> out;
         if (dense && launch_fill_words(P.state + sl.syn_base, d.wide + h.sp, initial_state(h), stream)) {
             err = cuda_msg("initial states", cudaGetLastError());
             return NC_ERR_CUDA;
@@ -283,10 +290,8 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
                 NC_CK(upload(P.out_ptr, outp, sl.ptr_base, stream));
                 NC_CK(upload(P.ring_off, h.ring_off, sl.ptr_base, stream));
                 NC_CK(upload_part(P.last_arr, never, sl.syn_base, 0, h.s, stream));
-                NC_CK(upload(P.out_post, h.out_post, sl.syn_base, stream));
-                NC_CK(upload(P.out_csc, h.out_csc, sl.syn_base, stream));
-                NC_CK(upload(P.out_delay, h.out_delay, sl.syn_base, stream));
-                NC_CK(upload(P.out_ringpos, h.out_ringpos, sl.syn_base, stream));
+                out = out_records(h);
+                NC_CK(upload(P.out, out, sl.syn_base, stream));
             }
         }
         NC_CK(upload(P.tables, h.tables, d.table_base, stream));

@@ -112,6 +112,8 @@ private:
 // Blocks of `threads` threads that the rows of `neurons` neurons are shared out to: one wave,
 // or a block for each 8 neurons.
 int dense_blocks(int64_t neurons, int threads);
+// Neurons per warp of the event form's kernels, for an engine of so many 32-neuron tiles.
+void event_rows(int64_t tiles, int sms, NcPools& P);
 // The CSC positions of a net's input synapses on the device (freed by the caller), or null
 // when there is no memory for them: the read-back then reorders on the host.
 uint32_t* upload_index(const std::vector<int64_t>& input_to_csc);

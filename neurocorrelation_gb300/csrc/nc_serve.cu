@@ -119,13 +119,13 @@ constexpr int kGroupsPerNet = 16;
 constexpr int64_t kBuiltHostCap = 8ll << 30;
 // host bytes of a prepared request's tables (CSC, CSR, weights, maps)
 int64_t host_bytes(const nc::NetHost& h) { return h.s * 64 + (int64_t)h.n * 64; }
-// per in-synapse position: w x | t_arr inh out_* last_arr (event form) or key state and a
+// per in-synapse position: w x | t_arr inh out last_arr (event form) or key state and a
 // quad's row and window bytes (dense)
-constexpr double kSynBytesEvent = 4 + 4 + 4 + 0.125 + 4 + 4 + 2 + 4 + 4;
+constexpr double kSynBytesEvent = 4 + 4 + 4 + 0.125 + 16 + 4;
 constexpr double kSynBytesDense = 4 + 4 + 4 + 4 + 0.5;
-// state, row starts, bitsets, tiles | fired list, out-row and ring starts (event form)
+// state, row starts, bitsets, tiles | out-row and ring starts (event form)
 constexpr double kNeuronBytesDense = 4 * 7 + 8 + 0.75 + 1;
-constexpr double kNeuronBytesEvent = 4 * 6 + 8 + 0.75 + 0.25 + 16 + 12;
+constexpr double kNeuronBytesEvent = 4 * 6 + 8 + 0.75 + 0.25 + 12;
 
 }  // namespace
 
@@ -260,10 +260,7 @@ int nc_server::init(std::string& err)
         S_AL(P.t_arr, int32_t, syn_cap);
         S_AL(P.out_ptr, int64_t, ptr_cap);
         S_AL(P.ring_off, int32_t, ptr_cap);
-        S_AL(P.out_post, int32_t, syn_cap);
-        S_AL(P.out_csc, int32_t, syn_cap);
-        S_AL(P.out_delay, int16_t, syn_cap);
-        S_AL(P.out_ringpos, uint32_t, syn_cap);
+        S_AL(P.out, NcOut, syn_cap);
         S_AL(P.last_arr, int32_t, syn_cap);
         S_AL(P.ring, uint32_t, ring_cap);
     }
@@ -271,14 +268,10 @@ int nc_server::init(std::string& err)
     S_AL(P.fired, uint32_t, 2 * word_cap);
     S_AL(P.forced, uint32_t, 2 * word_cap);
     S_AL(P.ufire, uint32_t, 2 * word_cap);
-    P.fired_cap = dense ? 0 : neuron_cap;
-    if (!dense) S_AL(P.fired_list, int2, 2 * neuron_cap);
-    S_AL(P.fired_count, int32_t, 2);
     S_AL(P.tables, float, table_cap);
     S_AL(P.groups, NcGroupDev, (int64_t)nets * kGroupsPerNet);
     S_AL(P.nets, NcNetDesc, nets);
     if (!dense) S_AL(P.tiles, NcTile, tile_cap);
-    S_AL(P.tick, int32_t, 1);
     S_AL(P.done_ctr, uint32_t, 1);
     S_AL(P.dev_err, uint32_t, 1);
     S_AL(d_stats, unsigned long long, 4 * (int64_t)nets);
@@ -287,6 +280,8 @@ int nc_server::init(std::string& err)
     P.n_nets = nets;
     P.n_tiles = 0;
     P.n_tiles_dev = d_ntiles;
+    P.warp_rows = 32;
+    P.launch_rows = 8;
     a_neuron.reset(neuron_cap);
     a_ptr.reset(ptr_cap);
     a_word.reset(word_cap);
@@ -294,9 +289,9 @@ int nc_server::init(std::string& err)
     a_ring.reset(ring_cap);
     a_table.reset(table_cap);
     for (int32_t q = nets - 1; q >= 0; --q) free_slots.push_back(q);
-    if (!dense) L.neuron_block = 256;
-    L.launch_block = 256;
-    L.launch_blocks = std::max(1, sms * NC_LAUNCH_MIN_BLOCKS);
+    if (!dense) L.neuron_block = NC_EVENT_BLOCK;
+    L.launch_block = 128;
+    L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
     S_CK(cudaStreamSynchronize(stream));
     return capture(err);
 }
@@ -453,6 +448,7 @@ int nc_server::admit(Resident& r, std::string& err)
     // upload: the same per-network layout as the static engine, state reset
     std::vector<float> pot((size_t)h.n, -70.0f);
     std::vector<int32_t> never_n((size_t)h.n, NC_NEVER), never_s(dense ? 0 : (size_t)h.sp, NC_NEVER);
+    std::vector<NcOut> out;
     const int64_t wide = dense && h.wide ? r.syn_len / 2 : 0;
     std::vector<int64_t> inp(h.in_ptr), outp(h.out_ptr);
     for (auto& v : inp) v += sb;
@@ -483,10 +479,8 @@ int nc_server::admit(Resident& r, std::string& err)
         S_CK(put(P.out_ptr, outp, pb, stream));
         S_CK(put(P.ring_off, h.ring_off, pb, stream));
         S_CK(put(P.last_arr, never_s, sb, stream));
-        S_CK(put(P.out_post, h.out_post, sb, stream));
-        S_CK(put(P.out_csc, h.out_csc, sb, stream));
-        S_CK(put(P.out_delay, h.out_delay, sb, stream));
-        S_CK(put(P.out_ringpos, h.out_ringpos, sb, stream));
+        out = nc::out_records(h);
+        S_CK(put(P.out, out, sb, stream));
         S_CK(cudaMemsetAsync(P.ring + rb, 0, sizeof(uint32_t) * r.ring_len, stream));
     }
     for (int par = 0; par < 2; ++par) {
