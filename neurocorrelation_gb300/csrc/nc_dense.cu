@@ -132,12 +132,83 @@ __device__ __forceinline__ void async4(uint32_t dst, const void* src)
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory"); }
 
+// *p where `in` is not zero, -0.0 elsewhere: a predicated load, so that nothing waits for the
+// value before it is used.
+__device__ __forceinline__ float load_or_absent(const float* p, uint32_t in)
+{
+    float v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f80000000;\n\t@q ld.global.f32 %0, [%1];\n\t}"
+                 : "=f"(v)
+                 : "l"(p), "r"(in));
+    return v;
+}
+
+// The window bits of one row, taken eight at a time.  nib: the tile's window bits, four to a
+// byte; q0, nq: the row's quads; x0: the tile's captured charges.  Eight bytes are packed to a
+// word of 32 synapses; a batch looks at the 32 from the first bit left on, across words.
+struct WindowBits {
+    const unsigned long long* words;
+    const float* x;        // charge of the first bit of `cur`
+    uint32_t cur, nxt;
+    int from;              // first bit left, 0..31
+    int w, nw;             // next word to read, words
+    uint32_t last;
+    __device__ __forceinline__ uint32_t word()
+    {
+        uint32_t v = 0u;
+        if (w < nw) {
+            const unsigned long long b = words[w++];
+            const uint32_t lo = (uint32_t)b, hi = (uint32_t)(b >> 32);
+            v = __byte_perm(lo | lo >> 4, hi | hi >> 4, 0x6420);
+            if (w == nw) v &= last;
+        }
+        return v;
+    }
+    __device__ __forceinline__ WindowBits(const uint8_t* nib, int q0, int nq, const float* x0)
+    {
+        const int skip = (int)((uintptr_t)(nib + q0) & 7);  // quads of the first word before the row
+        words = (const unsigned long long*)(nib + q0 - skip);
+        x = x0 + 4 * (int64_t)(q0 - skip);
+        w = 0;
+        nw = (skip + nq + 7) >> 3;
+        last = ((skip + nq) & 7) ? (1u << (4 * ((skip + nq) & 7))) - 1u : ~0u;
+        from = 0;
+        cur = word() & (~0u << (4 * skip));
+        nxt = word();
+    }
+    // The charges of the next eight bits, absent ones as -0.0; whether there are any.  (All
+    // branches come first, so that the rest runs between the terms of a sum.)
+    __device__ __forceinline__ bool next(float (&to)[8])
+    {
+        uint32_t m;
+        while (true) {
+            m = from < 32 ? __funnelshift_r(cur, nxt, from) : 0u;
+            if (m != 0u || !(nxt | (uint32_t)(w < nw))) break;
+            if (from >= 32) from -= 32;
+            cur = nxt;
+            nxt = word();
+            x += 32;
+        }
+        const bool any = m != 0u;
+        const float* xm = x + from;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            to[k] = load_or_absent(xm + __ffs((int)m) - 1, m);
+            m &= m - 1u;
+        }
+        from += m ? __ffs((int)m) - 1 : 32;
+        return any;
+    }
+};
+
 // charge_insynapses (src/NeuCor.cpp:688-700) of one row: the terms of the spikes that
-// arrived t-1 .. t-KC, in ascending source id, folded into pot.  nib: the tile's window
-// bits, four to a byte; q0, nq: the row's quads; x0: the tile's captured charges.  The bits
-// are read eight quads at a time and streamed in batches of 8 terms across word
-// boundaries, so that a warp's batch count is its busiest lane's, not a sum of per-word
-// maxima.
+// arrived t-1 .. t-KC, in ascending source id, folded into pot.  The bits are streamed in
+// batches of 8 terms across word boundaries, so that a warp's batch count is its busiest
+// lane's, not a sum of per-word maxima.  A batch takes some 1,100 cycles, a gather from L2 and a
+// serial sum; with the bits of 64-bit words taken one by one, and a branch at each for the next
+// word, it took 2,500, and 20k x 100 with inhibitory synapses 25.8 us a step (21.7 now).  A
+// batch gathered ahead of the sum gains half a microsecond where sums are long and costs 2 to
+// 5% where they stop early (more registers, and charges that are not needed).
 //
 // When no term of the net can be negative (nonneg_terms), the running sum only grows
 // (each `float += double` rounds a larger value, and rounding keeps the order), and so
@@ -149,33 +220,13 @@ __device__ __forceinline__ float fold_row(const uint8_t* nib, int q0, int nq, co
                                           const TermFactor& F, bool stop)
 {
     if (nq <= 0) return pot;
-    const int skip = (int)((uintptr_t)(nib + q0) & 7);  // quads of the first word before the row
-    const unsigned long long* words = (const unsigned long long*)(nib + q0 - skip);
-    const int nw = (skip + nq + 7) >> 3;
-    const unsigned long long last = ((skip + nq) & 7) ? (1ull << (8 * ((skip + nq) & 7))) - 1ull : ~0ull;
-    const float* x = x0 + 4 * (int64_t)(q0 - skip);
-    unsigned long long m = words[0] & (~0ull << (8 * skip));
-    if (nw == 1) m &= last;
-    int w = 0;
-    while (true) {
-        float xv[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            // on to the next word when this one is spent (an empty word costs a slot)
-            if (m == 0ull && w + 1 < nw) {
-                ++w;
-                m = words[w];
-                if (w + 1 == nw) m &= last;
-            }
-            const int p = __ffsll((long long)m) - 1;
-            xv[k] = -0.0f;
-            if (m) xv[k] = x[w * 32 + ((p >> 1) & ~3) + (p & 3)];
-            m &= m - 1ull;
-        }
+    WindowBits at(nib, q0, nq, x0);
+    float xv[8];
+    while (at.next(xv)) {
         pot = fold_terms(pot, xv, F);
-        if (m == 0ull && w + 1 >= nw) return pot;
-        if (stop && fires_at(pot, leak)) return pot;
+        if (stop && fires_at(pot, leak)) break;
     }
+    return pot;
 }
 
 // What a net's quads share.
@@ -630,6 +681,7 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh)
         // whatever its sum is, and it cannot cross the threshold; with no negative term a
         // neuron already over the threshold fires whatever its sum
         const bool can = lf == NC_NEVER || t - lf >= kc;
+        const TermFactor F = term_factor(D);
         const bool need = live && can && !(stop && fires_at(pot, leak));
         bar_sync<kBarFull>(b);
         if (at.ti < 0) {  // the block's last tile: all its warps have read the step counters
@@ -637,7 +689,7 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh)
             if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
         }
         const uint8_t* nib = tile.nq <= kNibCap ? sh.nib[b] : P.nib + tile.q0;
-        if (need) pot = fold_row(nib, q0, nq, P.x + 4 * (int64_t)tile.q0, pot, leak, term_factor(D), stop);
+        if (need) pot = fold_row(nib, q0, nq, P.x + 4 * (int64_t)tile.q0, pot, leak, F, stop);
         __syncwarp();
         if (ahead.ti >= 0) {
             give_rows(P, sh, ahead.ti, b, lane);
