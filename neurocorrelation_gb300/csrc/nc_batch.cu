@@ -78,7 +78,7 @@ int nc_batch_create(int32_t n_nets, const nc_net_spec* specs, nc_batch** out)
             if (sp.params.step_mode == NC_STEP_DENSE || sp.params.step_mode == NC_STEP_EVENT)
                 sp.params.step_mode = specs[0].params.step_mode;
             int rc = nc::build_net(sp.n_neurons, sp.xyz, sp.n_synapses, sp.syn_from, sp.syn_to, sp.syn_weight,
-                                   sp.syn_length, sp.syn_inhibitory, sp.params, b->hosts[(size_t)q], errs[(size_t)q]);
+                                   sp.syn_length, sp.syn_inhibitory, sp.params, b->hosts[(size_t)q], errs[(size_t)q], true);
             if (rc == NC_OK) rc = nc::set_groups(b->hosts[(size_t)q], sp.n_groups, sp.groups, errs[(size_t)q]);
             if (rc == NC_OK && sp.horizon < 0) {
                 rc = NC_ERR_INVALID;

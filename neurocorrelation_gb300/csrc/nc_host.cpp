@@ -4,9 +4,11 @@
 #include "nc_host.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <thread>
 
 namespace nc {
@@ -160,9 +162,87 @@ KnnGrid knn_grid(int32_t n, int32_t k, float density)
     return G;
 }
 
+// The synapses, as indexes into the input, by target slot and in each target's row by the
+// caller's source id, repeats in input order: two counting sorts, the first left out where
+// the input is in source order already (a kNN network's is).  start: n + 1 row starts.
+template <class Index>
+static std::unique_ptr<Index[]> rows_of_targets(const NetHost& h, int64_t n_syn, const int32_t* from, const int32_t* to,
+                                                bool by_source, const std::vector<int64_t>& start)
+{
+    std::unique_ptr<Index[]> first, order(new Index[(size_t)n_syn]);
+    if (!by_source) {
+        std::vector<int64_t> at((size_t)h.n + 1, 0);
+        for (int64_t k = 0; k < n_syn; ++k) at[(size_t)from[k] + 1]++;
+        for (int32_t i = 0; i < h.n; ++i) at[(size_t)i + 1] += at[(size_t)i];
+        first.reset(new Index[(size_t)n_syn]);
+        for (int64_t k = 0; k < n_syn; ++k) first[(size_t)at[(size_t)from[k]]++] = (Index)k;
+    }
+    std::vector<int64_t> at(start.begin(), start.end() - 1);
+    for (int64_t q = 0; q < n_syn; ++q) {
+        const int64_t k = by_source ? q : (int64_t)first[(size_t)q];
+        order[(size_t)at[(size_t)h.slot_of[(size_t)to[k]]]++] = (Index)k;
+    }
+    return order;
+}
+
+// The in-synapse rows (CSC): the first of repeated (source, target) pairs is kept
+// (createSynapse, src/NeuCor.cpp:189-191).  above: delay and same-step order flags of every
+// position, as in the upper part of a key; row_end: end of each row's synapses.
+template <class Index>
+static int fill_rows(NetHost& h, const Index* order, const std::vector<int64_t>& start, const int32_t* from,
+                     const float* weight, const float* length, std::vector<uint32_t>& above,
+                     std::vector<int64_t>& row_end, std::string& err)
+{
+    const int32_t n = h.n, pad = pad_slot(n);
+    int64_t size = 0;  // were no pair repeated
+    for (int32_t j = 0; j < n; ++j)
+        size = (size + start[(size_t)j + 1] - start[(size_t)j] + row_align(j) - 1) / row_align(j) * row_align(j);
+    h.csc_pre.resize((size_t)size);
+    h.w.resize((size_t)size);
+    above.resize((size_t)size);
+    int32_t* pre = h.csc_pre.data();
+    float* w = h.w.data();
+    int64_t c = 0;
+    for (int32_t j = 0; j < n; ++j) {
+        h.in_ptr[(size_t)j] = c;
+        const int32_t dst = h.orig_id[(size_t)j];
+        const float* at = &h.xyz[3 * (size_t)dst];
+        int32_t last_pre = -1;
+        for (int64_t q = start[(size_t)j]; q < start[(size_t)j + 1]; ++q) {
+            const int64_t k = (int64_t)order[q];
+            const int32_t src = from[k];
+            if (src == last_pre) continue;
+            last_pre = src;
+            h.input_to_csc[(size_t)k] = c;
+            pre[c] = h.slot_of[(size_t)src];
+            const float len = length ? length[k] : get_dist(&h.xyz[3 * (size_t)src], at);
+            const int32_t d = delay_steps(len, h.dt);
+            if (d < 0 || d > kMaxDelay) { err = "synapse delay exceeds 16383 steps"; return NC_ERR_INVALID; }
+            h.max_delay = std::max(h.max_delay, d);
+            // the same-step order rules compare the caller's ids of target and source
+            above[(size_t)c] = (uint32_t)d << NC_KEY_DELAY_SHIFT | (dst > src ? NC_KEY_AFTER : 0u) |
+                               (dst < src ? NC_KEY_BEFORE : 0u);
+            w[c++] = weight[k];
+        }
+        row_end[(size_t)j] = c;
+        h.s += c - h.in_ptr[(size_t)j];
+        for (; c & (row_align(j) - 1); ++c) {
+            pre[c] = pad;
+            above[(size_t)c] = 0u;
+            w[c] = 0.0f;
+        }
+    }
+    h.in_ptr[(size_t)n] = c;
+    h.sp = c;
+    h.csc_pre.resize((size_t)c);
+    h.w.resize((size_t)c);
+    above.resize((size_t)c);
+    return NC_OK;
+}
+
 int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, const int32_t* to,
               const float* weight, const float* length, const uint8_t* inhibitory, const nc_params& p,
-              NetHost& h, std::string& err)
+              NetHost& h, std::string& err, bool rows_only)
 {
     if (p.inhibitory_rule != NC_INHIBITORY_COPY_LOSS && p.inhibitory_rule != NC_INHIBITORY_SIGN) {
         err = "unknown inhibitory rule";
@@ -178,7 +258,10 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
         err = "trace decays must lie in (0, 1)";
         return NC_ERR_INVALID;
     }
+    bool by_source = true, negative = false;
     for (int64_t k = 0; k < n_syn; ++k) {
+        by_source = by_source && (k == 0 || from[k - 1] <= from[k]);
+        negative = negative || weight[k] < 0.0f;
         if (from[k] < 0 || from[k] >= n || to[k] < 0 || to[k] >= n) { err = "synapse endpoint out of range"; return NC_ERR_INVALID; }
         if (std::isnan(weight[k])) { err = "NaN weight"; return NC_ERR_INVALID; }
     }
@@ -209,51 +292,21 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
     }
     storage_order(h, xyz, p.storage_order);
 
-    // CSC: bucket by target slot in input order, sort each bucket by the caller's source
-    // id (stable), keep the first of repeated (source, target) pairs (createSynapse,
-    // src/NeuCor.cpp:189-191)
-    std::vector<int64_t> bstart((size_t)n + 1, 0);
-    for (int64_t k = 0; k < n_syn; ++k) bstart[(size_t)h.slot_of[(size_t)to[k]] + 1]++;
-    for (int32_t j = 0; j < n; ++j) bstart[j + 1] += bstart[j];
-    std::vector<int64_t> order((size_t)n_syn);
-    {
-        std::vector<int64_t> fill(bstart.begin(), bstart.end() - 1);
-        for (int64_t k = 0; k < n_syn; ++k) order[(size_t)fill[h.slot_of[(size_t)to[k]]]++] = k;
-    }
+    std::vector<int64_t> start((size_t)n + 1, 0), row_end((size_t)n, 0);
+    for (int64_t k = 0; k < n_syn; ++k) start[(size_t)h.slot_of[(size_t)to[k]] + 1]++;
+    for (int32_t j = 0; j < n; ++j) start[(size_t)j + 1] += start[(size_t)j];
     h.input_to_csc.assign((size_t)n_syn, -1);
     h.in_ptr.assign((size_t)n + 1, 0);
-    h.csc_pre.reserve((size_t)n_syn);
-    h.csc_delay.reserve((size_t)n_syn);
-    h.w.reserve((size_t)n_syn);
-    std::vector<int64_t> row_end((size_t)n, 0);
-    for (int32_t j = 0; j < n; ++j) {
-        auto b = order.begin() + bstart[j], e = order.begin() + bstart[j + 1];
-        std::stable_sort(b, e, [&](int64_t x, int64_t y) { return from[x] < from[y]; });
-        int32_t last_pre = -1;
-        for (auto it = b; it != e; ++it) {
-            const int64_t k = *it;
-            if (from[k] == last_pre) continue;
-            last_pre = from[k];
-            const int64_t c = (int64_t)h.csc_pre.size();
-            h.input_to_csc[(size_t)k] = c;
-            h.csc_pre.push_back(h.slot_of[(size_t)from[k]]);
-            const float len = length ? length[k] : get_dist(&h.xyz[3 * (size_t)from[k]], &h.xyz[3 * (size_t)to[k]]);
-            const int32_t d = delay_steps(len, h.dt);
-            if (d < 0 || d > kMaxDelay) { err = "synapse delay exceeds 16383 steps"; return NC_ERR_INVALID; }
-            h.csc_delay.push_back(d);
-            h.max_delay = std::max(h.max_delay, d);
-            h.w.push_back(weight[k]);
-        }
-        h.s += (int64_t)h.csc_pre.size() - h.in_ptr[j];
-        row_end[(size_t)j] = (int64_t)h.csc_pre.size();
-        while (h.csc_pre.size() & (size_t)(row_align(j) - 1)) {
-            h.csc_pre.push_back(pad_slot(n));
-            h.csc_delay.push_back(0);
-            h.w.push_back(0.0f);
-        }
-        h.in_ptr[j + 1] = (int64_t)h.csc_pre.size();
+    std::vector<uint32_t> above;
+    int rc = NC_OK;
+    if (n_syn < (1ll << 32)) {
+        auto order = rows_of_targets<uint32_t>(h, n_syn, from, to, by_source, start);
+        rc = fill_rows(h, order.get(), start, from, weight, length, above, row_end, err);
+    } else {
+        auto order = rows_of_targets<int64_t>(h, n_syn, from, to, by_source, start);
+        rc = fill_rows(h, order.get(), start, from, weight, length, above, row_end, err);
     }
-    h.sp = (int64_t)h.csc_pre.size();
+    if (rc != NC_OK) return rc;
     if (h.s >= (1ll << 31) || h.sp >= (1ll << 32)) { err = "too many synapses in one network"; return NC_ERR_INVALID; }
 
     // ring words per target: one bit per in-synapse
@@ -283,22 +336,51 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
     if (dense) {
         h.key.resize((size_t)(h.sp * key_words(h)));
         h.qrow.resize((size_t)(h.sp / 4));
-        for (int64_t c = 0; c < h.sp; ++c) h.key[(size_t)c] = (uint32_t)h.csc_pre[(size_t)c] << h.key_shift;
+        for (int64_t c = 0; c < h.sp; ++c)
+            h.key[(size_t)c] = (uint32_t)h.csc_pre[(size_t)c] << h.key_shift | (h.wide ? 0u : above[(size_t)c]);
+        if (h.wide) std::copy(above.begin(), above.end(), h.key.begin() + (size_t)h.sp);
         for (int32_t j = 0; j < n; ++j)
             for (int64_t q = h.in_ptr[j] / 4; q < h.in_ptr[j + 1] / 4; ++q) h.qrow[(size_t)q] = (uint8_t)(j & 31);
     }
 
-    // CSR: each source's out-synapses in creation order (Neuron::outSynapses)
-    h.out_ptr.assign((size_t)n + 1, 0);
-    for (int32_t j = 0; j < n; ++j)
-        for (int64_t c = h.in_ptr[j]; c < row_end[(size_t)j]; ++c) h.out_ptr[(size_t)h.csc_pre[c] + 1]++;
-    for (int32_t i = 0; i < n; ++i) h.out_ptr[i + 1] += h.out_ptr[i];
-    h.out_post.assign((size_t)h.s, 0);
-    h.out_csc.assign((size_t)h.s, 0);
-    h.out_delay.assign((size_t)h.s, 0);
+    // Synapse::inhibitory: setWeight's sign (src/NeuCor.cpp:576-579), lost by synapses
+    // the vector growth copied (rule COPY_LOSS), or the caller's own flags
+    h.inh_bits.assign((size_t)((h.sp + 31) / 32), 0u);
+    if (negative) {
+        // each source's synapses in creation order (Neuron::outSynapses)
+        std::vector<int64_t> size((size_t)n, 0), made((size_t)n, 0);
+        for (int64_t k = 0; k < n_syn; ++k) size[(size_t)from[k]] += h.input_to_csc[(size_t)k] >= 0 ? 1 : 0;
+        for (int64_t k = 0; k < n_syn; ++k) {
+            const int64_t c = h.input_to_csc[(size_t)k];
+            if (c < 0) continue;
+            const int64_t m = made[(size_t)from[k]]++;
+            if (!(weight[k] < 0.0f)) continue;
+            if (p.inhibitory_rule == NC_INHIBITORY_COPY_LOSS && grown_copy(m, size[(size_t)from[k]])) continue;
+            h.inh_bits[(size_t)(c >> 5)] |= 1u << (c & 31);
+        }
+    }
+    if (inhibitory) {
+        for (int64_t k = 0; k < n_syn; ++k) {
+            const int64_t c = h.input_to_csc[(size_t)k];
+            if (c < 0) continue;
+            if (inhibitory[k]) h.inh_bits[(size_t)(c >> 5)] |= 1u << (c & 31);
+            else h.inh_bits[(size_t)(c >> 5)] &= ~(1u << (c & 31));
+        }
+    }
+
+    // CSR: each source's out-synapses in creation order
     const bool event = p.step_mode != NC_STEP_DENSE;
-    if (event) h.out_ringpos.assign((size_t)h.s, 0);
-    {
+    if (event || !rows_only) {
+        h.csc_delay.resize((size_t)h.sp);
+        for (int64_t c = 0; c < h.sp; ++c) h.csc_delay[(size_t)c] = (int32_t)(above[(size_t)c] >> NC_KEY_DELAY_SHIFT);
+        h.out_ptr.assign((size_t)n + 1, 0);
+        for (int32_t j = 0; j < n; ++j)
+            for (int64_t c = h.in_ptr[j]; c < row_end[(size_t)j]; ++c) h.out_ptr[(size_t)h.csc_pre[c] + 1]++;
+        for (int32_t i = 0; i < n; ++i) h.out_ptr[i + 1] += h.out_ptr[i];
+        h.out_post.assign((size_t)h.s, 0);
+        h.out_csc.assign((size_t)h.s, 0);
+        h.out_delay.assign((size_t)h.s, 0);
+        if (event) h.out_ringpos.assign((size_t)h.s, 0);
         std::vector<int64_t> fill(h.out_ptr.begin(), h.out_ptr.end() - 1);
         for (int64_t k = 0; k < n_syn; ++k) {
             const int64_t c = h.input_to_csc[(size_t)k];
@@ -308,38 +390,10 @@ int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, c
             const int64_t b = c - h.in_ptr[j];
             h.out_post[(size_t)q] = j;
             h.out_csc[(size_t)q] = (int32_t)(uint32_t)c;
-            // the same-step order rules compare the caller's ids of target and source
             const uint32_t flags = (to[k] > from[k] ? 1u << kAfterBit : 0u) | (to[k] < from[k] ? 1u << kBeforeBit : 0u);
             h.out_delay[(size_t)q] = (int16_t)(uint16_t)((uint32_t)h.csc_delay[(size_t)c] | flags);
-            if (dense) {
-                const uint32_t hi = (uint32_t)h.csc_delay[(size_t)c] << NC_KEY_DELAY_SHIFT |
-                                    (to[k] > from[k] ? NC_KEY_AFTER : 0u) | (to[k] < from[k] ? NC_KEY_BEFORE : 0u);
-                if (h.wide) h.key[(size_t)(h.sp + c)] = hi;
-                else h.key[(size_t)c] |= hi;
-            }
             if (!event) continue;
             h.out_ringpos[(size_t)q] = ((uint32_t)(h.ring_off[j] + (int32_t)(b >> 5)) << 5) | (uint32_t)(b & 31);
-        }
-    }
-
-    // Synapse::inhibitory: setWeight's sign (src/NeuCor.cpp:576-579), lost by synapses
-    // the vector growth copied (rule COPY_LOSS), or the caller's own flags
-    h.inh_bits.assign((size_t)((h.sp + 31) / 32), 0u);
-    for (int32_t i = 0; i < n; ++i) {
-        const int64_t size = h.out_ptr[i + 1] - h.out_ptr[i];
-        for (int64_t m = 0; m < size; ++m) {
-            const int64_t c = (uint32_t)h.out_csc[(size_t)(h.out_ptr[i] + m)];
-            bool inh = h.w[(size_t)c] < 0.0f;
-            if (p.inhibitory_rule == NC_INHIBITORY_COPY_LOSS && grown_copy(m, size)) inh = false;
-            if (inh) h.inh_bits[(size_t)(c >> 5)] |= 1u << (c & 31);
-        }
-    }
-    if (inhibitory) {
-        for (int64_t k = 0; k < n_syn; ++k) {
-            const int64_t c = h.input_to_csc[(size_t)k];
-            if (c < 0) continue;
-            if (inhibitory[k]) h.inh_bits[(size_t)(c >> 5)] |= 1u << (c & 31);
-            else h.inh_bits[(size_t)(c >> 5)] &= ~(1u << (c & 31));
         }
     }
 
@@ -441,19 +495,6 @@ int set_groups(NetHost& h, int32_t n_groups, const nc_group* groups, std::string
 }  // namespace nc
 
 // ------------------------------------------------------------------ C ABI
-namespace {
-thread_local std::string g_build_err;
-using nc::kStreamPosition;
-using nc::kStreamWeight;
-using nc::unit24;
-
-struct Cand {
-    float d;
-    int32_t j;
-    bool operator<(const Cand& o) const { return d < o.d || (d == o.d && j < o.j); }
-};
-}  // namespace
-
 extern "C" int nc_philox4x32_10(const uint32_t ctr[4], const uint32_t key[2], uint32_t out[4])
 {
     if (!ctr || !key || !out) return NC_ERR_INVALID;
@@ -461,14 +502,16 @@ extern "C" int nc_philox4x32_10(const uint32_t ctr[4], const uint32_t key[2], ui
     return NC_OK;
 }
 
-extern "C" int nc_build_knn(int32_t n, int32_t k, float density, uint64_t seed, float* xyz, int32_t* syn_from,
-                            int32_t* syn_to, float* syn_weight)
+namespace nc {
+
+int build_knn(int32_t n, int32_t k, float density, uint64_t seed, int32_t threads, float* xyz, int32_t* syn_from,
+              int32_t* syn_to, float* syn_weight)
 {
     if (n < 0 || k < 0 || !(density > 0.0f) || !xyz || ((int64_t)n * k > 0 && (!syn_from || !syn_to || !syn_weight)))
         return NC_ERR_INVALID;
     if (n > 0 && k >= n) return NC_ERR_INVALID;
     const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-    const nc::KnnGrid grid = nc::knn_grid(n, k, density);
+    const KnnGrid grid = knn_grid(n, k, density);
     const float side = grid.side;
     for (int32_t i = 0; i < n; ++i) {
         uint32_t o[4];
@@ -489,64 +532,99 @@ extern "C" int nc_build_knn(int32_t n, int32_t k, float density, uint64_t seed, 
         cstart[(size_t)c + 1]++;
     }
     for (size_t c = 0; c + 1 < cstart.size(); ++c) cstart[c + 1] += cstart[c];
-    std::vector<int32_t> members((size_t)n);
+    // the points by cell, with their positions: a run of cells along z is a run of memory
+    struct Point {
+        float p[3];
+        int32_t id;
+    };
+    std::vector<Point> points((size_t)n);
     {
         std::vector<int32_t> fill(cstart.begin(), cstart.end() - 1);
-        for (int32_t i = 0; i < n; ++i) members[(size_t)fill[cell[i]]++] = i;
+        for (int32_t i = 0; i < n; ++i) {
+            const float* p = &xyz[3 * (size_t)i];
+            points[(size_t)fill[(size_t)cell[(size_t)i]]++] = Point{{p[0], p[1], p[2]}, i};
+        }
     }
+    // Shells of cells of growing Chebyshev radius r.  Once k candidates are known, only points
+    // up to the k-th distance so far (`far`) can be among the k nearest.  A candidate is its
+    // distance's bits, which order as the distance does, above its id.
     auto worker = [&](int32_t lo, int32_t hi) {
-        std::vector<Cand> cand;
+        std::vector<uint64_t> cand;
         for (int32_t i = lo; i < hi; ++i) {
             const float* pi = &xyz[3 * (size_t)i];
             const int32_t cx = cell_of(pi[0]), cy = cell_of(pi[1]), cz = cell_of(pi[2]);
             cand.clear();
-            for (int32_t r = 0;; ++r) {
-                for (int32_t x = cx - r; x <= cx + r; ++x) {
-                    if (x < 0 || x >= g) continue;
-                    for (int32_t y = cy - r; y <= cy + r; ++y) {
-                        if (y < 0 || y >= g) continue;
-                        for (int32_t z = cz - r; z <= cz + r; ++z) {
-                            if (z < 0 || z >= g) continue;
-                            if (std::max(std::abs(x - cx), std::max(std::abs(y - cy), std::abs(z - cz))) != r) continue;
-                            const int32_t c = (x * g + y) * g + z;
-                            for (int32_t q = cstart[c]; q < cstart[(size_t)c + 1]; ++q) {
-                                const int32_t j = members[(size_t)q];
-                                if (j == i) continue;
-                                cand.push_back(Cand{nc::get_dist(pi, &xyz[3 * (size_t)j]), j});
-                            }
-                        }
-                    }
+            float far2 = INFINITY;  // no less than the square of any distance up to `far`
+            auto visit = [&](int32_t x, int32_t y, int32_t z0, int32_t z1) {
+                const size_t row = ((size_t)x * g + y) * g;
+                for (int32_t q = cstart[row + z0], e = cstart[row + z1 + 1]; q < e; ++q) {
+                    const Point& pt = points[(size_t)q];
+                    const float dx = pi[0] - pt.p[0], dy = pi[1] - pt.p[1], dz = pi[2] - pt.p[2];
+                    if (dx * dx + dy * dy + dz * dz > far2 || pt.id == i) continue;
+                    const float d = get_dist(pi, pt.p);
+                    uint32_t bits;
+                    std::memcpy(&bits, &d, sizeof(bits));
+                    cand.push_back((uint64_t)bits << 32 | (uint32_t)pt.id);
                 }
+            };
+            for (int32_t r = 0;; ++r) {
+                const int32_t z0 = std::max(0, cz - r), z1 = std::min(g - 1, cz + r);
+                for (int32_t x = std::max(0, cx - r); x <= std::min(g - 1, cx + r); ++x)
+                    for (int32_t y = std::max(0, cy - r); y <= std::min(g - 1, cy + r); ++y) {
+                        if (std::max(std::abs(x - cx), std::abs(y - cy)) == r) {
+                            visit(x, y, z0, z1);
+                            continue;
+                        }
+                        if (cz - r >= 0) visit(x, y, cz - r, cz - r);
+                        if (cz + r < g) visit(x, y, cz + r, cz + r);
+                    }
                 const bool all = r >= g;
                 if ((int32_t)cand.size() >= k) {
                     // every unvisited point is at least r*h away
                     std::nth_element(cand.begin(), cand.begin() + (k - 1), cand.end());
-                    if (all || cand[(size_t)k - 1].d < (float)r * h) break;
+                    const uint32_t bits = (uint32_t)(cand[(size_t)k - 1] >> 32);
+                    float far;
+                    std::memcpy(&far, &bits, sizeof(far));
+                    if (all || far < (float)r * h) break;
+                    far2 = far * far * (1.0f + 0x1p-20f) + 0x1p-100f;
+                    cand.resize((size_t)k);  // those beyond stay beyond
                 } else if (all) {
                     break;
                 }
             }
-            std::partial_sort(cand.begin(), cand.begin() + k, cand.end());
+            std::sort(cand.begin(), cand.begin() + k);  // the k nearest, by distance and id
+            uint32_t o[4] = {0u, 0u, 0u, 0u};
             for (int32_t m = 0; m < k; ++m) {
                 const size_t q = (size_t)i * k + m;
                 syn_from[q] = i;
-                syn_to[q] = cand[(size_t)m].j;
-                uint32_t o[4];
-                nc_philox((uint32_t)i, (uint32_t)(m >> 2), kStreamWeight, 0u, k0, k1, o);
+                syn_to[q] = (int32_t)(uint32_t)cand[(size_t)m];
+                if ((m & 3) == 0) nc_philox((uint32_t)i, (uint32_t)(m >> 2), kStreamWeight, 0u, k0, k1, o);
                 syn_weight[q] = unit24(o[m & 3]);
             }
         }
     };
-    const int32_t threads = (int32_t)std::max(1u, std::min(64u, std::thread::hardware_concurrency()));
+    // chunks of points, taken in turn (a chunk is some milliseconds' worth at most)
+    constexpr int32_t kChunk = 128;
+    threads = std::max(1, std::min(std::min(threads, 64), (n + kChunk - 1) / kChunk));
+    std::atomic<int32_t> next{0};
+    auto chunks = [&] {
+        for (int64_t lo = (int64_t)kChunk * next++; lo < n; lo = (int64_t)kChunk * next++)
+            worker((int32_t)lo, (int32_t)std::min<int64_t>(n, lo + kChunk));
+    };
     std::vector<std::thread> pool;
-    const int32_t chunk = (n + threads - 1) / threads;
-    for (int32_t tb = 0; tb < threads; ++tb) {
-        const int32_t lo = tb * chunk, hi = std::min(n, lo + chunk);
-        if (lo >= hi) break;
-        pool.emplace_back(worker, lo, hi);
-    }
+    for (int32_t t = 1; t < threads; ++t) pool.emplace_back(chunks);
+    chunks();
     for (auto& th : pool) th.join();
     return NC_OK;
+}
+
+}  // namespace nc
+
+extern "C" int nc_build_knn(int32_t n, int32_t k, float density, uint64_t seed, float* xyz, int32_t* syn_from,
+                            int32_t* syn_to, float* syn_weight)
+{
+    return nc::build_knn(n, k, density, seed, (int32_t)std::max(1u, std::thread::hardware_concurrency()), xyz, syn_from,
+                         syn_to, syn_weight);
 }
 
 namespace {

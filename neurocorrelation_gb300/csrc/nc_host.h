@@ -88,10 +88,11 @@ void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTil
                std::vector<int32_t>& start);
 // The net's out-synapse records (event form).
 std::vector<NcOut> out_records(const NetHost& h);
-// Builds the layout; returns NC_OK or an NC_ERR_* code with `err` set.
+// Builds the layout; returns NC_OK or an NC_ERR_* code with `err` set.  rows_only: without the
+// out-synapses (csc_delay, out_*) where the form of the step does not need them.
 int build_net(int32_t n, const float* xyz, int64_t n_syn, const int32_t* from, const int32_t* to,
               const float* weight, const float* length, const uint8_t* inhibitory, const nc_params& p,
-              NetHost& out, std::string& err);
+              NetHost& out, std::string& err, bool rows_only = false);
 bool inhibitory_flag(const NetHost& h, int64_t csc);
 int set_groups(NetHost& net, int32_t n_groups, const nc_group* groups, std::string& err);
 
@@ -120,6 +121,9 @@ struct KnnGrid {
     float h;
 };
 KnnGrid knn_grid(int32_t n, int32_t k, float density);
+// nc_build_knn on `threads` threads.
+int build_knn(int32_t n, int32_t k, float density, uint64_t seed, int32_t threads, float* xyz, int32_t* syn_from,
+              int32_t* syn_to, float* syn_weight);
 float ap_value(float x);                              // Neuron::AP, src/NeuCor.cpp:706-714
 float step_ms(int64_t k, float dt);                   // k steps as a float time difference
 

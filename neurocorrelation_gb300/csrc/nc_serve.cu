@@ -106,6 +106,8 @@ struct Resident {
     int64_t neuron0 = -1, ptr0 = -1, word0 = -1, syn0 = -1, ring0 = -1, table0 = -1;
     int64_t syn_len = 0, ring_len = 0, table_len = 0, words = 0;
     int64_t bytes = 0;
+    // position of every given synapse (~0: an ignored duplicate), when results are kept
+    std::vector<uint32_t> index;
     int64_t steps_done = 0;
     int status = NC_OK;
     std::string err;
@@ -152,6 +154,7 @@ struct nc_server {
     int64_t next_id = 1;
     std::deque<std::unique_ptr<Request>> todo;              // awaiting a builder
     std::map<int64_t, std::unique_ptr<Resident>> built;     // prepared, awaiting admission
+    int32_t building = 0;                                   // builder threads at work
     // host memory the prepared, unadmitted requests hold; builders pause above
     // kBuiltHostCap so that a burst of submissions cannot fill the host
     int64_t built_host_bytes = 0;
@@ -163,7 +166,9 @@ struct nc_server {
     std::thread scheduler;
     std::chrono::steady_clock::time_point t0;
 
-    std::vector<std::unique_ptr<Resident>> active;  // scheduler thread only
+    // scheduler thread only: prepared requests that do not fit yet, resident networks
+    std::map<int64_t, std::unique_ptr<Resident>> waiting;
+    std::vector<std::unique_ptr<Resident>> active;
 
     double now() const
     {
@@ -174,6 +179,7 @@ struct nc_server {
     void builder_loop();
     void scheduler_loop();
     int admit(Resident& r, std::string& err);
+    int gather_weights(const Resident& r, float* out, std::string& err);
     int retire(Resident& r, std::string& err);
     int upload_tiles(std::string& err);
     int capture(std::string& err);
@@ -348,12 +354,17 @@ void nc_server::builder_loop()
 {
     for (;;) {
         std::unique_ptr<Request> rq;
+        int threads = 1;
         {
             std::unique_lock<std::mutex> lk(mu);
             cv.wait(lk, [&] { return stop || (!todo.empty() && built_host_bytes < kBuiltHostCap); });
             if (stop && todo.empty()) return;
             rq = std::move(todo.front());
             todo.pop_front();
+            // this request's share of the host's cores, or a little more: a large request
+            // last in line is what a burst waits for (12 requests of 77k-773k synapses on 16
+            // cores: 44 ms with a plain share, 38 with 4 threads at least)
+            threads = std::max(4, (int)std::thread::hardware_concurrency() / ++building);
         }
         auto r = std::make_unique<Resident>();
         r->id = rq->id;
@@ -368,8 +379,8 @@ void nc_server::builder_loop()
             rq->from.resize(m);
             rq->to.resize(m);
             rq->weight.resize(m);
-            rc = nc_build_knn(sp.n_neurons, rq->knn_k, rq->knn_density, rq->knn_seed, rq->xyz.data(), rq->from.data(),
-                              rq->to.data(), rq->weight.data());
+            rc = nc::build_knn(sp.n_neurons, rq->knn_k, rq->knn_density, rq->knn_seed, threads, rq->xyz.data(),
+                               rq->from.data(), rq->to.data(), rq->weight.data());
             if (rc != NC_OK) err = "bad kNN request";
             sp.n_synapses = (int64_t)m;
         }
@@ -381,7 +392,7 @@ void nc_server::builder_loop()
             rc = nc::build_net(sp.n_neurons, rq->xyz.empty() ? nullptr : rq->xyz.data(), sp.n_synapses,
                                rq->from.data(), rq->to.data(), rq->weight.data(),
                                rq->length.empty() ? nullptr : rq->length.data(), rq->inh.empty() ? nullptr : rq->inh.data(),
-                               sp.params, r->host, err);
+                               sp.params, r->host, err, true);
         if (rq->knn) {  // the arrays are not needed past the host layout
             std::vector<float>().swap(rq->xyz);
             std::vector<int32_t>().swap(rq->from);
@@ -405,10 +416,14 @@ void nc_server::builder_loop()
             }
             r->bytes = (int64_t)(r->syn_len * syn_bytes + h.n * neuron_bytes + r->ring_len * 4.0 + r->table_len * 4.0);
         }
+        if (cfg.keep_results) r->index.assign(r->host.input_to_csc.begin(), r->host.input_to_csc.end());
+        std::vector<int64_t>().swap(r->host.input_to_csc);
+        std::vector<int32_t>().swap(r->host.csc_pre);
         r->status = rc;
         r->err = err;
         {
             std::lock_guard<std::mutex> lk(mu);
+            --building;
             built_host_bytes += host_bytes(r->host);
             built.emplace(r->id, std::move(r));
         }
@@ -540,6 +555,26 @@ int nc_server::admit(Resident& r, std::string& err)
     return NC_OK;
 }
 
+// The final weights of a network that has run its last step, in the order they were given in,
+// gathered on the device (in the scheduler's loop on the host a random read each, some 20 ms for a dozen
+// networks of 3.7M synapses).  The network's own charges and arrival words, which nothing
+// reads any more, hold the result and the index.
+int nc_server::gather_weights(const Resident& r, float* out, std::string& err)
+{
+    uint32_t* index = (dense ? P.state : (uint32_t*)P.t_arr) + r.syn0;
+    float* part = P.x + r.syn0;
+    for (int64_t a = 0; a < (int64_t)r.index.size(); a += r.syn_len) {
+        const int64_t m = std::min(r.syn_len, (int64_t)r.index.size() - a);
+        S_CK(cudaMemcpyAsync(index, r.index.data() + a, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, stream));
+        if (nc::launch_gather(P.w + r.syn0, index, m, part, stream)) {
+            err = nc::cuda_msg("gather of weights", cudaGetLastError());
+            return NC_ERR_CUDA;
+        }
+        S_CK(cudaMemcpyAsync(out + a, part, sizeof(float) * m, cudaMemcpyDeviceToHost, stream));
+    }
+    return NC_OK;
+}
+
 int nc_server::retire(Resident& r, std::string& err)
 {
     const nc::NetHost& h = r.host;
@@ -596,42 +631,44 @@ void nc_server::scheduler_loop()
     const int G = cfg.steps_per_batch;
     for (;;) {
         std::string err;
-        // admission: prepared requests in submission order, each as soon as it fits
+        // admission: prepared requests in submission order, each as soon as it fits (uploaded
+        // without the lock, so that builders and callers go on)
         std::vector<std::unique_ptr<Resident>> rejected;
-        bool changed = false;
         {
             std::unique_lock<std::mutex> lk(mu);
-            if (active.empty())
+            if (active.empty() && waiting.empty())
                 cv.wait(lk, [&] { return stop || !built.empty(); });
             if (stop) return;  // destroy abandons resident and queued work
-            for (auto it = built.begin(); it != built.end();) {
-                Resident& r = *it->second;
-                if (r.status != NC_OK) {
-                    built_host_bytes -= host_bytes(r.host);
-                    rejected.push_back(std::move(it->second));
-                    it = built.erase(it);
-                    continue;
-                }
-                const int rc = admit(r, err);
-                if (rc == 1) {
-                    ++it;
-                    continue;
-                }
-                built_host_bytes -= host_bytes(r.host);
-                if (rc != NC_OK) {
-                    r.status = rc;
-                    r.err = err;
-                    rejected.push_back(std::move(it->second));
-                    it = built.erase(it);
-                    continue;
-                }
-                r.admit_s = now();
-                st.admitted++;
-                st.resident_bytes += r.bytes;
-                active.push_back(std::move(it->second));
-                it = built.erase(it);
-                changed = true;
+            for (auto& r : built) waiting.emplace(r.first, std::move(r.second));
+            built.clear();
+        }
+        int64_t left = 0, taken = 0, admitted = 0;  // host bytes no longer waiting, device bytes and networks admitted
+        for (auto it = waiting.begin(); it != waiting.end();) {
+            Resident& r = *it->second;
+            const int rc = r.status == NC_OK ? admit(r, err) : r.status;
+            if (r.status == NC_OK && rc == 1) {
+                ++it;
+                continue;
             }
+            left += host_bytes(r.host);
+            if (rc != NC_OK) {
+                if (r.status == NC_OK) r.err = err;
+                r.status = rc;
+                rejected.push_back(std::move(it->second));
+            } else {
+                r.admit_s = now();
+                taken += r.bytes;
+                ++admitted;
+                active.push_back(std::move(it->second));
+            }
+            it = waiting.erase(it);
+        }
+        const bool changed = admitted > 0;
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            built_host_bytes -= left;
+            st.admitted += admitted;
+            st.resident_bytes += taken;
             st.peak_resident_bytes = std::max(st.peak_resident_bytes, st.resident_bytes);
             st.peak_resident_networks = std::max<int64_t>(st.peak_resident_networks, (int64_t)active.size());
             for (auto& r : rejected) {
@@ -691,15 +728,11 @@ void nc_server::scheduler_loop()
             Kept k;
             if (cfg.keep_results) {
                 const nc::NetHost& h = r->host;
-                std::vector<float> w((size_t)h.sp), pot((size_t)h.n);
-                cudaMemcpyAsync(w.data(), P.w + r->syn0, sizeof(float) * h.sp, cudaMemcpyDeviceToHost, stream);
+                std::vector<float> pot((size_t)h.n);
                 cudaMemcpyAsync(pot.data(), P.pot + r->neuron0, sizeof(float) * h.n, cudaMemcpyDeviceToHost, stream);
-                cudaStreamSynchronize(stream);
                 k.weights.resize((size_t)h.n_input);
-                for (int64_t q = 0; q < h.n_input; ++q) {
-                    const int64_t c = h.input_to_csc[(size_t)q];
-                    k.weights[(size_t)q] = c < 0 ? NAN : w[(size_t)c];
-                }
+                if (gather_weights(*r, k.weights.data(), err) != NC_OK) return;
+                cudaStreamSynchronize(stream);
                 k.potentials.resize((size_t)h.n);
                 nc::to_caller_order(h, pot.data(), k.potentials.data());
             }
