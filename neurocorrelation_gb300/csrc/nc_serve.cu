@@ -555,9 +555,9 @@ int nc_server::admit(Resident& r, std::string& err)
     return NC_OK;
 }
 
-// The final weights of a network that has run its last step, in the order they were given in,
-// gathered on the device (in the scheduler's loop on the host a random read each, some 20 ms for a dozen
-// networks of 3.7M synapses).  The network's own charges and arrival words, which nothing
+// The final weights of a network that has run its last step, in the order they were given
+// in, gathered on the device (a random read per synapse on the host, in the loop that
+// launches the steps, before).  The network's own charges and arrival words, which nothing
 // reads any more, hold the result and the index.
 int nc_server::gather_weights(const Resident& r, float* out, std::string& err)
 {
