@@ -114,7 +114,7 @@ __device__ __forceinline__ void bar_arrive(int b)
 constexpr int kBarReady = 1, kBarFull = 3;
 
 // Programmatic dependent launch: a step's blocks may be scheduled while the previous step
-// drains, and wait here, before they read anything that a step writes, until it has
+// drains; they read what no step writes, and wait here for the rest until it has
 // completed and its writes are visible.  (A kernel launched without the attribute passes
 // the wait at once.)
 __device__ __forceinline__ void wait_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -142,6 +142,9 @@ __device__ __forceinline__ void async4(uint32_t dst, const void* src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// waits for all but the kRing groups committed last, and for all
+__device__ __forceinline__ void async_wait_first() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing) : "memory"); }
+__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory"); }
 
 // *p where `in` is not zero, -0.0 elsewhere: a predicated load, so that nothing waits for the
@@ -379,21 +382,32 @@ struct Ring {
         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(row + slot * (part >> 2)));
         return v;
     }
-    __device__ __forceinline__ void fetch(const NcPools& P, int slot, uint32_t Q) const
+    // the part of a quad that no step writes, and the part that steps write
+    __device__ __forceinline__ void fetch_key(const NcPools& P, int slot, uint32_t Q) const
+    {
+        async16(quad + slot * 3 * part, (const uint4*)P.key + Q);
+        async4(row + slot * (part >> 2), (const uint32_t*)P.qrow + (Q >> 2));
+    }
+    __device__ __forceinline__ void fetch_state(const NcPools& P, int slot, uint32_t Q) const
     {
         const uint32_t to = quad + slot * 3 * part;
-        async16(to, (const uint4*)P.key + Q);
         const uint64_t keep = keep_half();
         async16_kept(to + part, (const uint4*)P.state + Q, keep);
         async16_kept(to + 2 * part, (const uint4*)P.w + Q, keep);
-        async4(row + slot * (part >> 2), (const uint32_t*)P.qrow + (Q >> 2));
+    }
+    __device__ __forceinline__ void fetch(const NcPools& P, int slot, uint32_t Q) const
+    {
+        fetch_key(P, slot, Q);
+        fetch_state(P, slot, Q);
     }
 };
 
 // The tiles of a block that are due in a launch, in order: blocks take the plan's shares
-// blockIdx.x, blockIdx.x + gridDim.x, ...  Every other step goes through a share backwards:
-// what a step touched last is what the L2 cache still holds when the next one begins
-// (100k x 100, 160 MB of arrays against 129 MB of L2: 53.4 -> 48.5 us a step).
+// blockIdx.x, blockIdx.x + gridDim.x, ...  Every other launch goes through a share backwards
+// (`back`, the caller's): what a step touched last is what the L2 cache still holds when the
+// next one begins (100k x 100, 160 MB of arrays against 129 MB of L2: 53.4 -> 48.5 us a step).
+// The plan is known before the launch's wait for the step before it; what is due only after
+// (settle_first).
 template <bool kFlush>
 struct Tiles {
     const NcPools& P;
@@ -405,11 +419,11 @@ struct Tiles {
         const int32_t t = D.t;
         return D.active && (kFlush ? t >= 2 && D.stdp_done < t - 1 : t <= D.t_end);
     }
-    __device__ __forceinline__ explicit Tiles(const NcPools& p) : P(p), share(blockIdx.x)
+    __device__ __forceinline__ Tiles(const NcPools& p, bool back_) : P(p), share(blockIdx.x), back(back_) { enter(); }
+    __device__ __forceinline__ bool planned() const { return ti >= begin && ti < end; }
+    __device__ __forceinline__ void settle_first()
     {
         single = P.n_nets == 1 ? (due_net(P.nets[0]) ? 1 : 0) : -1;
-        back = P.nets[0].t & 1;
-        enter();
         settle();
     }
     __device__ __forceinline__ void enter()
@@ -428,7 +442,7 @@ struct Tiles {
                 ti = -1;
                 return;
             }
-            if (ti >= begin && ti < end) {
+            if (planned()) {
                 if (single > 0 || due_net(P.nets[P.rtiles[ti].net])) return;
                 ti += back ? -1 : 1;
                 continue;
@@ -510,34 +524,110 @@ __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst&
 }
 
 // The stream warps' part of a step (or of the flush of the last one).
-template <bool kFlush>
-__device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, unsigned char* dyn)
+template <bool kFlush, bool kAlone>
+__device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t threads = blockDim.x - 32;
     const Ring ring(dyn, threads);
-    Tiles<kFlush> at(P);
+    Tiles<kFlush> at(P, back);
     TileConst C;
     int net = -1, share = -1, slot = 0;
     const uint32_t step = at.back ? 0u - threads : threads;
     uint32_t Q = 0u, run0 = 0u, run = 0u;
     uint32_t f[4] = {0u, 0u, 0u, 0u};  // fired words of this thread's next quad
+    const uint32_t* fired = nullptr;   // the net's fired words, of even steps
     bool due = false, inh = false;
     unsigned nl = 0u, nf = 0u;  // launches, and synapses whose source fired
+    // the run of consecutive quads that `tile` begins, and this thread's first one of it
+    auto begin_run = [&](const NcRowTile& tile) {
+        int other = at.back ? at.begin : at.end - 1;  // the run's last tile in this order
+        while (P.rtiles[other].net != tile.net) other += at.back ? 1 : -1;
+        const NcRowTile& last = P.rtiles[other];
+        run0 = at.back ? last.q0 : tile.q0;
+        run = (at.back ? tile.q0 + (uint32_t)tile.nq : last.q0 + (uint32_t)last.nq) - run0;
+        // chunks of `threads` quads from run0 on, the last one short
+        Q = run0 + threadIdx.x + (at.back && run ? (run - 1u) / threads * threads : 0u);
+        if (at.back && Q - run0 >= run) Q -= threads;
+    };
+    // what no step writes of a net's descriptor
+    auto begin_net = [&](int n) {
+        net = n;
+        const NcNetDesc& D = P.nets[n];
+        inh = !D.nonneg_terms;
+        fired = P.fired + D.word_base;
+        C.tab_pre = P.tables + D.table_base;
+        C.tab_pre_len = D.tab_pre_len;
+        C.kc = D.kc;
+        C.key_shift = D.key_shift;
+        C.dt = D.dt;
+        C.c52 = D.c52;
+        C.pre = D.pre_factor;
+        C.lr = D.lr;
+        C.post0 = D.post_factor * 0.0f;
+        C.wide = D.wide;
+    };
+    auto begin_step = [&](int32_t t, int32_t done) {
+        C.prev = t - 1;
+        due = C.prev >= 1 && done < C.prev;  // launches and plasticity of prev
+        C.fprev = fired + (int64_t)(C.prev & 1) * P.total_words;
+        C.refresh = C.prev % NC_AGE_PERIOD == 0;
+    };
+    // Before the wait: the first tile, its net's constants and its first keys.  After it the
+    // step counter, the first states and the first fired words (of both parities, the counter
+    // tells which) come side by side: one round trip to L2 instead of five, while the step
+    // before drains (the sphere of 750 7.5 -> 6.5 us a step, 1k x 50 7.05 -> 6.7, 30k x 73 15.3
+    // -> 14.7, 20k x 100 with inhibitory synapses 21.5 -> 20.7, 100k x 100 46.1 -> 45.0).
+    const int first = at.planned() ? at.ti : -1;
+    if (kAlone && first >= 0) {
+        const NcRowTile tile = P.rtiles[first];
+        begin_run(tile);
+#pragma unroll 1
+        for (int k = 0; k < kRing; ++k)
+            if (Q + k * step - run0 < run) ring.fetch_key(P, k, Q + k * step);
+        async_commit();
+        begin_net(tile.net);
+    }
+    if (kAlone) {
+        wait_previous_step();
+        release_next_step();
+    }
+    if (kAlone && first >= 0) {
+        const NcNetDesc& D = P.nets[net];
+        const int32_t t = D.t, done = D.stdp_done;
+#pragma unroll 1
+        for (int k = 0; k < kRing; ++k) {
+            if (Q + k * step - run0 < run) ring.fetch_state(P, k, Q + k * step);
+            async_commit();
+        }
+        async_wait_first();
+        if (Q - run0 < run) {
+            uint32_t odd[4];
+            const uint4 key = ring.load(0, 0);
+            C.fprev = fired;
+            if (C.wide) fired_words<true>(C, key, f);
+            else fired_words<false>(C, key, f);
+            C.fprev = fired + P.total_words;
+            if (C.wide) fired_words<true>(C, key, odd);
+            else fired_words<false>(C, key, odd);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (!(t & 1)) f[u] = odd[u];
+        }
+        begin_step(t, done);
+        share = at.share;
+    }
+    at.settle_first();
+    if (kAlone && first >= 0 && (at.ti != first || at.share != share)) {  // it was not due
+        async_wait_all();
+        net = share = -1;
+    }
     for (int n = 0; at.ti >= 0; at.next(), ++n) {
         const NcRowTile tile = P.rtiles[at.ti];
         const bool new_run = tile.net != net || at.share != share;
         if (new_run) {
-            // the next run of consecutive quads: fetch this thread's first ones
             share = at.share;
-            int other = at.back ? at.begin : at.end - 1;  // the run's last tile in this order
-            while (P.rtiles[other].net != tile.net) other += at.back ? 1 : -1;
-            const NcRowTile& last = P.rtiles[other];
-            run0 = at.back ? last.q0 : tile.q0;
-            run = (at.back ? tile.q0 + (uint32_t)tile.nq : last.q0 + (uint32_t)last.nq) - run0;
-            // chunks of `threads` quads from run0 on, the last one short
-            Q = run0 + threadIdx.x + (at.back && run ? (run - 1u) / threads * threads : 0u);
-            if (at.back && Q - run0 >= run) Q -= threads;
+            begin_run(tile);
 #pragma unroll 1
             for (int k = 0; k < kRing; ++k) {
                 const uint32_t q = Q + k * step;
@@ -548,24 +638,8 @@ __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, u
         if (tile.net != net) {
             if (net >= 0) count_events(P.nets[net], nl, nf, lane);
             nl = nf = 0u;
-            net = tile.net;
-            const NcNetDesc& D = P.nets[net];
-            const int32_t prev = D.t - 1;
-            due = prev >= 1 && D.stdp_done < prev;  // launches and plasticity of prev
-            inh = !D.nonneg_terms;
-            C.fprev = P.fired + (int64_t)(prev & 1) * P.total_words + D.word_base;
-            C.tab_pre = P.tables + D.table_base;
-            C.tab_pre_len = D.tab_pre_len;
-            C.prev = prev;
-            C.kc = D.kc;
-            C.key_shift = D.key_shift;
-            C.dt = D.dt;
-            C.c52 = D.c52;
-            C.pre = D.pre_factor;
-            C.lr = D.lr;
-            C.post0 = D.post_factor * 0.0f;
-            C.refresh = prev % NC_AGE_PERIOD == 0;
-            C.wide = D.wide;
+            begin_net(tile.net);
+            begin_step(P.nets[net].t, P.nets[net].stdp_done);
         }
         if (new_run && due) {  // the first quad's fired words
             async_wait();
@@ -583,10 +657,10 @@ __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, u
                                               slot, f, nl, nf);
         else if (inh)
             tile_synapses<kFlush, false, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
-                                              slot, f, nl, nf);
+                                               slot, f, nl, nf);
         else
             tile_synapses<kFlush, false, false>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
-                                              slot, f, nl, nf);
+                                                slot, f, nl, nf);
         bar_arrive<kBarFull>(b);
     }
     if (net >= 0) count_events(P.nets[net], nl, nf, lane);
@@ -608,6 +682,12 @@ __device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
     if (lane == 0) *P.done_ctr = 0u;
 }
 
+// Row starts of a tile into L1, before the wait: nothing writes them.
+__device__ __forceinline__ void prefetch_tile(const NcPools& P, const NcRowTile& tile, int lane)
+{
+    if (lane < tile.count) asm volatile("prefetch.global.L1 [%0];" ::"l"(P.in_ptr + tile.ptr + lane));
+}
+
 // Rows of tile `ti` into sh.row[b], and the buffer handed to the stream warps.
 __device__ __forceinline__ void give_rows(const NcPools& P, BlockShared& sh, int ti, int b, int lane)
 {
@@ -623,11 +703,18 @@ __device__ __forceinline__ void give_rows(const NcPools& P, BlockShared& sh, int
 }
 
 // The neuron warp's part of a step.
-template <bool kFlush>
-__device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh)
+template <bool kFlush, bool kAlone>
+__device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, bool back)
 {
     const int lane = threadIdx.x & 31;
-    Tiles<kFlush> at(P);
+    Tiles<kFlush> at(P, back);
+    // (the first tile's rows, into the L1 or at least the L2)
+    if (kAlone && at.planned()) prefetch_tile(P, P.rtiles[at.ti], lane);
+    if (kAlone) {
+        wait_previous_step();
+        release_next_step();
+    }
+    at.settle_first();
     // the tile whose rows are given next: up to two ahead of the one being summed
     Tiles<kFlush> ahead = at;
     int given = 0;
@@ -754,13 +841,13 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh)
 }
 
 // One step (or the flush of the last one) of every tile of this block.
-template <bool kFlush>
-__device__ __forceinline__ void dense_pass(const NcPools& P, BlockShared& sh, unsigned char* dyn)
+template <bool kFlush, bool kAlone>
+__device__ __forceinline__ void dense_pass(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
     if (threadIdx.x >= blockDim.x - 32) {
-        neuron_role<kFlush>(P, sh);
+        neuron_role<kFlush, kAlone>(P, sh, back);
     } else {
-        stream_role<kFlush>(P, sh, dyn);
+        stream_role<kFlush, kAlone>(P, sh, dyn, back);
     }
 }
 
@@ -768,13 +855,11 @@ __device__ __forceinline__ void dense_pass(const NcPools& P, BlockShared& sh, un
 #define NC_DENSE_MIN_BLOCKS 3
 #endif
 template <bool kFlush>
-__global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_step(NcPools P)
+__global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_step(NcPools P, bool back)
 {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ BlockShared sh;
-    wait_previous_step();
-    release_next_step();
-    dense_pass<kFlush>(P, sh, dyn);
+    dense_pass<kFlush, true>(P, sh, dyn, back);
 }
 
 // ---------------------------------------------------------------- fused multi-step launch
@@ -824,7 +909,7 @@ __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_fuse
     unsigned gen = 0u;
     if (threadIdx.x == 0) gen = atomicAdd(&bar[1], 0u);
     for (int32_t k = 0; k < ticks; ++k) {
-        dense_pass<false>(P, sh, dyn);
+        dense_pass<false, false>(P, sh, dyn, k & 1);
         if (!grid_barrier(bar, gen, P.dev_err, sh)) return;
     }
 }
@@ -877,7 +962,7 @@ namespace nc {
 
 int dense_resident_blocks(int threads) { return resident_blocks(0, std::max(threads, 64)); }
 
-int launch_step_dense(const NcPools& P, const LaunchShape& L, void* stream)
+int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* stream)
 {
     // a net with no neuron has no tile, but its step counter still advances
     const int threads = block_threads(L);
@@ -892,7 +977,7 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, void* stream)
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_dense_step<false>, P) != cudaSuccess) return -1;
+    if (cudaLaunchKernelEx(&cfg, k_dense_step<false>, P, back) != cudaSuccess) return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -918,7 +1003,7 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, un
 int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
     const int threads = block_threads(L);
-    k_dense_step<true><<<P.row_blocks, threads, ring_bytes(threads - 32), (cudaStream_t)stream>>>(P);
+    k_dense_step<true><<<P.row_blocks, threads, ring_bytes(threads - 32), (cudaStream_t)stream>>>(P, false);
     k_dense_mark_flushed<<<1, 256, 0, (cudaStream_t)stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -56,11 +56,16 @@ struct NcGroupDev {
     int32_t index;       // group index within its net (first Philox counter word)
 };
 
-struct NcNetDesc {
+// What a step writes comes first, in a cache line of its own: the rest may be read, and stay
+// in L1, before a launch's wait for the step before it.
+struct alignas(128) NcNetDesc {
     int32_t t;            // step processed by the next launch pair (>= 1)
     int32_t t_end;        // last step to simulate (inclusive)
     int32_t stdp_done;    // last step whose deferred plasticity has been applied
-    int32_t n;            // neurons
+    float tsum;           // NeuCor::currentTime after t-1 steps: the float sum of t-1 runSpeeds
+    int32_t active;       // 0: skipped by the kernels
+    int32_t live;         // event form: the last neuron step advanced the net (its fires launch)
+    alignas(128) int32_t n; // neurons
     int32_t neuron_base;  // pool index of neuron 0
     int32_t ptr_base;     // pool index of in_ptr/out_ptr/ring_off entry 0 (n+1 entries)
     int32_t word_base;    // pool index of this net's first bitset word
@@ -78,8 +83,6 @@ struct NcNetDesc {
     int32_t ap_base;      // pool index of the AP shape table (kc entries)
     int32_t group_base;
     int32_t n_groups;
-    int32_t active;       // 0: skipped by the kernels
-    int32_t live;         // event form: the last neuron step advanced the net (its fires launch)
     int32_t raster_len;   // recorded steps capacity (0 = off)
     int32_t raster_t0;    // first recorded step
     int32_t permuted;     // neurons are stored in a different order than the caller's ids
@@ -93,7 +96,6 @@ struct NcNetDesc {
     unsigned long long* stats; // 4 counters: fires, launched, dropped, steps
     int64_t n_syn;        // synapses (out-synapse entries)
     int64_t wide;         // dense form: 0, or the offset of the second range (NcPools::key)
-    float tsum;           // NeuCor::currentTime after t-1 steps: the float sum of t-1 runSpeeds
     int32_t nonneg_terms; // 1: no launch can add a negative term (no inhibitory synapse, no
                           // negative weight), so a neuron's sum only grows within a step
     int32_t group_lo;     // caller ids [group_lo, group_hi) hold every input group's members
@@ -315,7 +317,7 @@ int launch_spike_launch(const NcPools& P, const LaunchShape& L, void* stream);
 int launch_stdp_flush(const NcPools& P, const LaunchShape& L, void* stream);
 // Dense form (nc_dense.cu): one step in one launch, and the plasticity flush (the launches
 // and plasticity of the last step's fires) before read-back.
-int launch_step_dense(const NcPools& P, const LaunchShape& L, void* stream);
+int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* stream);
 // Blocks of `threads` threads of the dense step that fit on the current device at once (0:
 // the device cannot run it); called before a stream capture, where it may not be asked.
 int dense_resident_blocks(int threads);

@@ -392,7 +392,7 @@ int Engine::step(int64_t ticks, std::string& err)
 int Engine::launch_tick(cudaStream_t s)
 {
     int rc = P.n_firers > 0 ? launch_input_firers(P, s) : 0;  // the step's run-call schedule first
-    rc |= dense ? launch_step_dense(P, L, s) : (launch_neuron_step(P, L, s) | launch_spike_launch(P, L, s));
+    rc |= dense ? launch_step_dense(P, L, back_ = !back_, s) : (launch_neuron_step(P, L, s) | launch_spike_launch(P, L, s));
     return rc;
 }
 
@@ -472,7 +472,7 @@ int Engine::time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::str
             return NC_ERR_CUDA;
         }
         NC_CK(cudaEventRecord(at[0], stream));
-        if (dense ? launch_step_dense(P, L, stream) : launch_neuron_step(P, L, stream)) {
+        if (dense ? launch_step_dense(P, L, back_ = !back_, stream) : launch_neuron_step(P, L, stream)) {
             err = "launch";
             return NC_ERR_CUDA;
         }

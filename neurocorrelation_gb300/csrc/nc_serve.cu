@@ -313,7 +313,7 @@ int nc_server::capture(std::string& err)
     S_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
     for (int k = 0; k < cfg.steps_per_batch && rc == 0; ++k) {
-        if (dense) rc |= nc::launch_step_dense(G, L, stream);
+        if (dense) rc |= nc::launch_step_dense(G, L, k & 1, stream);
         else rc |= nc::launch_neuron_step(G, L, stream) | nc::launch_spike_launch(G, L, stream);
     }
     cudaError_t e = cudaStreamEndCapture(stream, &g);
