@@ -162,7 +162,7 @@ struct KnnShared {
 
 __global__ void __launch_bounds__(32 * kKnnWarps) k_knn(int32_t n, int32_t k, float h, int32_t g, uint32_t k0,
                                                         uint32_t k1, const float* xyz, const int32_t* cstart,
-                                                        const int32_t* members, unsigned long long* scratch,
+                                                        const int32_t* members, unsigned long long* scratch, int32_t cand_cap,
                                                         int32_t* to, float* weight, uint32_t* flags,
                                                         uint32_t* far)
 {
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(32 * kKnnWarps) k_knn(int32_t n, int32_t k, fl
     const int wib = threadIdx.x >> 5;
     const int gw = blockIdx.x * kKnnWarps + wib;
     const int nw = gridDim.x * kKnnWarps;
-    unsigned long long* cand = scratch + (int64_t)gw * kCandCap;
+    unsigned long long* cand = scratch + (int64_t)gw * cand_cap;
     uint32_t* hist = sh.hist[wib];
     for (int32_t i = gw; i < n; i += nw) {
         const float pi[3] = {xyz[3 * (int64_t)i], xyz[3 * (int64_t)i + 1], xyz[3 * (int64_t)i + 2]};
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(32 * kKnnWarps) k_knn(int32_t n, int32_t k, fl
                 const int32_t b0 = c >= 0 ? cstart[c] : 0, b1 = c >= 0 ? cstart[c + 1] : 0;
                 int tot = 0;
                 const int off = warp_excl_scan(b1 - b0, lane, &tot);
-                if (count + tot > kCandCap) {
+                if (count + tot > cand_cap) {
                     overflow = true;
                     break;
                 }
@@ -351,18 +351,36 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_fill_rows(NcPools P, int32_t
     }
 }
 
-template <class T>
-T* dalloc(size_t count, std::vector<void*>& own, cudaError_t& e)
-{
-    void* p = nullptr;
-    if (e == cudaSuccess) e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
-    if (p) own.push_back(p);
-    return (T*)p;
-}
-
-struct Frees {
+// The build's device arrays, freed with it.  Small ones share blocks of 1 MiB (an allocation
+// takes some 40 us, its release as much).
+struct Arrays {
     std::vector<void*> v;
-    ~Frees()
+    char* block = nullptr;
+    size_t left = 0;
+    cudaError_t e = cudaSuccess;
+    template <class T>
+    T* get(size_t count, bool alone = false)
+    {
+        constexpr size_t kBlock = 1 << 20, kAlign = 256;
+        const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + kAlign - 1) / kAlign * kAlign;
+        const bool small = !alone && bytes <= kBlock / 4;
+        if (!small || bytes > left) {
+            void* p = nullptr;
+            if (e == cudaSuccess) e = cudaMalloc(&p, small ? kBlock : bytes);
+            if (!p) return nullptr;
+            v.push_back(p);
+            if (!small) return (T*)p;
+            block = (char*)p;
+            left = kBlock;
+        }
+        char* p = block;
+        block += bytes;
+        left -= bytes;
+        return (T*)p;
+    }
+    // no longer freed here
+    void give(void* p) { v.erase(std::remove(v.begin(), v.end(), p), v.end()); }
+    ~Arrays()
     {
         for (void* p : v) cudaFree(p);
     }
@@ -397,17 +415,19 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    Frees own;
-    cudaError_t e = cudaSuccess;
-    float* d_xyz = dalloc<float>(3 * (size_t)n, own.v, e);
-    int32_t* d_cell = dalloc<int32_t>((size_t)n, own.v, e);
-    int32_t* d_count = dalloc<int32_t>((size_t)cells + 1, own.v, e);
-    int32_t* d_members = dalloc<int32_t>((size_t)n, own.v, e);
-    int32_t* d_to = dalloc<int32_t>((size_t)edges, own.v, e);
-    float* d_w = dalloc<float>((size_t)edges, own.v, e);
-    uint32_t* d_flags = dalloc<uint32_t>(2, own.v, e);  // failure flags, the longest distance's bits
-    const int knn_blocks = std::max(1, sms * 8);
-    unsigned long long* d_scratch = dalloc<unsigned long long>((size_t)knn_blocks * kKnnWarps * kCandCap, own.v, e);
+    Arrays own;
+    cudaError_t& e = own.e;
+    float* d_xyz = own.get<float>(3 * (size_t)n);
+    int32_t* d_cell = own.get<int32_t>((size_t)n);
+    int32_t* d_count = own.get<int32_t>((size_t)cells + 1);
+    int32_t* d_members = own.get<int32_t>((size_t)n);
+    int32_t* d_to = own.get<int32_t>((size_t)edges, true);
+    float* d_w = own.get<float>((size_t)edges);
+    uint32_t* d_flags = own.get<uint32_t>(2);  // failure flags, the longest distance's bits
+    // candidates of a warp's point: never more than the other points
+    const int knn_blocks = std::max(1, std::min(sms * 8, (n + kKnnWarps - 1) / kKnnWarps));
+    const int32_t cand_cap = std::min(kCandCap, n);
+    unsigned long long* d_scratch = own.get<unsigned long long>((size_t)knn_blocks * kKnnWarps * cand_cap);
     if (e != cudaSuccess) {
         err = cuda_msg("device kNN build (allocation)", e);
         return e == cudaErrorMemoryAllocation ? NC_ERR_NOMEM : NC_ERR_CUDA;
@@ -420,14 +440,14 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     e = cudaMemcpy(cstart.data() + 1, d_count, sizeof(int32_t) * (size_t)cells, cudaMemcpyDeviceToHost);
     for (int64_t c = 0; c < cells; ++c) cstart[(size_t)c + 1] += cstart[(size_t)c];
     if (e == cudaSuccess) e = cudaMemcpy(d_count, cstart.data(), sizeof(int32_t) * cstart.size(), cudaMemcpyHostToDevice);
-    int32_t* d_cursor = dalloc<int32_t>((size_t)cells, own.v, e);
+    int32_t* d_cursor = own.get<int32_t>((size_t)cells);
     if (e == cudaSuccess) e = cudaMemcpy(d_cursor, cstart.data(), sizeof(int32_t) * (size_t)cells, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         err = cuda_msg("device kNN build (cells)", e);
         return NC_ERR_CUDA;
     }
     k_fill_cells<<<(n + 255) / 256, 256>>>(n, d_cell, d_cursor, d_members);
-    k_knn<<<knn_blocks, 32 * kKnnWarps>>>(n, k, G.h, G.g, k0, k1, d_xyz, d_count, d_members, d_scratch, d_to, d_w,
+    k_knn<<<knn_blocks, 32 * kKnnWarps>>>(n, k, G.h, G.g, k0, k1, d_xyz, d_count, d_members, d_scratch, cand_cap, d_to, d_w,
                                           d_flags, d_flags + 1);
     uint32_t found[2] = {0, 0};
     e = cudaMemcpy(found, d_flags, sizeof(found), cudaMemcpyDeviceToHost);
@@ -453,8 +473,8 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     // inhibitory, so no term of this network can be negative
     h.nonneg_terms = true;
     // in-degrees by target slot -> row starts
-    int32_t* d_slot = dalloc<int32_t>((size_t)n, own.v, e);
-    int32_t* d_deg = dalloc<int32_t>((size_t)n, own.v, e);
+    int32_t* d_slot = own.get<int32_t>((size_t)n);
+    int32_t* d_deg = own.get<int32_t>((size_t)n);
     if (e == cudaSuccess) e = cudaMemcpy(d_slot, h.slot_of.data(), sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_deg, 0, sizeof(int32_t) * (size_t)n);
     if (e != cudaSuccess) {
@@ -489,9 +509,9 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     std::vector<const NetHost*> nets{&h};
     rc = net->eng.build(nets, 64, err, nullptr, true);
     if (rc != NC_OK) return rc;
-    unsigned long long* d_cur = dalloc<unsigned long long>((size_t)n, own.v, e);
-    unsigned long long* d_rows = dalloc<unsigned long long>((size_t)h.sp, own.v, e);
-    uint32_t* d_i2c = dalloc<uint32_t>((size_t)edges, own.v, e);
+    unsigned long long* d_cur = own.get<unsigned long long>((size_t)n);
+    unsigned long long* d_rows = own.get<unsigned long long>((size_t)h.sp);
+    uint32_t* d_i2c = own.get<uint32_t>((size_t)edges, true);
     if (e == cudaSuccess)
         e = cudaMemcpy(d_cur, h.in_ptr.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -515,8 +535,8 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     // read-back tables stay on the device until a read-back asks for them
     net->dev_to = d_to;
     net->dev_i2c = d_i2c;
-    own.v.erase(std::remove(own.v.begin(), own.v.end(), (void*)d_to), own.v.end());
-    own.v.erase(std::remove(own.v.begin(), own.v.end(), (void*)d_i2c), own.v.end());
+    own.give(d_to);
+    own.give(d_i2c);
     net->knn_k = k;
     return NC_OK;
 }

@@ -98,8 +98,17 @@ static void storage_order(NetHost& h, const float* xyz, int32_t order_kind)
             }
             code[(size_t)i] = morton3(q[0], q[1], q[2]);
         }
-        std::stable_sort(h.orig_id.begin(), h.orig_id.end(),
-                         [&](int32_t a, int32_t b) { return code[(size_t)a] < code[(size_t)b]; });
+        // by code, equal ones by id: three stable passes over ten bits each (a comparison sort
+        // took 1.5 of the 4 ms that building 20k x 60 on the device takes, 8.6 ms of 15 at
+        // 100k x 100)
+        std::vector<int32_t> other((size_t)n);
+        for (int shift = 0; shift < 30; shift += 10) {
+            int32_t at[1025] = {0};
+            for (int32_t i = 0; i < n; ++i) at[(code[(size_t)i] >> shift & 1023u) + 1]++;
+            for (int b = 0; b < 1024; ++b) at[b + 1] += at[b];
+            for (int32_t id : h.orig_id) other[(size_t)at[code[(size_t)id] >> shift & 1023u]++] = id;
+            h.orig_id.swap(other);
+        }
     }
     h.permuted = false;
     for (int32_t s = 0; s < n; ++s) {

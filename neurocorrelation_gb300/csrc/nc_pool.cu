@@ -36,15 +36,33 @@ Engine::~Engine()
 template <class T>
 T* Engine::alloc(size_t count, std::string& err)
 {
+    // Small arrays lie 64 KiB apart in shared blocks: an allocation takes some 40 us and its
+    // release as much, and the allocator packs small ones 512 bytes apart, where a step's
+    // loads meet in few slices of L2 (three neurons 6.1 to 6.4 us a step, 1k x 50 6.8 to 7.1;
+    // 256 bytes to 20 KiB apart 5.8 to 6.6 and 6.5 to 7.0; 36 or 64 KiB apart 5.8 to 6.0 and
+    // 6.4 to 6.5).
+    constexpr size_t kBlock = 2 << 20, kApart = 64 << 10;
+    const size_t bytes = (std::max<size_t>(1, count) * sizeof(T) + kApart - 1) / kApart * kApart;
+    const bool shared = bytes <= kBlock / 8;
+    if (shared && bytes <= block_left_) {
+        void* p = block_;
+        block_ += bytes;
+        block_left_ -= bytes;
+        return (T*)p;
+    }
     void* p = nullptr;
-    const size_t bytes = std::max<size_t>(1, count) * sizeof(T);
-    cudaError_t e = cudaMalloc(&p, bytes);
+    const size_t size = shared ? kBlock : std::max<size_t>(1, count) * sizeof(T);
+    cudaError_t e = cudaMalloc(&p, size);
     if (e != cudaSuccess) {
         err = cuda_msg("cudaMalloc", e);
         return nullptr;
     }
     allocs_.push_back(p);
-    e = cudaMemsetAsync(p, 0, bytes, stream);
+    if (shared) {
+        block_ = (char*)p + bytes;
+        block_left_ = size - bytes;
+    }
+    e = cudaMemsetAsync(p, 0, size, stream);
     if (e != cudaSuccess) {
         err = cuda_msg("cudaMemsetAsync", e);
         return nullptr;

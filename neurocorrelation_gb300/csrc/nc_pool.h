@@ -99,6 +99,8 @@ private:
     size_t scratch_bytes_ = 0;
     bool flushed_ = false, unseen_ = false;
     std::vector<void*> allocs_;
+    char* block_ = nullptr;      // what is left of the last block of small arrays
+    size_t block_left_ = 0;
     cudaGraphExec_t graph_ = nullptr;
     void* firers_buf_ = nullptr;
     void* near_buf_ = nullptr;
