@@ -57,6 +57,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <vector>
 
 namespace {
 
@@ -70,10 +71,12 @@ constexpr int kNibCap = 2048;
 // slots of shared memory).  Two leave the memory idle (400k x 100: 215 us a step against
 // 180), four take L1 from the gathers of fired bits (188).
 constexpr int kRing = 3;
+// Quads of a tile whose captured charges fit in a block's shared memory beside the ring.
+constexpr int kStageQuads = 640;
 
 struct RowState {
     float chg;      // weight change of an arrival at prev, before the clamp
-    uint32_t tf;    // the neuron fired at prev
+    uint32_t tf;    // bit 0: the neuron fired at prev; bit 1: its sum counts (it is out of its AP)
 };
 
 struct BlockShared {
@@ -83,7 +86,7 @@ struct BlockShared {
 };
 
 constexpr int kRingBytes = kRing * (3 * 16 + 4);  // dynamic shared memory per stream thread
-size_t ring_bytes(int threads) { return (size_t)threads * kRingBytes; }
+size_t dyn_bytes(int threads, bool stage) { return (size_t)threads * kRingBytes + (stage ? 16 * kStageQuads : 0); }
 
 // Named barriers between the neuron warp and the stream warps, two of each: `ready` once a
 // tile's rows are in shared memory and its window bits may be written, `full` once they are.
@@ -148,19 +151,26 @@ __device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_a
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory"); }
 
 // *p where `in` is not zero, -0.0 elsewhere: a predicated load, so that nothing waits for the
-// value before it is used.
+// value before it is used.  kShared: p points into shared memory.
+template <bool kShared>
 __device__ __forceinline__ float load_or_absent(const float* p, uint32_t in)
 {
     float v;
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f80000000;\n\t@q ld.global.f32 %0, [%1];\n\t}"
-                 : "=f"(v)
-                 : "l"(p), "r"(in));
+    if (kShared)
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f80000000;\n\t@q ld.shared.f32 %0, [%1];\n\t}"
+            : "=f"(v)
+            : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(in));
+    else
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.f32 %0, 0f80000000;\n\t@q ld.global.f32 %0, [%1];\n\t}"
+            : "=f"(v)
+            : "l"(p), "r"(in));
     return v;
 }
 
 // The window bits of one row, taken eight at a time.  nib: the tile's window bits, four to a
 // byte; q0, nq: the row's quads; x0: the tile's captured charges.  Eight bytes are packed to a
 // word of 32 synapses; a batch looks at the 32 from the first bit left on, across words.
+template <bool kShared>
 struct WindowBits {
     const unsigned long long* words;
     const float* x;        // charge of the first bit of `cur`
@@ -208,7 +218,7 @@ struct WindowBits {
         const float* xm = x + from;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            to[k] = load_or_absent(xm + __ffs((int)m) - 1, m);
+            to[k] = load_or_absent<kShared>(xm + __ffs((int)m) - 1, m);
             m &= m - 1u;
         }
         from += m ? __ffs((int)m) - 1 : 32;
@@ -217,7 +227,10 @@ struct WindowBits {
 };
 
 // charge_insynapses (src/NeuCor.cpp:688-700) of one row: the terms of the spikes that
-// arrived t-1 .. t-KC, in ascending source id, folded into pot.  The bits are streamed in
+// arrived t-1 .. t-KC, in ascending source id, folded into pot.  x0: the tile's charges, in
+// global memory or (kShared) staged in shared memory by the stream warps, which copy those of
+// quads with window bits behind their own work: a batch then waits for its bits and its sum,
+// not for L2 as well.  The bits are streamed in
 // batches of 8 terms across word boundaries, so that a warp's batch count is its busiest
 // lane's, not a sum of per-word maxima.  A batch takes some 1,100 cycles, a gather from L2 and a
 // serial sum; with the bits of 64-bit words taken one by one, and a branch at each for the next
@@ -231,11 +244,12 @@ struct WindowBits {
 // whatever the remaining terms are, and its potential is then replaced by the AP table
 // (src/NeuCor.cpp:682-686, 706-714): the fold stops there and returns the partial sum,
 // which leads the update to the same decision.
+template <bool kShared>
 __device__ __forceinline__ float fold_row(const uint8_t* nib, int q0, int nq, const float* x0, float pot, float leak,
                                           const TermFactor& F, bool stop)
 {
     if (nq <= 0) return pot;
-    WindowBits at(nib, q0, nq, x0);
+    WindowBits<kShared> at(nib, q0, nq, x0);
     float xv[8];
     while (at.next(xv)) {
         pot = fold_terms(pot, xv, F);
@@ -292,7 +306,7 @@ __device__ __forceinline__ uint32_t quad_update(const NcPools& P, const TileCons
         hi[u] = inh ? 0.0f : 1.0f;
         w1[u] = cap[u] = w0[u];
     }
-    if (row.tf) {
+    if (row.tf & 1u) {
         // post-spike branch: the trace since the last arrival before prev
         float tr[4];
 #pragma unroll
@@ -342,7 +356,7 @@ __device__ __forceinline__ uint32_t quad_update(const NcPools& P, const TileCons
         for (int u = 0; u < 4; ++u)
             if (nc_state_age(s[u], C.prev) >= NC_AGE_LIMIT) s[u] = nc_state_word(C.prev, NC_AGE_OLD, 0);
     }
-    if (row.tf || arrived) *((float4*)P.w + Q) = make_float4(w2[0], w2[1], w2[2], w2[3]);
+    if ((row.tf & 1u) || arrived) *((float4*)P.w + Q) = make_float4(w2[0], w2[1], w2[2], w2[3]);
     if (nl != nl0 || (!kWide && C.refresh)) {
         *((uint4*)P.state + Q) = make_uint4(s[0], s[1], s[2], s[3]);
         if (kWide) *((uint4*)(P.state + C.wide) + Q) = make_uint4(bf[0], bf[1], bf[2], bf[3]);
@@ -486,10 +500,10 @@ __device__ __forceinline__ void fired_bits(const TileConst& C, const uint4& key,
 // The quads of one tile.  The block's quads of one net are consecutive, [run0, run0 + run):
 // this thread takes every threads-th of them, from Q on in steps of `step`, whichever tiles
 // they fall into (Q is left at its first past the tile), and keeps its next ones under way.
-template <bool kFlush, bool kWide, bool kInh>
+template <bool kFlush, bool kStage, bool kWide, bool kInh>
 __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst& C, uint32_t q0, uint32_t nq,
                                               uint32_t run0, uint32_t run, bool due, const RowState* row,
-                                              uint32_t row0, uint8_t* nib, const Ring& ring, uint32_t step,
+                                              uint32_t row0, uint8_t* nib, uint32_t stage, const Ring& ring, uint32_t step,
                                               uint32_t& Q, int& slot, uint32_t (&f)[4], unsigned& nl, unsigned& nf)
 {
     for (; Q - q0 < nq; Q += step) {
@@ -497,6 +511,7 @@ __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst&
         const int ahead = slot + 1 == kRing ? 0 : slot + 1;
         const uint4 st = ring.load(slot, 1);
         uint32_t win = 0u;
+        uint32_t sums = 0u;  // (staged) bit 1: the row's sum counts
         if (due) {
             const uint4 key = ring.load(slot, 0);
             uint32_t fired[4] = {f[0], f[1], f[2], f[3]};
@@ -505,8 +520,11 @@ __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst&
             if (Q + step - run0 < run) fired_words<kWide>(C, ring.load(ahead, 0), f);
             const uint4 w = ring.load(slot, 2);
             const uint32_t rb = ring.load_row(slot) >> (8 * (Q & 3u));
-            win = quad_update<kWide, kInh>(P, C, Q, row[(rb - row0) & 31u], key, st, w, fired, nl, nf);
+            const RowState rs = row[(rb - row0) & 31u];
+            if (kStage) sums = rs.tf;
+            win = quad_update<kWide, kInh>(P, C, Q, rs, key, st, w, fired, nl, nf);
         } else {
+            if (kStage) sums = row[((ring.load_row(slot) >> (8 * (Q & 3u))) - row0) & 31u].tf;
             const uint32_t s[4] = {st.x, st.y, st.z, st.w};
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -515,6 +533,7 @@ __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst&
             }
         }
         if (!kFlush) nib[Q] = (uint8_t)win;
+        if (kStage && win && (sums & 2u)) async16(stage + 16u * (Q - q0), (const float4*)P.x + Q);
         // the slot has been read: refill it
         const uint32_t next = Q + kRing * step;
         if (next - run0 < run) ring.fetch(P, slot, next);
@@ -524,12 +543,13 @@ __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst&
 }
 
 // The stream warps' part of a step (or of the flush of the last one).
-template <bool kFlush, bool kAlone>
+template <bool kFlush, bool kAlone, bool kStage>
 __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t threads = blockDim.x - 32;
     const Ring ring(dyn, threads);
+    const uint32_t stage = kStage ? (uint32_t)__cvta_generic_to_shared(dyn) + kRingBytes * threads : 0u;
     Tiles<kFlush> at(P, back);
     TileConst C;
     int net = -1, share = -1, slot = 0;
@@ -653,14 +673,15 @@ __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, u
         bar_sync<kBarReady>(b);
         const uint32_t row0 = (uint32_t)tile.first, nq = (uint32_t)tile.nq;
         if (C.wide)
-            tile_synapses<kFlush, true, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
+            tile_synapses<kFlush, kStage, true, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, stage, ring, step, Q,
                                               slot, f, nl, nf);
         else if (inh)
-            tile_synapses<kFlush, false, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
+            tile_synapses<kFlush, kStage, false, true>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, stage, ring, step, Q,
                                                slot, f, nl, nf);
         else
-            tile_synapses<kFlush, false, false>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, ring, step, Q,
+            tile_synapses<kFlush, kStage, false, false>(P, C, tile.q0, nq, run0, run, due, sh.row[b], row0, nib, stage, ring, step, Q,
                                                 slot, f, nl, nf);
+        if (kStage) async_wait_all();
         bar_arrive<kBarFull>(b);
     }
     if (net >= 0) count_events(P.nets[net], nl, nf, lane);
@@ -697,14 +718,15 @@ __device__ __forceinline__ void give_rows(const NcPools& P, BlockShared& sh, int
         // the target's trace at prev; the arriving synapse's own is 0
         const int32_t lf = P.lf[i];
         const float trT = P.pst[i];
-        sh.row[b][lane] = RowState{(D.pre_factor * 0.0f - D.post_factor * trT) * D.lr, lf == D.t - 1 ? 1u : 0u};
+        const uint32_t sums = lf == NC_NEVER || D.t - lf >= D.kc ? 2u : 0u;
+        sh.row[b][lane] = RowState{(D.pre_factor * 0.0f - D.post_factor * trT) * D.lr, lf == D.t - 1 ? 1u | sums : sums};
     }
     bar_arrive<kBarReady>(b);
 }
 
 // The neuron warp's part of a step.
-template <bool kFlush, bool kAlone>
-__device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, bool back)
+template <bool kFlush, bool kAlone, bool kStage>
+__device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
     const int lane = threadIdx.x & 31;
     Tiles<kFlush> at(P, back);
@@ -793,7 +815,8 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, b
             if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
         }
         const uint8_t* nib = tile.nq <= kNibCap ? sh.nib[b] : P.nib + tile.q0;
-        if (need) pot = fold_row(nib, q0, nq, P.x + 4 * (int64_t)tile.q0, pot, leak, F, stop);
+        const float* x = kStage ? (const float*)(dyn + kRingBytes * (blockDim.x - 32)) : P.x + 4 * (int64_t)tile.q0;
+        if (need) pot = fold_row<kStage>(nib, q0, nq, x, pot, leak, F, stop);
         __syncwarp();
         if (ahead.ti >= 0) {
             give_rows(P, sh, ahead.ti, b, lane);
@@ -841,25 +864,25 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, b
 }
 
 // One step (or the flush of the last one) of every tile of this block.
-template <bool kFlush, bool kAlone>
+template <bool kFlush, bool kAlone, bool kStage>
 __device__ __forceinline__ void dense_pass(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
     if (threadIdx.x >= blockDim.x - 32) {
-        neuron_role<kFlush, kAlone>(P, sh, back);
+        neuron_role<kFlush, kAlone, kStage>(P, sh, dyn, back);
     } else {
-        stream_role<kFlush, kAlone>(P, sh, dyn, back);
+        stream_role<kFlush, kAlone, kStage>(P, sh, dyn, back);
     }
 }
 
 #ifndef NC_DENSE_MIN_BLOCKS
 #define NC_DENSE_MIN_BLOCKS 3
 #endif
-template <bool kFlush>
+template <bool kFlush, bool kStage>
 __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_step(NcPools P, bool back)
 {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ BlockShared sh;
-    dense_pass<kFlush, true>(P, sh, dyn, back);
+    dense_pass<kFlush, true, kStage>(P, sh, dyn, back);
 }
 
 // ---------------------------------------------------------------- fused multi-step launch
@@ -909,7 +932,7 @@ __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_fuse
     unsigned gen = 0u;
     if (threadIdx.x == 0) gen = atomicAdd(&bar[1], 0u);
     for (int32_t k = 0; k < ticks; ++k) {
-        dense_pass<false, false>(P, sh, dyn, k & 1);
+        dense_pass<false, false, false>(P, sh, dyn, k & 1);
         if (!grid_barrier(bar, gen, P.dev_err, sh)) return;
     }
 }
@@ -923,28 +946,29 @@ __global__ void k_dense_mark_flushed(NcPools P)
     }
 }
 
-// Blocks of one wave of kernel `which` (0: a step, 1: several) with `threads` threads on the
-// current device (cached per device and block size).  Returns 0 when the device cannot run
-// it (the launch then reports an error).
+// Blocks of one wave of kernel `which` (0: a step, 1: several, 2: a step with staged charges)
+// with `threads` threads on the current device (cached per device and block size).  Returns 0
+// when the device cannot run it (the launch then reports an error).
 int resident_blocks(int which, int threads)
 {
-    static std::atomic<int> cache[2][64][kMaxThreads / 32 + 1];
+    static std::atomic<int> cache[3][64][kMaxThreads / 32 + 1];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     std::atomic<int>& c = cache[which][dev][threads / 32];
     int n = c.load(std::memory_order_relaxed);
     if (n == 0) {
         int sms = 0, per_sm = 0;
-        const void* fn = which ? (const void*)k_dense_fused : (const void*)k_dense_step<false>;
+        const size_t dyn = dyn_bytes(threads - 32, which == 2);
+        const void* fn = which == 1   ? (const void*)k_dense_fused
+                         : which == 2 ? (const void*)k_dense_step<false, true>
+                                      : (const void*)k_dense_step<false, false>;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, ring_bytes(threads - 32)) !=
-                cudaSuccess ||
-            sms * per_sm <= 0)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn) != cudaSuccess || sms * per_sm <= 0)
             return 0;
         // no more shared memory than the blocks need: the rest is L1 for the gathers
         cudaFuncAttributes fa;
         if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
-        const size_t need = (size_t)per_sm * (fa.sharedSizeBytes + ring_bytes(threads - 32) + 1024);
+        const size_t need = (size_t)per_sm * (fa.sharedSizeBytes + dyn + 1024);
         cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)std::min<size_t>(100, (need * 100 + 233471) / 233472));
         n = sms * per_sm;
@@ -960,6 +984,17 @@ int block_threads(const nc::LaunchShape& L) { return std::max(L.neuron_block, 64
 
 namespace nc {
 
+// Whether a step keeps its captured charges in shared memory: one tile to a block, and it fits.
+// (Blocks of several tiles would need two buffers, and large networks their L1.)
+bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t>& start)
+{
+    for (size_t b = 0; b + 1 < start.size(); ++b)
+        if (start[b + 1] - start[b] > 1) return false;
+    for (const NcRowTile& t : tiles)
+        if (t.nq > kStageQuads) return false;
+    return true;
+}
+
 int dense_resident_blocks(int threads) { return resident_blocks(0, std::max(threads, 64)); }
 
 int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* stream)
@@ -970,14 +1005,17 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* s
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = ring_bytes(threads - 32);
+    // (the plan was made for this kernel only if a wave of it holds every block)
+    const bool stage = P.stage && L.dense_blocks == 0 && resident_blocks(2, threads) >= blocks;
+    cfg.dynamicSmemBytes = dyn_bytes(threads - 32, stage);
     cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_dense_step<false>, P, back) != cudaSuccess) return -1;
+    if (cudaLaunchKernelEx(&cfg, stage ? k_dense_step<false, true> : k_dense_step<false, false>, P, back) != cudaSuccess)
+        return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -995,7 +1033,7 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, un
     NcPools p = P;
     void* args[] = {(void*)&p, (void*)&ticks, (void*)&bar};
     if (cudaLaunchCooperativeKernel((const void*)k_dense_fused, dim3((unsigned)blocks), dim3((unsigned)threads), args,
-                                    ring_bytes(threads - 32), s) != cudaSuccess)
+                                    dyn_bytes(threads - 32, false), s) != cudaSuccess)
         return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -1003,7 +1041,7 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, un
 int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
     const int threads = block_threads(L);
-    k_dense_step<true><<<P.row_blocks, threads, ring_bytes(threads - 32), (cudaStream_t)stream>>>(P, false);
+    k_dense_step<true, false><<<P.row_blocks, threads, dyn_bytes(threads - 32, false), (cudaStream_t)stream>>>(P, false);
     k_dense_mark_flushed<<<1, 256, 0, (cudaStream_t)stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -29,6 +29,8 @@
 #include <cstdint>
 #include <vector_types.h>
 
+#include <vector>
+
 #ifdef __CUDACC__
 #define NC_HD __host__ __device__
 #else
@@ -227,6 +229,7 @@ struct NcPools {
     NcRowTile* rtiles;   // in the order of the blocks that run them
     int32_t* rstart;     // first tile of each of row_blocks blocks (row_blocks + 1 entries)
     int32_t row_blocks;
+    int32_t stage;       // dense step: captured charges of the sums pass through shared memory (dense_stages)
     // ring and bitsets
     uint32_t* ring;
     uint32_t* fired;     // 2 parities x total_words
@@ -321,6 +324,7 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* s
 // Blocks of `threads` threads of the dense step that fit on the current device at once (0:
 // the device cannot run it); called before a stream capture, where it may not be asked.
 int dense_resident_blocks(int threads);
+bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t>& start);
 // `ticks` whole dense steps of every net in one cooperative launch (no periodic input
 // firers); bar: two zero-initialised words of device memory for its grid barrier.
 int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, unsigned* bar, void* stream);
