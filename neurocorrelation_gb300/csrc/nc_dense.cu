@@ -685,14 +685,20 @@ __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, u
         bar_arrive<kBarFull>(b);
     }
     if (net >= 0) count_events(P.nets[net], nl, nf, lane);
-    else if (!kFlush) bar_arrive<kBarFull>(0);  // nothing to do: the step counters have been read
+    else bar_arrive<kBarFull>(0);  // nothing to do: the step counters have been read
 }
 
-// Every block has read the step counters: one warp moves them on.
+// Every block has read the step counters: one warp moves them on (a flush: notes that the
+// launches and plasticity of every active net's last step are done).
+template <bool kFlush>
 __device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
 {
     for (int n = lane; n < P.n_nets; n += 32) {
         NcNetDesc* D = P.nets + n;
+        if (kFlush) {
+            if (D->active && D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
+            continue;
+        }
         if (D->active && D->t <= D->t_end) {
             if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
             D->stats[3] += 1ull;
@@ -751,6 +757,10 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
         at.next();
         if (kFlush) {
             bar_sync<kBarFull>(b);
+            if (at.ti < 0) {
+                counted = true;
+                if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
+            }
             if (ahead.ti >= 0) {
                 give_rows(P, sh, ahead.ti, b, lane);
                 ahead.next();
@@ -854,13 +864,12 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
         }
         fires += __popc(fmask);
     }
-    if (kFlush) return;
     if (net >= 0 && lane == 0 && fires) atomicAdd(P.nets[net].stats + 0, (unsigned long long)fires);
     if (!counted) {  // a block with nothing to do (its other warps have read the counters)
         bar_sync<kBarFull>(0);
         if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
     }
-    if (__shfl_sync(kFull, arrived, 0) == gridDim.x - 1u) advance_steps(P, lane);
+    if (__shfl_sync(kFull, arrived, 0) == gridDim.x - 1u) advance_steps<kFlush>(P, lane);
 }
 
 // One step (or the flush of the last one) of every tile of this block.
@@ -934,15 +943,6 @@ __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_fuse
     for (int32_t k = 0; k < ticks; ++k) {
         dense_pass<false, false, false>(P, sh, dyn, k & 1);
         if (!grid_barrier(bar, gen, P.dev_err, sh)) return;
-    }
-}
-
-// After a flush: the launches and plasticity of every active net's last step are done.
-__global__ void k_dense_mark_flushed(NcPools P)
-{
-    for (int n = threadIdx.x; n < P.n_nets; n += blockDim.x) {
-        NcNetDesc* D = P.nets + n;
-        if (D->active && D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
     }
 }
 
@@ -1042,7 +1042,6 @@ int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
     const int threads = block_threads(L);
     k_dense_step<true, false><<<P.row_blocks, threads, dyn_bytes(threads - 32, false), (cudaStream_t)stream>>>(P, false);
-    k_dense_mark_flushed<<<1, 256, 0, (cudaStream_t)stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

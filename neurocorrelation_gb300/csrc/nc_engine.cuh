@@ -341,7 +341,7 @@ int launch_force_bits(const NcPools& P, int net, const int32_t* d_ids, int count
 // Input firers (nc_inputs.cu), launched before a step's kernels: each firer's schedule
 // for the run call that starts at its net's step t; fires land in the ufire bits of
 // step t+1 (and, before the first step, those of the time-0 call in step 1's).
-int launch_input_firers(const NcPools& P, void* stream);
+int launch_input_firers(const NcPools& P, bool early, void* stream);
 // Mean potential of each detector's near neurons (caller ids; near_ptr has count+1 entries).
 int launch_detector_voltages(const NcPools& P, int32_t neuron_base, const int32_t* near, const int32_t* near_ptr,
                              int32_t count, float* out, void* stream);

@@ -60,8 +60,13 @@ __device__ void mark_near(const NcPools& P, const NcFirer& F, uint32_t* uf, int 
 
 // Warp per firer, before the kernels of its net's step t = D.t: lane 0 runs the
 // schedule, the warp marks the near neurons.
-__global__ void k_input_firers(NcPools P)
+// A programmatic dependent launch between two steps.  `early`: the step that follows reads
+// nothing before its own wait that this kernel writes (the dense step; the event form's
+// reads the fire requests), so its blocks may come as soon as the last step is done.
+__global__ void k_input_firers(NcPools P, bool early)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int f = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (f >= P.n_firers) return;
@@ -103,12 +108,21 @@ __global__ void k_detector_voltages(const float* pot, const int32_t* slot_of, in
 
 namespace nc {
 
-int launch_input_firers(const NcPools& P, void* stream)
+int launch_input_firers(const NcPools& P, bool early, void* stream)
 {
     if (P.n_firers <= 0) return 0;
     const int threads = 256;
     const int blocks = (int)(((int64_t)P.n_firers * 32 + threads - 1) / threads);
-    k_input_firers<<<blocks, threads, 0, (cudaStream_t)stream>>>(P);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_input_firers, P, early) != cudaSuccess) return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -96,6 +96,7 @@ private:
     // or kScratchMax of it at a time.
     static constexpr size_t kScratchMax = 64 << 20;
     void* scratch_ = nullptr;
+    bool shared_tables_ = false;  // the GPU uses the host's page tables: it can write ordinary host memory
     size_t scratch_bytes_ = 0;
     bool flushed_ = false, unseen_ = false;
     std::vector<void*> allocs_;
