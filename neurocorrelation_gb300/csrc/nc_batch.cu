@@ -200,11 +200,12 @@ int nc_batch_autotune(nc_batch* b, int32_t steps_per_trial, nc_launch_config* be
     const nc_launch_config cur = {b->eng.L.neuron_block, b->eng.L.launch_blocks, b->eng.L.launch_block,
                                   b->eng.graph_ticks, b->eng.L.dense_blocks, b->eng.L.fused_ticks};
     if (b->eng.dense) {
-        for (int nb : {64, 128, 256})
+        // (the plan's shares are a wave of NC_DENSE_BLOCK-thread blocks)
+        for (int nb : {64, NC_DENSE_BLOCK, 128, 256})
             for (int g : {16, 64}) cands.push_back(nc_launch_config{nb, cur.launch_blocks, cur.launch_block, g, 0, 0});
         if (b->eng.P.n_firers == 0)
             for (int k : {4, 16, 64})
-                cands.push_back(nc_launch_config{128, cur.launch_blocks, cur.launch_block, 16, 0, k});
+                cands.push_back(nc_launch_config{NC_DENSE_BLOCK, cur.launch_blocks, cur.launch_block, 16, 0, k});
     } else {
         for (int nb : {64, 128, 256})
             for (int lbm : {4, 8, 16})
