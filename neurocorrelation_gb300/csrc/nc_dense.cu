@@ -36,20 +36,21 @@
 //
 // What bounds it, and why this shape.  The step streams 12.25 bytes a synapse (key, state,
 // weight; a row byte per quad) and writes what changed; on networks past the L2 cache that
-// is 23 bytes a synapse of DRAM traffic at 5.2 TB/s (2M x 200: 2,815 -> 1,640 us a step),
+// is 23 bytes a synapse of DRAM traffic at 5.8 TB/s (2M x 200: 2,815 -> 1,597 us a step),
 // on smaller ones instruction issue and, below some 10k neurons, the chain of dependent
-// loads.  The two passes before it (synapses, then neurons) read 22 bytes a synapse, took
-// 184 warp instructions per 32 synapses against 75, and exchanged window bits, captured
-// terms and traces through memory.  100k x 100: 92 -> 48 us; 1k x 50: 18.0 -> 7.4;
-// 20k x 100 with inhibitory synapses: 45.8 -> 26; 30k x 73 at dt 0.5: 33 -> 16.5.
+// loads and the boundary between two launches.  The two passes before it (synapses, then
+// neurons) read 22 bytes a synapse, took 184 warp instructions per 32 synapses against 75,
+// and exchanged window bits, captured terms and traces through memory.  100k x 100: 92 -> 45
+// us; 1k x 50: 18.0 -> 6.6; 20k x 100 with inhibitory synapses: 45.8 -> 19; 30k x 73 at dt
+// 0.5: 33 -> 14.8.
 //   - Rows padded to quads: a thread's four synapses share their target's values, and move
 //     with one 16-byte access per array; every eighth row ends on a 128-byte line.
 //   - A warp of its own sums, so the others never wait for a sum: with block barriers
-//     between the two halves the 100k x 100 step took 78 us.
+//     between the two halves the 100k x 100 step took 78 us (48 then).
 //   - 96 threads (two stream warps to a neuron warp), 80 registers, 8 blocks an SM, the
 //     rest of shared memory left to the L1 (all of it for shared memory: 57 -> 66 us).
-//     128 threads: 49 us, and 19.6 us against 16.5 on 30k x 73, whose shares get uneven;
-//     64 registers spill (60 us).
+//     128 threads: 49 us against 48, and 19.6 against 16.5 on 30k x 73, whose shares get
+//     uneven; 64 registers spill (60 us).
 #include "nc_device.cuh"
 #include "nc_engine.cuh"
 
@@ -984,15 +985,16 @@ int block_threads(const nc::LaunchShape& L) { return std::max(L.neuron_block, 64
 
 namespace nc {
 
-// Whether a step keeps its captured charges in shared memory: one tile to a block, and it fits.
-// (Blocks of several tiles would need two buffers, and large networks their L1.)
-bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t>& start)
+// Whether a step of `threads`-thread blocks can keep its captured charges in shared memory: one
+// tile to a block, it fits, and a wave holds every block.  (Blocks of several tiles would need
+// two buffers, and large networks their L1.)
+bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t>& start, int threads)
 {
     for (size_t b = 0; b + 1 < start.size(); ++b)
         if (start[b + 1] - start[b] > 1) return false;
     for (const NcRowTile& t : tiles)
         if (t.nq > kStageQuads) return false;
-    return true;
+    return resident_blocks(2, std::max(threads, 64)) >= (int)start.size() - 1;
 }
 
 int dense_resident_blocks(int threads) { return resident_blocks(0, std::max(threads, 64)); }
@@ -1005,7 +1007,7 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* s
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3((unsigned)threads);
-    // (the plan was made for this kernel only if a wave of it holds every block)
+    // (another launch shape than the plan's may not hold every block in a wave)
     const bool stage = P.stage && L.dense_blocks == 0 && resident_blocks(2, threads) >= blocks;
     cfg.dynamicSmemBytes = dyn_bytes(threads - 32, stage);
     cfg.stream = (cudaStream_t)stream;

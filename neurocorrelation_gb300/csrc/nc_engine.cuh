@@ -324,7 +324,7 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* s
 // Blocks of `threads` threads of the dense step that fit on the current device at once (0:
 // the device cannot run it); called before a stream capture, where it may not be asked.
 int dense_resident_blocks(int threads);
-bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t>& start);
+bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t>& start, int threads);
 // `ticks` whole dense steps of every net in one cooperative launch (no periodic input
 // firers); bar: two zero-initialised words of device memory for its grid barrier.
 int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, unsigned* bar, void* stream);

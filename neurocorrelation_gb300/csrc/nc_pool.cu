@@ -335,9 +335,9 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         // sums that run to their last term (inhibitory or negative synapses) gain from it: the
         // sphere of 750 6.3 -> 5.9 us a step, 20k x 100 20.7 -> 19.0; those that stop early, after
         // a batch or two, do not (1k x 50 6.5 either way, 30k x 73 14.7 and 14.9)
-        P.stage = dense_stages(rows, start) ? 1 : 0;
-        for (const NetHost* h : nets)
-            if (h->nonneg_terms) P.stage = 0;
+        bool all_sum = true;
+        for (const NetHost* h : nets) all_sum = all_sum && !h->nonneg_terms;
+        P.stage = all_sum && dense_stages(rows, start, L.neuron_block) ? 1 : 0;
         NC_ALLOC(P.rtiles, NcRowTile, rows.size());
         NC_ALLOC(P.rstart, int32_t, start.size());
         NC_CK(upload(P.rtiles, rows, 0, stream));
