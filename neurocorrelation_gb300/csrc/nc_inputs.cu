@@ -60,9 +60,10 @@ __device__ void mark_near(const NcPools& P, const NcFirer& F, uint32_t* uf, int 
 
 // Warp per firer, before the kernels of its net's step t = D.t: lane 0 runs the
 // schedule, the warp marks the near neurons.
-// A programmatic dependent launch between two steps.  `early`: the step that follows reads
-// nothing before its own wait that this kernel writes (the dense step; the event form's
-// reads the fire requests), so its blocks may come as soon as the last step is done.
+// A programmatic dependent launch between two steps.  The step that follows reads nothing
+// before its own wait that this kernel writes.  `early`: nor anything that the last step
+// writes (the dense step; the event form's reads the neurons' state), so its blocks may
+// come while this kernel waits and runs.
 __global__ void k_input_firers(NcPools P, bool early)
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -209,8 +209,9 @@ __device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
 // One warp per warp_rows (8, 16 or 32) neurons of one net; blocks of any size, no block
 // barrier.  The chain of dependent loads bounds it (about 800 cycles each and more for what
 // is not in L2), so:
-//   - what the spike launch of the step before does not write (everything but charges, ring
-//     bits and arrival steps) is read, and the draws are made, before the wait for it;
+//   - what neither the spike launch of the step before nor a kernel between two steps writes
+//     (everything but charges, ring bits, arrival steps and fire requests) is read, and the
+//     draws are made, before the wait;
 //   - the ring words of the whole window come in one go, then the gathers of the arrivals'
 //     weights and of the sum's charges together;
 //   - a small network gives a warp fewer neurons, so that a warp has fewer fired rows and a
@@ -264,14 +265,12 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
             if (D.permuted) cid = __ldg(P.orig_id + pj);
         }
         const uint32_t was = (__ldcg(P.fired + (int64_t)(prev & 1) * P.total_words + word) & mask) >> shift;
-        const uint32_t fw = (__ldcg(P.forced + (int64_t)(t & 1) * P.total_words + word) & mask) >> shift;
-        const uint32_t uw = (__ldcg(P.ufire + (int64_t)(t & 1) * P.total_words + word) & mask) >> shift;
         // input requests, and the background target for step t+1 (src/NeuCor.cpp:604-607),
         // drawn per caller id
-        bool forced = (fw >> lane) & 1u;
+        bool forced = false;
         uint32_t bg = ~0u;
         if (live && act) {
-            if (!forced && D.n_groups) forced = input_request(P, D, cid, t);
+            if (D.n_groups) forced = input_request(P, D, cid, t);
             if (D.bg_period > 0) {
                 uint32_t o[4];
                 philox((uint32_t)cid, (uint32_t)t, NC_STREAM_BACKGROUND, 0u, D, o);
@@ -293,6 +292,10 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
         if (last_unit && lane == 0) arrived = atomicAdd(P.done_ctr, min(t, done_to) > NC_NEVER ? 1u : 0u);
         if (act) {
             const bool stdp = prev >= 1 && done_to < prev;
+            // fire requests: kernels between two steps set them, so not before the wait
+            const uint32_t fw = (__ldcg(P.forced + (int64_t)(t & 1) * P.total_words + word) & mask) >> shift;
+            const uint32_t uw = (__ldcg(P.ufire + (int64_t)(t & 1) * P.total_words + word) & mask) >> shift;
+            forced = forced || ((fw >> lane) & 1u);
             RowBits B;
             row_bits(B, ring, rw, ring_mask, r0, r1, t, kc);
             if (bg != ~0u)
