@@ -49,7 +49,7 @@ def workload_config(extra=None):
     cfg = {"workload": "plain single network: 100k neurons x 100 nearest targets (10M synapses), "
                        "200 inputs in 10 correlated Poisson groups 5-40 Hz, STDP on, 20,000 steps",
            "neurons": N_NEURONS, "synapses": N_NEURONS * FANOUT, "sim_steps_per_bench_step": SIM_STEPS_PER_STEP,
-           "dt_ms": 1.0, "l2": "inputs larger than L2 (synapse tables ~350 MB)", "parallelism": "replicas"}
+           "dt_ms": 1.0, "l2": "inputs larger than L2 (the step's arrays ~160 MB)", "parallelism": "replicas"}
     if extra:
         cfg.update(extra)
     return cfg
