@@ -981,6 +981,24 @@ int resident_blocks(int which, int threads)
 // Threads per block: a neuron warp and at least one stream warp.
 int block_threads(const nc::LaunchShape& L) { return std::max(L.neuron_block, 64); }
 
+// A step's or flush's kernel as a programmatic dependent launch.
+int launch_dependent(void (*fn)(NcPools, bool), int blocks, int threads, size_t dyn, const NcPools& P, bool back,
+                     void* stream)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = dyn;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, fn, P, back) != cudaSuccess) return -1;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
 }  // namespace
 
 namespace nc {
@@ -1004,21 +1022,10 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* s
     // a net with no neuron has no tile, but its step counter still advances
     const int threads = block_threads(L);
     const int blocks = L.dense_blocks > 0 ? std::min(L.dense_blocks, P.row_blocks) : P.row_blocks;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3((unsigned)threads);
     // (another launch shape than the plan's may not hold every block in a wave)
     const bool stage = P.stage && L.dense_blocks == 0 && resident_blocks(2, threads) >= blocks;
-    cfg.dynamicSmemBytes = dyn_bytes(threads - 32, stage);
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, stage ? k_dense_step<false, true> : k_dense_step<false, false>, P, back) != cudaSuccess)
-        return -1;
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_dependent(stage ? k_dense_step<false, true> : k_dense_step<false, false>, blocks, threads,
+                            dyn_bytes(threads - 32, stage), P, back, stream);
 }
 
 int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, unsigned* bar, void* stream)
@@ -1043,8 +1050,8 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, un
 int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
     const int threads = block_threads(L);
-    k_dense_step<true, false><<<P.row_blocks, threads, dyn_bytes(threads - 32, false), (cudaStream_t)stream>>>(P, false);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_dependent(k_dense_step<true, false>, P.row_blocks, threads, dyn_bytes(threads - 32, false), P, false,
+                            stream);
 }
 
 }  // namespace nc

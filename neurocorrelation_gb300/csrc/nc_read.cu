@@ -14,11 +14,33 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// The read-backs are programmatic dependent launches: they are scheduled while the step (or
+// flush) before them drains, and wait here before they read anything (a step and two
+// read-backs of three neurons 39.4 -> 36.3 us).
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+int launch_dependent(void (*fn)(P...), dim3 grid, void* stream, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, fn, args...) != cudaSuccess) return -1;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
 unsigned blocks_for(int64_t items) { return (unsigned)((items + kThreads - 1) / kThreads); }
 
 // out[k] = src[index[k]]; NaN where the index is ~0 (a synapse that was not kept).
 __global__ void k_gather(const float* src, const uint32_t* index, int64_t count, float* out)
 {
+    wait_previous();
     const int64_t k = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (k >= count) return;
     const uint32_t c = __ldg(index + k);
@@ -31,6 +53,7 @@ __global__ void k_gather(const float* src, const uint32_t* index, int64_t count,
 __global__ void k_potact(const float* pot, const uint32_t* firings, const int32_t* start, const int32_t* slot_of,
                          int32_t n, int64_t t, float dt, float2* out)
 {
+    wait_previous();
     const int32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const int32_t s = __ldg(slot_of + i);
@@ -46,6 +69,7 @@ __global__ void k_potact(const float* pot, const uint32_t* firings, const int32_
 // Last fire of every neuron in ms, NaN for none, in the caller's order.
 __global__ void k_last_fire(const int32_t* lf, const int32_t* slot_of, int32_t n, float dt, float* out)
 {
+    wait_previous();
     const int32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const int32_t t = lf[__ldg(slot_of + i)];
@@ -58,6 +82,7 @@ constexpr int kRows = 8;
 __global__ void k_raster_bytes(const uint32_t* in, uint8_t* out, const int32_t* slot_of, int32_t n, int32_t n_words,
                                int32_t row_bytes, int32_t rows)
 {
+    wait_previous();
     const int32_t b = blockIdx.x * kThreads + threadIdx.x;
     if (b >= row_bytes) return;
     const int32_t r0 = blockIdx.y * kRows;
@@ -74,8 +99,6 @@ __global__ void k_raster_bytes(const uint32_t* in, uint8_t* out, const int32_t* 
     }
 }
 
-int status() { return cudaGetLastError() == cudaSuccess ? 0 : -1; }
-
 }  // namespace
 
 namespace nc {
@@ -83,25 +106,22 @@ namespace nc {
 int launch_gather(const float* src, const uint32_t* index, int64_t count, float* out, void* stream)
 {
     if (count <= 0) return 0;
-    k_gather<<<blocks_for(count), kThreads, 0, (cudaStream_t)stream>>>(src, index, count, out);
-    return status();
+    return launch_dependent(k_gather, dim3(blocks_for(count)), stream, src, index, count, out);
 }
 
 int launch_potact(const NcPools& P, int32_t neuron_base, int32_t first, int32_t n, int64_t t, float dt, float* out, void* stream)
 {
     if (n <= 0) return 0;
-    k_potact<<<blocks_for(n), kThreads, 0, (cudaStream_t)stream>>>(P.pot + neuron_base, P.firings + neuron_base,
-                                                                   P.act_start + neuron_base, P.slot_of + neuron_base + first,
-                                                                   n, t, dt, (float2*)out);
-    return status();
+    return launch_dependent(k_potact, dim3(blocks_for(n)), stream, (const float*)(P.pot + neuron_base),
+                            (const uint32_t*)(P.firings + neuron_base), (const int32_t*)(P.act_start + neuron_base),
+                            (const int32_t*)(P.slot_of + neuron_base + first), n, t, dt, (float2*)out);
 }
 
 int launch_last_fire(const NcPools& P, int32_t neuron_base, int32_t first, int32_t n, float dt, float* out, void* stream)
 {
     if (n <= 0) return 0;
-    k_last_fire<<<blocks_for(n), kThreads, 0, (cudaStream_t)stream>>>(P.lf + neuron_base, P.slot_of + neuron_base + first,
-                                                                      n, dt, out);
-    return status();
+    return launch_dependent(k_last_fire, dim3(blocks_for(n)), stream, (const int32_t*)(P.lf + neuron_base),
+                            (const int32_t*)(P.slot_of + neuron_base + first), n, dt, out);
 }
 
 int launch_raster_bytes(const uint32_t* in, uint8_t* out, const int32_t* slot_of, int32_t n, int32_t n_words,
@@ -112,11 +132,11 @@ int launch_raster_bytes(const uint32_t* in, uint8_t* out, const int32_t* slot_of
     // (a grid's second dimension is at most 65,535)
     for (int32_t r = 0; r < rows; r += 65535 * kRows) {
         const int32_t m = rows - r < 65535 * kRows ? rows - r : 65535 * kRows;
-        k_raster_bytes<<<dim3(blocks_for(row_bytes), (unsigned)((m + kRows - 1) / kRows)), kThreads, 0,
-                         (cudaStream_t)stream>>>(in + (int64_t)r * n_words, out + (int64_t)r * row_bytes, slot_of, n,
-                                                 n_words, row_bytes, m);
+        if (launch_dependent(k_raster_bytes, dim3(blocks_for(row_bytes), (unsigned)((m + kRows - 1) / kRows)), stream,
+                             in + (int64_t)r * n_words, out + (int64_t)r * row_bytes, slot_of, n, n_words, row_bytes, m))
+            return -1;
     }
-    return status();
+    return 0;
 }
 
 }  // namespace nc
