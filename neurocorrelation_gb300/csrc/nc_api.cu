@@ -615,7 +615,7 @@ int nc_read_weights(nc_net* net, float* out_s)
     const nc::NetHost& h = net->host;
     if (!out_s && h.n_input) return fail(NC_ERR_INVALID, "null output");
     NC_CALL0(net->eng, flush_plasticity);
-    if (!net->dev_i2c) net->dev_i2c = nc::upload_index(h.input_to_csc);
+    if (!net->dev_i2c) net->dev_i2c = net->eng.upload_index(h.input_to_csc);
     if (net->dev_i2c) {
         std::string err;
         const int rc = net->eng.read_weights(0, net->dev_i2c, h.n_input, out_s, err);

@@ -19,7 +19,7 @@ struct nc_batch {
     std::vector<int32_t> horizon;
     nc::Engine eng;
     int64_t ticks = 0;  // steps issued
-    std::vector<uint32_t*> index;  // per net, once its weights have been read (nc::upload_index)
+    std::vector<uint32_t*> index;  // per net, once its weights have been read (Engine::upload_index)
     ~nc_batch()
     {
         for (uint32_t* p : index)
@@ -275,7 +275,7 @@ int nc_batch_read_weights(nc_batch* b, int32_t net, float* out)
     B_CALL0(b->eng, flush_plasticity);
     if (b->index.empty()) b->index.resize(b->hosts.size(), nullptr);
     uint32_t*& index = b->index[(size_t)net];
-    if (!index) index = nc::upload_index(h.input_to_csc);
+    if (!index) index = b->eng.upload_index(h.input_to_csc);
     if (index) {
         std::string err;
         const int rc = b->eng.read_weights(net, index, h.n_input, out, err);

@@ -647,12 +647,15 @@ int Engine::read_raster(int net, const uint32_t* d_raster, int32_t rows, uint8_t
                       err);
 }
 
-uint32_t* upload_index(const std::vector<int64_t>& input_to_csc)
+uint32_t* Engine::upload_index(const std::vector<int64_t>& input_to_csc)
 {
     std::vector<uint32_t> index(input_to_csc.begin(), input_to_csc.end());  // -1 becomes ~0
     void* d = nullptr;
+    // on the engine's stream, and waited for: the gather that reads it is launched there, and a
+    // copy from pageable memory on the legacy stream may still be on its way when it returns
     if (cudaMalloc(&d, sizeof(uint32_t) * std::max<size_t>(index.size(), 1)) != cudaSuccess ||
-        cudaMemcpy(d, index.data(), sizeof(uint32_t) * index.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpyAsync(d, index.data(), sizeof(uint32_t) * index.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess ||
+        cudaStreamSynchronize(stream) != cudaSuccess) {
         cudaGetLastError();
         if (d) cudaFree(d);
         return nullptr;

@@ -53,6 +53,9 @@ public:
     int read_last_fire(int net, float* out, std::string& err);
     // index: device array, the CSC position of each synapse (~0: not kept)
     int read_weights(int net, const uint32_t* index, int64_t count, float* out, std::string& err);
+    // The CSC positions of a net's input synapses on the device (freed by the caller), or null
+    // when there is no memory for them: the read-back then reorders on the host.
+    uint32_t* upload_index(const std::vector<int64_t>& input_to_csc);
     int read_raster(int net, const uint32_t* d_raster, int32_t rows, uint8_t* out, std::string& err);
     int sync(std::string& err);
 
@@ -118,9 +121,6 @@ private:
 int dense_blocks(int64_t neurons, int threads);
 // Neurons per warp of the event form's kernels, for an engine of so many 32-neuron tiles.
 void event_rows(int64_t tiles, int sms, NcPools& P);
-// The CSC positions of a net's input synapses on the device (freed by the caller), or null
-// when there is no memory for them: the read-back then reorders on the host.
-uint32_t* upload_index(const std::vector<int64_t>& input_to_csc);
 std::string cuda_msg(const char* what, cudaError_t e);
 // Records the calling thread's last error (nc_last_error) and returns `code`.
 int set_last_error(int code, const std::string& msg);

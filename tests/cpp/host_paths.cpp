@@ -1,0 +1,90 @@
+// The library's host code on a device of host memory (fake_device.h): host_paths <check>.
+#include "fake_device.h"
+
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <string>
+#include <vector>
+
+static int fails = 0;
+
+static void check(bool ok, const std::string& what)
+{
+    if (!ok) std::printf("FAIL %s\n", what.c_str());
+    fails += ok ? 0 : 1;
+}
+
+struct Made {
+    std::vector<float> xyz, w;
+    std::vector<int32_t> from, to;
+    nc_params p{};
+    int32_t n;
+    explicit Made(int32_t neurons, int32_t synapses, int mode = NC_STEP_DENSE) : n(neurons)
+    {
+        nc_default_params(&p);
+        p.step_mode = mode;
+        for (int32_t i = 0; i < 3 * n; ++i) xyz.push_back((float)(i * 7919 % 101) / 40.0f);
+        for (int32_t k = 0; k < synapses; ++k) {
+            from.push_back(k * 31 % n);
+            to.push_back(k * 17 % n);
+            w.push_back((float)(k + 1) / (float)(synapses + 1));
+        }
+    }
+    nc_net* create()
+    {
+        nc_net* net = nullptr;
+        const int rc = nc_create(n, xyz.data(), (int64_t)w.size(), from.data(), to.data(), w.data(), nullptr, nullptr, &p, &net);
+        check(rc == NC_OK, std::string("create: ") + nc_last_error());
+        return net;
+    }
+    nc_net_spec spec(int32_t horizon)
+    {
+        nc_net_spec s{};
+        s.n_neurons = n;
+        s.xyz = xyz.data();
+        s.n_synapses = (int64_t)w.size();
+        s.syn_from = from.data();
+        s.syn_to = to.data();
+        s.syn_weight = w.data();
+        s.params = p;
+        s.horizon = horizon;
+        return s;
+    }
+    // weights read back: as given, NaN where a pair is repeated
+    bool same(const std::vector<float>& got) const
+    {
+        for (size_t k = 0; k < w.size(); ++k)
+            if (!(got[k] == w[k] || std::isnan(got[k]))) return false;
+        return true;
+    }
+};
+
+// Weights read for the first time, however late the legacy stream's work is done.
+static void weights_order()
+{
+    for (int delay : {0, 1, 2, 3, 5, 9, 1000}) {
+        fake::legacy_delay = delay;
+        Made m(50, 400);
+        std::vector<float> got(m.w.size());
+        nc_net* net = m.create();
+        check(nc_read_weights(net, got.data()) == NC_OK && m.same(got), "weights, delay " + std::to_string(delay));
+        nc_destroy(net);
+        nc_net_spec specs[2] = {m.spec(5), m.spec(9)};
+        nc_batch* b = nullptr;
+        check(nc_batch_create(2, specs, &b) == NC_OK, "batch");
+        for (int32_t q = 0; q < 2; ++q)
+            check(nc_batch_read_weights(b, q, got.data()) == NC_OK && m.same(got), "batch weights, delay " + std::to_string(delay));
+        nc_batch_destroy(b);
+    }
+    check(fake::faults == 0, "positions out of range");
+}
+
+int main(int argc, char** argv)
+{
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "weights_order") weights_order();
+    else check(false, "no such check: " + what);
+    std::printf("%s\n", fails ? "FAILED" : "OK");
+    return fails != 0;
+}
