@@ -555,7 +555,9 @@ int nc_record_raster(nc_net* net, int32_t max_steps)
         const size_t words = (size_t)max_steps * net->eng.slots[0].n_words;
         cudaError_t e = cudaMalloc(&net->d_raster, std::max<size_t>(words, 1) * sizeof(uint32_t));
         if (e != cudaSuccess) return fail(NC_ERR_NOMEM, nc::cuda_msg("cudaMalloc raster", e));
-        e = cudaMemset(net->d_raster, 0, std::max<size_t>(words, 1) * sizeof(uint32_t));
+        // (on the handle's stream, which the steps that write the rows run on; the legacy
+        // stream's work may come after theirs)
+        e = cudaMemsetAsync(net->d_raster, 0, std::max<size_t>(words, 1) * sizeof(uint32_t), net->eng.stream);
         if (e != cudaSuccess) return fail(NC_ERR_CUDA, nc::cuda_msg("cudaMemset raster", e));
         net->raster_cap = max_steps;
     }

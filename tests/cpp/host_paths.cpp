@@ -80,10 +80,29 @@ static void weights_order()
     check(fake::faults == 0, "positions out of range");
 }
 
+// The raster's rows are cleared before the steps that write them.
+static void raster_order()
+{
+    for (int delay = 0; delay < 24; ++delay) {
+        fake::legacy_delay = delay;
+        Made m(64, 300);
+        nc_net* net = m.create();
+        std::vector<uint8_t> rows(5 * 8, 0);
+        int32_t steps = 0;
+        check(nc_record_raster(net, 5) == NC_OK && nc_run(net, 4) == NC_OK, "run");
+        check(nc_read_raster(net, rows.data(), (int64_t)rows.size(), &steps) == NC_OK && steps == 4, "read");
+        check(rows == std::vector<uint8_t>([] { std::vector<uint8_t> v(32, 0xff); v.resize(40, 0); return v; }()),
+              "rows of the steps, delay " + std::to_string(delay));
+        nc_destroy(net);
+    }
+    check(fake::faults == 0, "rows out of range");
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "weights_order") weights_order();
+    else if (what == "raster_order") raster_order();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
