@@ -547,6 +547,8 @@ int nc_record_raster(nc_net* net, int32_t max_steps)
     NC_CALL0(net->eng, sync);
     net->raster_t0 = (int32_t)net->step + 1;
     if (net->d_raster && max_steps != net->raster_cap) {
+        // (the steps' descriptor lets go of it first: a new one may not be had)
+        NC_CALL(net->eng, set_raster, 0, nullptr, net->raster_t0, 0);
         cudaFree(net->d_raster);
         net->d_raster = nullptr;
         net->raster_cap = 0;

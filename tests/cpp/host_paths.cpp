@@ -98,11 +98,29 @@ static void raster_order()
     check(fake::faults == 0, "rows out of range");
 }
 
+// A raster that cannot be replaced for want of memory is no longer written.
+static void raster_refused()
+{
+    Made m(64, 300);
+    nc_net* net = m.create();
+    check(nc_record_raster(net, 5) == NC_OK && nc_run(net, 2) == NC_OK, "run");
+    fake::fail_malloc_from = 8 * 70;
+    check(nc_record_raster(net, 70) == NC_ERR_NOMEM, "refused");
+    check(nc_run(net, 2) == NC_OK && fake::faults == 0, "steps after it");
+    int32_t steps = -1;
+    uint8_t none[1];
+    check(nc_read_raster(net, none, 1, &steps) == NC_OK && steps == 0, "no rows");
+    fake::fail_malloc_from = ~(size_t)0;
+    check(nc_record_raster(net, 70) == NC_OK && nc_run(net, 2) == NC_OK && fake::faults == 0, "made later");
+    nc_destroy(net);
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "weights_order") weights_order();
     else if (what == "raster_order") raster_order();
+    else if (what == "raster_refused") raster_refused();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
