@@ -384,7 +384,8 @@ int nc_set_detectors(nc_net* net, int32_t count, const float* xyz, const float* 
     cudaError_t e = cudaMalloc(&net->d_det, sizeof(int32_t) * flat.size());
     if (e == cudaSuccess) e = cudaMalloc(&net->d_volt, sizeof(float) * std::max<size_t>(n_det, 1));
     if (e == cudaSuccess)
-        e = cudaMemcpy(net->d_det, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(net->d_det, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice, net->eng.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(net->eng.stream);  // (`flat` goes)
     if (e != cudaSuccess) return fail(NC_ERR_CUDA, nc::cuda_msg("detector tables", e));
     return NC_OK;
 }

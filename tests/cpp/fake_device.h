@@ -249,12 +249,12 @@ int launch_detector_voltages(const NcPools& P, int32_t base, const int32_t* near
 {
     return fake::launch([=] {
         for (int32_t d = 0; d < count; ++d) {
-            out[d] = 0.0f;
-            if (!fake::device_range(near_ptr + d, 8) || near_ptr[d] < 0 || near_ptr[d + 1] < near_ptr[d] ||
+            if (!fake::device_range(out + d, 4) || !fake::device_range(near_ptr + d, 8) || near_ptr[d] < 0 || near_ptr[d + 1] < near_ptr[d] ||
                 !fake::device_range(near + near_ptr[d], 4 * (size_t)(near_ptr[d + 1] - near_ptr[d]))) {
                 ++fake::faults;
                 continue;
             }
+            out[d] = 0.0f;
             for (int32_t k = near_ptr[d]; k < near_ptr[d + 1]; ++k) out[d] += P.pot[base + P.slot_of[base + near[k]]];
             out[d] /= (float)(near_ptr[d + 1] - near_ptr[d]);
         }

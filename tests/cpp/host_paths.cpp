@@ -115,12 +115,30 @@ static void raster_refused()
     nc_destroy(net);
 }
 
+// Detectors' tables are on the device before they are read.
+static void detectors_order()
+{
+    for (int delay : {0, 1, 2, 5, 1000}) {
+        fake::legacy_delay = delay;
+        Made m(40, 100);
+        nc_net* net = m.create();
+        const float at[6] = {1, 1, 1, 0.5f, 1, 1.5f}, radius[2] = {9, 9};
+        float v[2] = {0, 0};
+        check(nc_set_detectors(net, 2, at, radius) == NC_OK, "set");
+        check(nc_get_detector_voltages(net, v, 2, nullptr) == NC_OK && v[0] == -70.0f && v[1] == -70.0f,
+              "voltages, delay " + std::to_string(delay));
+        nc_destroy(net);
+    }
+    check(fake::faults == 0, "neurons out of range");
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "weights_order") weights_order();
     else if (what == "raster_order") raster_order();
     else if (what == "raster_refused") raster_refused();
+    else if (what == "detectors_order") detectors_order();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
