@@ -358,6 +358,7 @@ int nc_set_detectors(nc_net* net, int32_t count, const float* xyz, const float* 
     if (count < 0 || count > (1 << 24)) return fail(NC_ERR_INVALID, "bad detector count");
     if (xyz && !radius) return fail(NC_ERR_INVALID, "positions given without radii");
     // NeuCor::setDetectors (src/NeuCor.cpp:70-77) appends `count` detectors
+    std::vector<int32_t> det_near(net->det_near), det_ptr(net->det_ptr);
     for (int32_t i = 0; i < count; ++i) {
         float a[3];
         float r = 1.0f;
@@ -370,23 +371,31 @@ int nc_set_detectors(nc_net* net, int32_t count, const float* xyz, const float* 
             for (int d = 0; d < 3; ++d) a[d] = (random_unit() - 0.5f) * 3.f;
         }
         const std::vector<int32_t> ids = near_ids(net->host, a, r);
-        net->det_near.insert(net->det_near.end(), ids.begin(), ids.end());
-        net->det_ptr.push_back((int32_t)net->det_near.size());
+        det_near.insert(det_near.end(), ids.begin(), ids.end());
+        det_ptr.push_back((int32_t)det_near.size());
     }
     // device copies: near ids, then the pointer array; one voltage per detector
+    std::vector<int32_t> flat(det_near);
+    flat.insert(flat.end(), det_ptr.begin(), det_ptr.end());
+    int32_t* d_det = nullptr;
+    float* d_volt = nullptr;
+    cudaError_t e = cudaMalloc(&d_det, sizeof(int32_t) * flat.size());
+    if (e == cudaSuccess) e = cudaMalloc(&d_volt, sizeof(float) * std::max<size_t>(det_ptr.size() - 1, 1));
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(d_det, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice, net->eng.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(net->eng.stream);  // (`flat` goes)
+    if (e != cudaSuccess) {  // the detectors there were stay
+        cudaGetLastError();
+        if (d_det) cudaFree(d_det);
+        if (d_volt) cudaFree(d_volt);
+        return fail(NC_ERR_CUDA, nc::cuda_msg("detector tables", e));
+    }
     if (net->d_det) cudaFree(net->d_det);
     if (net->d_volt) cudaFree(net->d_volt);
-    net->d_det = nullptr;
-    net->d_volt = nullptr;
-    std::vector<int32_t> flat(net->det_near);
-    flat.insert(flat.end(), net->det_ptr.begin(), net->det_ptr.end());
-    const size_t n_det = net->det_ptr.size() - 1;
-    cudaError_t e = cudaMalloc(&net->d_det, sizeof(int32_t) * flat.size());
-    if (e == cudaSuccess) e = cudaMalloc(&net->d_volt, sizeof(float) * std::max<size_t>(n_det, 1));
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(net->d_det, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice, net->eng.stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(net->eng.stream);  // (`flat` goes)
-    if (e != cudaSuccess) return fail(NC_ERR_CUDA, nc::cuda_msg("detector tables", e));
+    net->d_det = d_det;
+    net->d_volt = d_volt;
+    net->det_near.swap(det_near);
+    net->det_ptr.swap(det_ptr);
     return NC_OK;
 }
 

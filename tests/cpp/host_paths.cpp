@@ -132,6 +132,29 @@ static void detectors_order()
     check(fake::faults == 0, "neurons out of range");
 }
 
+// Detectors that cannot be added for want of memory leave the ones before them.
+static void detectors_refused()
+{
+    const float at[3] = {1, 1, 1}, radius[1] = {9};
+    for (int64_t call = 0; call < 2; ++call) {
+        Made m(40, 100);
+        nc_net* net = m.create();
+        for (int round = 0; round < 2; ++round) {
+            float v[2] = {0, 0};
+            int32_t count = -1;
+            fake::fail_malloc_at = fake::mallocs + call;
+            check(nc_set_detectors(net, 1, at, radius) == NC_ERR_CUDA, "refused");
+            fake::fail_malloc_at = -1;
+            check(nc_get_detector_voltages(net, v, 2, &count) == NC_OK && count == round, "as many as before");
+            check(fake::faults == 0 && v[0] == (round ? -70.0f : 0.0f), "voltages");
+            check(nc_set_detectors(net, 1, at, radius) == NC_OK, "added later");
+        }
+        const size_t held = fake::held;
+        nc_destroy(net);
+        check(held > 0 && fake::held == 0, "memory given back");
+    }
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -139,6 +162,7 @@ int main(int argc, char** argv)
     else if (what == "raster_order") raster_order();
     else if (what == "raster_refused") raster_refused();
     else if (what == "detectors_order") detectors_order();
+    else if (what == "detectors_refused") detectors_refused();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
