@@ -207,7 +207,7 @@ static int ensure_host_tables(nc_net* net)
     std::vector<uint32_t> index((size_t)S);
     std::vector<int32_t> to((size_t)S);
     std::vector<uint32_t> key((size_t)h.sp);
-    NC_CALL(net->eng, download, index.data(), (const uint32_t*)net->dev_i2c, (size_t)S);
+    NC_CALL(net->eng, download, index.data(), (const uint32_t*)net->eng.index(0), (size_t)S);
     std::vector<int64_t> i2c(index.begin(), index.end());
     NC_CALL(net->eng, download, to.data(), (const int32_t*)net->dev_to, (size_t)S);
     // the words with the delays: the second range of a wide net
@@ -629,15 +629,11 @@ int nc_read_weights(nc_net* net, float* out_s)
     const nc::NetHost& h = net->host;
     if (!out_s && h.n_input) return fail(NC_ERR_INVALID, "null output");
     NC_CALL0(net->eng, flush_plasticity);
-    if (!net->dev_i2c) net->dev_i2c = net->eng.upload_index(h.input_to_csc);
-    if (net->dev_i2c) {
-        std::string err;
-        const int rc = net->eng.read_weights(0, net->dev_i2c, h.n_input, out_s, err);
-        if (rc == NC_OK) return NC_OK;
-        if (rc != NC_ERR_NOMEM) return fail(rc, err);
+    if (net->eng.index(0)) {
+        NC_CALL(net->eng, read_weights, 0, out_s);
+        return NC_OK;
     }
-    // no device memory for the gather: reorder on the host
-    if (int rc = ensure_host_tables(net)) return rc;
+    // (no device memory for the index when the network was made)
     std::vector<float> w((size_t)h.sp);
     NC_CALL(net->eng, download, w.data(), (const float*)net->eng.P.w + net->eng.slots[0].syn_base, (size_t)h.sp);
     for (int64_t k = 0; k < h.n_input; ++k) {

@@ -19,12 +19,6 @@ struct nc_batch {
     std::vector<int32_t> horizon;
     nc::Engine eng;
     int64_t ticks = 0;  // steps issued
-    std::vector<uint32_t*> index;  // per net, once its weights have been read (Engine::upload_index)
-    ~nc_batch()
-    {
-        for (uint32_t* p : index)
-            if (p) cudaFree(p);
-    }
 };
 
 #define B_NEED(b)                                                    \
@@ -273,16 +267,11 @@ int nc_batch_read_weights(nc_batch* b, int32_t net, float* out)
     const nc::NetHost& h = b->hosts[(size_t)net];
     if (!out && h.n_input) return bfail(NC_ERR_INVALID, "null output");
     B_CALL0(b->eng, flush_plasticity);
-    if (b->index.empty()) b->index.resize(b->hosts.size(), nullptr);
-    uint32_t*& index = b->index[(size_t)net];
-    if (!index) index = b->eng.upload_index(h.input_to_csc);
-    if (index) {
-        std::string err;
-        const int rc = b->eng.read_weights(net, index, h.n_input, out, err);
-        if (rc == NC_OK) return NC_OK;
-        if (rc != NC_ERR_NOMEM) return bfail(rc, err);
+    if (b->eng.index(net)) {
+        B_CALL(b->eng, read_weights, net, out);
+        return NC_OK;
     }
-    // no device memory for the gather: reorder on the host
+    // (no device memory for the index when the batch was made)
     const auto& sl = b->eng.slots[(size_t)net];
     std::vector<float> w((size_t)h.sp);
     B_CALL(b->eng, download, w.data(), (const float*)b->eng.P.w + sl.syn_base, (size_t)h.sp);

@@ -511,7 +511,8 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     if (rc != NC_OK) return rc;
     unsigned long long* d_cur = own.get<unsigned long long>((size_t)n);
     unsigned long long* d_rows = own.get<unsigned long long>((size_t)h.sp);
-    uint32_t* d_i2c = own.get<uint32_t>((size_t)edges, true);
+    uint32_t* d_i2c = net->eng.index(0);
+    if (e == cudaSuccess && !d_i2c) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess)
         e = cudaMemcpy(d_cur, h.in_ptr.data(), sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -534,9 +535,7 @@ int build_knn_device(int32_t n, int32_t k, float density, uint64_t seed, const n
     }
     // read-back tables stay on the device until a read-back asks for them
     net->dev_to = d_to;
-    net->dev_i2c = d_i2c;
     own.give(d_to);
-    own.give(d_i2c);
     net->knn_k = k;
     return NC_OK;
 }

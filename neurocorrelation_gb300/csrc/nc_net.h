@@ -29,9 +29,6 @@ struct nc_net {
     std::vector<int32_t> det_near, det_ptr{0};
     int32_t* d_det = nullptr;      // det_near then det_ptr on the device
     float* d_volt = nullptr;
-    // CSC position of every input synapse on the device (~0: not kept): from nc_create_knn, or
-    // uploaded by the first weight read-back
-    uint32_t* dev_i2c = nullptr;
     // built on the device (nc_create_knn): targets in creation order, kept until a read-back
     // needs the host tables
     int32_t* dev_to = nullptr;
@@ -39,7 +36,6 @@ struct nc_net {
     ~nc_net()
     {
         if (dev_to) cudaFree(dev_to);
-        if (dev_i2c) cudaFree(dev_i2c);
         if (d_raster) cudaFree(d_raster);
         if (d_det) cudaFree(d_det);
         if (d_volt) cudaFree(d_volt);

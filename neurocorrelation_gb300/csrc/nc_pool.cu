@@ -151,7 +151,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
 
     // pool sizes
-    int64_t neurons = 0, ptrs = 0, words = 0, syn = 0, ring = 0, tables = 0, tiles = 0;
+    int64_t neurons = 0, ptrs = 0, words = 0, syn = 0, ring = 0, tables = 0, tiles = 0, inputs = 0;
     const int ngroups_each = std::max(group_capacity, 1);
     slots.clear();
     std::vector<NcNetDesc> desc;
@@ -167,6 +167,9 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         sl.ptr_base = (int32_t)ptrs;
         sl.word_base = (int32_t)words;
         sl.syn_base = syn;
+        sl.n_input = h.n_input;
+        sl.index_base = inputs;
+        inputs += h.n_input;
         sl.group_cap = ngroups_each;
         sl.group_base = (int32_t)(q * ngroups_each);
         NcNetDesc d;
@@ -342,6 +345,19 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         NC_ALLOC(P.rstart, int32_t, start.size());
         NC_CK(upload(P.rtiles, rows, 0, stream));
         NC_CK(upload(P.rstart, start, 0, stream));
+        NC_CK(cudaStreamSynchronize(stream));
+    }
+    // The positions of the given synapses, for the read-back of the weights: with the network's
+    // other arrays, so that no read-back allocates.  (Last: where memory is short the host
+    // reorders instead.)
+    index_ = alloc<uint32_t>((size_t)inputs, err);
+    if (!index_) {
+        cudaGetLastError();
+        err.clear();
+    }
+    for (size_t q = 0; index_ && !device_synapses && q < nets.size(); ++q) {
+        const std::vector<uint32_t> index(nets[q]->input_to_csc.begin(), nets[q]->input_to_csc.end());  // -1 becomes ~0
+        NC_CK(upload(index_, index, (size_t)slots[q].index_base, stream));
         NC_CK(cudaStreamSynchronize(stream));
     }
     NC_CK(cudaStreamSynchronize(stream));
@@ -628,11 +644,12 @@ int Engine::read_last_fire(int net, float* out, std::string& err)
                       err);
 }
 
-int Engine::read_weights(int net, const uint32_t* index, int64_t count, float* out, std::string& err)
+int Engine::read_weights(int net, float* out, std::string& err)
 {
     const float* w = P.w + slots[(size_t)net].syn_base;
-    return read_parts(count, sizeof(float), shared_tables_, scratch_, scratch_bytes_, out, stream,
-                      [&](int64_t a, int64_t m, void* buf) { return launch_gather(w, index + a, m, (float*)buf, stream); },
+    const uint32_t* at = index(net);
+    return read_parts(slots[(size_t)net].n_input, sizeof(float), shared_tables_, scratch_, scratch_bytes_, out, stream,
+                      [&](int64_t a, int64_t m, void* buf) { return launch_gather(w, at + a, m, (float*)buf, stream); },
                       err);
 }
 
@@ -645,22 +662,6 @@ int Engine::read_raster(int net, const uint32_t* d_raster, int32_t rows, uint8_t
                                                      sl.n, sl.n_words, (int32_t)m, stream);
                       },
                       err);
-}
-
-uint32_t* Engine::upload_index(const std::vector<int64_t>& input_to_csc)
-{
-    std::vector<uint32_t> index(input_to_csc.begin(), input_to_csc.end());  // -1 becomes ~0
-    void* d = nullptr;
-    // on the engine's stream, and waited for: the gather that reads it is launched there, and a
-    // copy from pageable memory on the legacy stream may still be on its way when it returns
-    if (cudaMalloc(&d, sizeof(uint32_t) * std::max<size_t>(index.size(), 1)) != cudaSuccess ||
-        cudaMemcpyAsync(d, index.data(), sizeof(uint32_t) * index.size(), cudaMemcpyHostToDevice, stream) != cudaSuccess ||
-        cudaStreamSynchronize(stream) != cudaSuccess) {
-        cudaGetLastError();
-        if (d) cudaFree(d);
-        return nullptr;
-    }
-    return (uint32_t*)d;
 }
 
 int Engine::set_form(bool to_dense, std::string& err)

@@ -17,6 +17,7 @@ struct NetSlot {       // host view of one packed net
     float dt = 1.0f;
     int32_t n_words = 0;
     int64_t syn_base = 0;
+    int64_t n_input = 0, index_base = 0;  // synapses given, the first one's place in the index
     int32_t neuron_base = 0, ptr_base = 0, word_base = 0, group_cap = 0, group_base = 0;
 };
 
@@ -51,13 +52,14 @@ public:
     int read_potentials(int net, float* out, std::string& err);
     int read_potact(int net, int64_t t, float* out_2n, std::string& err);
     int read_last_fire(int net, float* out, std::string& err);
-    // index: device array, the CSC position of each synapse (~0: not kept)
-    int read_weights(int net, const uint32_t* index, int64_t count, float* out, std::string& err);
-    // The CSC positions of a net's input synapses on the device (freed by the caller), or null
-    // when there is no memory for them: the read-back then reorders on the host.
-    uint32_t* upload_index(const std::vector<int64_t>& input_to_csc);
+    // (needs index(net))
+    int read_weights(int net, float* out, std::string& err);
     int read_raster(int net, const uint32_t* d_raster, int32_t rows, uint8_t* out, std::string& err);
     int sync(std::string& err);
+    // The CSC position of each of a net's given synapses (~0: not kept) on the device, made with
+    // the pools; null when there was no memory for them: the weights are then reordered on the
+    // host.  device_synapses: written by the caller.
+    uint32_t* index(int net) const { return index_ ? index_ + slots[(size_t)net].index_base : nullptr; }
 
     int set_groups(int net, const std::vector<NcGroupDev>& groups, std::string& err);
     int set_rates(int net, float lr, float pre_factor, float post_factor, std::string& err);
@@ -99,6 +101,7 @@ private:
     // or kScratchMax of it at a time.
     static constexpr size_t kScratchMax = 64 << 20;
     void* scratch_ = nullptr;
+    uint32_t* index_ = nullptr;
     bool shared_tables_ = false;  // the GPU uses the host's page tables: it can write ordinary host memory
     size_t scratch_bytes_ = 0;
     bool flushed_ = false, unseen_ = false;

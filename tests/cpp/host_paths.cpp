@@ -155,6 +155,76 @@ static void detectors_refused()
     }
 }
 
+// Every read-back of a network's results, once.
+static bool reads(nc_net* net, const Made& m)
+{
+    std::vector<float> w(m.w.size()), per(2 * (size_t)m.n);
+    std::vector<int32_t> d(m.w.size());
+    std::vector<uint8_t> inh(m.w.size()), rows(4 * (((size_t)m.n + 7) / 8));
+    std::vector<nc_synapse_snapshot> snap(m.w.size());
+    int64_t count = 0;
+    int32_t steps = 0;
+    nc_stats st;
+    return nc_read_weights(net, w.data()) == NC_OK && m.same(w) && nc_read_potentials(net, per.data()) == NC_OK &&
+           nc_read_potact(net, per.data()) == NC_OK && nc_read_last_fire(net, per.data()) == NC_OK &&
+           nc_read_delays(net, d.data()) == NC_OK && nc_read_inhibitory(net, inh.data()) == NC_OK &&
+           nc_read_raster(net, rows.data(), (int64_t)rows.size(), &steps) == NC_OK &&
+           nc_read_synapse_snapshots(net, snap.data(), (int64_t)snap.size(), &count) == NC_OK &&
+           nc_get_stats(net, &st) == NC_OK;
+}
+
+// A read-back allocates no device memory, the first one neither.
+static void reads_allocate_nothing()
+{
+    for (int mode : {NC_STEP_DENSE, NC_STEP_EVENT, NC_STEP_AUTO}) {
+        Made m(200, 3000, mode);
+        nc_net* net = m.create();
+        check(nc_record_raster(net, 4) == NC_OK && nc_run_noalloc(net, 4, nullptr) == NC_OK, "run");
+        const int64_t calls = fake::mallocs;
+        const size_t held = fake::held;
+        check(reads(net, m), std::string("reads: ") + nc_last_error());
+        check(fake::mallocs == calls && fake::held == held, "allocations in the reads of form " + std::to_string(mode));
+        nc_destroy(net);
+    }
+    Made a(200, 3000), b(31, 90);
+    nc_net_spec specs[2] = {a.spec(5), b.spec(9)};
+    nc_batch* batch = nullptr;
+    check(nc_batch_create(2, specs, &batch) == NC_OK, "batch");
+    const int64_t calls = fake::mallocs;
+    std::vector<float> got(a.w.size());
+    check(nc_batch_read_weights(batch, 0, got.data()) == NC_OK && a.same(got), "first network");
+    check(nc_batch_read_weights(batch, 1, got.data()) == NC_OK && b.same(got), "second network");
+    check(fake::mallocs == calls, "allocations in the reads of a batch");
+    nc_batch_destroy(batch);
+    check(fake::held == 0, "memory given back");
+}
+
+// Without memory for the weights' index a network is made all the same, and its weights read.
+static void no_index()
+{
+    for (int mode : {NC_STEP_DENSE, NC_STEP_EVENT}) {
+        Made m(2000, 100000, mode);  // (its index is too large for a block of small arrays)
+        int64_t before = fake::mallocs;
+        nc_destroy(m.create());
+        const int64_t calls = fake::mallocs - before;
+        fake::fail_malloc_at = fake::mallocs + calls - 1;
+        nc_net* net = m.create();
+        fake::fail_malloc_at = -1;
+        before = fake::mallocs;
+        check(net && reads(net, m), std::string("reads: ") + nc_last_error());
+        check(fake::mallocs == before, "allocations");
+        nc_destroy(net);
+        nc_net_spec spec = m.spec(5);
+        nc_batch* b = nullptr;
+        std::vector<float> got(m.w.size());
+        fake::fail_malloc_at = fake::mallocs + calls - 1;
+        check(nc_batch_create(1, &spec, &b) == NC_OK, "batch");
+        fake::fail_malloc_at = -1;
+        check(nc_batch_read_weights(b, 0, got.data()) == NC_OK && m.same(got), "batch weights");
+        nc_batch_destroy(b);
+    }
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -163,6 +233,8 @@ int main(int argc, char** argv)
     else if (what == "raster_refused") raster_refused();
     else if (what == "detectors_order") detectors_order();
     else if (what == "detectors_refused") detectors_refused();
+    else if (what == "reads_allocate_nothing") reads_allocate_nothing();
+    else if (what == "no_index") no_index();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
