@@ -1,12 +1,17 @@
 // nc_pool.cu — the device engine (see nc_pool.h).
 #include "nc_pool.h"
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
 #include <cstddef>
 #include <cstring>
 #include <string>
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23  // Linux 5.14; older kernels refuse it
+#endif
 
 namespace nc {
 
@@ -557,11 +562,13 @@ int Engine::flush_plasticity(std::string& err)
     return NC_OK;
 }
 
-// Writes a byte of every page of a buffer that is about to be filled, where it is ordinary
-// host memory (and says whether it is).  A bad pointer faults here, as in a copy; and a page that is not there
-// yet costs the host less than it costs the GPU, whose page tables are the host's: with a
-// copy into fresh pages, 400 KB 39 us instead of 151, 2 MB 99 instead of 218, 40 MB 1,516
-// instead of 1,525, and nothing where the GPU is still at work on the steps before.
+// Has the pages of a buffer that is about to be filled made present and writable, where it is
+// ordinary host memory (and says whether they are).  A page that is not there yet costs the
+// host less than it costs the GPU, whose page tables are the host's: with a copy into fresh
+// pages, 400 KB 39 us instead of 151, 2 MB 99 instead of 218, and nothing where the GPU is
+// still at work on the steps before (a byte written to each page, before: 40 MB 1,590 us, 1,480
+// now).  The contents stay as they are until the result is there; what cannot be written is
+// left to the copy to report.
 static bool bring_in(void* out, size_t bytes)
 {
     cudaPointerAttributes at;
@@ -570,10 +577,23 @@ static bool bring_in(void* out, size_t bytes)
         return false;
     }
     if (at.type != cudaMemoryTypeUnregistered) return false;
-    static const size_t page = (size_t)std::max<long>(4096, sysconf(_SC_PAGESIZE));
-    volatile char* p = (volatile char*)out;
-    for (size_t k = 0; k < bytes; k += page) p[k] = 0;  // (a read first would map the zero page)
-    p[bytes - 1] = 0;
+    if (bytes <= 4096) {  // a page or two, nearly always there: a store of what is there saves the system calls
+        __atomic_fetch_or((char*)out, 0, __ATOMIC_RELAXED);
+        __atomic_fetch_or((char*)out + bytes - 1, 0, __ATOMIC_RELAXED);
+        return true;
+    }
+    static const uintptr_t page = (uintptr_t)std::max<long>(4096, sysconf(_SC_PAGESIZE));
+    const uintptr_t from = (uintptr_t)out / page * page;
+    const size_t length = (uintptr_t)out + bytes - from;
+    constexpr size_t kChunk = 1024;
+    unsigned char there[kChunk];
+    for (size_t a = 0; a < length; a += kChunk * page) {
+        const size_t m = std::min(length - a, kChunk * page);
+        // (many pages that are there are only looked at: 40 MB 4 us instead of 80)
+        bool all = m >= 16 * page && mincore((void*)(from + a), m, there) == 0;
+        for (size_t k = 0; all && k * page < m; ++k) all = there[k] & 1;
+        if (!all && madvise((void*)(from + a), m, MADV_POPULATE_WRITE) != 0) return false;
+    }
     return true;
 }
 

@@ -225,6 +225,22 @@ static void no_index()
     }
 }
 
+// A read-back whose kernel cannot be launched leaves the caller's buffer as it was.
+static void failed_read()
+{
+    for (int32_t synapses : {300, 40000, 200000}) {  // one page, several, more than are written directly
+        Made m(1000, synapses);
+        nc_net* net = m.create();
+        std::vector<float> old(m.w.size()), got(m.w.size());
+        for (size_t k = 0; k < old.size(); ++k) old[k] = got[k] = -1.0f - (float)k;
+        fake::gathers_to_fail = 1;
+        check(nc_read_weights(net, got.data()) == NC_ERR_CUDA, "reported");
+        check(got == old, "contents, " + std::to_string(synapses) + " synapses");
+        check(nc_read_weights(net, got.data()) == NC_OK && m.same(got), "read later");
+        nc_destroy(net);
+    }
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -235,6 +251,7 @@ int main(int argc, char** argv)
     else if (what == "detectors_refused") detectors_refused();
     else if (what == "reads_allocate_nothing") reads_allocate_nothing();
     else if (what == "no_index") no_index();
+    else if (what == "failed_read") failed_read();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
