@@ -387,7 +387,9 @@ typedef struct {
 
 typedef struct {
     int64_t request_id;
-    int32_t status;    /* NC_OK, or why the request was refused (NC_ERR_BUDGET, NC_ERR_INVALID) */
+    int32_t status;    /* NC_OK, why the request was refused (NC_ERR_BUDGET, NC_ERR_INVALID), or
+                          NC_ERR_CUDA: its results could not be read, or the device was lost (every
+                          request then finishes so) */
     int32_t n_neurons;
     int32_t horizon;
     int32_t reserved;

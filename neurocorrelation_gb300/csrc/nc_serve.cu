@@ -169,6 +169,9 @@ struct nc_server {
     // scheduler thread only: prepared requests that do not fit yet, resident networks
     std::map<int64_t, std::unique_ptr<Resident>> waiting;
     std::vector<std::unique_ptr<Resident>> active;
+    // why the device can no longer be used (NC_OK: it can): every request left then finishes
+    // with it
+    int lost = NC_OK;
 
     double now() const
     {
@@ -180,7 +183,11 @@ struct nc_server {
     void scheduler_loop();
     int admit(Resident& r, std::string& err);
     int gather_weights(const Resident& r, float* out, std::string& err);
+    int collect(const Resident& r, nc_request_done& d, Kept& k, std::string& err);
     int retire(Resident& r, std::string& err);
+    int run_batch(float& ms, std::string& err);
+    nc_request_done outcome(const Resident& r, int status) const;
+    void fail_active(int status);
     int upload_tiles(std::string& err);
     int capture(std::string& err);
 };
@@ -575,6 +582,35 @@ int nc_server::gather_weights(const Resident& r, float* out, std::string& err)
     return NC_OK;
 }
 
+// The results of a network that has run its last step.  The stream is waited for on every way
+// out: the copies are into buffers of this call and of the caller.
+int nc_server::collect(const Resident& r, nc_request_done& d, Kept& k, std::string& err)
+{
+    const nc::NetHost& h = r.host;
+    unsigned long long s4[4] = {0, 0, 0, 0};
+    std::vector<float> pot;
+    auto copies = [&]() -> int {
+        S_CK(cudaMemcpyAsync(s4, d_stats + 4 * (int64_t)r.slot, sizeof(s4), cudaMemcpyDeviceToHost, stream));
+        if (!cfg.keep_results) return NC_OK;
+        pot.resize((size_t)h.n);
+        k.weights.resize((size_t)h.n_input);
+        S_CK(cudaMemcpyAsync(pot.data(), P.pot + r.neuron0, sizeof(float) * h.n, cudaMemcpyDeviceToHost, stream));
+        return gather_weights(r, k.weights.data(), err);
+    };
+    const int rc = copies();
+    S_CK(cudaStreamSynchronize(stream));
+    if (rc != NC_OK) return rc;
+    d.stats.fires = (int64_t)s4[0];
+    d.stats.launched = (int64_t)s4[1];
+    d.stats.dropped = (int64_t)s4[2];
+    d.stats.steps = (int64_t)s4[3];
+    if (cfg.keep_results) {
+        k.potentials.resize((size_t)h.n);
+        nc::to_caller_order(h, pot.data(), k.potentials.data());
+    }
+    return NC_OK;
+}
+
 int nc_server::retire(Resident& r, std::string& err)
 {
     const nc::NetHost& h = r.host;
@@ -625,6 +661,49 @@ int nc_server::upload_tiles(std::string& err)
     return NC_OK;
 }
 
+// One batch of steps of every resident network; ms: its device time.
+int nc_server::run_batch(float& ms, std::string& err)
+{
+    S_CK(cudaEventRecord(ev0, stream));
+    S_CK(cudaGraphLaunch(graph, stream));
+    S_CK(cudaEventRecord(ev1, stream));
+    S_CK(cudaEventSynchronize(ev1));
+    S_CK(cudaEventElapsedTime(&ms, ev0, ev1));
+    return NC_OK;
+}
+
+nc_request_done nc_server::outcome(const Resident& r, int status) const
+{
+    nc_request_done d{};
+    d.request_id = r.id;
+    d.status = status;
+    d.n_neurons = r.host.n;
+    d.horizon = r.horizon;
+    d.submit_s = r.submit_s;
+    d.done_s = now();
+    d.admit_s = r.slot >= 0 ? r.admit_s : d.done_s;
+    return d;
+}
+
+// The device is lost: the resident networks finish with `status`, and so will every request
+// still to be admitted (scheduler_loop).
+void nc_server::fail_active(int status)
+{
+    cudaStreamSynchronize(stream);
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        lost = status;
+        for (auto& r : active) {
+            finished.push_back(outcome(*r, status));
+            st.finished++;
+            outstanding--;
+            st.resident_bytes -= r->bytes;
+        }
+    }
+    active.clear();
+    cv_done.notify_all();
+}
+
 void nc_server::scheduler_loop()
 {
     cudaSetDevice(device);
@@ -645,7 +724,7 @@ void nc_server::scheduler_loop()
         int64_t left = 0, taken = 0, admitted = 0;  // host bytes no longer waiting, device bytes and networks admitted
         for (auto it = waiting.begin(); it != waiting.end();) {
             Resident& r = *it->second;
-            const int rc = r.status == NC_OK ? admit(r, err) : r.status;
+            const int rc = r.status != NC_OK ? r.status : lost != NC_OK ? lost : admit(r, err);
             if (r.status == NC_OK && rc == 1) {
                 ++it;
                 continue;
@@ -672,13 +751,8 @@ void nc_server::scheduler_loop()
             st.peak_resident_bytes = std::max(st.peak_resident_bytes, st.resident_bytes);
             st.peak_resident_networks = std::max<int64_t>(st.peak_resident_networks, (int64_t)active.size());
             for (auto& r : rejected) {
-                nc_request_done d{};
-                d.request_id = r->id;
-                d.status = r->status;
-                d.n_neurons = r->host.n;
-                d.horizon = r->horizon;
-                d.submit_s = r->submit_s;
-                d.admit_s = d.done_s = now();
+                nc_request_done d = outcome(*r, r->status);
+                d.admit_s = d.done_s;
                 finished.push_back(d);
                 st.rejected++;
                 st.finished++;
@@ -687,15 +761,15 @@ void nc_server::scheduler_loop()
         }
         if (!rejected.empty()) cv_done.notify_all();
         if (changed || !rejected.empty()) cv.notify_all();  // builders paused on the host cap
-        if (changed && upload_tiles(err) != NC_OK) return;
+        int rc = changed ? upload_tiles(err) : NC_OK;
         if (active.empty()) continue;
-        // one batch of G launch pairs over every resident network
-        cudaEventRecord(ev0, stream);
-        if (cudaGraphLaunch(graph, stream) != cudaSuccess) return;
-        cudaEventRecord(ev1, stream);
-        cudaEventSynchronize(ev1);
+        // one batch of G steps of every resident network
         float ms = 0.0f;
-        cudaEventElapsedTime(&ms, ev0, ev1);
+        if (rc == NC_OK) rc = run_batch(ms, err);
+        if (rc != NC_OK) {
+            fail_active(rc);
+            continue;
+        }
         // retire networks that reached their horizon
         std::vector<std::unique_ptr<Resident>> done;
         for (auto it = active.begin(); it != active.end();) {
@@ -710,46 +784,25 @@ void nc_server::scheduler_loop()
         if (!done.empty()) {
             NcPools F = P;  // flush launched directly with the current tile count
             F.n_tiles_dev = nullptr;
-            if (dense ? nc::launch_flush_dense(F, L, stream) : nc::launch_stdp_flush(F, L, stream)) return;
-            cudaStreamSynchronize(stream);
+            if (dense ? nc::launch_flush_dense(F, L, stream) : nc::launch_stdp_flush(F, L, stream)) rc = NC_ERR_CUDA;
+            if (cudaStreamSynchronize(stream) != cudaSuccess) rc = NC_ERR_CUDA;
         }
         std::vector<nc_request_done> out;
         for (auto& r : done) {
-            nc_request_done d{};
-            d.request_id = r->id;
-            d.status = NC_OK;
-            d.n_neurons = r->host.n;
-            d.horizon = r->horizon;
-            d.n_synapses = r->host.s;
-            d.submit_s = r->submit_s;
-            d.admit_s = r->admit_s;
-            unsigned long long s4[4];
-            cudaMemcpyAsync(s4, d_stats + 4 * (int64_t)r->slot, sizeof(s4), cudaMemcpyDeviceToHost, stream);
             Kept k;
-            if (cfg.keep_results) {
-                const nc::NetHost& h = r->host;
-                std::vector<float> pot((size_t)h.n);
-                cudaMemcpyAsync(pot.data(), P.pot + r->neuron0, sizeof(float) * h.n, cudaMemcpyDeviceToHost, stream);
-                k.weights.resize((size_t)h.n_input);
-                if (gather_weights(*r, k.weights.data(), err) != NC_OK) return;
-                cudaStreamSynchronize(stream);
-                k.potentials.resize((size_t)h.n);
-                nc::to_caller_order(h, pot.data(), k.potentials.data());
-            }
-            cudaStreamSynchronize(stream);
-            d.stats.fires = (int64_t)s4[0];
-            d.stats.launched = (int64_t)s4[1];
-            d.stats.dropped = (int64_t)s4[2];
-            d.stats.steps = (int64_t)s4[3];
-            retire(*r, err);
+            nc_request_done d = outcome(*r, NC_OK);
+            d.status = rc != NC_OK ? rc : collect(*r, d, k, err);
+            d.n_synapses = d.status == NC_OK ? r->host.s : 0;
+            const int gone = retire(*r, err);
+            if (rc == NC_OK) rc = gone;
             d.done_s = now();
             out.push_back(d);
-            if (cfg.keep_results) {
+            if (cfg.keep_results && d.status == NC_OK) {
                 std::lock_guard<std::mutex> lk(mu);
                 kept.emplace(r->id, std::move(k));
             }
         }
-        if (!done.empty() && upload_tiles(err) != NC_OK) return;
+        if (!done.empty() && rc == NC_OK) rc = upload_tiles(err);
         {
             std::lock_guard<std::mutex> lk(mu);
             st.steps_run += G;
@@ -761,6 +814,7 @@ void nc_server::scheduler_loop()
             }
             for (auto& r : done) st.resident_bytes -= r->bytes;
         }
+        if (rc != NC_OK) fail_active(rc);
         if (!out.empty()) cv_done.notify_all();
     }
 }

@@ -241,6 +241,76 @@ static void failed_read()
     }
 }
 
+// Submits `count` requests, waits for all, and returns their outcomes in the order they came.
+static std::vector<nc_request_done> served(nc_server* s, Made& m, int count)
+{
+    std::vector<int64_t> ids((size_t)count);
+    for (int q = 0; q < count; ++q) {
+        const nc_net_spec spec = m.spec(5 + 7 * q);
+        check(nc_server_submit(s, &spec, &ids[(size_t)q]) == NC_OK, "submit");
+    }
+    check(nc_server_drain(s) == NC_OK, "drain");
+    std::vector<nc_request_done> got((size_t)count + 1), out;
+    int32_t n = 0;
+    check(nc_server_poll(s, got.data(), count + 1, &n) == NC_OK && n == count, "one outcome a request");
+    for (int64_t id : ids)
+        for (int32_t k = 0; k < n; ++k)
+            if (got[(size_t)k].request_id == id) out.push_back(got[(size_t)k]);
+    return out;
+}
+
+static nc_server* server(int mode)
+{
+    nc_server_config c{};
+    c.memory_budget_bytes = 32 << 20;
+    c.max_networks = 2;
+    c.steps_per_batch = 4;
+    c.build_threads = 2;
+    c.keep_results = 1;
+    c.step_mode = mode;
+    nc_server* s = nullptr;
+    check(nc_server_create(&c, &s) == NC_OK, std::string("server: ") + nc_last_error());
+    return s;
+}
+
+// A request whose results cannot be read finishes with the error; the others go on.
+static void server_read_fails()
+{
+    for (int mode : {NC_STEP_DENSE, NC_STEP_EVENT}) {
+        Made m(60, 500, mode);
+        nc_server* s = server(mode);
+        fake::gathers_to_fail = 1;
+        int failed = 0;
+        for (const nc_request_done& d : served(s, m, 5)) {
+            std::vector<float> w(m.w.size()), pot((size_t)m.n);
+            const int rc = nc_server_fetch(s, d.request_id, w.data(), pot.data());
+            if (d.status == NC_OK) check(rc == NC_OK && m.same(w) && pot[0] == -70.0f, "results");
+            else check(d.status == NC_ERR_CUDA && rc == NC_ERR_INVALID, "error");
+            failed += d.status != NC_OK;
+        }
+        check(failed == 1, "one failure");
+        nc_server_stats st;
+        check(nc_server_get_stats(s, &st) == NC_OK && st.finished == 5 && st.resident_bytes == 0, "counts");
+        nc_server_destroy(s);
+    }
+}
+
+// When the device is lost every request, early and late, finishes with the error.
+static void server_device_lost()
+{
+    Made m(60, 500);
+    nc_server* s = server(NC_STEP_DENSE);
+    for (const nc_request_done& d : served(s, m, 3)) check(d.status == NC_OK, "before");
+    fake::graphs_to_fail = 1 << 30;
+    for (int round = 0; round < 2; ++round)
+        for (const nc_request_done& d : served(s, m, 5)) check(d.status == NC_ERR_CUDA, "after");
+    nc_server_stats st;
+    check(nc_server_get_stats(s, &st) == NC_OK && st.finished == 13 && st.resident_bytes == 0, "counts");
+    nc_server_destroy(s);
+    fake::graphs_to_fail = 0;
+    check(fake::held == 0, "memory given back");
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -252,6 +322,8 @@ int main(int argc, char** argv)
     else if (what == "reads_allocate_nothing") reads_allocate_nothing();
     else if (what == "no_index") no_index();
     else if (what == "failed_read") failed_read();
+    else if (what == "server_read_fails") server_read_fails();
+    else if (what == "server_device_lost") server_device_lost();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
