@@ -689,27 +689,6 @@ __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, u
     else bar_arrive<kBarFull>(0);  // nothing to do: the step counters have been read
 }
 
-// Every block has read the step counters: one warp moves them on (a flush: notes that the
-// launches and plasticity of every active net's last step are done).
-template <bool kFlush>
-__device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
-{
-    for (int n = lane; n < P.n_nets; n += 32) {
-        NcNetDesc* D = P.nets + n;
-        if (kFlush) {
-            if (D->active && D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
-            continue;
-        }
-        if (D->active && D->t <= D->t_end) {
-            if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
-            D->stats[3] += 1ull;
-            D->t += 1;
-            D->tsum = __fadd_rn(D->tsum, D->dt);  // currentTime = targetTime (src/NeuCor.cpp:616)
-        }
-    }
-    if (lane == 0) *P.done_ctr = 0u;
-}
-
 // Row starts of a tile into L1, before the wait: nothing writes them.
 __device__ __forceinline__ void prefetch_tile(const NcPools& P, const NcRowTile& tile, int lane)
 {
@@ -870,7 +849,7 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
         bar_sync<kBarFull>(0);
         if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
     }
-    if (__shfl_sync(kFull, arrived, 0) == gridDim.x - 1u) advance_steps<kFlush>(P, lane);
+    if (__shfl_sync(kFull, arrived, 0) == gridDim.x - 1u) advance_steps<kFlush ? kFlushed : kStep>(P, lane);
 }
 
 // One step (or the flush of the last one) of every tile of this block.

@@ -67,6 +67,8 @@ struct alignas(128) NcNetDesc {
     float tsum;           // NeuCor::currentTime after t-1 steps: the float sum of t-1 runSpeeds
     int32_t active;       // 0: skipped by the kernels
     int32_t live;         // event form: the last neuron step advanced the net (its fires launch)
+    float dt_again;       // dt, for what moves the counters on
+    int32_t pad;
     alignas(128) int32_t n; // neurons
     int32_t neuron_base;  // pool index of neuron 0
     int32_t ptr_base;     // pool index of in_ptr/out_ptr/ring_off entry 0 (n+1 entries)
@@ -95,7 +97,7 @@ struct alignas(128) NcNetDesc {
     double e_term;        // 0.9943 is applied separately; this is exp(0.3702*dt) (src/NeuCor.cpp:695)
     float term_hi, term_lo; // both factors as one: a float and the float of what it leaves
     uint32_t* raster;     // device raster rows of n_words words
-    unsigned long long* stats; // 4 counters: fires, launched, dropped, steps
+    unsigned long long* stats; // the net's four counters (NcPools::stats)
     int64_t n_syn;        // synapses (out-synapse entries)
     int64_t wide;         // dense form: 0, or the offset of the second range (NcPools::key)
     int32_t nonneg_terms; // 1: no launch can add a negative term (no inhibitory synapse, no
@@ -244,9 +246,11 @@ struct NcPools {
     NcGroupDev* groups;
     NcNetDesc* nets;
     int32_t n_nets;
+    unsigned long long* stats; // 4 counters a net: fires, launched, dropped, steps
     NcTile* tiles;
     int32_t n_tiles;
     int32_t* n_tiles_dev; // when set, the tile count is read from device memory (served engine)
+    int32_t* n_nets_dev;  // when set, the nets from *n_nets_dev on are not active (served engine)
     int32_t warp_rows;   // event form: neurons per warp of the neuron step: 8, 16 or 32
     int32_t launch_rows; // and of the spike launch: 1, 2, 4 or 8
     // engine

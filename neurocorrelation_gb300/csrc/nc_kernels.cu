@@ -189,23 +189,6 @@ __device__ __forceinline__ bool any_words(const uint32_t (&m)[4]) { return (m[0]
 
 constexpr int kBatch = 8;  // charges, or weights, of a row gathered together
 
-// Every warp has read the step counters: the last to say so moves them on.  The spike launch
-// that follows works on the step before the counter, for the nets this advanced (live).
-__device__ __forceinline__ void advance_steps(const NcPools& P, int lane)
-{
-    for (int n = lane; n < P.n_nets; n += 32) {
-        NcNetDesc* D = P.nets + n;
-        D->live = D->active && D->t <= D->t_end;
-        if (D->live) {
-            if (D->stdp_done < D->t - 1) D->stdp_done = D->t - 1;
-            D->stats[3] += 1ull;
-            D->t += 1;
-            D->tsum = __fadd_rn(D->tsum, D->dt);  // currentTime = targetTime (src/NeuCor.cpp:616)
-        }
-    }
-    if (lane == 0) *P.done_ctr = 0u;
-}
-
 // One warp per warp_rows (8, 16 or 32) neurons of one net; blocks of any size, no block
 // barrier.  The chain of dependent loads bounds it (about 800 cycles each and more for what
 // is not in L2), so:
@@ -399,11 +382,11 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
                     ((uint8_t*)(D.raster + (int64_t)(t - D.raster_t0) * D.n_words))[(first >> 3) + lane] = v;
             }
         }
-        if (last_unit && __shfl_sync(kFull, arrived, 0) == (unsigned)min(units, warps) - 1u) advance_steps(P, lane);
+        if (last_unit && __shfl_sync(kFull, arrived, 0) == (unsigned)min(units, warps) - 1u) advance_steps<kEvent>(P, lane);
     }
     if (units == 0 && blockIdx.x == 0 && threadIdx.x < 32) {  // nets without neurons still step
         if (!waited) wait_previous();
-        advance_steps(P, lane);
+        advance_steps<kEvent>(P, lane);
     }
 }
 

@@ -205,7 +205,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         d.active = 1;
         d.permuted = h.permuted ? 1 : 0;
         d.nonneg_terms = h.nonneg_terms ? 1 : 0;
-        d.dt = h.dt;
+        d.dt = d.dt_again = h.dt;
         d.leak = h.leak;
         d.c52 = h.c52;
         d.lr = h.p.learning_rate;
@@ -274,7 +274,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     NC_ALLOC(P.done_ctr, uint32_t, 1);
     NC_ALLOC(P.dev_err, uint32_t, 1);
     NC_ALLOC(d_bar_, unsigned, 2);
-    NC_ALLOC(d_stats_, unsigned long long, 4 * nets.size());
+    NC_ALLOC(P.stats, unsigned long long, 4 * nets.size());
     for (const NetHost* h : nets)
         scratch_bytes_ = std::max(scratch_bytes_, std::max(sizeof(float) * (size_t)h->n_input, 8 * (size_t)h->n));
     scratch_bytes_ = std::max<size_t>(256, std::min(scratch_bytes_, kScratchMax));
@@ -290,7 +290,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         const NetHost& h = *nets[q];
         const NetSlot& sl = slots[q];
         NcNetDesc& d = desc[q];
-        d.stats = d_stats_ + 4 * q;
+        d.stats = P.stats + 4 * q;
         std::vector<float> pot((size_t)h.n, -70.0f);  // setPotential(baselevel)
         std::vector<int32_t> lf((size_t)h.n, NC_NEVER);
         NC_CK(upload(P.pot, pot, sl.neuron_base, stream));
@@ -787,7 +787,7 @@ int Engine::set_raster(int net, uint32_t* d_raster, int32_t t0, int32_t len, std
 
 int Engine::read_stats(int net, unsigned long long out[4], std::string& err)
 {
-    NC_CK(cudaMemcpyAsync(out, d_stats_ + 4 * net, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
+    NC_CK(cudaMemcpyAsync(out, P.stats + 4 * net, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
     NC_CK(cudaStreamSynchronize(stream));
     return NC_OK;
 }

@@ -113,7 +113,6 @@ private:
     void* near_buf_ = nullptr;
     int32_t* d_ids_ = nullptr;
     int ids_cap_ = 0;
-    unsigned long long* d_stats_ = nullptr;
     bool back_ = false;          // direction of the last dense step's sweep
     unsigned* d_bar_ = nullptr;  // grid barrier of the fused launch (arrivals, generation)
     int64_t ring_words_total_ = 0;

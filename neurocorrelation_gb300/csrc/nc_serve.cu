@@ -143,8 +143,8 @@ struct nc_server {
     double syn_bytes = kSynBytesDense, neuron_bytes = kNeuronBytesDense;
     RangeAlloc a_neuron, a_ptr, a_word, a_syn, a_ring, a_table;
     std::vector<int32_t> free_slots;
-    unsigned long long* d_stats = nullptr;
     int32_t* d_ntiles = nullptr;
+    int32_t* d_nnets = nullptr;
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -287,12 +287,14 @@ int nc_server::init(std::string& err)
     if (!dense) S_AL(P.tiles, NcTile, tile_cap);
     S_AL(P.done_ctr, uint32_t, 1);
     S_AL(P.dev_err, uint32_t, 1);
-    S_AL(d_stats, unsigned long long, 4 * (int64_t)nets);
+    S_AL(P.stats, unsigned long long, 4 * (int64_t)nets);
     S_AL(d_ntiles, int32_t, 1);
+    S_AL(d_nnets, int32_t, 1);
 #undef S_AL
     P.n_nets = nets;
     P.n_tiles = 0;
     P.n_tiles_dev = d_ntiles;
+    P.n_nets_dev = d_nnets;
     P.warp_rows = 32;
     P.launch_rows = 8;
     a_neuron.reset(neuron_cap);
@@ -512,7 +514,7 @@ int nc_server::admit(Resident& r, std::string& err)
     }
     S_CK(put(P.tables, h.tables, tb, stream));
     if (!h.groups.empty()) S_CK(put(P.groups, h.groups, (int64_t)r.slot * kGroupsPerNet, stream));
-    S_CK(cudaMemsetAsync(d_stats + 4 * (int64_t)r.slot, 0, 4 * sizeof(unsigned long long), stream));
+    S_CK(cudaMemsetAsync(P.stats + 4 * (int64_t)r.slot, 0, 4 * sizeof(unsigned long long), stream));
     NcNetDesc d;
     std::memset(&d, 0, sizeof(d));
     d.t = 1;
@@ -541,7 +543,7 @@ int nc_server::admit(Resident& r, std::string& err)
     d.active = 1;
     d.permuted = h.permuted ? 1 : 0;
     d.nonneg_terms = h.nonneg_terms ? 1 : 0;
-    d.dt = h.dt;
+    d.dt = d.dt_again = h.dt;
     d.leak = h.leak;
     d.c52 = h.c52;
     d.lr = h.p.learning_rate;
@@ -552,7 +554,7 @@ int nc_server::admit(Resident& r, std::string& err)
     d.n_syn = h.s;
     d.key_shift = h.key_shift;
     d.wide = wide;
-    d.stats = d_stats + 4 * (int64_t)r.slot;
+    d.stats = P.stats + 4 * (int64_t)r.slot;
     S_CK(cudaMemcpyAsync(P.nets + r.slot, &d, sizeof(d), cudaMemcpyHostToDevice, stream));
     if (nc::launch_background_prologue(P, r.slot, h.n, stream)) {
         err = nc::cuda_msg("background prologue", cudaGetLastError());
@@ -590,7 +592,7 @@ int nc_server::collect(const Resident& r, nc_request_done& d, Kept& k, std::stri
     unsigned long long s4[4] = {0, 0, 0, 0};
     std::vector<float> pot;
     auto copies = [&]() -> int {
-        S_CK(cudaMemcpyAsync(s4, d_stats + 4 * (int64_t)r.slot, sizeof(s4), cudaMemcpyDeviceToHost, stream));
+        S_CK(cudaMemcpyAsync(s4, P.stats + 4 * (int64_t)r.slot, sizeof(s4), cudaMemcpyDeviceToHost, stream));
         if (!cfg.keep_results) return NC_OK;
         pot.resize((size_t)h.n);
         k.weights.resize((size_t)h.n_input);
@@ -630,6 +632,10 @@ int nc_server::retire(Resident& r, std::string& err)
 
 int nc_server::upload_tiles(std::string& err)
 {
+    // a step's end looks at the slots up to the last one taken (8,192 slots, one network: event
+    // form 46 us a step with all of them, 23 with one)
+    int32_t n_nets = 0;
+    for (const auto& r : active) n_nets = std::max(n_nets, r->slot + 1);
     if (dense) {
         std::vector<nc::RowNet> nets;
         std::vector<NcRowTile> rows;
@@ -641,6 +647,7 @@ int nc_server::upload_tiles(std::string& err)
             err = "tile table overflow";
             return NC_ERR_INVALID;
         }
+        S_CK(cudaMemcpyAsync(d_nnets, &n_nets, sizeof(n_nets), cudaMemcpyHostToDevice, stream));
         S_CK(put(P.rtiles, rows, 0, stream));
         S_CK(put(P.rstart, start, 0, stream));
         S_CK(cudaStreamSynchronize(stream));
@@ -654,6 +661,7 @@ int nc_server::upload_tiles(std::string& err)
         return NC_ERR_INVALID;
     }
     const int32_t n = (int32_t)tiles.size();
+    S_CK(cudaMemcpyAsync(d_nnets, &n_nets, sizeof(n_nets), cudaMemcpyHostToDevice, stream));
     S_CK(put(P.tiles, tiles, 0, stream));
     S_CK(cudaMemcpyAsync(d_ntiles, &n, sizeof(n), cudaMemcpyHostToDevice, stream));
     S_CK(cudaStreamSynchronize(stream));
