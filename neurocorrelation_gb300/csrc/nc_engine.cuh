@@ -320,7 +320,9 @@ struct LaunchShape {
                           // per step, replayed through CUDA graphs)
 };
 int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream);
-int launch_spike_launch(const NcPools& P, const LaunchShape& L, void* stream);
+// many: the warps have several units each (many_units of the live tiles).
+int launch_spike_launch(const NcPools& P, const LaunchShape& L, bool many, void* stream);
+bool many_units(int n_tiles, const NcPools& P, const LaunchShape& L);
 int launch_stdp_flush(const NcPools& P, const LaunchShape& L, void* stream);
 // Dense form (nc_dense.cu): one step in one launch, and the plasticity flush (the launches
 // and plasticity of the last step's fires) before read-back.

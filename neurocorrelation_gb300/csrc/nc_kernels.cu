@@ -390,11 +390,102 @@ __global__ void __launch_bounds__(256, NC_NEURON_MIN_BLOCKS) k_neuron_step(NcPoo
     }
 }
 
+// A warp's counts of the net it works on (nl, nd per lane), added when it passes to another.
+struct LaunchCounts {
+    int net = -1;
+    unsigned fires = 0, nl = 0, nd = 0;
+    __device__ __forceinline__ void turn_to(const NcPools& P, int n, int lane)
+    {
+        if (n == net) return;
+        if (net >= 0) {
+            nl = __reduce_add_sync(kFull, nl);
+            nd = __reduce_add_sync(kFull, nd);
+            if (lane == 0) {
+                unsigned long long* st = P.nets[net].stats;
+                atomicAdd(st + 0, (unsigned long long)fires);
+                atomicAdd(st + 1, (unsigned long long)nl);
+                atomicAdd(st + 2, (unsigned long long)nd);
+            }
+        }
+        net = n;
+        fires = nl = nd = 0;
+    }
+};
+
+// The out-synapses of the neurons whose bits are set in `fired` (all lanes call).  start: row
+// start of the unit's neuron `lane`.
+__device__ __forceinline__ void launch_unit(const NcPools& P, const NcNetDesc& D, uint32_t fired, int32_t t,
+                                            int64_t start, int lane, LaunchCounts& C)
+{
+    C.fires += __popc(fired);
+    const uint32_t* fired_t = P.fired + (int64_t)(t & 1) * P.total_words + D.word_base;
+    const float* tab_pre = P.tables + D.table_base;
+    uint32_t* ring = P.ring + D.ring_base;
+    // the descriptor's fields in registers: it lives in global memory, where every
+    // store below could alias it
+    const int32_t kc = D.kc, tpl = D.tab_pre_len, ring_mask = D.ring_mask;
+    const int64_t syn_base = D.syn_base, ring_words = D.ring_words;
+    const float dt = D.dt, c52 = D.c52;
+    const Rates R = rates_of(D);
+    for (; fired; fired &= fired - 1u) {
+        const int i = __ffs((int)fired) - 1;
+        const int64_t k0 = __shfl_sync(kFull, start, i), k1 = __shfl_sync(kFull, start, i + 1);
+        for (int64_t kb = k0; kb < k1; kb += 128) {
+            uint4 o[4];
+            int32_t la[4];
+            bool ok[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int64_t k = kb + lane + 32 * v;
+                ok[v] = k < k1;
+                if (ok[v]) {
+                    o[v] = __ldg((const uint4*)P.out + k);
+                    la[v] = P.last_arr[k];
+                }
+            }
+            float wv[4];
+            uint32_t fw[4];
+            bool acc[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                // freed by the target's update at t only if the target's id is not above
+                acc[v] = ok[v] && (la[v] == NC_NEVER || t - la[v] >= kc + (int32_t)((o[v].w >> 14) & 1u));
+                fw[v] = 0u;
+                if (acc[v]) {
+                    wv[v] = P.w[syn_base + o[v].x];
+                    // target id below the source's: its update ran first
+                    if ((o[v].w >> 15) & 1u) fw[v] = fired_t[o[v].y >> 5] >> (o[v].y & 31);
+                }
+                C.nl += acc[v] ? 1u : 0u;
+                C.nd += ok[v] && !acc[v] ? 1u : 0u;
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                if (!acc[v]) continue;
+                const int64_t k = kb + lane + 32 * v;
+                const int64_t s = syn_base + o[v].x;
+                float w = wv[v];
+                if (fw[v] & 1u)
+                    w = plasticity(w, inh_bit(P, s), trace_at(tab_pre, tpl, t, P.t_arr[s]), 0.0f, R);
+                // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
+                P.x[s] = dt * (c52 * w);
+                const int32_t d = (int32_t)(o[v].w & 0x3fffu);
+                P.last_arr[k] = t + d;
+                atomicOr(ring + (int64_t)((t + d) & ring_mask) * ring_words + (o[v].z >> 5), 1u << (o[v].z & 31));
+            }
+        }
+    }
+}
+
 // Synapse::fire (src/NeuCor.cpp:727-738) on the out-synapses of the neurons that fired at t,
-// a warp per launch_rows (1 to 8) neurons' fired bits, all lanes on a fired neuron's
+// a warp per launch_rows (1 to 8) neurons' fired bits (a unit), all lanes on a fired neuron's
 // out-synapses, four in flight each.  Its chain of loads bounds it: the fired byte (of both
 // parities, beside the step counter), the 16-byte out-synapse records, the weights and the
 // fired words of targets that came first.
+//   kMany: a warp has several units (many_units), and a lane looks at the fired byte of one of
+//   its next 32: one after the other, a quiet network of 2M neurons took 83 us for them, 26 so.
+//   With one unit a warp the row starts are read before the wait: 0.9 us less (50k x 80 quiet).
+template <bool kMany>
 __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPools P)
 {
     __shared__ int s_net[8];
@@ -411,110 +502,63 @@ __global__ void __launch_bounds__(256, NC_LAUNCH_MIN_BLOCKS) k_spike_launch(NcPo
     }
     const int rows = P.launch_rows, parts = 32 / rows;
     const int units = parts * n_tiles;
-    int acc_net = -1;
-    unsigned fires = 0, nl = 0, nd = 0;  // of acc_net; nl, nd per lane
-    for (int u = blockIdx.x * nwb + wib; u < units; u += gridDim.x * nwb) {
-        const NcTile tile = P.tiles[u / parts];
-        const NcNetDesc& D = P.nets[tile.net];
-        const int32_t first = tile.first + (u % parts) * rows;
-        if (first >= D.n) continue;
-        int64_t start = 0;  // row start of neuron first + lane
-        if (lane <= min(rows, D.n - first)) start = __ldg(P.out_ptr + D.ptr_base + first + lane);
-        const int64_t byte = 4 * (D.word_base + (int64_t)(first >> 5)) + ((first & 31) >> 3);
+    LaunchCounts C;
+    const int warps = gridDim.x * nwb;
+    for (int base = blockIdx.x * nwb + wib; base < units; base += (kMany ? 32 : 1) * warps) {
+        const int mine = base + (kMany ? lane * warps : 0);
+        int32_t net = -1, first = 0;
+        int64_t byte = 0, start = 0;
+        if (mine < units) {
+            const NcTile tile = P.tiles[mine / parts];
+            const NcNetDesc& D = P.nets[tile.net];
+            first = tile.first + (mine % parts) * rows;
+            if (first < D.n) {
+                net = tile.net;
+                byte = 4 * (D.word_base + (int64_t)(first >> 5)) + ((first & 31) >> 3);
+                if (!kMany && lane <= min(rows, D.n - first)) start = __ldg(P.out_ptr + D.ptr_base + first + lane);
+            }
+        }
+        if (!kMany && net < 0) continue;
         if (!waited) {
             wait_previous();
             release_next();
             waited = true;
         }
-        // both parities' bytes beside the counter that picks one
-        const uint32_t f0 = __ldcg((const uint8_t*)P.fired + byte);
-        const uint32_t f1 = __ldcg((const uint8_t*)(P.fired + P.total_words) + byte);
-        const int32_t t = __ldcg(&D.t) - 1;
-        uint32_t fired = ((t & 1 ? f1 : f0) >> (first & 7)) & ((1u << rows) - 1u);
-        if (!fired || !__ldcg(&D.live)) continue;
-        if (tile.net != acc_net) {
-            if (acc_net >= 0) {
-                nl = __reduce_add_sync(kFull, nl);
-                nd = __reduce_add_sync(kFull, nd);
-                if (lane == 0) {
-                    unsigned long long* st = P.nets[acc_net].stats;
-                    atomicAdd(st + 0, (unsigned long long)fires);
-                    atomicAdd(st + 1, (unsigned long long)nl);
-                    atomicAdd(st + 2, (unsigned long long)nd);
-                }
-            }
-            acc_net = tile.net;
-            fires = nl = nd = 0;
+        uint32_t fired = 0u;
+        int32_t t = 0;
+        if (net >= 0) {
+            // both parities' bytes beside the counter that picks one
+            const uint32_t f0 = __ldcg((const uint8_t*)P.fired + byte);
+            const uint32_t f1 = __ldcg((const uint8_t*)(P.fired + P.total_words) + byte);
+            t = __ldcg(&P.nets[net].t) - 1;
+            fired = ((t & 1 ? f1 : f0) >> (first & 7)) & ((1u << rows) - 1u);
+            if (fired && !__ldcg(&P.nets[net].live)) fired = 0u;
         }
-        fires += __popc(fired);
-        const uint32_t* fired_t = P.fired + (int64_t)(t & 1) * P.total_words + D.word_base;
-        const float* tab_pre = P.tables + D.table_base;
-        uint32_t* ring = P.ring + D.ring_base;
-        // the descriptor's fields in registers: it lives in global memory, where every
-        // store below could alias it
-        const int32_t kc = D.kc, tpl = D.tab_pre_len, ring_mask = D.ring_mask;
-        const int64_t syn_base = D.syn_base, ring_words = D.ring_words;
-        const float dt = D.dt, c52 = D.c52;
-        const Rates R = rates_of(D);
-        for (; fired; fired &= fired - 1u) {
-            const int i = __ffs((int)fired) - 1;
-            const int64_t k0 = __shfl_sync(kFull, start, i), k1 = __shfl_sync(kFull, start, i + 1);
-            for (int64_t kb = k0; kb < k1; kb += 128) {
-                uint4 o[4];
-                int32_t la[4];
-                bool ok[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int64_t k = kb + lane + 32 * v;
-                    ok[v] = k < k1;
-                    if (ok[v]) {
-                        o[v] = __ldg((const uint4*)P.out + k);
-                        la[v] = P.last_arr[k];
-                    }
-                }
-                float wv[4];
-                uint32_t fw[4];
-                bool acc[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    // freed by the target's update at t only if the target's id is not above
-                    acc[v] = ok[v] && (la[v] == NC_NEVER || t - la[v] >= kc + (int32_t)((o[v].w >> 14) & 1u));
-                    fw[v] = 0u;
-                    if (acc[v]) {
-                        wv[v] = P.w[syn_base + o[v].x];
-                        // target id below the source's: its update ran first
-                        if ((o[v].w >> 15) & 1u) fw[v] = fired_t[o[v].y >> 5] >> (o[v].y & 31);
-                    }
-                    nl += acc[v] ? 1u : 0u;
-                    nd += ok[v] && !acc[v] ? 1u : 0u;
-                }
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    if (!acc[v]) continue;
-                    const int64_t k = kb + lane + 32 * v;
-                    const int64_t s = syn_base + o[v].x;
-                    float w = wv[v];
-                    if (fw[v] & 1u)
-                        w = plasticity(w, inh_bit(P, s), trace_at(tab_pre, tpl, t, P.t_arr[s]), 0.0f, R);
-                    // AP_depolFac = 0.2f; *= 52.0; *= weight  (src/NeuCor.cpp:729-731)
-                    P.x[s] = dt * (c52 * w);
-                    const int32_t d = (int32_t)(o[v].w & 0x3fffu);
-                    P.last_arr[k] = t + d;
-                    atomicOr(ring + (int64_t)((t + d) & ring_mask) * ring_words + (o[v].z >> 5), 1u << (o[v].z & 31));
-                }
-            }
+        if (!kMany) {
+            if (!fired) continue;
+            C.turn_to(P, net, lane);
+            launch_unit(P, P.nets[net], fired, t, start, lane, C);
+            continue;
+        }
+        for (unsigned todo = __ballot_sync(kFull, fired != 0u); todo; todo &= todo - 1u) {
+            const int who = __ffs((int)todo) - 1;
+            const int32_t n = __shfl_sync(kFull, net, who), f = __shfl_sync(kFull, first, who);
+            const NcNetDesc& D = P.nets[n];
+            if (lane <= min(rows, D.n - f)) start = __ldg(P.out_ptr + D.ptr_base + f + lane);
+            C.turn_to(P, n, lane);
+            launch_unit(P, D, __shfl_sync(kFull, fired, who), __shfl_sync(kFull, t, who), start, lane, C);
         }
     }
     if (!waited) wait_previous();
     // per-block reduction of the counters, per net
-    if (!__syncthreads_or(acc_net >= 0)) return;
-    nl = __reduce_add_sync(kFull, nl);
-    nd = __reduce_add_sync(kFull, nd);
+    if (!__syncthreads_or(C.net >= 0)) return;
+    C.nl = __reduce_add_sync(kFull, C.nl);
+    C.nd = __reduce_add_sync(kFull, C.nd);
     if (lane == 0) {
-        s_net[wib] = acc_net;
-        s_acc[wib][0] = fires;
-        s_acc[wib][1] = nl;
-        s_acc[wib][2] = nd;
+        s_net[wib] = C.net;
+        s_acc[wib][0] = C.fires;
+        s_acc[wib][1] = C.nl;
+        s_acc[wib][2] = C.nd;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -634,9 +678,17 @@ int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream)
     return launch_dependent(k_neuron_step, (int)std::max<int64_t>(1, blocks), L.neuron_block, stream, P);
 }
 
-int launch_spike_launch(const NcPools& P, const LaunchShape& L, void* stream)
+bool many_units(int n_tiles, const NcPools& P, const LaunchShape& L)
 {
-    return launch_dependent(k_spike_launch, L.launch_blocks, L.launch_block, stream, P);
+    // two units a warp: 100k neurons (1.3 a warp) 25.2 us a step one after the other and 26.1
+    // with lanes, 200k (2.6) 31.3 and 29.6, 500k (6.4) 57 and 46
+    return (int64_t)n_tiles * (32 / P.launch_rows) > 2 * (int64_t)L.launch_blocks * (L.launch_block / 32);
+}
+
+int launch_spike_launch(const NcPools& P, const LaunchShape& L, bool many, void* stream)
+{
+    return launch_dependent(many ? k_spike_launch<true> : k_spike_launch<false>, L.launch_blocks,
+                            L.launch_block, stream, P);
 }
 
 int launch_stdp_flush(const NcPools& P, const LaunchShape& L, void* stream)

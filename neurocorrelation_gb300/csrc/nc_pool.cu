@@ -443,7 +443,7 @@ int Engine::step(int64_t ticks, std::string& err)
 int Engine::launch_tick(cudaStream_t s)
 {
     int rc = P.n_firers > 0 ? launch_input_firers(P, dense, s) : 0;  // the step's run-call schedule first
-    rc |= dense ? launch_step_dense(P, L, back_ = !back_, s) : (launch_neuron_step(P, L, s) | launch_spike_launch(P, L, s));
+    rc |= dense ? launch_step_dense(P, L, back_ = !back_, s) : (launch_neuron_step(P, L, s) | launch_spike_launch(P, L, many_units(P.n_tiles, P, L), s));
     return rc;
 }
 
@@ -529,7 +529,7 @@ int Engine::time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::str
         }
         NC_CK(cudaEventRecord(at[1], stream));
         if (dense) continue;
-        if (launch_spike_launch(P, L, stream)) {
+        if (launch_spike_launch(P, L, many_units(P.n_tiles, P, L), stream)) {
             err = "launch";
             return NC_ERR_CUDA;
         }

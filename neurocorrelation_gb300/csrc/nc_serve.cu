@@ -145,7 +145,7 @@ struct nc_server {
     std::vector<int32_t> free_slots;
     int32_t* d_ntiles = nullptr;
     int32_t* d_nnets = nullptr;
-    cudaGraphExec_t graph = nullptr;
+    cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // the event form's [1]: many units a warp of the spike launch
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
     std::mutex mu;
@@ -189,7 +189,7 @@ struct nc_server {
     nc_request_done outcome(const Resident& r, int status) const;
     void fail_active(int status);
     int upload_tiles(std::string& err);
-    int capture(std::string& err);
+    int capture(bool many, cudaGraphExec_t* graph, std::string& err);
 };
 
 #define S_CK(call)                                                   \
@@ -308,10 +308,11 @@ int nc_server::init(std::string& err)
     L.launch_block = 128;
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
     S_CK(cudaStreamSynchronize(stream));
-    return capture(err);
+    rc = capture(false, &graphs[0], err);
+    return rc == NC_OK && !dense ? capture(true, &graphs[1], err) : rc;
 }
 
-int nc_server::capture(std::string& err)
+int nc_server::capture(bool many, cudaGraphExec_t* graph, std::string& err)
 {
     // the event form's kernels stride over the tile table, whose live length they read from
     // the device, and the dense step's blocks find their tiles there: the grids need not
@@ -323,7 +324,7 @@ int nc_server::capture(std::string& err)
     int rc = 0;
     for (int k = 0; k < cfg.steps_per_batch && rc == 0; ++k) {
         if (dense) rc |= nc::launch_step_dense(G, L, k & 1, stream);
-        else rc |= nc::launch_neuron_step(G, L, stream) | nc::launch_spike_launch(G, L, stream);
+        else rc |= nc::launch_neuron_step(G, L, stream) | nc::launch_spike_launch(G, L, many, stream);
     }
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     if (rc != 0 || e != cudaSuccess) {
@@ -331,10 +332,10 @@ int nc_server::capture(std::string& err)
         err = nc::cuda_msg("server graph capture", e != cudaSuccess ? e : cudaGetLastError());
         return NC_ERR_CUDA;
     }
-    e = cudaGraphInstantiate(&graph, g, 0);
+    e = cudaGraphInstantiate(graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-        graph = nullptr;
+        *graph = nullptr;
         err = nc::cuda_msg("cudaGraphInstantiate", e);
         return NC_ERR_CUDA;
     }
@@ -351,7 +352,8 @@ nc_server::~nc_server()
     for (auto& t : builders)
         if (t.joinable()) t.join();
     if (scheduler.joinable()) scheduler.join();
-    if (graph) cudaGraphExecDestroy(graph);
+    for (cudaGraphExec_t g : graphs)
+        if (g) cudaGraphExecDestroy(g);
     if (stream) cudaStreamSynchronize(stream);
     for (void* p : allocs) cudaFree(p);
     if (ev0) cudaEventDestroy(ev0);
@@ -673,7 +675,7 @@ int nc_server::upload_tiles(std::string& err)
 int nc_server::run_batch(float& ms, std::string& err)
 {
     S_CK(cudaEventRecord(ev0, stream));
-    S_CK(cudaGraphLaunch(graph, stream));
+    S_CK(cudaGraphLaunch(graphs[!dense && nc::many_units(P.n_tiles, P, L)], stream));
     S_CK(cudaEventRecord(ev1, stream));
     S_CK(cudaEventSynchronize(ev1));
     S_CK(cudaEventElapsedTime(&ms, ev0, ev1));

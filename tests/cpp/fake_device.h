@@ -222,7 +222,8 @@ int launch_neuron_step(const NcPools& P, const LaunchShape&, void*)
 {
     return fake::launch([P] { fake::step(P); });
 }
-int launch_spike_launch(const NcPools&, const LaunchShape&, void*) { return fake::launch([] {}); }
+bool many_units(int, const NcPools&, const LaunchShape&) { return false; }
+int launch_spike_launch(const NcPools&, const LaunchShape&, bool, void*) { return fake::launch([] {}); }
 int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape&, unsigned*, void*)
 {
     return fake::launch([P, ticks] {
