@@ -320,6 +320,8 @@ struct LaunchShape {
                           // per step, replayed through CUDA graphs)
 };
 int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream);
+// Blocks of the neuron step that fit on the current device at once; asked before a capture.
+int event_resident_blocks(int threads);
 // many: the warps have several units each (many_units of the live tiles).
 int launch_spike_launch(const NcPools& P, const LaunchShape& L, bool many, void* stream);
 bool many_units(int n_tiles, const NcPools& P, const LaunchShape& L);

@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 namespace {
 
@@ -671,10 +672,34 @@ static int launch_dependent(void (*fn)(NcPools), int grid, int block, void* stre
     return check_launch();
 }
 
+// Blocks of `threads` threads of the neuron step that the current device holds at once (cached
+// per device and block size; 0 when it does not say).
+int event_resident_blocks(int threads)
+{
+    static std::atomic<int> cache[64][9];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::atomic<int>& c = cache[dev][threads / 32];
+    int n = c.load(std::memory_order_relaxed);
+    if (n == 0) {
+        int sms = 0, per_sm = 0;
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neuron_step, threads, 0) != cudaSuccess)
+            return 0;
+        n = sms * per_sm;
+        c.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream)
 {
     const int64_t warps = (int64_t)P.n_tiles * (32 / P.warp_rows);
-    const int64_t blocks = (warps + L.neuron_block / 32 - 1) / (L.neuron_block / 32);
+    int64_t blocks = (warps + L.neuron_block / 32 - 1) / (L.neuron_block / 32);
+    // at most a wave: a warp goes on to its next tile sooner than a block takes the place of
+    // another (2M neurons, 13 waves: 151 us a step, 134 so; 500k busy 312 either way)
+    const int resident = event_resident_blocks(L.neuron_block);
+    if (resident > 0) blocks = std::min<int64_t>(blocks, resident);
     return launch_dependent(k_neuron_step, (int)std::max<int64_t>(1, blocks), L.neuron_block, stream, P);
 }
 

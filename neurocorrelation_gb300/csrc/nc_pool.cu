@@ -135,6 +135,7 @@ void Engine::set_launch(const LaunchShape& shape, int ticks_per_graph)
 {
     release_graph();
     L = shape;
+    if (!dense || both) event_resident_blocks(L.neuron_block);
     graph_ticks = ticks_per_graph;
 }
 
@@ -254,6 +255,7 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     }
     L.neuron_block = dense ? NC_DENSE_BLOCK : NC_EVENT_BLOCK;
     if (event_tables) {
+        event_resident_blocks(L.neuron_block);
         NC_ALLOC(P.inh, uint32_t, (syn + 31) / 32 + 1);  // one spare word for 32-bit windows
         NC_ALLOC(P.t_arr, int32_t, syn);
         NC_ALLOC(P.out_ptr, int64_t, ptrs);

@@ -304,7 +304,7 @@ int nc_server::init(std::string& err)
     a_ring.reset(ring_cap);
     a_table.reset(table_cap);
     for (int32_t q = nets - 1; q >= 0; --q) free_slots.push_back(q);
-    if (!dense) L.neuron_block = NC_EVENT_BLOCK;
+    if (!dense) nc::event_resident_blocks(L.neuron_block = NC_EVENT_BLOCK);
     L.launch_block = 128;
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
     S_CK(cudaStreamSynchronize(stream));

@@ -222,6 +222,7 @@ int launch_neuron_step(const NcPools& P, const LaunchShape&, void*)
 {
     return fake::launch([P] { fake::step(P); });
 }
+int event_resident_blocks(int) { return 152 * 8; }
 bool many_units(int, const NcPools&, const LaunchShape&) { return false; }
 int launch_spike_launch(const NcPools&, const LaunchShape&, bool, void*) { return fake::launch([] {}); }
 int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape&, unsigned*, void*)
