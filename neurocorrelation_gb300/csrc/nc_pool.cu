@@ -43,14 +43,15 @@ Engine::~Engine()
 template <class T>
 T* Engine::alloc(size_t count, std::string& err)
 {
-    // Small arrays lie 64 KiB apart in shared blocks: an allocation takes some 40 us and its
-    // release as much, and the allocator packs small ones 512 bytes apart, where a step's
-    // loads meet in few slices of L2 (three neurons 6.1 to 6.4 us a step, 1k x 50 6.8 to 7.1;
-    // 256 bytes to 20 KiB apart 5.8 to 6.6 and 6.5 to 7.0; 36 or 64 KiB apart 5.8 to 6.0 and
-    // 6.4 to 6.5).
-    constexpr size_t kBlock = 2 << 20, kApart = 64 << 10;
+    // Small arrays share blocks: an allocation takes some 40 us and its release as much.  They lie
+    // 2 KiB apart: 512 bytes apart, as the allocator packs them, a step's loads meet in few slices
+    // of L2 (a step of three neurons 5.1 us, the sphere of 750 6.9, 1k x 50 6.7; 2 KiB apart 5.0,
+    // 6.7 and 6.6; 4 to 64 KiB 4.9 to 5.5, 6.7 to 6.9, 6.5 to 6.7).  A block is eight times the array
+    // that begins it, and 64 KiB at least: a network of three neurons takes one or two (two of
+    // 2 MiB with the arrays 64 KiB apart).
+    constexpr size_t kSmallest = 64 << 10, kLargest = 2 << 20, kApart = 2 << 10;
     const size_t bytes = (std::max<size_t>(1, count) * sizeof(T) + kApart - 1) / kApart * kApart;
-    const bool shared = bytes <= kBlock / 8;
+    const bool shared = bytes <= kLargest / 8;
     if (shared && bytes <= block_left_) {
         void* p = block_;
         block_ += bytes;
@@ -58,7 +59,7 @@ T* Engine::alloc(size_t count, std::string& err)
         return (T*)p;
     }
     void* p = nullptr;
-    const size_t size = shared ? kBlock : std::max<size_t>(1, count) * sizeof(T);
+    const size_t size = shared ? std::max(kSmallest, 8 * bytes) : std::max<size_t>(1, count) * sizeof(T);
     cudaError_t e = cudaMalloc(&p, size);
     if (e != cudaSuccess) {
         err = cuda_msg("cudaMalloc", e);

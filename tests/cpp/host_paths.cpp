@@ -311,6 +311,21 @@ static void server_device_lost()
     check(fake::held == 0, "memory given back");
 }
 
+// A small network takes little device memory.
+static void footprint()
+{
+    for (int mode : {NC_STEP_DENSE, NC_STEP_EVENT, NC_STEP_AUTO}) {
+        Made few(3, 2, mode), more(1000, 50000, mode);
+        nc_net* a = few.create();
+        check(fake::held <= 160 << 10, "three neurons: " + std::to_string(fake::held));
+        nc_destroy(a);
+        a = more.create();
+        // some 20 bytes a position dense, 40 event, and what is left of the last blocks
+        check(fake::held <= (size_t)(mode == NC_STEP_DENSE ? 4 : 7) << 20, "50,000 synapses: " + std::to_string(fake::held));
+        nc_destroy(a);
+    }
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -324,6 +339,7 @@ int main(int argc, char** argv)
     else if (what == "failed_read") failed_read();
     else if (what == "server_read_fails") server_read_fails();
     else if (what == "server_device_lost") server_device_lost();
+    else if (what == "footprint") footprint();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;
