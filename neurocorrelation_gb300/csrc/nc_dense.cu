@@ -45,6 +45,10 @@
 // 0.5: 33 -> 14.8.
 //   - Rows padded to quads: a thread's four synapses share their target's values, and move
 //     with one 16-byte access per array; every eighth row ends on a 128-byte line.
+//   - A run of 8 neurons with more quads than two blocks' shares is split over several blocks;
+//     the last of them to be done with its part updates the neurons (100k x 10 with one row of
+//     99,999 in-synapses 176 -> 19 us, with inhibitory synapses 373 -> 49; 200k x 25 with skewed
+//     rows 152 -> 45).
 //   - A warp of its own sums, so the others never wait for a sum: with block barriers
 //     between the two halves the 100k x 100 step took 78 us (48 then).
 //   - 96 threads (two stream warps to a neuron warp), 80 registers, 8 blocks an SM, the
@@ -74,6 +78,11 @@ constexpr int kNibCap = 2048;
 constexpr int kRing = 3;
 // Quads of a tile whose captured charges fit in a block's shared memory beside the ring.
 constexpr int kStageQuads = 640;
+
+// What a step's tiles are: whole; whole, one to a block, with their captured charges staged in
+// shared memory (NcPools::stage); some of them split over blocks (NcPools::split).  Kernels of
+// their own: the step's 80 registers hold one kind.
+enum Kind { kWhole, kStaged, kSplit };
 
 struct RowState {
     float chg;      // weight change of an arrival at prev, before the clamp
@@ -257,6 +266,69 @@ __device__ __forceinline__ float fold_row(const uint8_t* nib, int q0, int nq, co
         if (stop && fires_at(pot, leak)) break;
     }
     return pot;
+}
+
+// fold_row by a whole warp (all lanes call, with the same values, and get the sum), for rows
+// long enough to be split over blocks: the window bits of 1,024 synapses at a time are listed in
+// shared memory (`list`, 1,024 entries) and the charges gathered 32 at once, so that empty
+// stretches cost a load per 1,024 synapses and a term its place in the sum alone.  One lane took
+// 188 us for a row of 100k in-synapses of which 600 were in the window.
+__device__ __noinline__ float fold_long_row(const uint8_t* nib, int64_t q0, int nq, const float* x, float pot, float leak,
+                                            float hi, float lo, double e_term, bool stop, uint16_t* list)
+{
+    const int lane = threadIdx.x & 31;
+    const int skip = (int)((uintptr_t)(nib + q0) & 7);  // quads of the first word before the row
+    const unsigned long long* words = (const unsigned long long*)(nib + q0 - skip);
+    const int nw = (skip + nq + 7) >> 3;
+    x += 4 * (q0 - skip);
+    const TermFactor F{hi, lo, e_term};
+    unsigned long long next = lane < nw ? __ldcg(words + lane) : 0ull;
+    for (int w0 = 0; w0 < nw; w0 += 32, x += 1024) {
+        const int w = w0 + lane;
+        const uint32_t b0 = (uint32_t)next, b1 = (uint32_t)(next >> 32);
+        uint32_t m = __byte_perm(b0 | b0 >> 4, b1 | b1 >> 4, 0x6420);
+        if (w == 0) m &= ~0u << (4 * skip);
+        if (w == nw - 1 && ((skip + nq) & 7)) m &= (1u << (4 * ((skip + nq) & 7))) - 1u;
+        if (w >= nw) m = 0u;
+        next = w + 32 < nw ? __ldcg(words + w + 32) : 0ull;
+        int at = __popc(m);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, at, o);
+            if (lane >= o) at += y;
+        }
+        const int total = __shfl_sync(kFull, at, 31);
+        for (at -= __popc(m); m; m &= m - 1u) list[at++] = (uint16_t)(32 * lane + __ffs((int)m) - 1);
+        __syncwarp();
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const float xv = k0 + lane < total ? x[list[k0 + lane]] : -0.0f;
+            for (int k = 0; k < min(32, total - k0); k += 8) {
+                float t[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) t[u] = __shfl_sync(kFull, xv, k + u);
+                pot = fold_terms(pot, t, F);
+                if (stop && fires_at(pot, leak)) return pot;
+            }
+        }
+        __syncwarp();
+    }
+    return pot;
+}
+
+// Whether this block is the last of those that stream the parts of a split tile (the neuron
+// warp calls, after its stream warps have arrived): it updates the neurons, the others' window
+// bits are there to read.
+__device__ __forceinline__ bool last_part(const NcPools& P, int32_t part, int lane)
+{
+    unsigned n = 0u;
+    if (lane == 0) {
+        uint32_t* ctr = P.split_ctr + (part & 0xffff) - 1;
+        __threadfence();
+        n = atomicAdd(ctr, 1u) + 1u;
+        if (n == (unsigned)part >> 16) *ctr = 0u;
+        __threadfence();
+    }
+    return __shfl_sync(kFull, n, 0) == (unsigned)part >> 16;
 }
 
 // What a net's quads share.
@@ -544,9 +616,10 @@ __device__ __forceinline__ void tile_synapses(const NcPools& P, const TileConst&
 }
 
 // The stream warps' part of a step (or of the flush of the last one).
-template <bool kFlush, bool kAlone, bool kStage>
+template <bool kFlush, bool kAlone, Kind kKind>
 __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
+    constexpr bool kStage = kKind == kStaged;
     const int lane = threadIdx.x & 31;
     const uint32_t threads = blockDim.x - 32;
     const Ring ring(dyn, threads);
@@ -670,7 +743,8 @@ __device__ __forceinline__ void stream_role(const NcPools& P, BlockShared& sh, u
             }
         }
         const int b = n & 1;
-        uint8_t* nib = (tile.nq <= kNibCap ? sh.nib[b] - tile.q0 : P.nib);  // by pool index of the quad
+        // by pool index of the quad (a part's are read by whichever block ends last)
+        uint8_t* nib = (tile.nq <= kNibCap && !(kKind == kSplit && tile.part) ? sh.nib[b] - tile.q0 : P.nib);
         bar_sync<kBarReady>(b);
         const uint32_t row0 = (uint32_t)tile.first, nq = (uint32_t)tile.nq;
         if (C.wide)
@@ -711,9 +785,10 @@ __device__ __forceinline__ void give_rows(const NcPools& P, BlockShared& sh, int
 }
 
 // The neuron warp's part of a step.
-template <bool kFlush, bool kAlone, bool kStage>
+template <bool kFlush, bool kAlone, Kind kKind>
 __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
+    constexpr bool kStage = kKind == kStaged;
     const int lane = threadIdx.x & 31;
     Tiles<kFlush> at(P, back);
     // (the first tile's rows, into the L1 or at least the L2)
@@ -756,7 +831,20 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
         const int32_t t = D.t;
         const int32_t kc = D.kc;
         const int32_t i = tile.first + lane, pj = tile.neuron + lane;
-        const bool live = lane < tile.count;
+        auto streamed = [&] {
+            bar_sync<kBarFull>(b);
+            if (at.ti < 0) {  // the block's last tile: all its warps have read the step counters
+                counted = true;
+                if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
+            }
+        };
+        // the neurons of a split tile are the last block's
+        bool mine = true;
+        if (kKind == kSplit && tile.part) {
+            streamed();
+            mine = last_part(P, tile.part, lane);
+        }
+        const bool live = mine && lane < tile.count;
         const bool stop = D.nonneg_terms != 0;
         const float leak = D.leak;
         const float* tables = P.tables + D.table_base;
@@ -799,14 +887,20 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
         const bool can = lf == NC_NEVER || t - lf >= kc;
         const TermFactor F = term_factor(D);
         const bool need = live && can && !(stop && fires_at(pot, leak));
-        bar_sync<kBarFull>(b);
-        if (at.ti < 0) {  // the block's last tile: all its warps have read the step counters
-            counted = true;
-            if (lane == 0) arrived = atomicAdd(P.done_ctr, 1u);
+        if (kKind != kSplit || !tile.part) {
+            streamed();
+            const uint8_t* nib = tile.nq <= kNibCap ? sh.nib[b] : P.nib + tile.q0;
+            const float* x = kStage ? (const float*)(dyn + kRingBytes * (blockDim.x - 32)) : P.x + 4 * (int64_t)tile.q0;
+            if (need) pot = fold_row<kStage>(nib, q0, nq, x, pot, leak, F, stop);
+        } else {
+            for (unsigned todo = __ballot_sync(kFull, need); todo; todo &= todo - 1u) {
+                const int j = __ffs((int)todo) - 1;
+                const float sum =
+                    fold_long_row(P.nib, (int64_t)tile.q0 + __shfl_sync(kFull, q0, j), __shfl_sync(kFull, nq, j), P.x,
+                                  __shfl_sync(kFull, pot, j), leak, F.hi, F.lo, F.e_term, stop, (uint16_t*)sh.nib[b]);
+                if (lane == j) pot = sum;
+            }
         }
-        const uint8_t* nib = tile.nq <= kNibCap ? sh.nib[b] : P.nib + tile.q0;
-        const float* x = kStage ? (const float*)(dyn + kRingBytes * (blockDim.x - 32)) : P.x + 4 * (int64_t)tile.q0;
-        if (need) pot = fold_row<kStage>(nib, q0, nq, x, pot, leak, F, stop);
         __syncwarp();
         if (ahead.ti >= 0) {
             give_rows(P, sh, ahead.ti, b, lane);
@@ -833,7 +927,7 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
         }
         const uint32_t fmask = __ballot_sync(kFull, fired);
         // a tile may hold part of a word: bytes (8 neurons) are written on their own
-        if (lane < 4 && 8 * lane < tile.count) {
+        if (mine && lane < 4 && 8 * lane < tile.count) {
             const int32_t at_byte = tile.first / 8 + lane;
             const uint8_t v = (uint8_t)(fmask >> (8 * lane));
             fired_t[at_byte] = v;
@@ -853,25 +947,25 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
 }
 
 // One step (or the flush of the last one) of every tile of this block.
-template <bool kFlush, bool kAlone, bool kStage>
+template <bool kFlush, bool kAlone, Kind kKind>
 __device__ __forceinline__ void dense_pass(const NcPools& P, BlockShared& sh, unsigned char* dyn, bool back)
 {
     if (threadIdx.x >= blockDim.x - 32) {
-        neuron_role<kFlush, kAlone, kStage>(P, sh, dyn, back);
+        neuron_role<kFlush, kAlone, kKind>(P, sh, dyn, back);
     } else {
-        stream_role<kFlush, kAlone, kStage>(P, sh, dyn, back);
+        stream_role<kFlush, kAlone, kKind>(P, sh, dyn, back);
     }
 }
 
 #ifndef NC_DENSE_MIN_BLOCKS
 #define NC_DENSE_MIN_BLOCKS 3
 #endif
-template <bool kFlush, bool kStage>
+template <bool kFlush, Kind kKind>
 __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_step(NcPools P, bool back)
 {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ BlockShared sh;
-    dense_pass<kFlush, true, kStage>(P, sh, dyn, back);
+    dense_pass<kFlush, true, kKind>(P, sh, dyn, back);
 }
 
 // ---------------------------------------------------------------- fused multi-step launch
@@ -913,6 +1007,7 @@ __device__ bool grid_barrier(unsigned* bar, unsigned& gen, uint32_t* dev_err, Bl
     return sh.ok != 0;
 }
 
+template <Kind kKind>
 __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_fused(NcPools P, int32_t ticks,
                                                                                 unsigned* bar)
 {
@@ -921,27 +1016,37 @@ __global__ void __launch_bounds__(kMaxThreads, NC_DENSE_MIN_BLOCKS) k_dense_fuse
     unsigned gen = 0u;
     if (threadIdx.x == 0) gen = atomicAdd(&bar[1], 0u);
     for (int32_t k = 0; k < ticks; ++k) {
-        dense_pass<false, false, false>(P, sh, dyn, k & 1);
+        dense_pass<false, false, kKind>(P, sh, dyn, k & 1);
         if (!grid_barrier(bar, gen, P.dev_err, sh)) return;
     }
 }
 
-// Blocks of one wave of kernel `which` (0: a step, 1: several, 2: a step with staged charges)
-// with `threads` threads on the current device (cached per device and block size).  Returns 0
-// when the device cannot run it (the launch then reports an error).
-int resident_blocks(int which, int threads)
+// The kernels by kind, of one step and of several.
+const void* step_kernel(Kind kind)
 {
-    static std::atomic<int> cache[3][64][kMaxThreads / 32 + 1];
+    return kind == kStaged ? (const void*)k_dense_step<false, kStaged>
+           : kind == kSplit ? (const void*)k_dense_step<false, kSplit>
+                            : (const void*)k_dense_step<false, kWhole>;
+}
+const void* fused_kernel(Kind kind)
+{
+    return kind == kSplit ? (const void*)k_dense_fused<kSplit> : (const void*)k_dense_fused<kWhole>;
+}
+
+// Blocks of one wave of a kind's kernel with `threads` threads on the current device (cached per
+// device and block size).  Returns 0 when the device cannot run it (the launch then reports an
+// error).
+int resident_blocks(bool fused, Kind kind, int threads)
+{
+    static std::atomic<int> cache[2][3][64][kMaxThreads / 32 + 1];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    std::atomic<int>& c = cache[which][dev][threads / 32];
+    std::atomic<int>& c = cache[fused][kind][dev][threads / 32];
     int n = c.load(std::memory_order_relaxed);
     if (n == 0) {
         int sms = 0, per_sm = 0;
-        const size_t dyn = dyn_bytes(threads - 32, which == 2);
-        const void* fn = which == 1   ? (const void*)k_dense_fused
-                         : which == 2 ? (const void*)k_dense_step<false, true>
-                                      : (const void*)k_dense_step<false, false>;
+        const size_t dyn = dyn_bytes(threads - 32, kind == kStaged);
+        const void* fn = fused ? fused_kernel(kind) : step_kernel(kind);
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, dyn) != cudaSuccess || sms * per_sm <= 0)
             return 0;
@@ -990,11 +1095,15 @@ bool dense_stages(const std::vector<NcRowTile>& tiles, const std::vector<int32_t
     for (size_t b = 0; b + 1 < start.size(); ++b)
         if (start[b + 1] - start[b] > 1) return false;
     for (const NcRowTile& t : tiles)
-        if (t.nq > kStageQuads) return false;
-    return resident_blocks(2, std::max(threads, 64)) >= (int)start.size() - 1;
+        if (t.nq > kStageQuads || t.part) return false;
+    return resident_blocks(false, kStaged, std::max(threads, 64)) >= (int)start.size() - 1;
 }
 
-int dense_resident_blocks(int threads) { return resident_blocks(0, std::max(threads, 64)); }
+int dense_resident_blocks(int threads)
+{
+    resident_blocks(false, kSplit, std::max(threads, 64));
+    return resident_blocks(false, kWhole, std::max(threads, 64));
+}
 
 int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* stream)
 {
@@ -1002,16 +1111,19 @@ int launch_step_dense(const NcPools& P, const LaunchShape& L, bool back, void* s
     const int threads = block_threads(L);
     const int blocks = L.dense_blocks > 0 ? std::min(L.dense_blocks, P.row_blocks) : P.row_blocks;
     // (another launch shape than the plan's may not hold every block in a wave)
-    const bool stage = P.stage && L.dense_blocks == 0 && resident_blocks(2, threads) >= blocks;
-    return launch_dependent(stage ? k_dense_step<false, true> : k_dense_step<false, false>, blocks, threads,
-                            dyn_bytes(threads - 32, stage), P, back, stream);
+    const bool stage = P.stage && L.dense_blocks == 0 && resident_blocks(false, kStaged, threads) >= blocks;
+    return launch_dependent(stage     ? k_dense_step<false, kStaged>
+                            : P.split ? k_dense_step<false, kSplit>
+                                      : k_dense_step<false, kWhole>,
+                            blocks, threads, dyn_bytes(threads - 32, stage), P, back, stream);
 }
 
 int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, unsigned* bar, void* stream)
 {
     if (ticks <= 0) return 0;
     const int threads = block_threads(L);
-    const int resident = resident_blocks(1, threads);
+    const Kind kind = P.split ? kSplit : kWhole;
+    const int resident = resident_blocks(true, kind, threads);
     if (resident <= 0) return -1;
     // at most one wave
     const int blocks = std::min(resident, P.row_blocks);
@@ -1020,7 +1132,7 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, un
     if (cudaMemsetAsync(bar, 0, sizeof(unsigned), s) != cudaSuccess) return -1;
     NcPools p = P;
     void* args[] = {(void*)&p, (void*)&ticks, (void*)&bar};
-    if (cudaLaunchCooperativeKernel((const void*)k_dense_fused, dim3((unsigned)blocks), dim3((unsigned)threads), args,
+    if (cudaLaunchCooperativeKernel(fused_kernel(kind), dim3((unsigned)blocks), dim3((unsigned)threads), args,
                                     dyn_bytes(threads - 32, false), s) != cudaSuccess)
         return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
@@ -1029,7 +1141,7 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape& L, un
 int launch_flush_dense(const NcPools& P, const LaunchShape& L, void* stream)
 {
     const int threads = block_threads(L);
-    return launch_dependent(k_dense_step<true, false>, P.row_blocks, threads, dyn_bytes(threads - 32, false), P, false,
+    return launch_dependent(k_dense_step<true, kWhole>, P.row_blocks, threads, dyn_bytes(threads - 32, false), P, false,
                             stream);
 }
 

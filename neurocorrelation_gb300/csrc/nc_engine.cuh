@@ -167,7 +167,8 @@ struct alignas(16) NcRowTile {  // dense form: up to NC_TILE_ROWS consecutive ne
     int32_t neuron;      // pool index of the first neuron
     int32_t ptr;         // pool index of its row start
     int32_t count;       // neurons
-    int32_t pad;
+    int32_t part;        // 0: all quads of its neurons; otherwise one of (part >> 16) tiles of the same
+                         // neurons, which count on NcPools::split_ctr[(part & 0xffff) - 1]
 };
 
 constexpr int NC_TILE_ROWS = 32;  // neurons of a dense tile at most: one per lane
@@ -231,6 +232,8 @@ struct NcPools {
     NcRowTile* rtiles;   // in the order of the blocks that run them
     int32_t* rstart;     // first tile of each of row_blocks blocks (row_blocks + 1 entries)
     int32_t row_blocks;
+    int32_t split;       // dense step: some tiles are split
+    uint32_t* split_ctr; // parts of a split tile that are streamed (a counter each, row_blocks of them)
     int32_t stage;       // dense step: captured charges of the sums pass through shared memory (dense_stages)
     // ring and bitsets
     uint32_t* ring;

@@ -457,30 +457,64 @@ void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTil
     for (const RowNet& r : nets) total += r.h->sp / 4 + kNeuronWeight * r.h->n;
     tiles.clear();
     start.assign(1, 0);
+    int32_t splits = 0;
     for (const RowNet& r : nets) {
         const NetHost& h = *r.h;
         bool open = false;  // the last tile may grow
-        for (int32_t f = 0; f < h.n; f += 8) {
-            const int32_t count = std::min(h.n - f, 8);
-            const int64_t a = h.in_ptr[(size_t)f], b = h.in_ptr[(size_t)(f + count)];
-            const int64_t weight = (b - a) / 4 + kNeuronWeight * count;
-            // the block its middle falls to
-            const int64_t block = std::min<int64_t>(blocks - 1, (int64_t)((done + 0.5 * weight) * blocks / total));
-            done += weight;
+        auto reach = [&](int64_t block) {
             while ((int64_t)start.size() <= block) {
                 start.push_back((int32_t)tiles.size());
                 open = false;
             }
-            if (!open || tiles.back().count + count > NC_TILE_ROWS) {
-                tiles.push_back(NcRowTile{(uint32_t)((r.syn_base + a) / 4), 0, r.net, f, r.neuron_base + f,
-                                          r.ptr_base + f, 0, 0});
+        };
+        for (int32_t f = 0; f < h.n; f += 8) {
+            const int32_t count = std::min(h.n - f, 8);
+            const int64_t a = h.in_ptr[(size_t)f] / 4, quads = h.in_ptr[(size_t)(f + count)] / 4 - a;
+            const int64_t weight = quads + kNeuronWeight * count;
+            const NcRowTile run{(uint32_t)(r.syn_base / 4 + a), (int32_t)quads, r.net, f, r.neuron_base + f,
+                                r.ptr_base + f, count, 0};
+            const int64_t first = std::min<int64_t>(blocks - 1, (int64_t)((double)done * blocks / total));
+            // a run of more than two shares (rows of many in-synapses) is split over the blocks it
+            // reaches into
+            int64_t parts = 1;
+            if (quads > kSplitQuads && weight * blocks > 2 * total)
+                parts = std::min<int64_t>({(weight * blocks + total - 1) / total, quads / kPartQuads, blocks - first});
+            if (parts > 1) {
+                ++splits;
+                int64_t from = 0;
+                for (int64_t p = 0; p < parts; ++p) {
+                    reach(first + p);
+                    // (parts begin on a 128-byte line of the streams)
+                    const int64_t to = p + 1 == parts ? quads : quads * (p + 1) / parts / 8 * 8;
+                    NcRowTile t = run;
+                    t.q0 += (uint32_t)from;
+                    t.nq = (int32_t)(to - from);
+                    t.part = (int32_t)(parts << 16) | splits;
+                    tiles.push_back(t);
+                    from = to;
+                }
+                open = false;
+                done += weight;
+                continue;
+            }
+            // the block its middle falls to
+            reach(std::min<int64_t>(blocks - 1, (int64_t)((done + 0.5 * weight) * blocks / total)));
+            done += weight;
+            if (open && tiles.back().count + count <= NC_TILE_ROWS) {
+                tiles.back().nq += run.nq;
+                tiles.back().count += count;
+            } else {
+                tiles.push_back(run);
                 open = true;
             }
-            tiles.back().nq += (int32_t)((b - a) / 4);
-            tiles.back().count += count;
         }
     }
     while ((int)start.size() <= blocks) start.push_back((int32_t)tiles.size());
+}
+
+bool has_parts(const std::vector<NcRowTile>& tiles)
+{
+    return std::any_of(tiles.begin(), tiles.end(), [](const NcRowTile& t) { return t.part != 0; });
 }
 
 int set_groups(NetHost& h, int32_t n_groups, const nc_group* groups, std::string& err)

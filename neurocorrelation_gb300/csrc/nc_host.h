@@ -75,9 +75,16 @@ inline void term_pair(const NetHost& h, float& hi, float& lo)
 }
 // Initial state word (never launched) of the net's positions.
 inline uint32_t initial_state(const NetHost& h) { return h.wide ? (uint32_t)NC_WIDE_NEVER : nc_state_never(); }
+// A run of up to 1,536 quads, 24 rounds of a block's threads, is as fast whole: with a row of
+// 1,999 in-synapses 8.4 us a step whole and 15.0 split, of 3,999 12.9 and 14.7, of 7,999 20.4 and
+// 14.0.
+constexpr int64_t kSplitQuads = 1536;
+constexpr int64_t kPartQuads = 256;   // of a part, at least
 // The row tiles of an engine's nets, and the first tile of each of `blocks` blocks (blocks
 // + 1 entries): consecutive runs of neurons with an even share of the quads each, cut at
-// multiples of 8 neurons and into tiles of at most NC_TILE_ROWS.
+// multiples of 8 neurons and into tiles of at most NC_TILE_ROWS; 8 neurons with many more quads
+// than a share (and kSplitQuads) are split over several blocks (NcRowTile::part).  At most two tiles a block more
+// than the nets' own.
 struct RowNet {              // a net and its pool indexes
     const NetHost* h;
     int32_t net;
@@ -86,6 +93,7 @@ struct RowNet {              // a net and its pool indexes
 };
 void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTile>& tiles,
                std::vector<int32_t>& start);
+bool has_parts(const std::vector<NcRowTile>& tiles);
 // The net's out-synapse records (event form).
 std::vector<NcOut> out_records(const NetHost& h);
 // Builds the layout; returns NC_OK or an NC_ERR_* code with `err` set.  rows_only: without the

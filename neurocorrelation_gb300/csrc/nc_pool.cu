@@ -351,6 +351,8 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         P.stage = all_sum && dense_stages(rows, start, L.neuron_block) ? 1 : 0;
         NC_ALLOC(P.rtiles, NcRowTile, rows.size());
         NC_ALLOC(P.rstart, int32_t, start.size());
+        NC_ALLOC(P.split_ctr, uint32_t, P.row_blocks);
+        P.split = has_parts(rows) ? 1 : 0;
         NC_CK(upload(P.rtiles, rows, 0, stream));
         NC_CK(upload(P.rstart, start, 0, stream));
         NC_CK(cudaStreamSynchronize(stream));

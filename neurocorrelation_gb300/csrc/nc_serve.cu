@@ -145,7 +145,9 @@ struct nc_server {
     std::vector<int32_t> free_slots;
     int32_t* d_ntiles = nullptr;
     int32_t* d_nnets = nullptr;
-    cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // the event form's [1]: many units a warp of the spike launch
+    // a batch of steps; [1] with many units a warp of the spike launch (event form), or with split
+    // tiles (dense form)
+    cudaGraphExec_t graphs[2] = {nullptr, nullptr};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
     std::mutex mu;
@@ -262,12 +264,14 @@ int nc_server::init(std::string& err)
         S_AL(P.qrow, uint8_t, syn_cap / 4);
         S_AL(P.pst, float, neuron_cap);
         S_AL(P.nib, uint8_t, syn_cap / 4 + 8);
-        // every block may cut a tile short, and every network's last one is
+        // every block may cut a tile short or hold a part of one, and every network's last one is
+        // short
         L.neuron_block = NC_DENSE_BLOCK;
         P.row_blocks = nc::dense_blocks(neuron_cap, L.neuron_block);
-        rtile_cap = tile_cap + P.row_blocks;
+        rtile_cap = tile_cap + 2 * (int64_t)P.row_blocks;
         S_AL(P.rtiles, NcRowTile, rtile_cap);
         S_AL(P.rstart, int32_t, P.row_blocks + 1);
+        S_AL(P.split_ctr, uint32_t, P.row_blocks);
     } else {
         S_AL(P.inh, uint32_t, syn_cap / 32 + 1);
         S_AL(P.t_arr, int32_t, syn_cap);
@@ -309,7 +313,7 @@ int nc_server::init(std::string& err)
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
     S_CK(cudaStreamSynchronize(stream));
     rc = capture(false, &graphs[0], err);
-    return rc == NC_OK && !dense ? capture(true, &graphs[1], err) : rc;
+    return rc == NC_OK ? capture(true, &graphs[1], err) : rc;
 }
 
 int nc_server::capture(bool many, cudaGraphExec_t* graph, std::string& err)
@@ -318,6 +322,7 @@ int nc_server::capture(bool many, cudaGraphExec_t* graph, std::string& err)
     // the device, and the dense step's blocks find their tiles there: the grids need not
     // follow the resident networks
     NcPools G = P;
+    G.split = many;
     G.n_tiles = (int32_t)std::min<int64_t>(tile_cap, 152 * 16 * (L.neuron_block / 32));
     cudaGraph_t g = nullptr;
     S_CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -653,6 +658,7 @@ int nc_server::upload_tiles(std::string& err)
         S_CK(put(P.rtiles, rows, 0, stream));
         S_CK(put(P.rstart, start, 0, stream));
         S_CK(cudaStreamSynchronize(stream));
+        P.split = nc::has_parts(rows) ? 1 : 0;
         return NC_OK;
     }
     std::vector<NcTile> tiles;
@@ -675,7 +681,7 @@ int nc_server::upload_tiles(std::string& err)
 int nc_server::run_batch(float& ms, std::string& err)
 {
     S_CK(cudaEventRecord(ev0, stream));
-    S_CK(cudaGraphLaunch(graphs[!dense && nc::many_units(P.n_tiles, P, L)], stream));
+    S_CK(cudaGraphLaunch(graphs[dense ? P.split : nc::many_units(P.n_tiles, P, L)], stream));
     S_CK(cudaEventRecord(ev1, stream));
     S_CK(cudaEventSynchronize(ev1));
     S_CK(cudaEventElapsedTime(&ms, ev0, ev1));

@@ -326,6 +326,75 @@ static void footprint()
     }
 }
 
+// The dense step's tiles: every quad of every network once and in order, runs of 8 neurons whole
+// or split over consecutive blocks, no more tiles than a server has room for.
+static void row_plan()
+{
+    unsigned seed = 1;
+    auto rnd = [&](int n) { return (int)((seed = seed * 1664525u + 1013904223u) >> 8) % n; };
+    int splits_seen = 0;
+    for (int trial = 0; trial < 300; ++trial) {
+        std::vector<nc::NetHost> hosts((size_t)(1 + rnd(4)));
+        std::vector<nc::RowNet> nets;
+        int64_t syn = 0, words = 0;
+        int32_t neurons = 0;
+        for (size_t q = 0; q < hosts.size(); ++q) {
+            nc::NetHost& h = hosts[q];
+            h.n = rnd(5) ? 1 + rnd(300) : 8 * rnd(20);
+            h.in_ptr.assign(1, 0);
+            for (int32_t j = 0; j < h.n; ++j) {
+                const int64_t fan = rnd(40) ? rnd(60) : rnd(3) ? 1000 + rnd(3000) : 20000 + rnd(60000);
+                const int64_t a = nc::row_align(j), end = h.in_ptr.back() + fan;
+                h.in_ptr.push_back((end + a - 1) / a * a);
+            }
+            h.sp = h.in_ptr.back();
+            nets.push_back({&h, (int32_t)q, syn, neurons, neurons + (int32_t)q});
+            syn += (h.sp + 31) / 32 * 32;
+            neurons += h.n;
+            words += (h.n + 31) / 32;
+        }
+        const int blocks = 1 + rnd(trial % 2 ? 1216 : 40);
+        std::vector<NcRowTile> tiles;
+        std::vector<int32_t> start;
+        nc::plan_rows(nets, blocks, tiles, start);
+        check((int)start.size() == blocks + 1 && start[0] == 0 && start[(size_t)blocks] == (int32_t)tiles.size(), "starts");
+        check((int64_t)tiles.size() <= words + 2 * blocks, "number of tiles");
+        size_t k = 0;
+        for (size_t q = 0; q < nets.size(); ++q) {
+            const nc::NetHost& h = hosts[q];
+            int64_t quad = nets[q].syn_base / 4;
+            for (int32_t f = 0; f < h.n;) {
+                check(k < tiles.size(), "tiles end early");
+                if (k >= tiles.size()) return;
+                const NcRowTile first = tiles[k];
+                check(first.first == f && first.first % 8 == 0 && first.count > 0 && first.count <= NC_TILE_ROWS, "neurons");
+                check(first.neuron == nets[q].neuron_base + f && first.ptr == nets[q].ptr_base + f, "bases");
+                const int parts = first.part ? first.part >> 16 : 1;
+                check(!first.part || (parts > 1 && first.count <= 8 && (first.part & 0xffff) <= blocks), "part");
+                for (int p = 0; p < parts; ++p, ++k) {
+                    const NcRowTile& t = tiles[k];
+                    check(t.net == (int32_t)q && t.q0 == quad && t.part == first.part && t.count == first.count &&
+                              t.first == f && (parts == 1 || t.nq > 0),
+                          "quads");
+                    quad += t.nq;
+                }
+                splits_seen += parts > 1;
+                f += first.count;
+                check(quad == (nets[q].syn_base + h.in_ptr[(size_t)f]) / 4, "rows of the neurons");
+            }
+        }
+        check(k == tiles.size(), "tiles left");
+        for (int b = 0; b < blocks; ++b) {
+            check(start[(size_t)b] <= start[(size_t)b + 1], "blocks in order");
+            for (int32_t t = start[(size_t)b] + 1; t < start[(size_t)b + 1]; ++t)
+                check(!tiles[(size_t)t].part || tiles[(size_t)t].part != tiles[(size_t)t - 1].part ||
+                          tiles[(size_t)t].net != tiles[(size_t)t - 1].net, "one part of a run to a block");
+        }
+        if (fails) return;
+    }
+    check(splits_seen > 100, "runs were split");
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -340,6 +409,7 @@ int main(int argc, char** argv)
     else if (what == "server_read_fails") server_read_fails();
     else if (what == "server_device_lost") server_device_lost();
     else if (what == "footprint") footprint();
+    else if (what == "row_plan") row_plan();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;

@@ -34,7 +34,8 @@ def host_paths(tmp_path_factory):
 @pytest.mark.parametrize("check", ["weights_order", "raster_order", "raster_refused",
                                    "detectors_order", "detectors_refused",
                                    "reads_allocate_nothing", "no_index",
-                                   "failed_read", "server_read_fails", "server_device_lost", "footprint"])
+                                   "failed_read", "server_read_fails", "server_device_lost", "footprint",
+                                   "row_plan"])
 def test_host_path(host_paths, check):
     r = subprocess.run([host_paths, check], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
