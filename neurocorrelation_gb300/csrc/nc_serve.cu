@@ -146,7 +146,7 @@ struct nc_server {
     int32_t* d_ntiles = nullptr;
     int32_t* d_nnets = nullptr;
     // a batch of steps; [1] with many units a warp of the spike launch (event form), or with split
-    // tiles (dense form)
+    // tiles (dense form), captured when first needed
     cudaGraphExec_t graphs[2] = {nullptr, nullptr};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
@@ -312,8 +312,7 @@ int nc_server::init(std::string& err)
     L.launch_block = 128;
     L.launch_blocks = std::max(1, sms * NC_LAUNCH_BLOCKS);
     S_CK(cudaStreamSynchronize(stream));
-    rc = capture(false, &graphs[0], err);
-    return rc == NC_OK ? capture(true, &graphs[1], err) : rc;
+    return capture(false, &graphs[0], err);
 }
 
 int nc_server::capture(bool many, cudaGraphExec_t* graph, std::string& err)
@@ -680,8 +679,11 @@ int nc_server::upload_tiles(std::string& err)
 // One batch of steps of every resident network; ms: its device time.
 int nc_server::run_batch(float& ms, std::string& err)
 {
+    const int kind = dense ? P.split : nc::many_units(P.n_tiles, P, L);
+    if (!graphs[kind])
+        if (const int rc = capture(kind != 0, &graphs[kind], err)) return rc;
     S_CK(cudaEventRecord(ev0, stream));
-    S_CK(cudaGraphLaunch(graphs[dense ? P.split : nc::many_units(P.n_tiles, P, L)], stream));
+    S_CK(cudaGraphLaunch(graphs[kind], stream));
     S_CK(cudaEventRecord(ev1, stream));
     S_CK(cudaEventSynchronize(ev1));
     S_CK(cudaEventElapsedTime(&ms, ev0, ev1));
