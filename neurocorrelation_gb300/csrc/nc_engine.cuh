@@ -322,7 +322,10 @@ struct LaunchShape {
     int fused_ticks = 0;  // dense form: steps per fused cooperative launch (0: one launch
                           // per step, replayed through CUDA graphs)
 };
-int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream);
+// whole: it waits for the kernel before it as a whole.  For the step after a kernel that writes
+// what the step reads before its own wait (potentials, last fires, fired bits, or the counters:
+// launch_stdp_flush does).
+int launch_neuron_step(const NcPools& P, const LaunchShape& L, bool whole, void* stream);
 // Blocks of the neuron step that fit on the current device at once; asked before a capture.
 int event_resident_blocks(int threads);
 // many: the warps have several units each (many_units of the live tiles).

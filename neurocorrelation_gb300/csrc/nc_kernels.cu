@@ -195,7 +195,8 @@ constexpr int kBatch = 8;  // charges, or weights, of a row gathered together
 // is not in L2), so:
 //   - what neither the spike launch of the step before nor a kernel between two steps writes
 //     (everything but charges, ring bits, arrival steps and fire requests) is read, and the
-//     draws are made, before the wait;
+//     draws are made, before the wait.  A flush writes stdp_done too: the step after one waits
+//     for it as a whole (launch_neuron_step);
 //   - the ring words of the whole window come in one go, then the gathers of the arrivals'
 //     weights and of the sum's charges together;
 //   - a small network gives a warp fewer neurons, so that a warp has fewer fired rows and a
@@ -656,8 +657,8 @@ static int check_launch()
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// Launches fn<<<grid, block, 0, s>>>(P) as a programmatic dependent launch.
-static int launch_dependent(void (*fn)(NcPools), int grid, int block, void* stream, const NcPools& P)
+// Launches fn<<<grid, block, 0, s>>>(P), as a programmatic dependent launch unless `whole`.
+static int launch_dependent(void (*fn)(NcPools), int grid, int block, void* stream, const NcPools& P, bool whole = false)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -667,7 +668,7 @@ static int launch_dependent(void (*fn)(NcPools), int grid, int block, void* stre
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = whole ? 0 : 1;
     if (cudaLaunchKernelEx(&cfg, fn, P) != cudaSuccess) return -1;
     return check_launch();
 }
@@ -692,7 +693,7 @@ int event_resident_blocks(int threads)
     return n;
 }
 
-int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream)
+int launch_neuron_step(const NcPools& P, const LaunchShape& L, bool whole, void* stream)
 {
     const int64_t warps = (int64_t)P.n_tiles * (32 / P.warp_rows);
     int64_t blocks = (warps + L.neuron_block / 32 - 1) / (L.neuron_block / 32);
@@ -700,7 +701,7 @@ int launch_neuron_step(const NcPools& P, const LaunchShape& L, void* stream)
     // another (2M neurons, 13 waves: 151 us a step, 134 so; 500k busy 312 either way)
     const int resident = event_resident_blocks(L.neuron_block);
     if (resident > 0) blocks = std::min<int64_t>(blocks, resident);
-    return launch_dependent(k_neuron_step, (int)std::max<int64_t>(1, blocks), L.neuron_block, stream, P);
+    return launch_dependent(k_neuron_step, (int)std::max<int64_t>(1, blocks), L.neuron_block, stream, P, whole);
 }
 
 bool many_units(int n_tiles, const NcPools& P, const LaunchShape& L)

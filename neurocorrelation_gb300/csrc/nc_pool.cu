@@ -448,7 +448,9 @@ int Engine::step(int64_t ticks, std::string& err)
 int Engine::launch_tick(cudaStream_t s)
 {
     int rc = P.n_firers > 0 ? launch_input_firers(P, dense, s) : 0;  // the step's run-call schedule first
-    rc |= dense ? launch_step_dense(P, L, back_ = !back_, s) : (launch_neuron_step(P, L, s) | launch_spike_launch(P, L, many_units(P.n_tiles, P, L), s));
+    const bool whole = counters_written_;
+    counters_written_ = false;
+    rc |= dense ? launch_step_dense(P, L, back_ = !back_, s) : (launch_neuron_step(P, L, whole, s) | launch_spike_launch(P, L, many_units(P.n_tiles, P, L), s));
     return rc;
 }
 
@@ -528,7 +530,9 @@ int Engine::time_kernels(int ticks, float* neuron_ms, float* launch_ms, std::str
             return NC_ERR_CUDA;
         }
         NC_CK(cudaEventRecord(at[0], stream));
-        if (dense ? launch_step_dense(P, L, back_ = !back_, stream) : launch_neuron_step(P, L, stream)) {
+        const bool whole = counters_written_;
+        counters_written_ = false;
+        if (dense ? launch_step_dense(P, L, back_ = !back_, stream) : launch_neuron_step(P, L, whole, stream)) {
             err = "launch";
             return NC_ERR_CUDA;
         }
@@ -563,7 +567,7 @@ int Engine::flush_plasticity(std::string& err)
         err = cuda_msg("plasticity flush", cudaGetLastError());
         return NC_ERR_CUDA;
     }
-    flushed_ = true;
+    flushed_ = counters_written_ = true;
     return NC_OK;
 }
 

@@ -105,6 +105,7 @@ private:
     bool shared_tables_ = false;  // the GPU uses the host's page tables: it can write ordinary host memory
     size_t scratch_bytes_ = 0;
     bool flushed_ = false, unseen_ = false;
+    bool counters_written_ = false;  // by a flush, since the last step that was launched
     std::vector<void*> allocs_;
     char* block_ = nullptr;      // what is left of the last block of small arrays
     size_t block_left_ = 0;

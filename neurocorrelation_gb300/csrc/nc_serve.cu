@@ -328,7 +328,7 @@ int nc_server::capture(bool many, cudaGraphExec_t* graph, std::string& err)
     int rc = 0;
     for (int k = 0; k < cfg.steps_per_batch && rc == 0; ++k) {
         if (dense) rc |= nc::launch_step_dense(G, L, k & 1, stream);
-        else rc |= nc::launch_neuron_step(G, L, stream) | nc::launch_spike_launch(G, L, many, stream);
+        else rc |= nc::launch_neuron_step(G, L, false, stream) | nc::launch_spike_launch(G, L, many, stream);
     }
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     if (rc != 0 || e != cudaSuccess) {

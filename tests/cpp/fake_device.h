@@ -33,6 +33,8 @@ size_t fail_malloc_from = ~(size_t)0;  // allocations of so many bytes and more 
 int faults = 0;
 int legacy_delay = 0;
 int gathers_to_fail = 0, graphs_to_fail = 0;
+bool flush_open = false;  // the event form's flush was launched, and nothing has waited for it
+int early_steps = 0;      // steps that may read what it writes before it is done
 
 struct Late {
     int left;
@@ -175,7 +177,7 @@ cudaError_t cudaMemset(void* p, int v, size_t bytes)
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return *s = (cudaStream_t)1, cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return fake::flush_open = false, cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = (cudaEvent_t)1, cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
@@ -218,8 +220,12 @@ int launch_step_dense(const NcPools& P, const LaunchShape&, bool, void*)
 {
     return fake::launch([P] { fake::step(P); });
 }
-int launch_neuron_step(const NcPools& P, const LaunchShape&, void*)
+int launch_neuron_step(const NcPools& P, const LaunchShape&, bool whole, void*)
 {
+    if (!fake::capturing) {
+        fake::early_steps += fake::flush_open && !whole;
+        fake::flush_open = false;
+    }
     return fake::launch([P] { fake::step(P); });
 }
 int event_resident_blocks(int) { return 152 * 8; }
@@ -231,7 +237,11 @@ int launch_fused_dense(const NcPools& P, int32_t ticks, const LaunchShape&, unsi
         for (int32_t k = 0; k < ticks; ++k) fake::step(P);
     });
 }
-int launch_stdp_flush(const NcPools&, const LaunchShape&, void*) { return fake::launch([] {}); }
+int launch_stdp_flush(const NcPools&, const LaunchShape&, void*)
+{
+    fake::flush_open = true;
+    return fake::launch([] {});
+}
 int launch_flush_dense(const NcPools&, const LaunchShape&, void*) { return fake::launch([] {}); }
 int launch_form_to_event(const NcPools&, int, int64_t, int64_t, void*) { return fake::launch([] {}); }
 int launch_form_to_dense(const NcPools&, int, int64_t, void*) { return fake::launch([] {}); }

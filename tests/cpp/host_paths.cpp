@@ -395,6 +395,24 @@ static void row_plan()
     check(splits_seen > 100, "runs were split");
 }
 
+// A step of the event form after a flush that no call has waited for waits for it as a whole.
+static void flush_then_step()
+{
+    for (int32_t synapses : {0, 300}) {
+        Made m(40, synapses, NC_STEP_EVENT);
+        nc_net* net = m.create();
+        std::vector<nc_synapse_snapshot> snap((size_t)synapses + 1);
+        int64_t count = 0;
+        for (int round = 0; round < 2; ++round) {
+            check(nc_run(net, 3) == NC_OK, "run");
+            check(nc_read_synapse_snapshots(net, snap.data(), synapses + 1, &count) == NC_OK, "snapshots");
+            check(nc_run_noalloc(net, 1, nullptr) == NC_OK, "step");
+        }
+        check(fake::early_steps == 0, "steps that may be early, " + std::to_string(synapses) + " synapses");
+        nc_destroy(net);
+    }
+}
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -410,6 +428,7 @@ int main(int argc, char** argv)
     else if (what == "server_device_lost") server_device_lost();
     else if (what == "footprint") footprint();
     else if (what == "row_plan") row_plan();
+    else if (what == "flush_then_step") flush_then_step();
     else check(false, "no such check: " + what);
     std::printf("%s\n", fails ? "FAILED" : "OK");
     return fails != 0;

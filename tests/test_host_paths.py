@@ -35,7 +35,7 @@ def host_paths(tmp_path_factory):
                                    "detectors_order", "detectors_refused",
                                    "reads_allocate_nothing", "no_index",
                                    "failed_read", "server_read_fails", "server_device_lost", "footprint",
-                                   "row_plan"])
+                                   "row_plan", "flush_then_step"])
 def test_host_path(host_paths, check):
     r = subprocess.run([host_paths, check], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
