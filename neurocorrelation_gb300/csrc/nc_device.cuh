@@ -147,9 +147,6 @@ static __device__ __forceinline__ float fold_terms(float p, const float (&x)[8],
 // only grows (rounding keeps the order) and so does this result, so a fold may stop once
 // it holds: the neuron fires whatever the remaining terms are, and its potential is then
 // replaced by the AP table (src/NeuCor.cpp:706-714).
-#ifndef NC_FOLD_EARLY_EXIT
-#define NC_FOLD_EARLY_EXIT 1
-#endif
 static __device__ __forceinline__ bool fires_at(float pot, float leak)
 {
     return -55.0f < (pot - -70.0f) * leak + -70.0f;

@@ -117,19 +117,6 @@ static void storage_order(NetHost& h, const float* xyz, int32_t order_kind)
     }
 }
 
-int64_t NetHost::device_bytes() const
-{
-    const int64_t per_neuron = 4 + 4 + 4 + 4 + 8 + 8 + 4;             // pot lf firings act_start in_ptr out_ptr ring_off
-    const bool dense = p.step_mode != NC_STEP_EVENT, event = p.step_mode != NC_STEP_DENSE;
-    // w x | key state (dense) and/or t_arr out last_arr (event); rows are
-    // padded to quads, and a quad has a row byte and a window byte
-    const int64_t per_syn = 4 + 4 + (dense ? 8 * key_words(*this) + 1 : 0) + (event ? 4 + 16 + 4 : 0);
-    const int64_t words = ((int64_t)n + 31) / 32;
-    const int64_t ring_bytes = event ? 4 * (int64_t)ring_slots * ring_words : 0;
-    return per_neuron * (n + 1) + per_syn * sp + ring_bytes + 4 * 4 * words +
-           8 * 2 * (int64_t)n + 4 * (int64_t)tables.size() + (int64_t)sizeof(NcGroupDev) * (int64_t)groups.size();
-}
-
 // Trace table powf(decay, k*dt) for k = 0.. until it underflows to zero, with the
 // reference's "a trace of exactly 1 counts as 0" rule (src/NeuCor.cpp:744-745).
 static bool trace_table(float decay, float dt, std::vector<float>& out, int32_t& len)

@@ -51,8 +51,6 @@ struct NetHost {
     int32_t tab_pre_len = 0, tab_post_len = 0, ap_len = 0;
     std::vector<NcGroupDev> groups;
     bool nonneg_terms = true;               // no inhibitory synapse and no negative weight
-
-    int64_t device_bytes() const;
 };
 
 // Source slot of a padding position: past the net's last slot, in the spare word of its
