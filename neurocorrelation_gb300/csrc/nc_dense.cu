@@ -47,8 +47,8 @@
 //     with one 16-byte access per array; every eighth row ends on a 128-byte line.
 //   - A run of 8 neurons with more quads than two blocks' shares is split over several blocks;
 //     the last of them to be done with its part updates the neurons (100k x 10 with one row of
-//     99,999 in-synapses 176 -> 19 us, with inhibitory synapses 373 -> 49; 200k x 25 with skewed
-//     rows 152 -> 45).
+//     99,999 in-synapses 176 -> 18 us, with inhibitory synapses 373 -> 49; 200k x 25 with skewed
+//     rows 152 -> 47).
 //   - A warp of its own sums, so the others never wait for a sum: with block barriers
 //     between the two halves the 100k x 100 step took 78 us (48 then).
 //   - 96 threads (two stream warps to a neuron warp), 80 registers, 8 blocks an SM, the
@@ -234,6 +234,27 @@ struct WindowBits {
         from += m ? __ffs((int)m) - 1 : 32;
         return any;
     }
+    // The same for windows of few bits: the next eight wherever they lie, a branch at each.
+    __device__ __forceinline__ bool next_of_few(float (&to)[8])
+    {
+        bool any = false;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            uint32_t m = from < 32 ? cur >> from : 0u;
+            while (m == 0u && (nxt | (uint32_t)(w < nw))) {
+                cur = nxt;
+                nxt = word();
+                x += 32;
+                from = 0;
+                m = cur;
+            }
+            const int b = from + __ffs((int)m) - 1;
+            to[k] = load_or_absent<kShared>(x + b, m);
+            any = any || m != 0u;
+            from = m ? b + 1 : 32;
+        }
+        return any;
+    }
 };
 
 // charge_insynapses (src/NeuCor.cpp:688-700) of one row: the terms of the spikes that
@@ -254,14 +275,14 @@ struct WindowBits {
 // whatever the remaining terms are, and its potential is then replaced by the AP table
 // (src/NeuCor.cpp:682-686, 706-714): the fold stops there and returns the partial sum,
 // which leads the update to the same decision.
-template <bool kShared>
+template <bool kShared, bool kFew = false>
 __device__ __forceinline__ float fold_row(const uint8_t* nib, int q0, int nq, const float* x0, float pot, float leak,
                                           const TermFactor& F, bool stop)
 {
     if (nq <= 0) return pot;
     WindowBits<kShared> at(nib, q0, nq, x0);
     float xv[8];
-    while (at.next(xv)) {
+    while (kFew ? at.next_of_few(xv) : at.next(xv)) {
         pot = fold_terms(pot, xv, F);
         if (stop && fires_at(pot, leak)) break;
     }
@@ -315,6 +336,72 @@ __device__ __noinline__ float fold_long_row(const uint8_t* nib, int64_t q0, int 
     return pot;
 }
 
+// The sums of a split tile, whose window bits lie in global memory (all lanes call): lane j's row is the
+// nq quads (0: no sum) from q0 on.  A few long rows are summed one after the other, by the whole
+// warp, which takes half as long for a term; rows of much the same length side by side, a lane
+// each, from shared memory (`buf`, kNibCap bytes) that the warp fills a piece of every row at a
+// time (one word after the other from L2: 160 us in the case below).
+__device__ __noinline__ float fold_split_rows(const uint8_t* nib, const float* x, int64_t q0, int nq, float pot, float leak,
+                                             float hi, float lo, double e_term, bool stop, uint8_t* buf)
+{
+    const int lane = threadIdx.x & 31;
+    const int longest = __reduce_max_sync(kFull, nq), all = __reduce_add_sync(kFull, nq);
+    if (all <= 2 * longest) {
+        for (unsigned todo = __ballot_sync(kFull, nq > 0); todo; todo &= todo - 1u) {
+            const int j = __ffs((int)todo) - 1;
+            const float sum = fold_long_row(nib, __shfl_sync(kFull, q0, j), __shfl_sync(kFull, nq, j), x,
+                                            __shfl_sync(kFull, pot, j), leak, hi, lo, e_term, stop, (uint16_t*)buf);
+            if (lane == j) pot = sum;
+        }
+        return pot;
+    }
+    const TermFactor F{hi, lo, e_term};
+    uint8_t* lane_of = buf + kNibCap - 32;  // the lanes of the rows left
+    unsigned todo;
+    for (int done = 0, piece; (todo = __ballot_sync(kFull, nq > done)) != 0u; done += piece) {
+        // a row's piece, with up to 7 quads before it in its first word
+        // (a short one first: most sums of a busy network stop in it)
+        const int rows = __popc(todo), stride = min((kNibCap - 32) / rows & ~7, done || !stop ? kNibCap : 56);
+        const int words = stride >> 3, total = words * rows;
+        piece = stride - 8;
+        const int64_t at = q0 + done;
+        const int skip = (int)((uintptr_t)(nib + at) & 7), mine = __popc(todo & ((1u << lane) - 1u));
+        if (nq > done) lane_of[mine] = (uint8_t)lane;
+        __syncwarp();
+        int bits = 0;
+        for (int k0 = 0; k0 < total; k0 += 128) {
+            unsigned long long v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = min(k0 + 32 * u + lane, total - 1), row = lane_of[k / words], w = k % words;
+                const int64_t from = __shfl_sync(kFull, at - skip, row);
+                const int left = __shfl_sync(kFull, skip + nq - done, row);
+                v[u] = 8 * w < left ? __ldcg((const unsigned long long*)(nib + from) + w) : 0ull;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = k0 + 32 * u + lane;
+                if (k < total) *((unsigned long long*)buf + k) = v[u];
+                if (k < total) bits += __popcll(v[u]);
+            }
+        }
+        // a batch looks at 32 synapses: with fewer than 3 of each in the window, the next eight are
+        // looked for instead (every neuron of 3,000 driving every other, inhibitory, quiet: 83 -> 73
+        // us a step, 120 with the rows whole)
+        const bool few = __reduce_add_sync(kFull, bits) < 3 * total;
+        __syncwarp();
+        if (nq > done) {
+            const uint8_t* row = buf + stride * mine + skip;
+            const int n = min(piece, nq - done);
+            pot = few ? fold_row<false, true>(row, 0, n, x + 4 * at, pot, leak, F, stop)
+                      : fold_row<false>(row, 0, n, x + 4 * at, pot, leak, F, stop);
+            if (stop && fires_at(pot, leak)) nq = 0;
+        }
+        __syncwarp();
+    }
+    return pot;
+}
+
 // Whether this block is the last of those that stream the parts of a split tile (the neuron
 // warp calls, after its stream warps have arrived): it updates the neurons, the others' window
 // bits are there to read.
@@ -328,6 +415,7 @@ __device__ __forceinline__ bool last_part(const NcPools& P, int32_t part, int la
         if (n == (unsigned)part >> 16) *ctr = 0u;
         __threadfence();
     }
+    __syncwarp();  // what lane 0 has seen, all lanes read
     return __shfl_sync(kFull, n, 0) == (unsigned)part >> 16;
 }
 
@@ -893,13 +981,8 @@ __device__ __forceinline__ void neuron_role(const NcPools& P, BlockShared& sh, u
             const float* x = kStage ? (const float*)(dyn + kRingBytes * (blockDim.x - 32)) : P.x + 4 * (int64_t)tile.q0;
             if (need) pot = fold_row<kStage>(nib, q0, nq, x, pot, leak, F, stop);
         } else {
-            for (unsigned todo = __ballot_sync(kFull, need); todo; todo &= todo - 1u) {
-                const int j = __ffs((int)todo) - 1;
-                const float sum =
-                    fold_long_row(P.nib, (int64_t)tile.q0 + __shfl_sync(kFull, q0, j), __shfl_sync(kFull, nq, j), P.x,
-                                  __shfl_sync(kFull, pot, j), leak, F.hi, F.lo, F.e_term, stop, (uint16_t*)sh.nib[b]);
-                if (lane == j) pot = sum;
-            }
+            pot = fold_split_rows(P.nib, P.x, (int64_t)tile.q0 + q0, need ? nq : 0, pot, leak, F.hi, F.lo, F.e_term, stop,
+                                  sh.nib[b]);
         }
         __syncwarp();
         if (ahead.ti >= 0) {

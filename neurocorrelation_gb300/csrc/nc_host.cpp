@@ -461,11 +461,18 @@ void plan_rows(const std::vector<RowNet>& nets, int blocks, std::vector<NcRowTil
             const NcRowTile run{(uint32_t)(r.syn_base / 4 + a), (int32_t)quads, r.net, f, r.neuron_base + f,
                                 r.ptr_base + f, count, 0};
             const int64_t first = std::min<int64_t>(blocks - 1, (int64_t)((double)done * blocks / total));
-            // a run of more than two shares (rows of many in-synapses) is split over the blocks it
-            // reaches into
+            // a run of several shares (rows of many in-synapses) is split over as many blocks, from the
+            // one it begins in: where one row is most of it, over all that it reaches into (there are
+            // few such runs); where its rows are even, so that no two runs' parts fall to one block
             int64_t parts = 1;
-            if (quads > kSplitQuads && weight * blocks > 2 * total)
-                parts = std::min<int64_t>({(weight * blocks + total - 1) / total, quads / kPartQuads, blocks - first});
+            if (quads > kSplitQuads) {
+                int64_t longest = 0;
+                for (int32_t j = f; j < f + count; ++j)
+                    longest = std::max(longest, h.in_ptr[(size_t)j + 1] / 4 - h.in_ptr[(size_t)j] / 4);
+                if (2 * longest > quads && weight * blocks > 2 * total) parts = (weight * blocks + total - 1) / total;
+                else if (quads > kSplitEvenQuads) parts = (4 * weight * blocks + total) / (4 * total);
+                parts = std::min<int64_t>({parts, quads / kPartQuads, blocks - first});
+            }
             if (parts > 1) {
                 ++splits;
                 int64_t from = 0;

@@ -75,14 +75,15 @@ inline void term_pair(const NetHost& h, float& hi, float& lo)
 inline uint32_t initial_state(const NetHost& h) { return h.wide ? (uint32_t)NC_WIDE_NEVER : nc_state_never(); }
 // A run of up to 1,536 quads, 24 rounds of a block's threads, is as fast whole: with a row of
 // 1,999 in-synapses 8.4 us a step whole and 15.0 split, of 3,999 12.9 and 14.7, of 7,999 20.4 and
-// 14.0.
-constexpr int64_t kSplitQuads = 1536;
+// 14.0.  So is one of up to 2,560 in rows of much the same length (every neuron of 1,000 driving
+// every other, inhibitory, quiet 28.9 and 30.7, of 1,500 50.6 and 38.9).
+constexpr int64_t kSplitQuads = 1536, kSplitEvenQuads = 2560;
 constexpr int64_t kPartQuads = 256;   // of a part, at least
 // The row tiles of an engine's nets, and the first tile of each of `blocks` blocks (blocks
 // + 1 entries): consecutive runs of neurons with an even share of the quads each, cut at
 // multiples of 8 neurons and into tiles of at most NC_TILE_ROWS; 8 neurons with many more quads
-// than a share (and kSplitQuads) are split over several blocks (NcRowTile::part).  At most two tiles a block more
-// than the nets' own.
+// than a share (and kSplitQuads) are split over several blocks (NcRowTile::part).  At most two
+// tiles a block more than the nets' own.
 struct RowNet {              // a net and its pool indexes
     const NetHost* h;
     int32_t net;

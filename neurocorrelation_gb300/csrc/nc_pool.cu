@@ -127,9 +127,14 @@ void event_rows(int64_t tiles, int sms, NcPools& P)
         P.launch_rows /= 2;
 }
 
-int dense_blocks(int64_t neurons, int threads)
+int dense_blocks(int64_t neurons, int64_t quads, int threads)
 {
-    return (int)std::max<int64_t>(1, std::min<int64_t>(dense_resident_blocks(threads), (neurons + 7) / 8));
+    // fewer blocks than a wave where there are fewer runs of 8 neurons: one for each, or as many
+    // for each as its rows are split into (every neuron of 3,000 driving every other 63 -> 46 us
+    // a step, with inhibitory synapses 248 -> 222)
+    const int64_t most = dense_resident_blocks(threads), runs = std::max<int64_t>(1, (neurons + 7) / 8);
+    const int64_t parts = quads / runs > kSplitEvenQuads ? std::min(2 * quads / runs / kSplitEvenQuads, most / runs) : 1;
+    return (int)std::max<int64_t>(1, std::min(most, runs * std::max<int64_t>(1, parts)));
 }
 
 void Engine::set_launch(const LaunchShape& shape, int ticks_per_graph)
@@ -341,7 +346,9 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
     if (dense) {
         std::vector<NcRowTile> rows;
         std::vector<int32_t> start;
-        P.row_blocks = dense_blocks(neurons, L.neuron_block);
+        int64_t quads = 0;
+        for (const NetHost* h : nets) quads += h->sp / 4;
+        P.row_blocks = dense_blocks(neurons, quads, L.neuron_block);
         plan_rows(row_nets, P.row_blocks, rows, start);
         // sums that run to their last term (inhibitory or negative synapses) gain from it: the
         // sphere of 750 6.3 -> 5.9 us a step, 20k x 100 20.7 -> 19.0; those that stop early, after

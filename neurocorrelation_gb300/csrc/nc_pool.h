@@ -119,9 +119,9 @@ private:
     int64_t ring_words_total_ = 0;
 };
 
-// Blocks of `threads` threads that the rows of `neurons` neurons are shared out to: one wave,
-// or a block for each 8 neurons.
-int dense_blocks(int64_t neurons, int threads);
+// Blocks of `threads` threads that the rows of `neurons` neurons, `quads` in all, are shared out
+// to: one wave, or a block for each 8 neurons (more where their rows are long).
+int dense_blocks(int64_t neurons, int64_t quads, int threads);
 // Neurons per warp of the event form's kernels, for an engine of so many 32-neuron tiles.
 void event_rows(int64_t tiles, int sms, NcPools& P);
 std::string cuda_msg(const char* what, cudaError_t e);

@@ -264,10 +264,9 @@ int nc_server::init(std::string& err)
         S_AL(P.qrow, uint8_t, syn_cap / 4);
         S_AL(P.pst, float, neuron_cap);
         S_AL(P.nib, uint8_t, syn_cap / 4 + 8);
-        // every block may cut a tile short or hold a part of one, and every network's last one is
-        // short
+        // (what cuts tiles short: plan_rows)
         L.neuron_block = NC_DENSE_BLOCK;
-        P.row_blocks = nc::dense_blocks(neuron_cap, L.neuron_block);
+        P.row_blocks = nc::dense_blocks(neuron_cap, syn_cap / 4, L.neuron_block);
         rtile_cap = tile_cap + 2 * (int64_t)P.row_blocks;
         S_AL(P.rtiles, NcRowTile, rtile_cap);
         S_AL(P.rstart, int32_t, P.row_blocks + 1);

@@ -1,7 +1,7 @@
 """The dense step with rows of so many in-synapses that they are split over blocks, against the
 oracle, bit for bit: runs just below and above the rule's size, several long rows in one run of 8,
 in the first and the last one, sparse and full windows, whole step counters, batches in every
-launch shape, and a served network."""
+launch shape, and a served network, rows of even length and of one long one."""
 import numpy as np
 import pytest
 
@@ -33,8 +33,9 @@ NETS = {
     "1537_quads": (lambda s: long_rows(6500, {3: 6145}, 0, 2, s), {}),
     "one_long_row": (lambda s: long_rows(7000, {1234: 6999}, 8000, 3, s), {}),
     "run_of_long_rows": (lambda s: long_rows(3000, {j: 1500 + 101 * (j - 16) for j in range(16, 24)}, 6000, 4, s), {}),
-    "first_and_last": (lambda s: long_rows(6501, {0: 4000, 7: 4000, 6500: 6500}, 3000, 5, s), {}),
+    "first_and_last": (lambda s: long_rows(6501, {0: 4000, 7: 3000, 6500: 6500}, 3000, 5, s), {}),
     "many": (lambda s: long_rows(6600, {j: 6400 for j in range(0, 6600, 597)}, 4000, 6, s), {}),
+    "even_rows": (lambda s: long_rows(1397, {j: 1396 - j % 5 for j in range(1397)}, 0, 9, s), {}),
     "whole_counters": (lambda s: long_rows(6500, {5: 6499}, 3000, 7, s), dict(presynaptic_trace_decay=0.9995)),
     "half_step": (lambda s: long_rows(4000, {5: 3999, 6: 3000}, 3000, 8, s), dict(run_speed=0.5)),
 }
@@ -68,7 +69,7 @@ def test_split_rows_match_the_oracle(nc, oracle_mod, name, negative, rate):
 
 
 def mixed():
-    return [long_rows(6500, {9: 6499}, 2000, 11, 0.2), random_net(40, 300, 12), long_rows(1500, {j: 1499 for j in range(5)}, 0, 13),
+    return [long_rows(6500, {9: 6499}, 2000, 11, 0.2), random_net(40, 300, 12), long_rows(1500, {j: 1499 for j in range(7)}, 0, 13),
             random_net(700, 9000, 14)]
 
 
