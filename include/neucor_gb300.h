@@ -83,11 +83,11 @@ typedef struct {
  *                  sums and updates the neurons beside it.  Its cost grows with the
  *                  synapse count, not with activity: the fast form when a large share
  *                  of neurons fires every step.
- *   NC_STEP_EVENT  two launches per step; fired neurons are compacted into a list and
- *                  only their out-synapses and the arrived spikes are touched.  Its cost
+ *   NC_STEP_EVENT  two launches per step: the neurons, then the out-synapses of those that
+ *                  fired; of the in-synapses only arrived spikes are touched.  Its cost
  *                  grows with the synaptic events: the faster form for sparse activity.
  *   NC_STEP_AUTO   a single network (nc_create, nc_create_knn) holds the tables of both
- *                  forms and switches between them at run-call boundaries from the share
+ *                  forms and switches between them, between two steps, from the share
  *                  of neurons that fired in the last window of steps (see nc_run); the
  *                  switch keeps every bit of the state.  It costs the memory of both forms.
  * Networks batched into one engine (nc_batch_create) run in the first network's form
@@ -209,9 +209,12 @@ int nc_schedule_fire(nc_net* net, int32_t count, const int32_t* neuron_ids);
  * calls) and reads its fire count at the end of each (a synchronisation): it moves to
  * the event form when fewer than
  * NC_AUTO_TO_EVENT_PERMILLE per mille of its neurons fired per step in the window, and
- * back to the dense form above NC_AUTO_TO_DENSE_PERMILLE (the measured crossover of the
- * two forms lies between: 100k x 100 at 1.1% of neurons firing per step, 38 us a step in
- * either form; 50k x 80 at 2.8%, 22.5 us). */
+ * back to the dense form above NC_AUTO_TO_DENSE_PERMILLE.  Measured, the two forms cross at
+ * 1.1% of neurons firing per step on 100k x 100 (38 us a step in either form) and at 2.8% on
+ * 50k x 80 (22.5 us): between 2% and 2.8% the smaller network runs in the dense form, where
+ * the event form would be some 10% faster.  There is no rule on size: networks of some
+ * 10k neurons and fewer are faster dense at any rate, and move to the event form all the same
+ * when they are quiet (nc_set_step_form pins a form). */
 #define NC_AUTO_WINDOW 256
 #define NC_AUTO_TO_EVENT_PERMILLE 10
 #define NC_AUTO_TO_DENSE_PERMILLE 20
@@ -239,6 +242,10 @@ int nc_record_raster(nc_net* net, int32_t max_steps);
 int nc_read_raster(nc_net* net, uint8_t* out, int64_t capacity_bytes, int32_t* steps);
 
 /* ------------------------------------------------------------ read-back */
+/* Read-backs allocate no device memory: their scratch (up to 64 MB) and the index of the
+ * weights (4 bytes a given synapse; without memory for it the host reorders them) are made
+ * with the network.  A read-back that fails before its result is there leaves the caller's
+ * buffer as it was. */
 /* NeuCor::potAct (src/NeuCor.h:105): potential, activity interleaved, 2*N floats. */
 int nc_read_potact(nc_net* net, float* out_2n);
 int nc_read_potentials(nc_net* net, float* out_n);
@@ -306,7 +313,7 @@ int nc_philox4x32_10(const uint32_t ctr[4], const uint32_t key[2], uint32_t out[
 
 /* ------------------------------------------------------ batched networks */
 /* Many independent networks packed into one device engine and advanced together:
- * every launch pair steps every unfinished network once.  Each network keeps its own
+ * every step's launches step every unfinished network once.  Each network keeps its own
  * constants, seed, inputs and horizon, and no state is shared, so a network computes
  * the same bits alone (nc_create) or packed.  There is no reference counterpart: the
  * reference simulates one NeuCor at a time (src/NeuCor.cpp:583-617). */
@@ -405,7 +412,7 @@ typedef struct {
     int64_t resident_bytes;      /* footprint of the networks resident now */
     int64_t peak_resident_bytes;
     int64_t peak_resident_networks;
-    int64_t steps_run;           /* launch pairs issued */
+    int64_t steps_run;           /* steps issued */
     double device_busy_s;        /* device time of the step batches */
 } nc_server_stats;
 
@@ -439,7 +446,9 @@ int nc_server_destroy(nc_server* server);
  * first use.  This call launches the same kernels directly on `stream` (NULL = the
  * handle's own stream) and calls no cudaMalloc, cudaFree or allocating library routine;
  * neither form's kernels need scratch.  In the event form it serves networks of at most
- * NC_NOALLOC_MAX_NEURONS neurons; larger ones are refused with NC_ERR_INVALID.
+ * NC_NOALLOC_MAX_NEURONS neurons; larger ones are refused with NC_ERR_INVALID (the limit of
+ * a scratch array of earlier versions, kept: callers are promised the refusal).  Read-backs
+ * allocate no device memory either.
  * Order the call after the handle's earlier work, and synchronise `stream`
  * before any other call on the handle when it is not the handle's stream.  After this
  * call the handle reads its step counter and simulated time back from the device

@@ -24,7 +24,7 @@ _LIB = os.path.join(_HERE, "_lib", "libneucor_gb300.so")
 
 NC_OK = 0
 NC_STEP_DENSE = 0  # step_mode: every in-row streamed in order each step, the neurons summed beside it
-NC_STEP_EVENT = 1  # step_mode: fired-list compaction and spike launch (sparse activity)
+NC_STEP_EVENT = 1  # step_mode: the neurons, then the out-synapses of those that fired (sparse activity)
 NC_STEP_AUTO = 2   # step_mode: both forms' tables; nc_run switches by the fire share
 _ERRORS = {-1: "invalid argument", -2: "CUDA error", -3: "out of memory", -4: "unsupported", -5: "no CUDA device",
            -6: "device wait timed out", -7: "over memory budget"}

@@ -61,7 +61,7 @@ struct NcGroupDev {
 // What a step writes comes first, in a cache line of its own: the rest may be read, and stay
 // in L1, before a launch's wait for the step before it.
 struct alignas(128) NcNetDesc {
-    int32_t t;            // step processed by the next launch pair (>= 1)
+    int32_t t;            // step processed by the next launch (>= 1)
     int32_t t_end;        // last step to simulate (inclusive)
     int32_t stdp_done;    // last step whose deferred plasticity has been applied
     float tsum;           // NeuCor::currentTime after t-1 steps: the float sum of t-1 runSpeeds

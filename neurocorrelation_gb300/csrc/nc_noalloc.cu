@@ -23,6 +23,7 @@ extern "C" int nc_run_noalloc(nc_net* net, int32_t n_steps, void* stream)
     cudaError_t e = cudaSetDevice(net->eng.device);
     if (e != cudaSuccess) return nc::set_last_error(NC_ERR_CUDA, nc::cuda_msg("cudaSetDevice", e));
     cudaStream_t s = stream ? (cudaStream_t)stream : net->eng.stream;
+    // (the size of a scratch array that the event form once needed; callers are promised the refusal)
     if (!net->eng.dense && net->host.n > NC_NOALLOC_MAX_NEURONS)
         return nc::set_last_error(NC_ERR_INVALID, "nc_run_noalloc serves event-form networks of at most " +
                                                       std::to_string(NC_NOALLOC_MAX_NEURONS) + " neurons; this one has " +

@@ -5,11 +5,12 @@
 // (the same host layout as nc_create), then the scheduler thread admits it as soon as
 // a network slot and room in every pool are free: its arrays are uploaded into free
 // ranges, its descriptor is activated and its tiles join the tile table.  Between
-// admissions the scheduler replays a captured CUDA graph of `steps_per_batch` launch
-// pairs; every resident network advances one step per pair until its horizon, so
-// networks admitted at different times share the same launches.  A network that
-// reached its horizon has its plasticity flushed, its counters (and, if kept, weights
-// and potentials) copied out, and its ranges and slot released.
+// admissions the scheduler replays a captured CUDA graph of `steps_per_batch` steps; every
+// resident network advances by each of them until its horizon, so networks admitted at
+// different times share the same launches.  A network that reached its horizon has its
+// plasticity flushed, its counters (and, if kept, weights and potentials) copied out, and
+// its ranges and slot released.  What cannot be read or launched is reported as its
+// request's status; when the device is lost, as every request's.
 //
 // The kernels read the tile count from device memory, so the graph stays valid while
 // the resident set changes; nothing is shared between networks, so each computes the
