@@ -351,7 +351,8 @@ int Engine::build(const std::vector<const NetHost*>& nets, int group_capacity, s
         P.row_blocks = dense_blocks(neurons, quads, L.neuron_block);
         plan_rows(row_nets, P.row_blocks, rows, start);
         // sums that run to their last term (inhibitory or negative synapses) gain from it: the
-        // sphere of 750 6.3 -> 5.9 us a step, 20k x 100 20.7 -> 19.0; those that stop early, after
+        // sphere of 750 6.3 -> 5.9 us a step, 20k x 100 20.7 -> 19.0 (at the limit: networks of that
+        // size whose largest tile has some quads more are not staged); those that stop early, after
         // a batch or two, do not (1k x 50 6.5 either way, 30k x 73 14.7 and 14.9)
         bool all_sum = true;
         for (const NetHost* h : nets) all_sum = all_sum && !h->nonneg_terms;
